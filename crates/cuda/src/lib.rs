@@ -86,6 +86,8 @@ mod ffi {
         pub fn tm_cuda_buffer_contents(ctx: *mut TmCudaCtx, buffer: *mut TmCudaBuffer) -> *mut c_void;
         pub fn tm_cuda_buffer_len(ctx: *const TmCudaCtx, buffer: *const TmCudaBuffer) -> usize;
         pub fn tm_cuda_buffer_zero(ctx: *mut TmCudaCtx, buffer: *mut TmCudaBuffer, off: usize, len: usize, err: *mut c_char, err_cap: usize) -> c_int;
+        pub fn tm_cuda_buffer_zero_2d(ctx: *mut TmCudaCtx, buffer: *mut TmCudaBuffer, off: usize, pitch: usize, width: usize, height: usize, err: *mut c_char, err_cap: usize) -> c_int;
+        pub fn tm_cuda_store_u32(ctx: *mut TmCudaCtx, dst: *mut TmCudaBuffer, index: *const u32, first: u32, values: *const u32, n: u32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_upload(ctx: *mut TmCudaCtx, dst: *mut TmCudaBuffer, off: usize, src: *const c_void, len: usize, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_download(ctx: *mut TmCudaCtx, src: *mut TmCudaBuffer, off: usize, dst: *mut c_void, len: usize, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_buffer_view(ctx: *mut TmCudaCtx, parent: *mut TmCudaBuffer, off: usize, len: usize, err: *mut c_char, err_cap: usize) -> *mut TmCudaBuffer;
@@ -127,6 +129,8 @@ mod ffi {
         pub fn tm_cuda_begin_group(ctx: *mut TmCudaCtx, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_end_group(ctx: *mut TmCudaCtx, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_abort_group(ctx: *mut TmCudaCtx, err: *mut c_char, err_cap: usize) -> c_int;
+        pub fn tm_cuda_begin_burst(ctx: *mut TmCudaCtx, err: *mut c_char, err_cap: usize) -> c_int;
+        pub fn tm_cuda_end_burst(ctx: *mut TmCudaCtx, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_end_group_retain(ctx: *mut TmCudaCtx, out: *mut *mut TmCudaGraph, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_graph_launch(ctx: *mut TmCudaCtx, graph: *mut TmCudaGraph, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_graph_free(ctx: *mut TmCudaCtx, graph: *mut TmCudaGraph);

@@ -68,6 +68,13 @@ size_t tm_cuda_buffer_len(const tm_cuda_ctx *ctx, const tm_cuda_buffer *buffer);
 /* tm_metal.h:78 tm_metal_buffer_zero. */
 int tm_cuda_buffer_zero(tm_cuda_ctx *ctx, tm_cuda_buffer *buffer, size_t off, size_t len,
                         char *err, size_t err_cap);
+/* No counterpart: zeroes `width` bytes of each of `height` rows that lie `pitch` bytes apart. */
+int tm_cuda_buffer_zero_2d(tm_cuda_ctx *ctx, tm_cuda_buffer *buffer, size_t off, size_t pitch, size_t width, size_t height,
+                           char *err, size_t err_cap);
+/* No counterpart: dst[index[i]] = values[i] (dst[first + i] when `index` is NULL) for i < n, as an operator:
+ * the words are taken before the call returns and stored in stream order, so nothing waits for a copy. */
+int tm_cuda_store_u32(tm_cuda_ctx *ctx, tm_cuda_buffer *dst, const uint32_t *index, uint32_t first, const uint32_t *values,
+                      uint32_t n, char *err, size_t err_cap);
 /* tm_metal.h:82,84 tm_metal_upload / tm_metal_download -- ordered after all
  * committed work; return when the copy is complete.  No open group. */
 int tm_cuda_upload(tm_cuda_ctx *ctx, tm_cuda_buffer *dst, size_t off, const void *src, size_t len,
@@ -273,6 +280,10 @@ int tm_cuda_q8_0_gemm_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer 
 int tm_cuda_begin_group(tm_cuda_ctx *ctx, char *err, size_t err_cap);
 int tm_cuda_end_group(tm_cuda_ctx *ctx, char *err, size_t err_cap);
 int tm_cuda_abort_group(tm_cuda_ctx *ctx, char *err, size_t err_cap);
+/* No counterpart: a group that will run once.  Its operators go to the stream as they are encoded (no graph is
+ * built); the group counts as one dispatch.  What was encoded before an error has been submitted: end the burst. */
+int tm_cuda_begin_burst(tm_cuda_ctx *ctx, char *err, size_t err_cap);
+int tm_cuda_end_burst(tm_cuda_ctx *ctx, char *err, size_t err_cap);
 /* No counterpart: end the open group WITHOUT running it and keep it as a
  * replayable graph; each launch is one committed dispatch.  A decode step
  * whose position lives on the device (below) is recorded once and replayed

@@ -56,6 +56,19 @@ public:
         cuda_check(tm_cuda_buffer_zero(ctx_, h_, off, n, e, sizeof e), e);
     }
     void zero() const { zero(0, len()); }
+    void zero_2d(size_t off, size_t pitch, size_t width, size_t height) const {
+        char e[256] = "";
+        cuda_check(tm_cuda_buffer_zero_2d(ctx_, h_, off, pitch, width, height, e, sizeof e), e);
+    }
+    // Words stored in stream order; nothing waits (tm_cuda_store_u32).
+    void store_u32(uint32_t first, const uint32_t *values, size_t n) const {
+        char e[256] = "";
+        cuda_check(tm_cuda_store_u32(ctx_, h_, nullptr, first, values, (uint32_t)n, e, sizeof e), e);
+    }
+    void store_u32(const uint32_t *index, const uint32_t *values, size_t n) const {
+        char e[256] = "";
+        cuda_check(tm_cuda_store_u32(ctx_, h_, index, 0, values, (uint32_t)n, e, sizeof e), e);
+    }
     void upload(size_t off, const void *src, size_t n) const {
         char e[256] = "";
         cuda_check(tm_cuda_upload(ctx_, h_, off, src, n, e, sizeof e), e);
@@ -117,6 +130,12 @@ private:
     do {                                                          \
         char e_[256] = "";                                        \
         cuda_check(fn(ctx_, __VA_ARGS__, e_, sizeof e_), e_);     \
+    } while (0)
+
+#define TM_CALL0(fn)                                              \
+    do {                                                          \
+        char e_[256] = "";                                        \
+        cuda_check(fn(ctx_, e_, sizeof e_), e_);                  \
     } while (0)
 
 class CudaContext {
@@ -446,18 +465,18 @@ public:
         cuda_check(tm_cuda_symm_status(ctx_, b.raw(), &st, e, sizeof e), e);
         return st;
     }
-    // One dispatch per step: a failure inside `encode` aborts the group so no
-    // partial work reaches the device.
+    // One dispatch that runs once: its operators go to the stream as they are encoded.
     template <class F>
-    void grouped(F &&encode) const {
-        begin_group();
+    void burst(F &&encode) const {
+        TM_CALL0(tm_cuda_begin_burst);
         try {
             encode();
         } catch (...) {
-            abort_group();
+            char e[256] = "";
+            tm_cuda_end_burst(ctx_, e, sizeof e);
             throw;
         }
-        end_group();
+        TM_CALL0(tm_cuda_end_burst);
     }
     void fence() const {
         char e[256] = "";

@@ -43,6 +43,18 @@ struct GatherArena {
     size_t off = 0;
 };
 
+// The KV planes of every layer live in one buffer, so that a reset is one memory operation.
+struct KvArena {
+    CudaBuffer buf;
+    size_t off = 0;
+    CudaBuffer take(size_t n) {
+        if (n % 16 != 0) throw TuckmillError(ErrorCode::InvalidRequest, "a KV plane is not a 16-byte multiple");
+        CudaBuffer v = buf.view(off, n);
+        off += n;
+        return v;
+    }
+};
+
 struct Shard {
     uint32_t rank = 0, world = 1;
     GatherArena *arena = nullptr;  // set while loading a split model
@@ -549,7 +561,7 @@ struct AttentionBlock {
         if (sh.world > 1) p.scratch_f32(hidden);  // proj_local
     }
     static AttentionBlock load(const CudaContext &ctx, const WeightSource &src, const AttentionSpec &s, float eps,
-                               size_t cap, size_t hidden, Shard sh, size_t seqs) {
+                               size_t cap, size_t hidden, Shard sh, size_t seqs, KvArena &kv_arena) {
         if (s.head_dim % 32 != 0 || (s.head_dim / 32 > 4 && s.head_dim != 256) || s.rope_dims % 2 != 0)
             throw TuckmillError(ErrorCode::UnsupportedArchitecture,
                                 "attention head size " + std::to_string(s.head_dim) + " has no CUDA block");
@@ -575,8 +587,8 @@ struct AttentionBlock {
         b.inv_freq = ctx.floats(rope_inv_freq(s.rope_dims, s.rope_base));
         b.seqs = seqs;
         const size_t plane = kv_plane_bytes(s, cap, sh);
-        b.k_cache = ctx.buffer(plane * seqs);
-        b.v_cache = ctx.buffer(plane * seqs);
+        b.k_cache = kv_arena.take(plane * seqs);
+        b.v_cache = kv_arena.take(plane * seqs);
         if (seqs > 1) {
             if (plane % 16 != 0)
                 throw TuckmillError(ErrorCode::InvalidRequest, "KV plane of one sequence is not a 16-byte multiple");
@@ -600,10 +612,6 @@ struct AttentionBlock {
                                                                                (uint32_t)s.head_dim, (uint32_t)cap));
         if (sh.world > 1) b.proj_local = zeros_f32(ctx, hidden);
         return b;
-    }
-    void reset() const {
-        k_cache.zero();
-        v_cache.zero();
     }
     float scale() const { return 1.0f / std::sqrt((float)spec.head_dim); }
 
@@ -703,13 +711,13 @@ struct Layer {
         SwiGluBlock::plan(l.ffn, l.has_ffn_out_norm, l.ffn_out_norm, g.hidden, src, sh, p);
     }
     static Layer load(const CudaContext &ctx, const WeightSource &src, const LayerSpec &l, const ModelGraph &g,
-                      size_t cap, Shard sh, size_t seqs) {
+                      size_t cap, Shard sh, size_t seqs, KvArena &kv_arena) {
         Layer L;
         L.pre_norm = vector(ctx, src, l.pre_norm);
         if (l.has_mixer_out_norm) L.mixer_out_norm = vector(ctx, src, l.mixer_out_norm);
         L.post_norm = vector(ctx, src, l.post_norm);
         L.proj = gather_target_f32(ctx, g.hidden * sh.world * (sh.world > 1 ? 2 : 1), sh);
-        L.mixer = AttentionBlock::load(ctx, src, l.mixer, g.eps, cap, g.hidden, sh, seqs);
+        L.mixer = AttentionBlock::load(ctx, src, l.mixer, g.eps, cap, g.hidden, sh, seqs, kv_arena);
         L.ffn = SwiGluBlock::load(ctx, src, l.ffn, l.has_ffn_out_norm, l.ffn_out_norm, g.hidden, g.eps, sh);
         return L;
     }
@@ -846,6 +854,9 @@ struct EngineModel::Impl {
     Matrix embedding, head_own;
     bool tied = false;
     Shard sh;
+    KvArena kv;         // likewise before the blocks' views of it
+    size_t kv_pitch = 0;  // bytes of one head's plane when all layers agree (0: they do not)
+    size_t kv_rows = 0;   // cache rows any sequence may have written since the last reset (an upper bound)
     GatherArena arena;  // declared before the blocks that hold views of it (views are released first)
     CudaBuffer tied_view;  // row split of a tied head: this rank's rows of the (replicated) embedding
     uint32_t head_rows = 0;  // rows of the head this rank multiplies (vocab / world)
@@ -1012,7 +1023,12 @@ std::unique_ptr<EngineModel> EngineModel::load_with(std::shared_ptr<CudaContext>
     I.seqs = opts.sequences;
     I.log_stride = token_log_stride(capacity, I.seqs);
     I.pos_b.assign(I.seqs, 0);
-    for (const LayerSpec &l : graph.layers) I.layers.push_back(Layer::load(c, src, l, graph, capacity, sh, I.seqs));
+    I.kv.buf = c.buffer(m->plan_.state);
+    I.kv_pitch = capacity * graph.layers[0].mixer.head_dim * 2;
+    for (const LayerSpec &l : graph.layers)
+        if (capacity * l.mixer.head_dim * 2 != I.kv_pitch) I.kv_pitch = 0;
+    I.kv_rows = capacity;  // fresh memory: every row is cleared by the first reset
+    for (const LayerSpec &l : graph.layers) I.layers.push_back(Layer::load(c, src, l, graph, capacity, sh, I.seqs, I.kv));
     I.embedding = Matrix::load(c, src, {graph.embedding});
     I.tied = graph.head == graph.embedding;
     I.head_rows = (uint32_t)(graph.vocab / sh.world);
@@ -1211,14 +1227,14 @@ void EngineModel::step_ungrouped() {
                             "position " + std::to_string(pos_) + " exceeds KV capacity " + std::to_string(capacity_));
     encode_decode_step();
     pos_ += 1;
+    impl_->kv_rows = std::min(impl_->kv_rows + 1, capacity_);
 }
 
 void EngineModel::check_device_status() {
     Impl &I = *impl_;
     ctx_->fence();
-    uint32_t st = 0;
-    I.status.download(0, &st, 4);
-    if (st != 0) throw TuckmillError(ErrorCode::Internal, "a decode step ran past the KV capacity on the device");
+    if (*(const volatile uint32_t *)I.status.contents() != 0)
+        throw TuckmillError(ErrorCode::Internal, "a decode step ran past the KV capacity on the device");
     if (!opts_.exact && ctx_->mma_aborted())
         throw TuckmillError(ErrorCode::Internal,
                             "a pipeline wait of the tensor-core GEMM ran out; the prefill results are undefined");
@@ -1247,13 +1263,29 @@ EngineModel::~EngineModel() {
     }
 }
 
+// The caches are cleared up to the last row that can have been written since the previous reset, all layers and
+// sequences in one operation: clearing the whole capacity (58 memsets, 470 MB on a 0.6B decoder at 4096 positions)
+// cost 0.6 ms of host launches before a request's first kernel.  Stream order is all that later work needs.
 void EngineModel::reset() {
-    for (const Layer &L : impl_->layers) L.mixer.reset();
-    impl_->pos_buf.zero();
-    impl_->status.zero();
-    ctx_->fence();
+    Impl &I = *impl_;
+    if (I.kv_rows > 0) {
+        if (I.kv_pitch && I.kv_rows < capacity_)
+            I.kv.buf.zero_2d(0, I.kv_pitch, I.kv_pitch / capacity_ * I.kv_rows, I.kv.buf.len() / I.kv_pitch);
+        else
+            I.kv.buf.zero();
+    }
+    I.kv_rows = 0;
+    I.pos_buf.zero();
+    I.status.zero();
     pos_ = 0;
-    std::fill(impl_->pos_b.begin(), impl_->pos_b.end(), 0);
+    std::fill(I.pos_b.begin(), I.pos_b.end(), 0);
+}
+
+// A recorded step of all sequences (or of the one) advances every device position by at most a row.
+void EngineModel::launch_step(bool batch) {
+    Impl &I = *impl_;
+    (batch ? I.batch_graph : I.decode_graph).launch();
+    I.kv_rows = std::min(I.kv_rows + 1, capacity_);
 }
 
 size_t EngineModel::sequences() const { return impl_->seqs; }
@@ -1278,7 +1310,7 @@ void EngineModel::prefill_seq(size_t seq, const uint32_t *tokens, size_t n, bool
     Impl &I = *impl_;
     const CudaContext &c = *ctx_;
     const size_t log0 = seq * I.log_stride;  // this sequence's token log
-    I.tokens.upload((log0 + pos_) * 4, tokens, n * 4);
+    I.kv_rows = std::max(I.kv_rows, pos_ + n);
     const size_t batch = std::min<size_t>(opts_.prefill_batch, capacity_);
     RowsAre rows;
     rows.seq = seq;
@@ -1286,7 +1318,8 @@ void EngineModel::prefill_seq(size_t seq, const uint32_t *tokens, size_t n, bool
         const size_t k = std::min(batch, n - t0);
         const bool last = t0 + k == n;
         const uint32_t pos0 = (uint32_t)(pos_ + t0), slot0 = (uint32_t)(log0 + pos_ + t0);
-        c.grouped([&] {
+        c.burst([&] {
+            I.tokens.store_u32(slot0, tokens + t0, k);
             if (I.embedding.type == 1)
                 c.f16_rows_indirect(I.embedding.buf, I.embedding.rows, I.embedding.cols, I.tokens, slot0, (uint32_t)k,
                                     graph_.embedding_scale, I.scratch.x);
@@ -1295,6 +1328,10 @@ void EngineModel::prefill_seq(size_t seq, const uint32_t *tokens, size_t n, bool
                                 graph_.embedding_scale, I.scratch.x);
             for (const Layer &L : I.layers)
                 L.prefill(c, I.scratch, k, pos0, graph_.hidden, graph_.eps, opts_.exact, rows);
+            if (last) {
+                const uint32_t p32 = (uint32_t)(pos_ + n);
+                I.pos_buf.store_u32((uint32_t)seq, &p32, 1);
+            }
             if (last && want_token) {
                 // Vocabulary projection for the last row only (engine/metal.rs:2610-2617).
                 c.copy_f32(I.scratch.x, (uint32_t)((k - 1) * graph_.hidden), I.x, 0, (uint32_t)graph_.hidden);
@@ -1302,15 +1339,14 @@ void EngineModel::prefill_seq(size_t seq, const uint32_t *tokens, size_t n, bool
                 if (I.sh.world > 1)
                     c.argmax_sharded(I.logits, I.head_rows, I.sh.rank * I.head_rows, I.partial, I.pairs, I.tokens,
                                      slot0 + (uint32_t)k, nullptr, 0, (uint32_t)(I.log_stride * I.seqs), nullptr);
-                else
-                    c.argmax_f32(I.logits, (uint32_t)graph_.vocab, I.partial, I.tokens, slot0 + (uint32_t)k);
+                else  // appended at this sequence's position, like a decode step's
+                    c.argmax_dev(I.logits, (uint32_t)graph_.vocab, I.partial, I.tokens, (uint32_t)log0, I.pos_buf,
+                                 (uint32_t)seq, (uint32_t)(I.log_stride * I.seqs), &I.tokens_mirror);
             }
         });
     }
     I.pos_b[seq] = pos_ + n;
     if (seq == 0) this->pos_ = I.pos_b[0];
-    const uint32_t p32 = (uint32_t)I.pos_b[seq];
-    I.pos_buf.upload(seq * 4, &p32, 4);
 }
 
 uint32_t EngineModel::prefill_token() { return prefill_token_of(0); }
@@ -1318,7 +1354,9 @@ uint32_t EngineModel::prefill_token() { return prefill_token_of(0); }
 uint32_t EngineModel::prefill_token_of(size_t seq) {
     if (seq >= impl_->seqs) throw TuckmillError(ErrorCode::InvalidRequest, "sequence outside the engine's");
     uint32_t t = 0;
-    impl_->tokens.download((seq * impl_->log_stride + impl_->pos_b[seq]) * 4, &t, 4);
+    const size_t at = (seq * impl_->log_stride + impl_->pos_b[seq]) * 4;
+    if (impl_->sh.world > 1) impl_->tokens.download(at, &t, 4);
+    else impl_->tokens_mirror.download_after(at, &t, 4, ctx_->committed());
     return t;
 }
 
@@ -1335,8 +1373,10 @@ void EngineModel::step_batch(const uint32_t *tokens) {
                                                                      std::to_string(I.pos_b[s]) + " exceeds KV capacity " +
                                                                      std::to_string(capacity_));
     }
-    for (size_t s = 0; s < I.seqs; ++s) I.tokens.upload((s * I.log_stride + I.pos_b[s]) * 4, &tokens[s], 4);
-    I.batch_graph.launch();
+    std::vector<uint32_t> slots(I.seqs);
+    for (size_t s = 0; s < I.seqs; ++s) slots[s] = (uint32_t)(s * I.log_stride + I.pos_b[s]);
+    I.tokens.store_u32(slots.data(), tokens, I.seqs);
+    launch_step(true);
     for (size_t s = 0; s < I.seqs; ++s) I.pos_b[s] += 1;
     pos_ = I.pos_b[0];
 }
@@ -1347,7 +1387,7 @@ void EngineModel::submit_batch_greedy() {
     for (size_t s = 0; s < I.seqs; ++s)
         if (I.pos_b[s] >= capacity_)
             throw TuckmillError(ErrorCode::ContextExceedsBudget, "sequence " + std::to_string(s) + " is at capacity");
-    I.batch_graph.launch();
+    launch_step(true);
     for (size_t s = 0; s < I.seqs; ++s) I.pos_b[s] += 1;
     pos_ = I.pos_b[0];
 }
@@ -1381,15 +1421,6 @@ std::vector<std::vector<uint32_t>> EngineModel::generate_batch(const std::vector
         return t == 0xFFFFFFFFu || (!ignore_eos && graph_.has_eos && t == graph_.eos_token_id);
     };
     std::vector<char> done(R, 0);
-    for (size_t s = 0; s < R; ++s) {
-        const uint32_t tok = prefill_token_of(s);
-        if (tok == 0xFFFFFFFFu)
-            throw TuckmillError(ErrorCode::Internal, "every logit was NaN; refusing to guess a token");
-        out[s].push_back(tok);
-        done[s] = is_stop(tok);
-    }
-    const uint64_t t_first = now_ns();
-    uint64_t t_last = t_first;
     // A step advances every sequence on the device; the host follows the ones still wanted.  Step
     // i + 1 is submitted before step i is read (executor.rs:1080-1087), so a sequence that stops runs
     // one step too many, whose token is dropped.
@@ -1411,12 +1442,26 @@ std::vector<std::vector<uint32_t>> EngineModel::generate_batch(const std::vector
                 host_pos[s] += 1;
                 submitted[s] += 1;
             }
-        I.batch_graph.launch();
+        launch_step(true);
         f.dispatch = ctx_->committed();
         return f;
     };
     std::vector<Flight> inflight;
-    if (any_wants()) inflight.push_back(submit());
+    const uint64_t prefilled = ctx_->committed();
+    if (I.sh.world <= 1 && any_wants()) inflight.push_back(submit());
+    for (size_t s = 0; s < R; ++s) {
+        uint32_t tok = 0;
+        const size_t at = s * I.log_stride + I.pos_b[s];
+        if (I.sh.world > 1) tok = prefill_token_of(s);  // a split model's prefill has no mirror
+        else I.tokens_mirror.download_after(at * 4, &tok, 4, prefilled);
+        if (tok == 0xFFFFFFFFu)
+            throw TuckmillError(ErrorCode::Internal, "every logit was NaN; refusing to guess a token");
+        out[s].push_back(tok);
+        done[s] = is_stop(tok);
+    }
+    const uint64_t t_first = now_ns();
+    uint64_t t_last = t_first;
+    if (inflight.empty() && any_wants()) inflight.push_back(submit());
     while (!inflight.empty()) {
         if (any_wants()) inflight.push_back(submit());
         const Flight f = inflight.front();
@@ -1461,8 +1506,8 @@ void EngineModel::step(uint32_t token) {
     if (pos_ >= capacity_)
         throw TuckmillError(ErrorCode::ContextExceedsBudget,
                             "position " + std::to_string(pos_) + " exceeds KV capacity " + std::to_string(capacity_));
-    impl_->tokens.upload(pos_ * 4, &token, 4);
-    impl_->decode_graph.launch();
+    impl_->tokens.store_u32((uint32_t)pos_, &token, 1);
+    launch_step(false);
     pos_ += 1;
     impl_->pos_b[0] = pos_;
 }
@@ -1483,7 +1528,7 @@ EngineModel::Ticket EngineModel::submit_greedy() {
     if (pos_ >= capacity_)
         throw TuckmillError(ErrorCode::ContextExceedsBudget,
                             "position " + std::to_string(pos_) + " exceeds KV capacity " + std::to_string(capacity_));
-    impl_->decode_graph.launch();
+    launch_step(false);
     Ticket t;
     t.dispatch = ctx_->committed();
     t.slot = pos_ + 1;
@@ -1506,7 +1551,17 @@ std::vector<uint32_t> EngineModel::generate(const uint32_t *prompt, size_t n_pro
     const uint64_t t_start = now_ns();
     reset();
     prefill(prompt, n_prompt, true);
-    uint32_t tok = prefill_token();
+    // Step i+1 is submitted before step i is collected (executor.rs:1080-1087), the first one before the prompt's
+    // own token is read: the device already has token i in its log.
+    std::vector<Ticket> inflight;
+    size_t submitted = 0;
+    const size_t want = max_new - 1;
+    auto can_submit = [&] { return submitted < want && pos_ < capacity_; };
+    const size_t first_slot = pos_;
+    const uint64_t first_dispatch = ctx_->committed();
+    const uint32_t first_split = impl_->sh.world > 1 ? prefill_token() : 0u;  // a split model's prefill has no mirror
+    if (can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
+    uint32_t tok = impl_->sh.world > 1 ? first_split : collect_greedy(Ticket{first_dispatch, first_slot});
     const uint64_t t_first = now_ns();
     uint64_t t_last = t_first;
     auto is_stop = [&](uint32_t t) {
@@ -1516,13 +1571,6 @@ std::vector<uint32_t> EngineModel::generate(const uint32_t *prompt, size_t n_pro
     if (tok == 0xFFFFFFFFu)
         throw TuckmillError(ErrorCode::Internal, "every logit was NaN; refusing to guess a token");
     if (!is_stop(tok)) {
-        // Step i+1 is submitted before step i is collected (executor.rs:1080-1087):
-        // the device already has token i in its log.
-        std::vector<Ticket> inflight;
-        size_t submitted = 0;
-        const size_t want = max_new - 1;
-        auto can_submit = [&] { return submitted < want && pos_ < capacity_; };
-        if (can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
         while (!inflight.empty()) {
             if (can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
             const Ticket t = inflight.front();

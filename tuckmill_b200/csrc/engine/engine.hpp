@@ -135,6 +135,7 @@ public:
     // graph): the attribution mode of engine/metal.rs:1964-1968, used with the
     // context's per-operator profile table.
     void step_ungrouped();
+    void launch_step(bool batch);
     // Throws Internal naming the wait when a bounded device-side wait ran out (tensor-core GEMM
     // pipeline, peer-memory exchange, persistent decode program) or a step ran past the KV capacity:
     // the results of such a dispatch are undefined and must not be returned as tokens.  Waits for

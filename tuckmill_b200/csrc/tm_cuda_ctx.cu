@@ -7,6 +7,7 @@
 #include <cstdlib>
 
 #include "tm_cuda_internal.cuh"
+#include "tm_cuda_device.cuh"
 
 namespace {
 
@@ -82,12 +83,12 @@ int tm_op_begin(tm_cuda_ctx *ctx, const char *label, char *err, size_t err_cap) 
     if (ctx->program)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED,
                        "operator %s cannot be recorded into a persistent program", label);
-    if (ctx->group_open) return TM_CUDA_OK;
+    if (ctx->group_open || ctx->burst_open) return TM_CUDA_OK;
     return commit_begin(ctx, &ctx->open_commit, label, err, err_cap);
 }
 
 int tm_op_end(tm_cuda_ctx *ctx, uint64_t kernels, char *err, size_t err_cap) {
-    if (ctx->group_open) {
+    if (ctx->group_open || ctx->burst_open) {
         ctx->group_kernels += kernels;
         return TM_CUDA_OK;
     }
@@ -199,6 +200,7 @@ void tm_cuda_destroy(tm_cuda_ctx *ctx) {
         poll_locked(ctx, true);
         for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
         if (ctx->mma_scratch) cudaFree(ctx->mma_scratch);
+        if (ctx->mma_abort) cudaFreeHost((void *)ctx->mma_abort);
     }
     if (ctx->side) {
         cudaStreamSynchronize(ctx->side);
@@ -316,10 +318,56 @@ int tm_cuda_buffer_zero(tm_cuda_ctx *ctx, tm_cuda_buffer *buffer, size_t off, si
     TM_OP_END(1);
 }
 
+int tm_cuda_buffer_zero_2d(tm_cuda_ctx *ctx, tm_cuda_buffer *buffer, size_t off, size_t pitch, size_t width, size_t height,
+                           char *err, size_t err_cap) {
+    TM_ENTER();
+    if (width == 0 || height == 0 || width > pitch || height > SIZE_MAX / pitch || off > SIZE_MAX - height * pitch)
+        return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "zero range is empty or overflows");
+    TM_CHECK_BUF(buffer, off + (height - 1) * pitch + width, "zero target");
+    TM_OP_BEGIN("buffer_zero_2d");
+    TM_CUDA_TRY(cudaMemset2DAsync(buffer->dev + off, pitch, 0, width, height, ctx->stream));
+    TM_OP_END(1);
+}
+
+// The words travel as kernel arguments: no staging buffer, no copy to wait for.
+constexpr uint32_t kStoreWords = 448;
+struct store_words {
+    uint32_t index[kStoreWords], value[kStoreWords];
+};
+__global__ void store_u32_kernel(uint32_t *out, const __grid_constant__ store_words w, uint32_t n) {
+    tmdev::pdl_wait();
+    tmdev::pdl_trigger();
+    if (threadIdx.x < n) out[w.index[threadIdx.x]] = w.value[threadIdx.x];
+}
+
+int tm_cuda_store_u32(tm_cuda_ctx *ctx, tm_cuda_buffer *dst, const uint32_t *index, uint32_t first, const uint32_t *values,
+                      uint32_t n, char *err, size_t err_cap) {
+    TM_ENTER();
+    if (!values || n == 0) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "no words to store");
+    uint64_t top = (uint64_t)first + n - 1;
+    if (index) {
+        top = 0;
+        for (uint32_t i = 0; i < n; ++i) top = index[i] > top ? index[i] : top;
+    }
+    TM_CHECK_BUF(dst, (top + 1) * 4, "store target");
+    TM_OP_BEGIN("store_u32");
+    uint64_t kernels = 0;
+    for (uint32_t at = 0; at < n; at += kStoreWords, ++kernels) {
+        const uint32_t k = n - at < kStoreWords ? n - at : kStoreWords;
+        store_words w;
+        for (uint32_t i = 0; i < k; ++i) {
+            w.index[i] = index ? index[at + i] : first + at + i;
+            w.value[i] = values[at + i];
+        }
+        TM_CUDA_TRY(tm_launch_pdl(ctx, store_u32_kernel, dim3(1), dim3(kStoreWords), 0, (uint32_t *)dst->dev, w, k));
+    }
+    TM_OP_END(kernels);
+}
+
 int tm_cuda_upload(tm_cuda_ctx *ctx, tm_cuda_buffer *dst, size_t off, const void *src, size_t len,
                    char *err, size_t err_cap) {
     TM_ENTER();
-    if (ctx->group_open)
+    if (ctx->group_open || ctx->burst_open)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "upload with a dispatch group open");
     if (!src || len == 0 || off > SIZE_MAX - len)
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "upload range is empty or overflows");
@@ -333,7 +381,7 @@ int tm_cuda_upload(tm_cuda_ctx *ctx, tm_cuda_buffer *dst, size_t off, const void
 int tm_cuda_download(tm_cuda_ctx *ctx, tm_cuda_buffer *src, size_t off, void *dst, size_t len,
                      char *err, size_t err_cap) {
     TM_ENTER();
-    if (ctx->group_open)
+    if (ctx->group_open || ctx->burst_open)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "download with a dispatch group open");
     if (!dst || len == 0 || off > SIZE_MAX - len)
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "download range is empty or overflows");
@@ -401,7 +449,7 @@ int tm_cuda_prefetch_l2(tm_cuda_ctx *ctx, tm_cuda_buffer *const *bufs, uint32_t 
         l2_prefetch_kernel<<<8, 256, 0, ctx->side>>>((const char *)bufs[i]->dev, bufs[i]->len);
     TM_CUDA_TRY(cudaGetLastError());
     ctx->side_pending = true;
-    if (ctx->group_open) ctx->group_kernels += n;
+    if (ctx->group_open || ctx->burst_open) ctx->group_kernels += n;
     else {
         ctx->launches.fetch_add(n);
         join_side(ctx);
@@ -411,7 +459,7 @@ int tm_cuda_prefetch_l2(tm_cuda_ctx *ctx, tm_cuda_buffer *const *bufs, uint32_t 
 
 int tm_cuda_begin_group(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
     TM_ENTER();
-    if (ctx->group_open || ctx->program)
+    if (ctx->group_open || ctx->burst_open || ctx->program)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "a dispatch group is already open");
     TM_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
     ctx->group_open = true;
@@ -472,6 +520,30 @@ int tm_cuda_end_group(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
     return rc;
 }
 
+// A group that runs once: capturing and instantiating a graph of a few hundred kernels costs the host more
+// than launching them (a 286-launch prefill: 1.7 ms before the first kernel runs, against 0.6 ms of launches
+// that overlap with it), so its operators go straight to the stream; only the book-keeping is a group's --
+// one dispatch, one pair of timing events.
+int tm_cuda_begin_burst(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
+    TM_ENTER();
+    if (ctx->group_open || ctx->burst_open || ctx->program)
+        return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "a dispatch group is already open");
+    const int rc = commit_begin(ctx, &ctx->open_commit, "group", err, err_cap);
+    if (rc != TM_CUDA_OK) return rc;
+    ctx->burst_open = true;
+    ctx->group_kernels = 0;
+    return TM_CUDA_OK;
+}
+
+int tm_cuda_end_burst(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
+    TM_ENTER();
+    if (!ctx->burst_open) return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "no burst is open");
+    join_side(ctx);
+    ctx->burst_open = false;
+    ctx->launches.fetch_add(ctx->group_kernels);
+    return commit_end(ctx, &ctx->open_commit, err, err_cap);
+}
+
 int tm_cuda_abort_group(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
     TM_ENTER();
     if (!ctx->group_open)
@@ -498,7 +570,7 @@ int tm_cuda_end_group_retain(tm_cuda_ctx *ctx, tm_cuda_graph **out, char *err, s
 
 int tm_cuda_graph_launch(tm_cuda_ctx *ctx, tm_cuda_graph *graph, char *err, size_t err_cap) {
     TM_ENTER();
-    if (ctx->group_open)
+    if (ctx->group_open || ctx->burst_open)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "graph launch with a dispatch group open");
     if (!graph || ctx->graphs.find(graph) == ctx->graphs.end())
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "graph does not belong to this context");
@@ -533,7 +605,7 @@ void tm_cuda_graph_free(tm_cuda_ctx *ctx, tm_cuda_graph *graph) {
 
 int tm_cuda_fence(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
     TM_ENTER();
-    if (ctx->group_open)
+    if (ctx->group_open || ctx->burst_open)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "fence with a dispatch group open");
     TM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     poll_locked(ctx, true);

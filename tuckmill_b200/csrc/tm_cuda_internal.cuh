@@ -76,7 +76,8 @@ struct tm_cuda_ctx {
     std::atomic<uint64_t> gpu_nanos{0};
     std::atomic<uint64_t> launches{0};
     std::atomic<uint64_t> last_gpu_ns{0};
-    bool group_open = false;
+    bool group_open = false;             // capturing a group into a graph
+    bool burst_open = false;             // a group whose operators go to the stream as they are encoded
     uint64_t group_kernels = 0;
     bool profiling = false;
     bool pdl = true;                     // chain kernels with programmatic dependent launch
@@ -87,6 +88,9 @@ struct tm_cuda_ctx {
     // Scratch owned by the context for the tensor-core GEMM (f16 copy of X).
     unsigned char *mma_scratch = nullptr;
     size_t mma_scratch_bytes = 0;
+    // Set by a tensor-core GEMM whose bounded wait ran out: host memory the device can write, so that the
+    // host looks at it without a copy.
+    volatile uint32_t *mma_abort = nullptr;
     int mma_last_bn = 0;                 // token sub-tile width of the last tensor-core GEMM launch
     int mma_last_ksplit = 0;             // K parts per output tile of that launch
     void *comm = nullptr;  // multi-GPU communicator state (tm_cuda_comm.cu)

@@ -169,7 +169,7 @@ struct mma_args {
     float *const *peer;
     uint32_t push_world, push_rank, push_off, push_tail;
     uint32_t rows, cols, batch;
-    uint32_t *abort_flag;  // set when a bounded wait gave up
+    uint32_t *abort_flag;  // host memory, set when a bounded wait gave up
 };
 
 // Ring bookkeeping over a running step count g: stage g % D, the consumer waits
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     // ---------------- teardown: everyone meets, tensor memory goes back ----------------
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (tid == 0 && *abort_s) atomicOr(a.abort_flag, 1u);
+    if (tid == 0 && *abort_s) *(volatile uint32_t *)a.abort_flag = 1u;
     if (a.push_world) {
         __shared__ uint32_t s_flag[2];
         tm_symm_finish(a.peer, a.push_tail, a.push_world, a.push_rank, s_flag);
@@ -683,7 +683,16 @@ int tm_cuda_mma_workspace_reserve(tm_cuda_ctx *ctx, size_t bytes, char *err, siz
         ctx->mma_scratch_bytes = 0;
     }
     void *p = nullptr;
-    const size_t total = tm_round_up(bytes, 256) + 256;  // + the abort flag word
+    if (!ctx->mma_abort) {
+        void *f = nullptr;
+        if (cudaHostAlloc(&f, 4, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return tm_fail(err, err_cap, TM_CUDA_ERR_ALLOC, "allocating the GEMM's status word failed");
+        }
+        ctx->mma_abort = (volatile uint32_t *)f;
+        *ctx->mma_abort = 0u;
+    }
+    const size_t total = tm_round_up(bytes, 256);
     if (cudaMalloc(&p, total) != cudaSuccess) {
         cudaGetLastError();
         return tm_fail(err, err_cap, TM_CUDA_ERR_ALLOC, "allocating the %zu-byte GEMM workspace failed", total);
@@ -725,7 +734,7 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     if (!encode)
         return tm_fail(err, err_cap, TM_CUDA_ERR_INTERNAL, "the driver does not export cuTensorMapEncodeTiled");
     __half *xh = (__half *)ctx->mma_scratch;
-    uint32_t *abort_flag = (uint32_t *)(ctx->mma_scratch + tm_round_up(ctx->mma_scratch_bytes, 256));
+    uint32_t *abort_flag = (uint32_t *)ctx->mma_abort;
     // Sub-tile width BN (a tile is 128 rows x 2*BN tokens): the one whose rounds of the persistent
     // grid cost the fewest cycles.  Fitted to measurements: a K step takes the larger of the
     // tensor-pipe time plus hand-over (4*BN + 94 cycles for the two issuers' eight MMAs) and the
@@ -962,12 +971,10 @@ int tm_cuda_mma_last_split(tm_cuda_ctx *ctx) {
 int tm_cuda_mma_aborted(tm_cuda_ctx *ctx) {
     if (!ctx) return 0;
     std::lock_guard<std::mutex> lock(ctx->mu);
-    if (!ctx->mma_scratch) return 0;
-    uint32_t v = 0;
+    if (!ctx->mma_abort) return 0;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    cudaMemcpy(&v, ctx->mma_scratch + tm_round_up(ctx->mma_scratch_bytes, 256), 4, cudaMemcpyDeviceToHost);
-    return v != 0;
+    return *ctx->mma_abort != 0;
 }
 
 }  // extern "C"

@@ -39,6 +39,10 @@ _ERR = [C.c_char_p, C.c_size_t]
 # name -> argument types WITHOUT the trailing (err, err_cap); all return int.
 _OPS = {
     "buffer_zero": [_P, _P, _SZ, _SZ],
+    "buffer_zero_2d": [_P, _P, _SZ, _SZ, _SZ, _SZ],
+    "store_u32": [_P, _P, _P, _U32, _P, _U32],
+    "begin_burst": [_P],
+    "end_burst": [_P],
     "upload": [_P, _P, _SZ, _P, _SZ],
     "download": [_P, _P, _SZ, _P, _SZ],
     "download_after": [_P, _P, _SZ, _P, _SZ, C.c_uint64],
@@ -232,6 +236,15 @@ class CudaBuffer:
 
     def zero(self, off: int = 0, length: int | None = None):
         self.ctx._call("buffer_zero", self.handle, off, len(self) if length is None else length)
+
+    def zero_2d(self, off: int, pitch: int, width: int, height: int):
+        self.ctx._call("buffer_zero_2d", self.handle, off, pitch, width, height)
+
+    def store_u32(self, values, first: int = 0, index=None):
+        """self[index[i]] = values[i] (self[first + i] without an index), in stream order."""
+        v = np.ascontiguousarray(values, dtype=np.uint32)
+        i = None if index is None else np.ascontiguousarray(index, dtype=np.uint32)
+        self.ctx._call("store_u32", self.handle, None if i is None else i.ctypes.data, first, v.ctypes.data, v.size)
 
     def upload(self, off: int, data) -> None:
         a = np.ascontiguousarray(data)
