@@ -199,6 +199,11 @@ cudaError_t tm_attention_decode_mma_launch(tm_cuda_ctx *ctx, const float *q, con
                                            float eps, float scale, uint32_t n_seq, size_t sq, size_t skv, size_t so,
                                            size_t scache, size_t sscratch, uint32_t count_off);
 
+// Tensor-core GEMM workspace and the f16 copy of X in it (tm_cuda_mma.cu).
+extern "C" int tm_mma_ensure_workspace(tm_cuda_ctx *ctx, uint32_t cols, uint32_t batch, char *err, size_t err_cap);
+cudaError_t tm_x_prep_launch(tm_cuda_ctx *ctx, int prologue, const float *x, const float *pro, uint32_t cols, uint32_t batch,
+                             float eps);
+
 cudaError_t tm_argmax_partial_launch(tm_cuda_ctx *ctx, const float *x, uint32_t n, float *pv, uint32_t *pi);
 cudaError_t tm_argmax_rows_partial_launch(tm_cuda_ctx *ctx, const float *x, uint32_t n_rows, uint32_t n, float *pv,
                                           uint32_t *pi);

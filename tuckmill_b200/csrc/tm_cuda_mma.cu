@@ -19,8 +19,8 @@
 //  * a weight tile converted once now serves 2*BN tokens.
 // Tensor memory: two BN-column accumulators + (512 - 2*BN)/32 A stages of 32 columns.
 // Roles by warp:
-//   0-7    converters: warps q and q+4 own tensor-memory lanes 32q..32q+31 and
-//          take alternate K steps; a thread reads its row's 64 raw bytes (TMA,
+//   0-7    converters (0-15 at up to 64 tokens): warps q, q+4, ... own tensor-memory lanes 32q..32q+31 and
+//          take K steps in turn; a thread reads its row's 64 raw bytes (TMA,
 //          64-byte swizzle), turns them into f16 d*q (byte permute into 1024+u,
 //          subtract 1152, multiply by d) and writes them with tcgen05.st; block
 //          scales come straight from global memory, several K steps ahead
@@ -42,11 +42,7 @@ namespace {
 
 constexpr int kBM = 128;        // weight rows per tile (UMMA M)
 constexpr int kBK = 64;         // K per stage: 64 f16 = one 128-byte swizzle row
-constexpr int kRawStages = 4;   // raw int8 weight tiles in flight (8 KB each)
-constexpr int kConvWarps = 8, kIssuers = 2, kEpiWarps = 4;
-constexpr int kWarpRaw = kConvWarps + kEpiWarps, kWarpTok = kWarpRaw + 1, kWarpMma = kWarpRaw + 2;
-constexpr int kMmaThreads = (kWarpMma + kIssuers) * 32;
-constexpr int kScaleAhead = 4;  // a converter's own steps (every other K step) between a scale's load and its use
+constexpr int kEpiWarps = 4;
 constexpr uint32_t kSpinLimit = 1u << 20;  // a healthy wait is microseconds; this is ~seconds
 // Split-K: when it shortens the longest CTA's run (few output tiles on many SMs: a decode batch, a narrow
 // projection, a last round that leaves most SMs idle) the K range of every tile is cut into `ksplit`
@@ -151,6 +147,22 @@ __device__ __forceinline__ void dequant8(uint32_t w0, uint32_t w1, __half2 d2, u
     }
 }
 
+// 32 accumulator columns of this warp's lanes.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
+        "%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+          "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
+          "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
+          "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 struct mma_args {
     const __half *d;       // [rows][cols/32] block scales
     // The rows may be cut into up to three consecutive parts (q | k | v, gate | up), each with its own
@@ -182,43 +194,71 @@ struct ring {
     static __device__ __forceinline__ uint32_t empty_parity(uint32_t g) { return (g / D - 1u) & 1u; }
 };
 
-template <int BN>
+// BN tokens per issuer, ISS issuers, SETS converter sets of four warps.  A set's own K step is one serial chain of
+// about 0.7 us (raw tile -> registers -> f16 -> tensor memory), so two sets hand over a step of 8 KB of weights
+// every 0.35-0.4 us: enough for the tensor pipe at 128 tokens and more, but 3 TB/s of weights at a decode batch.
+// Up to 64 tokens one issuer suffices and the accumulator leaves room for twelve A stages: four sets then keep
+// the weights streaming (24576 x 4096 at 32 tokens).
+template <int BN, int ISS, int SETS, bool WIDE>
 struct mma_smem {
+    static constexpr int kIssuers = ISS, kConvWarps = 4 * SETS;
+    static constexpr int kWarpRaw = kConvWarps + kEpiWarps, kWarpTok = kWarpRaw + 1, kWarpMma = kWarpRaw + 2;
+    static constexpr int kThreads = (kWarpMma + ISS) * 32;
+    static constexpr int kScaleAhead = SETS > 2 ? 2 : 4;  // a set's own steps between a scale's load and its use
+    // Raw int8 weight tiles in flight.  The copy engine spends the same time on a 64-byte row of a box as on a
+    // 128-byte one: boxes of 64 columns stream at most 3.3-3.7 TB/s of weights, boxes of 128 columns (two K steps)
+    // 5.0-6.5 TB/s.  The wide tiles serve the forms whose shared memory has room for six of them; the others are
+    // bound by the tensor pipe, which asks for less.
+    static constexpr int kRawCols = WIDE ? 128 : 64;
+    static constexpr int kRawStages = WIDE ? 6 : 4;
     // One ring hands both operands of a K step to the issuers: stage s holds the converted weight tile
     // (tensor-memory columns kACol0 + 32 s) and the token sub-tiles (shared memory), behind ONE full
     // barrier (converter arrivals + the TMA's bytes) and ONE empty barrier (the issuers' commits), so
     // an issuer pays one wait and one commit per step.
-    static constexpr int kATmemStages = (512 - kIssuers * BN) / 32;  // what the accumulators leave
-    static constexpr int kStages = BN > 128 ? 4 : 6;
-    static constexpr uint32_t kRawBytes = kBM * kBK;             // int8
+    // A second set of accumulators where tensor memory has room for it: the next tile's MMAs run while the
+    // epilogue stores this one.
+    static constexpr int kAccs = SETS > 2 && 2 * ISS * BN <= 256 ? 2 : 1;
+    static constexpr int kATmemStages = (512 - kAccs * kIssuers * BN) / 32;  // what the accumulators leave
+    static constexpr int kStages = SETS > 2 ? 8 : BN > 128 ? 4 : 6;
+    static constexpr uint32_t kRawBytes = kBM * kRawCols;        // int8
     static constexpr uint32_t kSubBytes = BN * kBK * 2;          // one token sub-tile, f16
-    static constexpr uint32_t kBBytes = kIssuers * kSubBytes;    // a stage
+    // Four converter sets: every issuer multiplies the SAME tokens and takes K steps in turn, each into its own
+    // accumulator.  MMAs into one accumulator run one after the other, and at up to 64 tokens an MMA is all latency
+    // (64 busy cycles of about 250), so one chain would hold a K step at 0.37 us whatever feeds it.
+    static constexpr bool kTurns = SETS > 2;
+    static constexpr int kSubs = kTurns ? 1 : ISS;               // token sub-tiles of a tile
+    static constexpr uint32_t kBBytes = kSubs * kSubBytes;       // a stage
     static constexpr uint32_t kBOff = 0;
     static constexpr uint32_t kRawOff = kBOff + kStages * kBBytes;
     static constexpr uint32_t kBarOff = kRawOff + kRawStages * kRawBytes;
-    static constexpr uint32_t kBars = 2 * kRawStages + 2 * kStages + kIssuers + 1;
+    static constexpr uint32_t kBars = 2 * kRawStages + 2 * kStages + kAccs * (kIssuers + 1);
     static constexpr uint32_t kBytes = 1024 + kBarOff + kBars * 8 + 16;
-    static constexpr uint32_t kACol0 = kIssuers * BN;  // tensor-memory column of A stage 0, after the accumulators
+    static constexpr uint32_t kACol0 = kAccs * kIssuers * BN;  // tensor-memory column of A stage 0, after the accumulators
     static constexpr uint32_t kTmemCols = 512;
-    static_assert(kStages % 2 == 0 && kStages <= kATmemStages, "each converter set needs its own A stages");
+    static_assert(kStages % SETS == 0 && kStages <= kATmemStages, "each converter set needs its own A stages");
     static_assert(kBytes <= 232448, "shared memory per CTA");
 };
 
-template <int BN>
-__global__ void __launch_bounds__(kMmaThreads, 1)
+template <int BN, int ISS, int SETS, bool WIDE>
+__global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
     q8_gemm_mma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
                        const mma_args a) {
-    using L = mma_smem<BN>;
+    using L = mma_smem<BN, ISS, SETS, WIDE>;
+    constexpr int kRawStages = L::kRawStages, kConvWarps = L::kConvWarps, kIssuers = ISS;
+    constexpr int kScaleAhead = L::kScaleAhead;
+    constexpr int kWarpRaw = L::kWarpRaw, kWarpTok = L::kWarpTok, kWarpMma = L::kWarpMma;
     constexpr int kStages = L::kStages;
-    constexpr uint32_t kTB = kIssuers * BN;  // tokens per tile
+    constexpr bool kTurns = L::kTurns;
+    constexpr uint32_t kAccs = L::kAccs;
+    constexpr uint32_t kTB = L::kSubs * BN;  // tokens per tile
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte aligned stage buffers (swizzle atoms), then the barriers.
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char *sB = smem + L::kBOff, *sRaw = smem + L::kRawOff;
     uint64_t *raw_full = (uint64_t *)(smem + L::kBarOff), *raw_empty = raw_full + kRawStages;
     uint64_t *full = raw_empty + kRawStages, *empty = full + kStages;
-    uint64_t *acc_full = empty + kStages, *acc_empty = acc_full + kIssuers;
-    uint32_t *tmem_slot = (uint32_t *)(acc_empty + 1);
+    uint64_t *acc_full = empty + kStages, *acc_empty = acc_full + kAccs * kIssuers;
+    uint32_t *tmem_slot = (uint32_t *)(acc_empty + kAccs);
     volatile uint32_t *abort_s = tmem_slot + 1;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -232,14 +272,14 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     if (tid == 0) {
         for (int s = 0; s < kRawStages; ++s) {
             mbar_init(&raw_full[s], 1);            // the TMA thread's expect_tx arrival
-            mbar_init(&raw_empty[s], kConvWarps / 2);  // one arrival per converter warp of the set that read it
+            mbar_init(&raw_empty[s], WIDE ? 8 : 4);  // one arrival per converter warp and K step in it
         }
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(&full[s], kConvWarps / 2 + 1);  // the converter set's warps + the TMA thread's expect_tx arrival
-            mbar_init(&empty[s], kIssuers);           // one tcgen05.commit per issuer
+            mbar_init(&full[s], 4 + 1);  // the converter set's warps + the TMA thread's expect_tx arrival
+            mbar_init(&empty[s], kTurns ? 1 : kIssuers);  // one tcgen05.commit per issuer that reads the stage
         }
-        for (int s = 0; s < kIssuers; ++s) mbar_init(&acc_full[s], 1);  // tcgen05.commit after a tile's last MMA
-        mbar_init(acc_empty, kEpiWarps);                                    // one arrival per epilogue warp
+        for (uint32_t s = 0; s < kAccs * kIssuers; ++s) mbar_init(&acc_full[s], 1);  // tcgen05.commit after a tile's last MMA
+        for (uint32_t s = 0; s < kAccs; ++s) mbar_init(&acc_empty[s], kEpiWarps);                                    // one arrival per epilogue warp
         *abort_s = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -261,28 +301,34 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     // by those roles after their wait, so at most this kernel's direct predecessor can still be running.
     if (warp < kConvWarps) {
         // ---------------- converters ----------------
-        // Warps q and q + 4 reach tensor-memory lanes 32q..32q+31; set 0 (warps 0-3) converts the even K
-        // steps of the running count, set 1 the odd ones.  A thread owns tile row 32q + lane.
+        // Warps q, q + 4, ... reach tensor-memory lanes 32q..32q+31; set s (warps 4s..4s+3) converts K steps
+        // s, s + SETS, ... of the running count.  A thread owns tile row 32q + lane.
         const uint32_t set = (uint32_t)warp >> 2, quarter = (uint32_t)warp & 3u;
         const uint32_t trow = quarter * 32u + (uint32_t)lane;
-        const uint32_t rsw = (trow >> 1) & 3u;  // the TMA's 64-byte swizzle: 16-byte piece c of row r sits at c ^ ((r >> 1) & 3)
+        // The TMA's swizzle: 16-byte piece c of row r sits at c ^ ((r >> 1) & 3) (64-byte rows), c ^ (r & 7) (128).
+        const uint32_t rsw = WIDE ? trow & 7u : (trow >> 1) & 3u;
         const bool pair_load = (nb & 1u) == 0u;  // both scales of a K step in one aligned 4-byte load
         // Scale look-ahead: the position (tile, kb) of this set's step kScaleAhead own-steps in front.
         uint32_t la_tile = blockIdx.x, la_kb = 0;
-        auto la_advance = [&](uint32_t n) {
-            for (uint32_t i = 0; i < n; ++i)
-                if (++la_kb == nkb) {
-                    la_kb = 0;
-                    la_tile += gridDim.x;
-                }
+        const unsigned short *la_row = nullptr;  // this row's scales from the tile's first K step on
+        auto la_point = [&]() {
+            const uint32_t ot = la_tile / ksplit, r = min((ot % row_tiles) * kBM + trow, a.rows - 1u);
+            la_row = (const unsigned short *)a.d + (size_t)r * nb + (la_tile - ot * ksplit) * nkb * 2u;
         };
+        la_point();
+        auto la_advance = [&](uint32_t n) {
+            la_kb += n;
+            if (la_kb >= nkb) {
+                for (; la_kb >= nkb; la_kb -= nkb) la_tile += gridDim.x;
+                la_point();
+            }
+        };
+        const uint32_t last_blk = nb - 1u;
         auto scale_load = [&]() -> uint32_t {
             if (la_tile >= n_tiles) return 0u;
-            const uint32_t r = min(((la_tile / ksplit) % row_tiles) * kBM + trow, a.rows - 1u);
-            const uint32_t blk = ((la_tile % ksplit) * nkb + la_kb) * 2u;
-            const unsigned short *p = (const unsigned short *)a.d + (size_t)r * nb + blk;
+            const unsigned short *p = la_row + la_kb * 2u;
             if (pair_load) return __ldg((const uint32_t *)p);
-            const uint32_t lo = __ldg(p), hi = blk + 1u < nb ? (uint32_t)__ldg(p + 1) : 0u;
+            const uint32_t lo = __ldg(p), hi = la_kb * 2u < last_blk ? (uint32_t)__ldg(p + 1) : 0u;  // (never split)
             return lo | (hi << 16);
         };
         la_advance(set);
@@ -293,21 +339,27 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
 #pragma unroll
         for (int i = 0; i < kScaleAhead; ++i) {
             ring_d[i] = scale_load();
-            la_advance(2);
+            la_advance(SETS);
         }
-        // This set's steps, flat over the CTA's tiles: own step j is running step g = 2j + set.
+        // This set's steps, flat over the CTA's tiles: own step j is running step g = SETS * j + set.
         const uint32_t my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1u - blockIdx.x) / gridDim.x + 1u : 0u;
-        const uint32_t total = my_tiles * nkb, n_own = total > set ? (total - set + 1u) / 2u : 0u;
+        const uint32_t total = my_tiles * nkb, n_own = total > set ? (total - set + SETS - 1u) / SETS : 0u;
+        // Where own step j lies in the raw ring: its K step of the tile and, for wide tiles, the tile's first pair.
+        uint32_t kb = set, pair0 = 0;
+        const uint32_t pairs = (nkb + 1u) / 2u;
+        for (; WIDE && kb >= nkb; kb -= nkb) pair0 += pairs;
         bool ok = true;
         for (uint32_t j0 = 0; j0 < n_own && ok; j0 += kScaleAhead) {
 #pragma unroll
             for (int u = 0; u < kScaleAhead; ++u) {
                 if (j0 + (uint32_t)u >= n_own || !ok) break;
-                const uint32_t g = 2u * (j0 + (uint32_t)u) + set;
-                const uint32_t sr = ring<kRawStages>::stage(g), sa = ring<kStages>::stage(g);
+                const uint32_t g = (uint32_t)SETS * (j0 + (uint32_t)u) + set;
+                const uint32_t gr = WIDE ? pair0 + (kb >> 1) : g;  // raw fill number
+                const uint32_t sr = ring<kRawStages>::stage(gr), sa = ring<kStages>::stage(g);
                 // Convert into registers first; the A stage is needed only for the store.
-                ok = mbar_wait(&raw_full[sr], ring<kRawStages>::full_parity(g), abort_s);
-                const unsigned char *raw = sRaw + sr * L::kRawBytes + trow * kBK;
+                ok = mbar_wait(&raw_full[sr], ring<kRawStages>::full_parity(gr), abort_s);
+                const unsigned char *raw = sRaw + sr * L::kRawBytes + trow * (uint32_t)L::kRawCols;
+                const uint32_t c_first = WIDE ? (kb & 1u) * 4u : 0u;
                 const uint32_t dd = ring_d[u];
                 const __half2 d_lo = __half2half2(__ushort_as_half((unsigned short)(dd & 0xffffu)));
                 const __half2 d_hi = __half2half2(__ushort_as_half((unsigned short)(dd >> 16)));
@@ -315,16 +367,21 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                 // raw stage then goes back to the TMA thread, not after the stores below have completed.
                 int4 w4[4];
 #pragma unroll
-                for (uint32_t c = 0; c < 4; ++c) w4[c] = *(const int4 *)(raw + ((c ^ rsw) << 4));
+                for (uint32_t c = 0; c < 4; ++c) w4[c] = *(const int4 *)(raw + (((c_first + c) ^ rsw) << 4));
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&raw_empty[sr]);
+                if (lane == 0) {
+                    mbar_arrive(&raw_empty[sr]);
+                    if (WIDE && (kb & 1u) == 0u && kb + 1u == nkb) mbar_arrive(&raw_empty[sr]);  // no second step in it
+                }
+                if (WIDE)
+                    for (kb += SETS; kb >= nkb; kb -= nkb) pair0 += pairs;
                 uint32_t v[32];
                 dequant8((uint32_t)w4[0].x, (uint32_t)w4[0].y, d_lo, v);
                 dequant8((uint32_t)w4[0].z, (uint32_t)w4[0].w, d_lo, v + 4);
                 dequant8((uint32_t)w4[1].x, (uint32_t)w4[1].y, d_lo, v + 8);
                 dequant8((uint32_t)w4[1].z, (uint32_t)w4[1].w, d_lo, v + 12);
                 ring_d[u] = scale_load();
-                la_advance(2);
+                la_advance(SETS);
                 if (ok && ring<kStages>::must_wait_empty(g))
                     ok = mbar_wait(&empty[sa], ring<kStages>::empty_parity(g), abort_s);
                 ok = __all_sync(0xffffffffu, ok);  // the tensor-memory stores below are warp-collective
@@ -364,6 +421,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
         tmdev::pdl_trigger();
         for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
           const uint32_t ot = tile / ksplit, part = tile % ksplit;
+          const uint32_t acc0 = (it % kAccs) * (uint32_t)kIssuers;  // this tile's accumulators
           // Split K, pass 0: the accumulators go to this part's workspace slot; pass 1 (only the warp that
           // arrived last for this tile's row quarter): the parts are added in order and stored.
           for (uint32_t pass = 0; pass < (ksplit > 1u ? 2u : 1u) && ok; ++pass) {
@@ -377,7 +435,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
               __threadfence();
               if (lane == 0) a.kcount[ot * 4u + quarter] = 0u;  // ready for the next launch
           }
-          for (uint32_t sub = 0; sub < (uint32_t)kIssuers && ok; ++sub) {
+          for (uint32_t sub = 0; sub < (uint32_t)L::kSubs && ok; ++sub) {
             const uint32_t tile_row0 = (ot % row_tiles) * kBM;
             const uint32_t rr = tile_row0 + quarter * 32u + (uint32_t)lane;
             const uint32_t tok0 = (ot / row_tiles) * kTB + sub * BN;
@@ -388,7 +446,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
             const size_t stride = part_row1 - part_row0;  // rows of this part = token stride of its output
             float *ybase = (p0 ? a.y[0] : p1 ? a.y[1] : a.y[2]) + (rr - part_row0);
             if (pass == 0u) {
-                if (ok) ok = mbar_wait(&acc_full[sub], it & 1u, abort_s);
+                if (ok) ok = mbar_wait(&acc_full[acc0 + sub], (it / kAccs) & 1u, abort_s);
+                for (uint32_t i = 1; kTurns && i < (uint32_t)kIssuers; ++i)
+                    if (ok) ok = mbar_wait(&acc_full[acc0 + i], (it / kAccs) & 1u, abort_s);
                 ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads below are warp-collective
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -412,19 +472,18 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                         for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(pp == 0u ? f[j] : __uint_as_float(v[j]) + f[j]);
                     }
                 } else {
-                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + sub * BN + (uint32_t)c0;
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
-                    "%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                      "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
-                      "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
-                      "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (acc0 + sub) * BN + (uint32_t)c0, v);
+                if (kTurns) {
+                    // the other issuers' accumulators, in order (a tile of fewer K steps than issuers skips some)
+                    for (uint32_t i = 1; i < (uint32_t)kIssuers; ++i) {
+                        const uint32_t g0 = it * nkb, first = (i + (uint32_t)kIssuers - g0 % kIssuers) % kIssuers;
+                        if (nkb < (uint32_t)kIssuers && first >= nkb) continue;
+                        uint32_t f[32];
+                        tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (acc0 + i) * BN + (uint32_t)c0, f);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(f[j]));
+                    }
+                }
                 }
                 if (ksplit > 1u && pass == 0u) {
                     float *dst = a.kpart + (size_t)(ot * ksplit + part) * a.kslot +
@@ -470,7 +529,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                 // The accumulator may be overwritten once every warp has its values in registers.
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty);
+                if (lane == 0) mbar_arrive(&acc_empty[it % kAccs]);
             }
           }
             if (!ok) break;
@@ -484,7 +543,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
             for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
                 const int row0 = (int)(((tile / ksplit) % row_tiles) * kBM);
                 const uint32_t kb0 = (tile % ksplit) * nkb;
-                for (uint32_t kb = 0; kb < nkb; ++kb, ++g) {
+                for (uint32_t kb = 0; kb < nkb; kb += L::kRawCols / kBK, ++g) {
                     const uint32_t s = ring<kRawStages>::stage(g);
                     if (ring<kRawStages>::must_wait_empty(g))
                         ok = mbar_wait(&raw_empty[s], ring<kRawStages>::empty_parity(g), abort_s);
@@ -509,7 +568,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                 const uint32_t tok0 = (tile / ksplit / row_tiles) * kTB;
                 const uint32_t kb0 = (tile % ksplit) * nkb;
                 // A sub-tile wholly past the batch is neither loaded nor multiplied.
-                const uint32_t subs = tok0 + BN < a.batch ? (uint32_t)kIssuers : 1u;
+                const uint32_t subs = tok0 + BN < a.batch ? (uint32_t)L::kSubs : 1u;
                 for (uint32_t kb = 0; kb < nkb; ++kb, ++g) {
                     const uint32_t s = ring<kStages>::stage(g);
                     if (ring<kStages>::must_wait_empty(g))
@@ -531,31 +590,37 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
         // Stage indices and parities advance by increment: no divisions, no descriptor built from scratch.
         if (lane == 0) {
             constexpr uint32_t idesc = umma_idesc(kBM, BN);
-            const uint32_t sub = (uint32_t)(warp - kWarpMma);
+            const uint32_t me = (uint32_t)(warp - kWarpMma), sub = kTurns ? 0u : me;
+            constexpr uint32_t kStep = kTurns ? (uint32_t)kIssuers : 1u;  // K steps from one of this issuer's to the next
+            static_assert(kStages % kStep == 0, "an issuer's stages repeat");
             const uint64_t db0 = umma_desc(smem_u32(sB + sub * L::kSubBytes));
             const uint32_t db_lo = (uint32_t)db0, db_hi = (uint32_t)(db0 >> 32);
-            const uint32_t ta0 = tmem_base + L::kACol0, d_tmem = tmem_base + sub * BN;
-            uint32_t it = 0, st = 0, par = 0;
+            const uint32_t ta0 = tmem_base + L::kACol0;
+            uint32_t it = 0, st = kTurns ? me : 0u, par = 0;
+            uint32_t kb = st;  // this issuer's next K step, counted from the current tile's first
             bool ok = true;
             for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++it) {
                 const bool live = (tile / ksplit / row_tiles) * kTB + sub * BN < a.batch;  // else: the barrier protocol only
-                if (it >= 1u) ok = mbar_wait(acc_empty, (it - 1u) & 1u, abort_s);
+                const uint32_t buf = it % kAccs, d_tmem = tmem_base + (buf * (uint32_t)kIssuers + me) * BN;
+                if (it >= kAccs) ok = mbar_wait(&acc_empty[buf], (it / kAccs - 1u) & 1u, abort_s);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t accumulate = 0u;
-                for (uint32_t kb = 0; kb < nkb; ++kb) {
+                for (; kb < nkb; kb += kStep) {
                     ok = mbar_wait(&full[st], par, abort_s);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (live) umma_f16_ts_x4(d_tmem, ta0 + st * 32u, db_lo + st * (L::kBBytes >> 4), db_hi, idesc, accumulate);
                     accumulate = 1u;
                     umma_commit(&empty[st]);  // frees the stage once this issuer's MMAs have read it
-                    if (++st == (uint32_t)kStages) {
-                        st = 0;
+                    st += kStep;
+                    if (st >= (uint32_t)kStages) {
+                        st -= (uint32_t)kStages;
                         par ^= 1u;
                     }
                 }
-                if (ok) umma_commit(&acc_full[sub]);  // fires when every MMA of the tile has completed
+                kb -= nkb;
+                if (ok) umma_commit(&acc_full[buf * (uint32_t)kIssuers + me]);  // fires when every MMA of the tile has completed
             }
         }
     }
@@ -631,6 +696,26 @@ __global__ void __launch_bounds__(256) x_prep_f16_kernel(const float *x, const f
     }
 }
 
+}  // namespace
+
+// The f16 copy of X (with its prologue) into the context's GEMM workspace.
+cudaError_t tm_x_prep_launch(tm_cuda_ctx *ctx, int prologue, const float *x, const float *pro, uint32_t cols, uint32_t batch,
+                             float eps) {
+    __half *xh = (__half *)ctx->mma_scratch;
+    switch (prologue) {
+        case TM_CUDA_PRO_RMSNORM:
+            return tm_launch_pdl(ctx, x_prep_f16_kernel<TM_CUDA_PRO_RMSNORM>, dim3(batch), dim3(256), 0, x, pro, xh, cols, eps);
+        case TM_CUDA_PRO_SILU_MUL:
+            return tm_launch_pdl(ctx, x_prep_f16_kernel<TM_CUDA_PRO_SILU_MUL>, dim3(batch), dim3(256), 0, x, pro, xh, cols, eps);
+        case TM_CUDA_PRO_GELU_MUL:
+            return tm_launch_pdl(ctx, x_prep_f16_kernel<TM_CUDA_PRO_GELU_MUL>, dim3(batch), dim3(256), 0, x, pro, xh, cols, eps);
+        default:
+            return tm_launch_pdl(ctx, x_prep_f16_kernel<TM_CUDA_PRO_NONE>, dim3(batch), dim3(256), 0, x, pro, xh, cols, eps);
+    }
+}
+
+namespace {
+
 typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                     const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -651,17 +736,17 @@ encode_tiled_fn get_encode_tiled() {
     return fn;
 }
 
-template <int BN>
+template <int BN, int ISS, int SETS, bool WIDE>
 cudaError_t launch_mma(tm_cuda_ctx *ctx, const CUtensorMap &wmap, const CUtensorMap &xmap, const mma_args &a, int grid) {
     const int device = ctx->device;
     static std::atomic<bool> attr_done[64] = {};  // per device; contexts of a process share it
     if (device < 0 || device >= 64 || !attr_done[device].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(q8_gemm_mma_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)mma_smem<BN>::kBytes);
+        const cudaError_t e = cudaFuncSetAttribute(q8_gemm_mma_kernel<BN, ISS, SETS, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)mma_smem<BN, ISS, SETS, WIDE>::kBytes);
         if (e != cudaSuccess) return e;
         if (device >= 0 && device < 64) attr_done[device].store(true, std::memory_order_release);
     }
-    return tm_launch_pdl(ctx, q8_gemm_mma_kernel<BN>, dim3(grid), dim3(kMmaThreads), mma_smem<BN>::kBytes, wmap, xmap, a);
+    return tm_launch_pdl(ctx, q8_gemm_mma_kernel<BN, ISS, SETS, WIDE>, dim3(grid), dim3(mma_smem<BN, ISS, SETS, WIDE>::kThreads), mma_smem<BN, ISS, SETS, WIDE>::kBytes, wmap, xmap, a);
 }
 
 }  // namespace
@@ -710,7 +795,7 @@ size_t tm_cuda_mma_workspace_bytes(uint32_t cols, uint32_t batch) {
 }
 
 // Grows the f16 workspace when the call needs more (outside a dispatch group only).
-static int mma_ensure_workspace(tm_cuda_ctx *ctx, uint32_t cols, uint32_t batch, char *err, size_t err_cap) {
+int tm_mma_ensure_workspace(tm_cuda_ctx *ctx, uint32_t cols, uint32_t batch, char *err, size_t err_cap) {
     const size_t need = tm_cuda_mma_workspace_bytes(cols, batch);
     bool small;
     {
@@ -754,12 +839,17 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
             }
         }
     }
+    // Up to 128 tokens, the forms with four converter sets (one token tile, as with two 64-token sub-tiles, so the
+    // split below is the same): 24576 x 4096 46 -> 36 us at 32 tokens, 60 -> 50 us at 128.  From 65 tokens on they
+    // pay only where an SM has at least eight K steps to stream (4096 x 1024 at 128: 19 us against 16).
+    const uint64_t sm_steps = (uint64_t)row_tiles * ((cols + kBK - 1) / kBK) / sms;
+    const int few = push.world ? 0 : batch <= 32u ? 32 : batch <= 64u ? 64 : batch <= 128u && sm_steps >= 8u ? 128 : 0;
     CUtensorMap xmap, wmap;
     const cuuint32_t estr[2] = {1, 1};
     {
         const cuuint64_t gdim[2] = {cols, batch};
         const cuuint64_t gstride[1] = {(cuuint64_t)cols * 2};
-        const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)bn};
+        const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)(few ? few : bn)};
         const CUresult cr = encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)xh, gdim, gstride, box, estr,
                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -767,12 +857,13 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
             return tm_fail(err, err_cap, TM_CUDA_ERR_INTERNAL, "cuTensorMapEncodeTiled (tokens) failed (%d)", (int)cr);
     }
     {
-        // The int8 plane as bytes, 64 x 128 boxes, 64-byte swizzle; rows and columns past the end read as zero.
+        // The int8 plane as bytes, boxes of 128 rows by 64 or 128 columns; rows and columns past the end read as zero.
+        const bool wide = few != 0 || bn == 64;
         const cuuint64_t gdim[2] = {cols, rows};
         const cuuint64_t gstride[1] = {(cuuint64_t)cols};
-        const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)kBM};
+        const cuuint32_t box[2] = {(cuuint32_t)(wide ? 2 * kBK : kBK), (cuuint32_t)kBM};
         const CUresult cr = encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)w->qp, gdim, gstride, box, estr,
-                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                                   CU_TENSOR_MAP_INTERLEAVE_NONE, wide ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS)
             return tm_fail(err, err_cap, TM_CUDA_ERR_INTERNAL, "cuTensorMapEncodeTiled (weights) failed (%d)", (int)cr);
@@ -825,9 +916,12 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     ctx->mma_last_ksplit = (int)a.ksplit;
     const uint32_t n_tiles = row_tiles * ((batch + 2 * bn - 1) / (2 * bn)) * a.ksplit;
     const int grid = (int)(n_tiles < (uint32_t)ctx->sm_count ? n_tiles : (uint32_t)ctx->sm_count);
-    TM_CUDA_TRY(bn == 192   ? launch_mma<192>(ctx, wmap, xmap, a, grid)
-                : bn == 128 ? launch_mma<128>(ctx, wmap, xmap, a, grid)
-                            : launch_mma<64>(ctx, wmap, xmap, a, grid));
+    TM_CUDA_TRY(few == 32   ? (launch_mma<32, 4, 4, true>(ctx, wmap, xmap, a, grid))
+                : few == 64 ? (launch_mma<64, 2, 4, true>(ctx, wmap, xmap, a, grid))
+                : few == 128 ? (launch_mma<128, 2, 4, true>(ctx, wmap, xmap, a, grid))
+                : bn == 192 ? (launch_mma<192, 2, 2, false>(ctx, wmap, xmap, a, grid))
+                : bn == 128 ? (launch_mma<128, 2, 2, false>(ctx, wmap, xmap, a, grid))
+                            : (launch_mma<64, 2, 2, true>(ctx, wmap, xmap, a, grid)));
     return TM_CUDA_OK;
 }
 
@@ -840,7 +934,7 @@ int tm_cuda_q8_0_gemm_mma(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x
         return tm_cuda_q8_0_gemm(ctx, w, x, y, rows, cols, batch, x_off, y_off, err, err_cap);
     }
     {
-        const int rc = mma_ensure_workspace(ctx, cols, batch, err, err_cap);
+        const int rc = tm_mma_ensure_workspace(ctx, cols, batch, err, err_cap);
         if (rc != TM_CUDA_OK) return rc;
     }
     TM_ENTER();
@@ -867,7 +961,7 @@ int tm_cuda_q8_0_gemm_mma_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buf
                                 const uint32_t *part_rows, int prologue, tm_cuda_buffer *pro, float eps, int epilogue,
                                 char *err, size_t err_cap) {
     {
-        const int rc = mma_ensure_workspace(ctx, cols, batch, err, err_cap);
+        const int rc = tm_mma_ensure_workspace(ctx, cols, batch, err, err_cap);
         if (rc != TM_CUDA_OK) return rc;
     }
     TM_ENTER();
@@ -896,21 +990,8 @@ int tm_cuda_q8_0_gemm_mma_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buf
     if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_BUF(pro, (size_t)cols * 4, "norm weight");
     else if (prologue != TM_CUDA_PRO_NONE) TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate operand");
     TM_OP_BEGIN("q8_0_gemm_mma_fused");
-    __half *xh = (__half *)ctx->mma_scratch;
-    const float *xp = (const float *)x->dev, *pp = pro ? (const float *)pro->dev : nullptr;
-    switch (prologue) {
-        case TM_CUDA_PRO_RMSNORM:
-            TM_CUDA_TRY(tm_launch_pdl(ctx, x_prep_f16_kernel<TM_CUDA_PRO_RMSNORM>, dim3(batch), dim3(256), 0, xp, pp, xh, cols, eps));
-            break;
-        case TM_CUDA_PRO_SILU_MUL:
-            TM_CUDA_TRY(tm_launch_pdl(ctx, x_prep_f16_kernel<TM_CUDA_PRO_SILU_MUL>, dim3(batch), dim3(256), 0, xp, pp, xh, cols, eps));
-            break;
-        case TM_CUDA_PRO_GELU_MUL:
-            TM_CUDA_TRY(tm_launch_pdl(ctx, x_prep_f16_kernel<TM_CUDA_PRO_GELU_MUL>, dim3(batch), dim3(256), 0, xp, pp, xh, cols, eps));
-            break;
-        default:
-            TM_CUDA_TRY(tm_launch_pdl(ctx, x_prep_f16_kernel<TM_CUDA_PRO_NONE>, dim3(batch), dim3(256), 0, xp, pp, xh, cols, eps));
-    }
+    TM_CUDA_TRY(tm_x_prep_launch(ctx, prologue, (const float *)x->dev, pro ? (const float *)pro->dev : nullptr, cols, batch,
+                                 eps));
     rc = mma_launch(ctx, w, rows, cols, batch, ys, ends, epilogue == TM_CUDA_EPI_ADD, err, err_cap);
     if (rc != TM_CUDA_OK) return rc;
     TM_OP_END(2);
@@ -919,7 +1000,7 @@ int tm_cuda_q8_0_gemm_mma_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buf
 int tm_cuda_q8_0_gemm_mma_push(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, tm_cuda_buffer *dst,
                                uint32_t rows, uint32_t cols, uint32_t batch, char *err, size_t err_cap) {
     {
-        const int rc = mma_ensure_workspace(ctx, cols, batch, err, err_cap);
+        const int rc = tm_mma_ensure_workspace(ctx, cols, batch, err, err_cap);
         if (rc != TM_CUDA_OK) return rc;
     }
     TM_ENTER();
