@@ -250,8 +250,10 @@ int tm_cuda_rows_indirect_f32(tm_cuda_ctx *ctx, tm_cuda_buffer *w, uint32_t rows
  *             | 3 x = gelu_tanh(x) * px            (pw/px: `pro` buffer)
  *   epilogue: 0 y = Wx  | 1 y += Wx */
 enum { TM_CUDA_PRO_NONE = 0, TM_CUDA_PRO_RMSNORM = 1, TM_CUDA_PRO_SILU_MUL = 2,
-       TM_CUDA_PRO_GELU_MUL = 3 };
-enum { TM_CUDA_EPI_STORE = 0, TM_CUDA_EPI_ADD = 1 };
+       TM_CUDA_PRO_GELU_MUL = 3,
+       TM_CUDA_PRO_F16 = 4 }; /* tm_cuda_q8_0_gemm_rows: x holds binary16 values */
+enum { TM_CUDA_EPI_STORE = 0, TM_CUDA_EPI_ADD = 1,
+       TM_CUDA_EPI_SILU_MUL_F16 = 2, TM_CUDA_EPI_GELU_MUL_F16 = 3 }; /* tm_cuda_q8_0_gemm_rows */
 int tm_cuda_q8_0_gemv_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x,
                             tm_cuda_buffer *y, uint32_t rows, uint32_t cols, int prologue,
                             tm_cuda_buffer *pro, float eps, int epilogue, char *err,
@@ -433,6 +435,17 @@ int tm_cuda_q8_0_gemm_mma_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buf
                                 uint32_t cols, uint32_t batch, uint32_t n_parts,
                                 tm_cuda_buffer *const *y_parts, const uint32_t *part_rows, int prologue,
                                 tm_cuda_buffer *pro, float eps, int epilogue, char *err, size_t err_cap);
+/* No counterpart: the same multiply, arguments and numerical profile for the rows of a decode step of several
+ * sequences or of a short prompt (batch <= TM_CUDA_GEMM_ROWS_MAX_BATCH, cols a multiple of 64).  Parts need
+ * multiples of 32 rows.  TM_CUDA_PRO_F16: x is [batch][cols] binary16, used as it is.  TM_CUDA_EPI_SILU_MUL_F16 /
+ * _GELU_MUL_F16: w is gate rows above as many up rows; y_parts[0] receives act(gate x) * (up x) as
+ * [batch][rows / 2] binary16, the operand of the next call's TM_CUDA_PRO_F16.  _pays: whether it is the faster of
+ * the two kernels for this size. */
+#define TM_CUDA_GEMM_ROWS_MAX_BATCH 32
+int tm_cuda_q8_0_gemm_rows_pays(uint32_t rows, uint32_t cols, uint32_t batch, int gated);
+int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, uint32_t rows, uint32_t cols,
+                           uint32_t batch, uint32_t n_parts, tm_cuda_buffer *const *y_parts, const uint32_t *part_rows,
+                           int prologue, tm_cuda_buffer *pro, float eps, int epilogue, char *err, size_t err_cap);
 /* No counterpart: tm_cuda_rmsnorm_f32 (q heads), tm_cuda_rmsnorm_f32 (k heads),
  * tm_cuda_qwen35_rope_partial_chunk and tm_cuda_qwen35_kv_store_f16_chunk as one
  * launch for a chunk of n token rows at pos0: q [n][heads][head_dim] is normed and

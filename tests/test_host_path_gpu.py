@@ -14,7 +14,7 @@ def test_store_u32_lands_where_asked_and_nowhere_else(ctx, n, indexed):
     size = 2 * n + 5
     buf = ctx.buffer(size * 4)
     buf.zero()
-    vals = (np.arange(n, dtype=np.uint32) * 2654435761 % 2 ** 32).astype(np.uint32)
+    vals = (np.arange(n, dtype=np.uint64) * 2654435761 % 2 ** 32).astype(np.uint32)
     idx = np.random.default_rng(n).permutation(size)[:n].astype(np.uint32) if indexed else np.arange(3, 3 + n)
     buf.store_u32(vals, first=3, index=idx if indexed else None)
     want = np.zeros(size, np.uint32)

@@ -238,6 +238,18 @@ public:
         TM_CALL(tm_cuda_q8_0_gemm_mma_fused, w.raw(), x.raw(), rows, cols, batch, n, yp, pr, prologue,
                 pro ? pro->raw() : nullptr, eps, epilogue);
     }
+    void q8_0_gemm_rows(const CudaBuffer &w, const CudaBuffer &x, uint32_t rows, uint32_t cols, uint32_t batch,
+                             std::initializer_list<const CudaBuffer *> ys, std::initializer_list<uint32_t> part_rows,
+                             int prologue, const CudaBuffer *pro, float eps, int epilogue) const {
+        tm_cuda_buffer *yp[3] = {nullptr, nullptr, nullptr};
+        uint32_t pr[3] = {0, 0, 0};
+        uint32_t n = 0;
+        for (const CudaBuffer *b : ys) yp[n++] = b->raw();
+        n = 0;
+        for (uint32_t r : part_rows) pr[n++] = r;
+        TM_CALL(tm_cuda_q8_0_gemm_rows, w.raw(), x.raw(), rows, cols, batch, n, yp, pr, prologue,
+                pro ? pro->raw() : nullptr, eps, epilogue);
+    }
     void qk_prep_chunk(const CudaBuffer &q, const CudaBuffer &k, const CudaBuffer &v, const CudaBuffer &qn,
                        const CudaBuffer &kn, const CudaBuffer &inv_freq, const CudaBuffer &kc, const CudaBuffer &vc,
                        uint32_t heads, uint32_t kvh, uint32_t hd, uint32_t n_rot, uint32_t pos0, uint32_t cap, uint32_t n,

@@ -288,6 +288,17 @@ struct Matrix {
     void gemm_all(const CudaContext &ctx, const CudaBuffer &x, const CudaBuffer &y, uint32_t batch, bool exact) const {
         gemm(ctx, buf, rows, cols, x, y, batch, exact, type);
     }
+    // The f16-operand multiply with its neighbours folded in (cut into `part_rows` outputs): a few rows take the
+    // register-operand kernel, whose units are short enough to fill the machine, a prefill chunk the tcgen05 one.
+    static bool few_rows(const Matrix &m, uint32_t n, bool gated = false) {
+        return m.type == 8 && tm_cuda_q8_0_gemm_rows_pays(m.rows, m.cols, n, gated);
+    }
+    void gemm_f16(const CudaContext &ctx, const CudaBuffer &x, uint32_t n, std::initializer_list<const CudaBuffer *> ys,
+                  std::initializer_list<uint32_t> rows_of, int prologue, const CudaBuffer *pro, float eps,
+                  int epilogue) const {
+        if (few_rows(*this, n)) ctx.q8_0_gemm_rows(buf, x, rows, cols, n, ys, rows_of, prologue, pro, eps, epilogue);
+        else ctx.q8_0_gemm_mma_fused(buf, x, rows, cols, n, ys, rows_of, prologue, pro, eps, epilogue);
+    }
     // One token, with the neighbouring elementwise operators folded in (include/tm_cuda.h).
     void gemv_fused(const CudaContext &ctx, const CudaBuffer &x, const CudaBuffer &y, int prologue, const CudaBuffer *pro,
                     float eps, int epilogue) const {
@@ -483,17 +494,26 @@ struct SwiGluBlock {
     void prefill_fused(const CudaContext &ctx, const PrefillScratch &s, size_t n, const CudaBuffer &post_norm,
                        size_t hidden) const {
         const uint32_t nn = (uint32_t)n;
-        ctx.q8_0_gemm_mma_fused(gate_up.buf, s.x, gate_up.rows, gate_up.cols, nn, {&s.g, &s.u},
-                                {(uint32_t)width, (uint32_t)width}, TM_CUDA_PRO_RMSNORM, &post_norm, eps,
-                                TM_CUDA_EPI_STORE);
-        const int pro = act == GluActivation::Silu ? TM_CUDA_PRO_SILU_MUL : TM_CUDA_PRO_GELU_MUL;
-        if (out_norm) {
-            ctx.q8_0_gemm_mma_fused(down.buf, s.g, down.rows, down.cols, nn, {&s.d2}, {down.rows}, pro, &s.u, 0.0f,
+        const bool silu = act == GluActivation::Silu;
+        const CudaBuffer *x = &s.g, *up = &s.u;
+        int pro = silu ? TM_CUDA_PRO_SILU_MUL : TM_CUDA_PRO_GELU_MUL;
+        if (Matrix::few_rows(gate_up, nn, true) && Matrix::few_rows(down, nn)) {
+            // s.g holds the activated product in binary16, ready for the down projection
+            ctx.q8_0_gemm_rows(gate_up.buf, s.x, gate_up.rows, gate_up.cols, nn, {&s.g}, {(uint32_t)width},
+                               TM_CUDA_PRO_RMSNORM, &post_norm, eps,
+                               silu ? TM_CUDA_EPI_SILU_MUL_F16 : TM_CUDA_EPI_GELU_MUL_F16);
+            pro = TM_CUDA_PRO_F16;
+            up = nullptr;
+        } else {
+            ctx.q8_0_gemm_mma_fused(gate_up.buf, s.x, gate_up.rows, gate_up.cols, nn, {&s.g, &s.u},
+                                    {(uint32_t)width, (uint32_t)width}, TM_CUDA_PRO_RMSNORM, &post_norm, eps,
                                     TM_CUDA_EPI_STORE);
+        }
+        if (out_norm) {
+            down.gemm_f16(ctx, *x, nn, {&s.d2}, {down.rows}, pro, up, 0.0f, TM_CUDA_EPI_STORE);
             ctx.rmsnorm_add(s.d2, out_norm, s.x, nn, (uint32_t)hidden, eps);
         } else {
-            ctx.q8_0_gemm_mma_fused(down.buf, s.g, down.rows, down.cols, nn, {&s.x}, {down.rows}, pro, &s.u, 0.0f,
-                                    TM_CUDA_EPI_ADD);
+            down.gemm_f16(ctx, *x, nn, {&s.x}, {down.rows}, pro, up, 0.0f, TM_CUDA_EPI_ADD);
         }
     }
     // x += ffn(h2) for the n chunk rows of s.h2 / s.x (engine/metal.rs:514-534).
@@ -650,9 +670,8 @@ struct AttentionBlock {
     void prefill_fused(const CudaContext &ctx, const PrefillScratch &s, size_t n, uint32_t pos0,
                        const CudaBuffer &pre_norm, const RowsAre &rows) const {
         const uint32_t nn = (uint32_t)n, heads = (uint32_t)heads_l, kv = (uint32_t)kv_l, hd = (uint32_t)spec.head_dim;
-        ctx.q8_0_gemm_mma_fused(qkv.buf, s.x, qkv.rows, qkv.cols, nn, {&s.a, &s.b, &s.c},
-                                {qkv.part_rows[0], qkv.part_rows[1], qkv.part_rows[2]}, TM_CUDA_PRO_RMSNORM, &pre_norm,
-                                eps, TM_CUDA_EPI_STORE);
+        qkv.gemm_f16(ctx, s.x, nn, {&s.a, &s.b, &s.c}, {qkv.part_rows[0], qkv.part_rows[1], qkv.part_rows[2]},
+                     TM_CUDA_PRO_RMSNORM, &pre_norm, eps, TM_CUDA_EPI_STORE);
         if (rows.pos_buf) {  // one row per sequence
             attend_batch(ctx, s.a, s.b, s.c, 0, 0, s.e, n, *rows.pos_buf, *rows.status, false);
             return;
@@ -808,11 +827,15 @@ struct Layer {
         if (!exact && mixer.fusable() && ffn.fusable()) {
             mixer.prefill_fused(ctx, s, n, pos0, pre_norm, rows);
             if (mixer_out_norm) {
-                mixer.o.gemm_all(ctx, s.e, s.proj, nn, false);
+                // (a handful of rows of a narrow matrix keep the exact GEMV: tm_cuda_q8_0_gemm_mma)
+                if (Matrix::few_rows(mixer.o, nn) && nn >= 3 && (nn >= 9 || mixer.o.cols >= 2048))
+                    mixer.o.gemm_f16(ctx, s.e, nn, {&s.proj}, {mixer.o.rows}, TM_CUDA_PRO_NONE, nullptr, 0.0f,
+                                     TM_CUDA_EPI_STORE);
+                else
+                    mixer.o.gemm_all(ctx, s.e, s.proj, nn, false);
                 ctx.rmsnorm_add(s.proj, mixer_out_norm, s.x, nn, (uint32_t)hidden, eps);
             } else {
-                ctx.q8_0_gemm_mma_fused(mixer.o.buf, s.e, mixer.o.rows, mixer.o.cols, nn, {&s.x}, {mixer.o.rows},
-                                        TM_CUDA_PRO_NONE, nullptr, 0.0f, TM_CUDA_EPI_ADD);
+                mixer.o.gemm_f16(ctx, s.e, nn, {&s.x}, {mixer.o.rows}, TM_CUDA_PRO_NONE, nullptr, 0.0f, TM_CUDA_EPI_ADD);
             }
             ffn.prefill_fused(ctx, s, n, post_norm, hidden);
             return;
@@ -874,6 +897,7 @@ struct EngineModel::Impl {
     CudaGraph batch_graph;
     std::vector<size_t> pos_b;  // host copy of every sequence's position
     const CudaBuffer &head_buf() const { return tied ? (sh.world > 1 ? tied_view : embedding.buf) : head_own.buf; }
+    const Matrix &head() const { return tied ? embedding : head_own; }  // single device only
     uint32_t head_cols() const { return embedding.cols; }
     uint32_t head_type() const { return tied ? embedding.type : head_own.type; }
     // Final norm folded into the vocabulary projection of the one row in `x`.
@@ -1206,6 +1230,9 @@ void EngineModel::encode_batch_step() {
     if (slices) {
         c.q8_0_gemm_fused(I.head_buf(), I.scratch.x, I.logits, I.head_rows, I.head_cols(), (uint32_t)S,
                           TM_CUDA_PRO_RMSNORM, &I.final_norm, g.eps, TM_CUDA_EPI_STORE);
+    } else if (!opts_.exact && S > slice_limit && I.sh.world == 1 && Matrix::few_rows(I.head(), (uint32_t)S)) {
+        I.head().gemm_f16(c, I.scratch.x, (uint32_t)S, {&I.logits}, {I.head_rows}, TM_CUDA_PRO_RMSNORM, &I.final_norm,
+                          g.eps, TM_CUDA_EPI_STORE);
     } else {
         c.rmsnorm(I.scratch.x, I.final_norm, I.scratch.h, (uint32_t)S, (uint32_t)g.hidden, g.eps);
         Matrix::gemm(c, I.head_buf(), I.head_rows, I.head_cols(), I.scratch.h, I.logits, (uint32_t)S, opts_.exact,

@@ -1,0 +1,421 @@
+// The f16-operand multiply for a few rows of activations (a decode step of several sequences, a short prompt):
+// Y[b, :] = W X[b, :] for b < batch <= 32, the numerical profile of the tcgen05 GEMM in tm_cuda_mma.cu (x and
+// d * q rounded to binary16 once each, products summed in f32) on a kernel shaped like the decode GEMV.
+//
+// What bounds it: the weights' bytes, and below ~8 MB the chain launch -> activations -> products -> sum.  The
+// tcgen05 kernel is bound by neither at these batches: its weight tile goes TMA -> shared memory -> registers ->
+// tensor memory -> MMA as one serial chain of 0.7 us per 64 columns, 12-15 us for a 4096 x 1024 projection of 32
+// rows that is 0.7 us of HBM traffic.  Here a warp reads int8 quants the way the GEMV does (16 bytes per lane
+// and row through a cp.async ring), turns them into the A operand in registers -- 7 instructions per 4 weights,
+// once for all rows of X -- and multiplies with m16n8k16 at most four token tiles.  At 32 rows that is 0.4 of the
+// issue slots the weight stream leaves, so mma.sync suffices; from 33 rows on the tcgen05 kernel serves.
+//
+// Split.  A unit is 32 weight rows (two 16-row tiles, so that one read of the token fragments feeds two tiles).
+// A cluster of P CTAs owns a unit, each CTA a P-th of K, each of its 8 warps every 8th 64-column chunk of that;
+// the CTA's share of X (f16) stays in shared memory for all units it serves.  Sums meet in a fixed order: the
+// 8 warps through shared memory, the P CTAs through distributed shared memory -- no workspace, no counters.
+// P is the smallest cost of rounds x chunks a warp streams (see plan_rows).
+#include "tm_cuda_internal.cuh"
+#include "tm_cuda_device.cuh"
+
+namespace {
+
+constexpr int kWarps = 8, kThreads = 256;
+constexpr uint32_t kSlot = 2048u + 128u;  // 32 rows x 64 quants, 32 rows x 2 scales
+constexpr uint32_t kRowPad = 36;          // floats per token of a partial sum: lanes (g, t) land in 32 banks
+
+enum : uint32_t { kPlain = 0, kSilu = 1, kGelu = 2 };
+
+struct rows_args {
+    const signed char *q;
+    const unsigned short *d;
+    const __half *x;       // [batch][cols]
+    float *y[3];           // up to three consecutive row ranges with dense outputs of their own
+    uint32_t part_end[3];  // exclusive row bound of each (multiples of 32 but the last)
+    __half *act;           // gated forms: act(gate) * up, [batch][rows / 2]
+    uint32_t rows, cols, batch, units, accumulate, mode, ring;
+};
+
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Four quants -> two half2 of RN(d * q): bytes become f16 1024 + (q + 128) by permutes, minus 1152, times d.
+__device__ __forceinline__ void dequant4(uint32_t w, __half2 d2, uint32_t &lo, uint32_t &hi) {
+    const __half2 bias = __half2half2(__ushort_as_half((unsigned short)0x6480));
+    const uint32_t u = w ^ 0x80808080u;
+    const uint32_t p = __byte_perm(u, 0x64646464u, 0x4140), s = __byte_perm(u, 0x64646464u, 0x4342);
+    const __half2 a = __hmul2(__hsub2(*(const __half2 *)&p, bias), d2);
+    const __half2 b = __hmul2(__hsub2(*(const __half2 *)&s, bias), d2);
+    lo = *(const uint32_t *)&a;
+    hi = *(const uint32_t *)&b;
+}
+
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t v;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t v;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote));
+    return v;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kThreads) q8_gemm_rows_kernel(const rows_args a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr uint32_t kTok = NT * 8;
+    const uint32_t P = cluster_size(), rank = P > 1 ? cluster_rank() : 0u;
+    const uint32_t n_clusters = gridDim.x / P, cluster = blockIdx.x / P;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const uint32_t n_chunks = a.cols / 64u, nb = a.cols / 32u;
+    const uint32_t c0 = n_chunks * rank / P, c1 = n_chunks * (rank + 1) / P;
+    const uint32_t kc_max = (n_chunks + P - 1) / P;
+    const uint32_t xstride = kc_max * 128u + 16u;  // 16 mod 128: the 16-byte reads of 8 lanes hit distinct banks
+    unsigned char *xs = smem;
+    float *red = (float *)(smem + kTok * xstride);      // [warp][token][kRowPad]
+    float *part = red + kWarps * kTok * kRowPad;        // [2][token][32]
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(part + (P > 1 ? 2 * kTok * 32 : 0)) + warp * a.ring * kSlot;
+    const uint32_t half_rows = a.rows / 2u;
+
+    // Row r (0..31) of a unit: consecutive rows, or 16 gate rows and the 16 up rows they gate.
+    auto row_of = [&](uint32_t unit, uint32_t r) -> uint32_t {
+        if (a.mode == kPlain) return min(unit * 32u + r, a.rows - 1u);
+        return unit * 16u + (r & 15u) + (r >= 16u ? half_rows : 0u);
+    };
+    uint32_t ld_unit = cluster, ld_c = c0 + warp;
+    if (ld_c >= c1) ld_unit = a.units;  // fewer chunks than warps: this one only adds zeros
+    auto issue = [&](uint32_t slot) {
+        if (ld_unit < a.units) {
+            const uint32_t dst = ring + slot * kSlot;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const signed char *p = a.q + (size_t)row_of(ld_unit, g + 8u * i) * a.cols + ld_c * 64u + t4 * 16u;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 512u + lane * 16u), "l"(p) : "memory");
+            }
+            const unsigned short *s = a.d + (size_t)row_of(ld_unit, lane) * nb + ld_c * 2u;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 2048u + lane * 4u), "l"(s) : "memory");
+            ld_c += kWarps;
+            if (ld_c >= c1) {
+                ld_c = c0 + warp;
+                ld_unit += n_clusters;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const uint32_t depth = a.ring;
+    for (uint32_t i = 0; i < depth; ++i) issue(i);
+
+    tmdev::pdl_trigger();
+    tmdev::pdl_wait();
+    {   // this CTA's columns of X; rows past the batch are zero
+        const uint32_t q16 = (c1 - c0) * 8u, total = kTok * q16;  // 16-byte pieces
+        constexpr uint32_t kBatch = 8;
+        for (uint32_t b = threadIdx.x; b < total; b += kThreads * kBatch) {
+            int4 v[kBatch];
+#pragma unroll
+            for (uint32_t i = 0; i < kBatch; ++i) {
+                const uint32_t at = b + i * kThreads, t = at / q16, c = at % q16;
+                v[i] = make_int4(0, 0, 0, 0);
+                if (at < total && t < a.batch) v[i] = __ldcg((const int4 *)(a.x + (size_t)t * a.cols + c0 * 64u) + c);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < kBatch; ++i) {
+                const uint32_t at = b + i * kThreads, t = at / q16, c = at % q16;
+                if (at < total) *(int4 *)(xs + t * xstride + c * 16u) = v[i];
+            }
+        }
+    }
+    __syncthreads();
+
+    uint32_t slot = 0, it = 0;
+    for (uint32_t unit = cluster; unit < a.units; unit += n_clusters, ++it) {
+        float acc[2][NT][4];
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.0f;
+#pragma unroll 1
+        for (uint32_t c = c0 + warp; c < c1; c += kWarps) {
+            // The oldest group has landed when at most depth - 1 are outstanding (depth is 2, 3, 4 or 6).
+            if (depth == 6) asm volatile("cp.async.wait_group 5;" ::: "memory");
+            else if (depth == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+            else if (depth == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+            else asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            const uint32_t src = ring + slot * kSlot;
+            uint32_t w[4][4];
+            __half2 d2[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[i][0]), "=r"(w[i][1]), "=r"(w[i][2]), "=r"(w[i][3]) : "r"(src + i * 512u + lane * 16u));
+                unsigned short h;
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(src + 2048u + (g + 8u * i) * 4u + (t4 >> 1) * 2u));
+                d2[i] = __half2half2(__ushort_as_half(h));
+            }
+            __syncwarp();
+            issue(slot);
+            slot = slot + 1u == depth ? 0u : slot + 1u;
+            const unsigned char *xp = xs + g * xstride + (c - c0) * 128u + t4 * 32u;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {  // two 16-byte pieces of x, two MMAs of K = 16 each
+                uint32_t af[2][2][4];
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        dequant4(w[2 * m][2 * h + j], d2[2 * m], af[j][m][0], af[j][m][2]);
+                        dequant4(w[2 * m + 1][2 * h + j], d2[2 * m + 1], af[j][m][1], af[j][m][3]);
+                    }
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    const uint4 b = *(const uint4 *)(xp + n * 8u * xstride + h * 16u);
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        mma_f16(acc[m][n], af[0][m][0], af[0][m][1], af[0][m][2], af[0][m][3], b.x, b.y);
+                        mma_f16(acc[m][n], af[1][m][0], af[1][m][1], af[1][m][2], af[1][m][3], b.z, b.w);
+                    }
+                }
+            }
+        }
+        // ---- the 8 warps' sums, then the CTAs' ----
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                float *r = red + (warp * kTok + n * 8u + 2u * t4) * kRowPad + m * 16u + g;
+                r[0] = acc[m][n][0];
+                r[kRowPad] = acc[m][n][1];
+                r[8] = acc[m][n][2];
+                r[kRowPad + 8] = acc[m][n][3];
+            }
+        __syncthreads();
+        float *mine = part + (it & 1u) * kTok * 32u;
+        float sum[NT];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const uint32_t tok = warp + 8u * i;
+            float v = 0.0f;
+#pragma unroll
+            for (int k = 0; k < kWarps; ++k) v += red[(k * kTok + tok) * kRowPad + lane];
+            sum[i] = v;
+            if (P > 1) mine[tok * 32u + lane] = v;
+        }
+        if (P > 1) cluster_sync();  // also: every warp has read `red`
+        else __syncthreads();
+        // Token tok of the unit is finished by CTA tok % P (all of them when P is 1).
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const uint32_t tok = P > 1 ? rank + P * (warp + 8u * i) : warp + 8u * i;
+            if (tok >= a.batch) break;
+            float v = sum[i];
+            if (P > 1) {
+                const uint32_t at = (uint32_t)__cvta_generic_to_shared(mine + tok * 32u + lane);
+                float pv[8];
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) pv[k] = k < P ? ld_cluster(at, k) : 0.0f;
+                v = pv[0];
+#pragma unroll
+                for (uint32_t k = 1; k < 8; ++k)
+                    if (k < P) v += pv[k];
+            }
+            if (a.mode == kPlain) {
+                const uint32_t row0 = unit * 32u, row = row0 + lane;
+                const bool p0 = row0 < a.part_end[0], p1 = row0 < a.part_end[1];
+                const uint32_t lo = p0 ? 0u : p1 ? a.part_end[0] : a.part_end[1];
+                const uint32_t hi = p0 ? a.part_end[0] : p1 ? a.part_end[1] : a.part_end[2];
+                if (row < a.rows) {
+                    float *yp = (p0 ? a.y[0] : p1 ? a.y[1] : a.y[2]) + (size_t)tok * (hi - lo) + (row - lo);
+                    *yp = a.accumulate ? *yp + v : v;
+                }
+            } else {
+                const float up = __shfl_down_sync(0xffffffffu, v, 16);
+                if (lane < 16u) {
+                    const float r = (a.mode == kSilu ? tmdev::silu_f(v) : tmdev::gelu_tanh_f(v)) * up;
+                    a.act[(size_t)tok * half_rows + unit * 16u + lane] = __float2half_rn(r);
+                }
+            }
+        }
+    }
+    if (P > 1) cluster_sync();  // nobody leaves while its sums are being read
+}
+
+size_t rows_smem(uint32_t cols, uint32_t nt, uint32_t p, uint32_t ring) {
+    const uint32_t tok = nt * 8u, kc = (cols / 64u + p - 1u) / p;
+    return (size_t)tok * (kc * 128u + 16u) + (size_t)kWarps * tok * kRowPad * 4u + (p > 1 ? 2u * tok * 32u * 4u : 0u) +
+           (size_t)kWarps * ring * kSlot;
+}
+
+struct rows_plan {
+    uint32_t p = 0, ring = 0;
+};
+
+// K parts and ring depth.  A CTA's time in cycles, fitted to measurements at 8 and 32 tokens (151936 x 1024:
+// 2.7k and 4.6k cycles per unit of two chunks a warp): its rounds of units, each the chunks one warp streams plus
+// the ordered sum, and once its share of X.  P is the part count with the least of that whose share of X leaves
+// room for a ring; the ring is as deep as a warp's stream is long, at most 6.
+rows_plan plan_rows(const tm_cuda_ctx *ctx, uint32_t units, uint32_t cols, uint32_t nt) {
+    const uint32_t chunks = cols / 64u, sms = (uint32_t)ctx->sm_count;
+    rows_plan best;
+    uint32_t cost = 0;
+    for (uint32_t p = 1; p <= 8u && p <= chunks; ++p) {
+        const uint32_t kc = (chunks + p - 1u) / p, rounds = (units * p + sms - 1u) / sms;
+        const uint32_t per_warp = (kc + kWarps - 1u) / kWarps;
+        const uint32_t c = rounds * (per_warp * (500u + 200u * nt) + 900u + 200u * nt + (p > 1u ? 300u : 0u)) + kc * 20u * nt;
+        if (best.p && c >= cost) continue;
+        uint32_t ring = 0;
+        for (uint32_t r : {6u, 4u, 3u, 2u})
+            if ((r <= rounds * per_warp || r == 2u) && rows_smem(cols, nt, p, r) <= ctx->smem_optin) {
+                ring = r;
+                break;
+            }
+        if (!ring) continue;
+        best.p = p;
+        best.ring = ring;
+        cost = c;
+    }
+    return best;
+}
+
+bool rows_ok(uint32_t rows, uint32_t cols, uint32_t batch, bool gated) {
+    return batch >= 1u && batch <= TM_CUDA_GEMM_ROWS_MAX_BATCH && rows > 0u && cols > 0u && cols % 64u == 0u &&
+           cols <= 16384u && (!gated || rows % 32u == 0u);
+}
+
+template <int NT>
+cudaError_t launch_rows(tm_cuda_ctx *ctx, const rows_args &args, const rows_plan &pl) {
+    rows_args a = args;
+    a.ring = pl.ring;
+    const size_t smem = rows_smem(a.cols, NT, pl.p, pl.ring);
+    static std::atomic<bool> attr_set[64] = {};  // per device; contexts of a process share it
+    const int dev = ctx->device;
+    if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(q8_gemm_rows_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)ctx->smem_optin);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+    }
+    // Resident clusters: by shared memory (1 KB per CTA is the system's) and registers at most two CTAs per SM.
+    const uint32_t per_sm = 2u * (smem + 1024u) <= 228u * 1024u ? 2u : 1u;
+    uint32_t clusters = (uint32_t)ctx->sm_count * per_sm / pl.p;
+    if (clusters > a.units) clusters = a.units;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * pl.p);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = pl.p;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = ctx->pdl ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, q8_gemm_rows_kernel<NT>, a);
+}
+
+}  // namespace
+
+extern "C" {
+
+// Where the multiply for a few rows beats the tcgen05 GEMM (measured, us against us, with the f16 copy of X): up to 8
+// tokens everywhere (24576 x 4096: 32 / 36, 151936 x 1024: 49 / 47); the more tokens, the sooner its MMAs and token
+// fragments cost more than the other kernel's hand-overs: at 16 tokens 12288 x 4096 is 22 / 23 but 24576 x 4096
+// 38 / 36, at 24 tokens 4096 x 4096 14 / 15, at 32 tokens 6144 x 1024 8.7 / 10.4 but 13824 x 1152 14 / 13.
+int tm_cuda_q8_0_gemm_rows_pays(uint32_t rows, uint32_t cols, uint32_t batch, int gated) {
+    if (!rows_ok(rows, cols, batch, gated != 0)) return 0;
+    const uint64_t weights = (uint64_t)rows * cols, limit[4] = {160u << 20, 32u << 20, 17u << 20, 7u << 20};
+    return weights <= limit[(batch - 1u) / 8u];
+}
+
+int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, uint32_t rows, uint32_t cols,
+                           uint32_t batch, uint32_t n_parts, tm_cuda_buffer *const *y_parts, const uint32_t *part_rows,
+                           int prologue, tm_cuda_buffer *pro, float eps, int epilogue, char *err, size_t err_cap) {
+    if (prologue != TM_CUDA_PRO_F16) {
+        const int rc = tm_mma_ensure_workspace(ctx, cols, batch, err, err_cap);
+        if (rc != TM_CUDA_OK) return rc;
+    }
+    TM_ENTER();
+    int rc = tm_check_packed(ctx, w, rows, cols, err, err_cap);
+    if (rc != TM_CUDA_OK) return rc;
+    const bool gated = epilogue == TM_CUDA_EPI_SILU_MUL_F16 || epilogue == TM_CUDA_EPI_GELU_MUL_F16;
+    if (!rows_ok(rows, cols, batch, gated))
+        return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "%u x %u for %u rows: 1..%d rows, whole 64-column chunks%s", rows,
+                       cols, batch, TM_CUDA_GEMM_ROWS_MAX_BATCH, gated ? ", gate and up of whole 16-row tiles" : "");
+    if (prologue < TM_CUDA_PRO_NONE || prologue > TM_CUDA_PRO_F16 ||
+        (!gated && epilogue != TM_CUDA_EPI_STORE && epilogue != TM_CUDA_EPI_ADD))
+        return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "unknown prologue %d / epilogue %d", prologue, epilogue);
+    if (n_parts < 1 || n_parts > 3 || !y_parts || !part_rows || (gated && n_parts != 1))
+        return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "1 to 3 output parts (1 for a gated output), got %u", n_parts);
+    rows_args a = {};
+    if (gated) {
+        if (part_rows[0] != rows / 2u) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "a gated output has %u rows", rows / 2u);
+        TM_CHECK_BUF(y_parts[0], (size_t)batch * (rows / 2u) * 2, "gated output");
+        a.act = (__half *)y_parts[0]->dev;
+        a.units = rows / 32u;
+        a.mode = epilogue == TM_CUDA_EPI_SILU_MUL_F16 ? kSilu : kGelu;
+    } else {
+        uint32_t sum = 0;
+        for (uint32_t p = 0; p < 3; ++p) a.part_end[p] = rows;
+        for (uint32_t p = 0; p < n_parts; ++p) {
+            if (part_rows[p] == 0 || (p + 1 < n_parts && part_rows[p] % 32u != 0))
+                return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED,
+                               "part %u has %u rows: every part but the last must be a multiple of 32", p, part_rows[p]);
+            TM_CHECK_BUF(y_parts[p], (size_t)batch * part_rows[p] * 4, "output part");
+            a.y[p] = (float *)y_parts[p]->dev;
+            sum += part_rows[p];
+            a.part_end[p] = sum;
+        }
+        if (sum != rows) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "parts cover %u of %u rows", sum, rows);
+        a.units = (rows + 31u) / 32u;
+        a.mode = kPlain;
+    }
+    a.q = (const signed char *)w->qp;
+    a.d = (const unsigned short *)w->dp;
+    a.rows = rows;
+    a.cols = cols;
+    a.batch = batch;
+    a.accumulate = epilogue == TM_CUDA_EPI_ADD;
+    const uint32_t nt = (batch + 7u) / 8u;
+    const rows_plan pl = plan_rows(ctx, a.units, cols, nt);
+    if (!pl.p) return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "cols %u exceeds the activation stage of a cluster", cols);
+    if (prologue == TM_CUDA_PRO_F16) {
+        TM_CHECK_BUF(x, (size_t)batch * cols * 2, "activation");
+        if (((size_t)x->dev & 15u) != 0) return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "f16 activations are not 16-byte aligned");
+        a.x = (const __half *)x->dev;
+    } else {
+        TM_CHECK_BUF(x, (size_t)batch * cols * 4, "activation");
+        if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_BUF(pro, (size_t)cols * 4, "norm weight");
+        else if (prologue != TM_CUDA_PRO_NONE) TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate operand");
+        a.x = (const __half *)ctx->mma_scratch;
+    }
+    TM_OP_BEGIN("q8_0_gemm_rows");
+    if (prologue != TM_CUDA_PRO_F16)
+        TM_CUDA_TRY(tm_x_prep_launch(ctx, prologue, (const float *)x->dev, pro ? (const float *)pro->dev : nullptr, cols,
+                                     batch, eps));
+    TM_CUDA_TRY(nt == 1   ? launch_rows<1>(ctx, a, pl)
+                : nt == 2 ? launch_rows<2>(ctx, a, pl)
+                : nt == 3 ? launch_rows<3>(ctx, a, pl)
+                          : launch_rows<4>(ctx, a, pl));
+    TM_OP_END(prologue == TM_CUDA_PRO_F16 ? 1 : 2);
+}
+
+}  // extern "C"

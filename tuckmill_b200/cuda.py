@@ -21,8 +21,8 @@ ERR_NAMES = {0: "OK", -1: "NO_DEVICE", -2: "SOURCE", -3: "ALLOC", -4: "BOUNDS", 
 ARGMAX_NONE = 0xFFFFFFFF
 GEMM_MAX_BATCH = 32
 GEMM_MMA_MAX_BATCH = 8192
-PRO_NONE, PRO_RMSNORM, PRO_SILU_MUL, PRO_GELU_MUL = 0, 1, 2, 3
-EPI_STORE, EPI_ADD = 0, 1
+PRO_NONE, PRO_RMSNORM, PRO_SILU_MUL, PRO_GELU_MUL, PRO_F16 = 0, 1, 2, 3, 4
+EPI_STORE, EPI_ADD, EPI_SILU_MUL_F16, EPI_GELU_MUL_F16 = 0, 1, 2, 3
 
 
 class CudaError(RuntimeError):
@@ -107,6 +107,7 @@ _OPS = {
     "q8_0_gemm_mma_push": [_P, _P, _P, _P, _U32, _U32, _U32],
     "symm_status": [_P, _P, C.POINTER(C.c_uint32)],
     "q8_0_gemm_mma_fused": [_P, _P, _P, _U32, _U32, _U32, _U32, C.POINTER(C.c_void_p), C.POINTER(C.c_uint32), _I, _P, _F, _I],
+    "q8_0_gemm_rows": [_P, _P, _P, _U32, _U32, _U32, _U32, C.POINTER(C.c_void_p), C.POINTER(C.c_uint32), _I, _P, _F, _I],
     "qk_prep_chunk": [_P] * 9 + [_U32] * 7 + [_F],
     "attention_chunk_mma": [_P, _P, _P, _P, _P, _U32, _U32, _U32, _U32, _U32, _F, _U32, _U32],
     "attention_decode_dev": [_P] * 12 + [_U32, _P] + [_U32] * 6 + [_F, _F, _I],
@@ -499,6 +500,13 @@ class CudaContext:
         yp = (C.c_void_p * len(ys))(*[y.handle for y in ys])
         pr = (C.c_uint32 * len(ys))(*part_rows)
         self._call("q8_0_gemm_mma_fused", w.handle, x.handle, rows, cols, batch, len(ys), yp, pr, prologue,
+                   self._h(pro), eps, epilogue)
+
+    def q8_0_gemm_rows(self, w, x, rows, cols, batch, ys, part_rows, prologue=PRO_NONE, pro=None, eps=0.0,
+                            epilogue=EPI_STORE):
+        yp = (C.c_void_p * len(ys))(*[y.handle for y in ys])
+        pr = (C.c_uint32 * len(ys))(*part_rows)
+        self._call("q8_0_gemm_rows", w.handle, x.handle, rows, cols, batch, len(ys), yp, pr, prologue,
                    self._h(pro), eps, epilogue)
 
     def qk_prep_chunk(self, q, k, v, q_norm, k_norm, inv_freq, k_cache, v_cache, heads, kv_heads, head_dim, n_rot, pos0,
