@@ -199,6 +199,14 @@ cudaError_t tm_attention_decode_mma_launch(tm_cuda_ctx *ctx, const float *q, con
                                            float eps, float scale, uint32_t n_seq, size_t sq, size_t skv, size_t so,
                                            size_t scache, size_t sscratch, uint32_t count_off);
 
+// Decode attention, latency form (tm_cuda_attn_decode.cu).
+bool tm_attention_decode_fast_ok(uint32_t heads, uint32_t kv_heads, uint32_t hd, uint32_t n_rot);
+cudaError_t tm_attention_decode_fast_launch(tm_cuda_ctx *ctx, const float *q, const float *k, const float *v,
+                                            const float *qn, const float *kn, const float *inv_freq, void *kc, void *vc,
+                                            float *out, const uint32_t *pos, uint32_t *status, uint32_t heads,
+                                            uint32_t kv_heads, uint32_t hd, uint32_t cap, uint32_t window, float eps,
+                                            float scale, uint32_t n_seq, size_t sq, size_t skv, size_t so, size_t scache);
+
 // Tensor-core GEMM workspace and the f16 copy of X in it (tm_cuda_mma.cu).
 extern "C" int tm_mma_ensure_workspace(tm_cuda_ctx *ctx, uint32_t cols, uint32_t batch, char *err, size_t err_cap);
 cudaError_t tm_x_prep_launch(tm_cuda_ctx *ctx, int prologue, const float *x, const float *pro, uint32_t cols, uint32_t batch,

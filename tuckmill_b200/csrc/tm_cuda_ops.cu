@@ -672,411 +672,6 @@ __global__ void __launch_bounds__(32) attention_decode_kernel(
     if (lane == 0) *count = 0u;  // ready for the next launch on this stream
 }
 
-// ---- decode attention, latency-optimised form ---------------------------------
-// Same mathematics as attention_decode_kernel, tolerance-qualified instead of
-// bit-identical to the prefill kernel (the engine uses it unless `exact` is
-// asked): one CTA of 128 threads per (KV head, 64-key split) serves all G query
-// heads of the group, so K and V are read once; the per-thread instruction
-// chain is short (two threads share a key's dot product, the value sum is
-// spread over dim pairs x key halves) and the last CTA to arrive for a KV head
-// merges the splits with a two-pass softmax, one thread per value dim.
-//   scratch: float part[kv_heads][nsplit][G][HD + 2], then u32 count[kv_heads]
-constexpr int kFastSplit = 64;
-constexpr int kFastThreads = 128;
-
-template <int G, int HD>
-__global__ void __launch_bounds__(kFastThreads) attention_decode_fast_kernel(
-    const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm,
-    const float *inv_freq, __half *kc, __half *vc, float *out, float *scratch, const uint32_t *pos_p,
-    uint32_t *status, uint32_t kv_heads, uint32_t n_rot, uint32_t cap, uint32_t window, float eps, float scale,
-    const decode_seq_strides seqs) {
-    TM_DECODE_SEQ_OFFSETS(seqs)
-    constexpr int EPL = HD / 32;          // elements of a head vector per lane (strided by 32)
-    constexpr int PAIRS = HD / 2;         // value dim pairs
-    constexpr int KP = kFastThreads / PAIRS > 0 ? kFastThreads / PAIRS : 1;  // key parts in the value sum
-    constexpr int PPT = PAIRS / kFastThreads > 0 ? PAIRS / kFastThreads : 1; // dim pairs per thread
-    __shared__ __align__(16) float qs[G][HD];
-    __shared__ __align__(16) __half kh[HD];
-    __shared__ __align__(16) __half vh[HD];
-    __shared__ float sc[G][kFastSplit];
-    __shared__ float stat[G][2];
-    __shared__ float opart[KP][G][HD];
-    __shared__ uint32_t s_last;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t kvh = blockIdx.x, split = blockIdx.y;
-    const uint32_t nsplit = (cap + kFastSplit - 1) / kFastSplit;
-    const __half *kp = kc + (size_t)kvh * cap * HD, *vp = vc + (size_t)kvh * cap * HD;
-    {   // value rows of this split: towards L2 (coherent; see the note on row pos - 1 below)
-        const uint32_t j = min(split * kFastSplit + (tid >> 1), cap - 1u);
-        const uint32_t half_bytes = HD;  // half a row of f16
-        for (uint32_t off = 0; off < half_bytes; off += 128u)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)(vp + (size_t)j * HD) + (tid & 1) * half_bytes + off));
-    }
-    // This thread's half of key row split*64 + tid/2: written by an earlier step's kernel (or is a row past
-    // the sequence, masked below; or the current position's row, replaced below by the fresh one), so it
-    // is read before the predecessor finishes.  One row is the exception: the attention call of the
-    // PREVIOUS token (two kernels back in a chain of programmatic launches) may still be storing row
-    // pos - 1; that row is read again after the wait.  Calls further back have finished, because an
-    // attention kernel lets its successor start only after its own predecessor is complete.
-    constexpr int NL0 = HD / 16;  // 16-byte loads per thread
-    int4 kraw[NL0];
-    {
-        const uint32_t j = min(split * kFastSplit + ((uint32_t)tid >> 1), cap - 1u);
-        const __half *kr = kp + (size_t)j * HD + (tid & 1) * (HD / 2);
-#pragma unroll
-        for (int c = 0; c < NL0; ++c) kraw[c] = *(const int4 *)(kr + c * 8);
-    }
-    // The same for this thread's value elements (one dim pair of up to 32 cached rows), when they fit.
-    constexpr int KEYS0 = kFastSplit / KP;
-    constexpr bool kHoistV = PPT == 1 && KEYS0 <= 32;
-    __half2 vpre[kHoistV ? KEYS0 : 1];
-    if constexpr (kHoistV) {
-        const uint32_t kpart0 = tid / PAIRS < KP ? tid / PAIRS : 0, dp00 = tid % PAIRS;
-#pragma unroll
-        for (int c = 0; c < KEYS0; ++c) {
-            const uint32_t j = min(split * kFastSplit + kpart0 * KEYS0 + (uint32_t)c, cap - 1u);
-            vpre[c] = *(const __half2 *)(vp + (size_t)j * HD + 2 * dp00);
-        }
-    }
-    tmdev::pdl_wait();
-    // The successor may start only now, when this kernel's own predecessor has finished: a kernel that
-    // let its successor start at once would let a whole chain of launches run ahead, and a later
-    // attention call could read cache rows early that a call several places back is still storing.
-    // This way only the call directly before can still be running: the row it stores is read again below.
-    tmdev::pdl_trigger();
-    // The first vector this warp will normalise (q_warp, or k for warp G) does not depend on the
-    // position: its loads are issued together with the position's, one memory trip instead of two.
-    constexpr int EPL0 = HD / 32;
-    float x0[EPL0], w0[EPL0], v0[EPL0], f0[EPL0 / 2];
-    {
-        const bool pre_k = warp == G;
-        const float *src = pre_k ? k + (size_t)blockIdx.x * HD : q + ((size_t)blockIdx.x * G + (warp < G ? warp : 0)) * HD;
-        const float *nw = pre_k ? k_norm : q_norm;
-#pragma unroll
-        for (int r = 0; r < EPL0; ++r) {
-            x0[r] = src[lane + 32 * r];
-            w0[r] = nw[lane + 32 * r];
-            v0[r] = pre_k ? v[(size_t)blockIdx.x * HD + lane + 32 * r] : 0.0f;
-        }
-#pragma unroll
-        for (int r = 0; r < EPL0 / 2; ++r) f0[r] = inv_freq[lane + 32 * r];
-    }
-    const uint32_t pos = *pos_p;
-    if (pos >= cap) {
-        if (tid == 0 && split == 0 && kvh == 0) atomicOr(status, 1u);
-        return;
-    }
-    const uint32_t seq = pos + 1u, start = attn_start(seq, window);
-    const uint32_t first = start / kFastSplit, last = pos / kFastSplit;
-    if (split < first || split > last) return;
-    const bool owns_new = split == last;
-    (void)n_rot;
-    if (pos > 0u) {  // the previous token's row, now certainly complete (read past L1)
-        const uint32_t prev = pos - 1u;
-        if (split * kFastSplit + ((uint32_t)tid >> 1) == prev) {
-            const int4 *kr = (const int4 *)(kp + (size_t)prev * HD + (tid & 1) * (HD / 2));
-#pragma unroll
-            for (int c = 0; c < NL0; ++c) kraw[c] = __ldcg(kr + c);
-        }
-        if constexpr (kHoistV) {
-            const uint32_t kpart0 = tid / PAIRS < KP ? tid / PAIRS : 0, dp00 = tid % PAIRS;
-#pragma unroll
-            for (int c = 0; c < KEYS0; ++c)
-                if (split * kFastSplit + kpart0 * KEYS0 + (uint32_t)c == prev) {
-                    const uint32_t raw = __ldcg((const unsigned int *)(vp + (size_t)prev * HD + 2 * dp00));
-                    vpre[c] = *(const __half2 *)&raw;
-                }
-        }
-    }
-
-    // ---- vectors q_0..q_{G-1} (and k for the owning split): RMS norm + RoPE, one warp each ----
-    for (int vec = warp; vec < G + (owns_new ? 1 : 0); vec += kFastThreads / 32) {
-        const bool is_k = vec == G;
-        const float *src = is_k ? k + (size_t)kvh * HD : q + ((size_t)kvh * G + vec) * HD;
-        const float *nw = is_k ? k_norm : q_norm;
-        float x[EPL], w[EPL];
-        const bool preloaded = vec == warp;  // the loop's first trip: the values are already here
-#pragma unroll
-        for (int r = 0; r < EPL; ++r) {
-            x[r] = preloaded ? x0[r] : src[lane + 32 * r];
-            w[r] = preloaded ? w0[r] : nw[lane + 32 * r];
-        }
-        float ss = 0.0f;
-#pragma unroll
-        for (int r = 0; r < EPL; ++r) ss = fmaf(x[r], x[r], ss);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-        const float inv = 1.0f / sqrtf(ss / (float)HD + eps);
-#pragma unroll
-        for (int r = 0; r < EPL; ++r) x[r] = x[r] * inv * w[r];
-        // full rotation (n_rot == HD, checked by the host): pair (i, i + HD/2), i = lane + 32 r,
-        // has both members in this lane
-#pragma unroll
-        for (int r = 0; r < EPL / 2; ++r) {
-            float sn, cs;
-            sincosf((float)pos * f0[r], &sn, &cs);
-            const float a0 = x[r], b0 = x[r + EPL / 2];
-            x[r] = a0 * cs - b0 * sn;
-            x[r + EPL / 2] = a0 * sn + b0 * cs;
-        }
-        if (is_k) {
-            const float *vsrc = v + (size_t)kvh * HD;
-#pragma unroll
-            for (int r = 0; r < EPL; ++r) {
-                const uint32_t e = lane + 32 * r;
-                const __half hk = __float2half_rn(x[r]), hv = __float2half_rn(preloaded ? v0[r] : vsrc[e]);
-                kh[e] = hk;
-                vh[e] = hv;
-                kc[((size_t)kvh * cap + pos) * HD + e] = hk;
-                vc[((size_t)kvh * cap + pos) * HD + e] = hv;
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < EPL; ++r) qs[vec][lane + 32 * r] = x[r];
-        }
-    }
-    __syncthreads();
-    // ---- scores: two threads per key, half the dims each ----
-    {
-        const uint32_t jj = tid >> 1, hsel = tid & 1, j = split * kFastSplit + jj;
-        const bool valid = j >= start && j < seq;
-        float dot[G][2];
-#pragma unroll
-        for (int g = 0; g < G; ++g) dot[g][0] = dot[g][1] = 0.0f;
-        if (valid) {
-            constexpr int NL = HD / 16;  // 16-byte loads per thread
-            int4 raw[NL];
-            const bool fresh = owns_new && j == pos;  // this step's own key: from shared memory
-#pragma unroll
-            for (int c = 0; c < NL; ++c) raw[c] = fresh ? *(const int4 *)(kh + hsel * (HD / 2) + c * 8) : kraw[c];
-#pragma unroll
-            for (int c = 0; c < NL; ++c) {
-                const __half2 *h2 = (const __half2 *)&raw[c];
-                float kf[8];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 f = __half22float2(h2[e]);
-                    kf[2 * e] = f.x;
-                    kf[2 * e + 1] = f.y;
-                }
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const float *qp = &qs[g][hsel * (HD / 2) + c * 8];
-                    const float4 q0 = *(const float4 *)qp, q1 = *(const float4 *)(qp + 4);
-                    float t = dot[g][c & 1];
-                    t = fmaf(q0.x, kf[0], t); t = fmaf(q0.y, kf[1], t); t = fmaf(q0.z, kf[2], t); t = fmaf(q0.w, kf[3], t);
-                    t = fmaf(q1.x, kf[4], t); t = fmaf(q1.y, kf[5], t); t = fmaf(q1.z, kf[6], t); t = fmaf(q1.w, kf[7], t);
-                    dot[g][c & 1] = t;
-                }
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            float d = dot[g][0] + dot[g][1];
-            d += __shfl_xor_sync(0xffffffffu, d, 1);
-            if (hsel == 0) sc[g][jj] = valid ? d * scale : -INFINITY;
-        }
-    }
-    __syncthreads();
-    // ---- split softmax: warp g owns head g ----
-    for (int g = warp; g < G; g += kFastThreads / 32) {
-        const float s0 = sc[g][lane], s1 = sc[g][lane + 32];
-        float mx = fmaxf(s0, s1);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        const float p0 = s0 == -INFINITY ? 0.0f : expf(s0 - mx), p1 = s1 == -INFINITY ? 0.0f : expf(s1 - mx);
-        float sum = p0 + p1;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        sc[g][lane] = p0;
-        sc[g][lane + 32] = p1;
-        if (lane == 0) {
-            stat[g][0] = mx;
-            stat[g][1] = sum;
-        }
-    }
-    __syncthreads();
-    // ---- values: thread = (dim pair(s), key part); keys of a part in order ----
-    {
-        const uint32_t kpart = tid / PAIRS < KP ? tid / PAIRS : 0, dp0 = tid % PAIRS;
-        constexpr int KEYS = kFastSplit / KP;
-        const uint32_t jbase = split * kFastSplit + kpart * KEYS;
-        float acc[PPT][G][2];
-#pragma unroll
-        for (int pp = 0; pp < PPT; ++pp)
-#pragma unroll
-            for (int g = 0; g < G; ++g) acc[pp][g][0] = acc[pp][g][1] = 0.0f;
-        if constexpr (kHoistV) {
-#pragma unroll
-            for (int c = 0; c < KEYS; ++c) {
-                const uint32_t j = jbase + (uint32_t)c;
-                __half2 hv = vpre[c];
-                if (owns_new && j == pos) hv = *(const __half2 *)(vh + 2 * dp0);  // this step's own row
-                if (j >= seq) hv = __float2half2_rn(0.0f);  // weight 0 there; never multiply stale bytes
-                const float2 f = __half22float2(hv);
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const float pj = sc[g][kpart * KEYS + c];
-                    acc[0][g][0] = fmaf(pj, f.x, acc[0][g][0]);
-                    acc[0][g][1] = fmaf(pj, f.y, acc[0][g][1]);
-                }
-            }
-        }
-        if constexpr (!kHoistV) {
-#pragma unroll 1
-        for (int kb = 0; kb < KEYS; kb += 8) {
-            __half2 vv[8][PPT];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint32_t j = jbase + kb + c;
-                const uint32_t jc = j < seq ? j : pos;  // rows past the sequence carry weight 0
-                const __half *vr = owns_new && jc == pos ? vh : vp + (size_t)jc * HD;
-#pragma unroll
-                for (int pp = 0; pp < PPT; ++pp) vv[c][pp] = *(const __half2 *)(vr + 2 * (dp0 + pp * kFastThreads));
-            }
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const float pj = sc[g][kpart * KEYS + kb + c];
-#pragma unroll
-                    for (int pp = 0; pp < PPT; ++pp) {
-                        const float2 f = __half22float2(vv[c][pp]);
-                        acc[pp][g][0] = fmaf(pj, f.x, acc[pp][g][0]);
-                        acc[pp][g][1] = fmaf(pj, f.y, acc[pp][g][1]);
-                    }
-                }
-            }
-        }
-        }  // !kHoistV
-#pragma unroll
-        for (int pp = 0; pp < PPT; ++pp)
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const uint32_t d = 2 * (dp0 + pp * kFastThreads);
-                opart[kpart][g][d] = acc[pp][g][0];
-                opart[kpart][g][d + 1] = acc[pp][g][1];
-            }
-    }
-    __syncthreads();
-    // ---- this split's (m, l, o); finish here when it is the only one ----
-    const bool single = first == last;
-    constexpr uint32_t stride = HD + 2;
-    float *part = scratch + ((size_t)kvh * nsplit + split) * G * stride;
-    for (uint32_t i = tid; i < G * HD; i += kFastThreads) {
-        const uint32_t g = i / HD, d = i % HD;
-        float o = 0.0f;
-#pragma unroll
-        for (int kq = 0; kq < KP; ++kq) o += opart[kq][g][d];
-        if (single) out[((size_t)kvh * G + g) * HD + d] = o / stat[g][1];
-        else part[g * stride + 2 + d] = o;
-    }
-    if (single) return;
-    if (tid < G) {
-        part[tid * stride] = stat[tid][0];
-        part[tid * stride + 1] = stat[tid][1];
-    }
-    __threadfence();
-    __syncthreads();
-    uint32_t *count = (uint32_t *)(scratch + (size_t)kv_heads * nsplit * G * stride) + kvh;
-    if (tid == 0) s_last = atomicAdd(count, 1u) == last - first ? 1u : 0u;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // ---- merge: warp w takes splits w, w + 4, ... with its own running (max, sum, output) per head, a
-    // lane two value dims per 64; the loads of several splits and all heads are issued together, so the
-    // loop costs one memory trip per 8 (16) splits of the CTA -- the merge is the serial tail of a
-    // decode step at long contexts -- and the four warps' states meet in shared memory. ----
-    {
-        constexpr int DJ = HD / 64;            // float2 pieces of a head vector per lane
-        constexpr int B = G > 2 ? 2 : 4;       // own splits fetched together
-        __shared__ __align__(8) float mrg[kFastThreads / 32][G][HD + 2];
-        const uint32_t nact = last - first + 1;
-        const float *base0 = scratch + ((size_t)kvh * nsplit + first) * G * stride;
-        float Mg[G], Lg[G], Og[G][2 * DJ];
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            Mg[g] = -INFINITY;
-            Lg[g] = 0.0f;
-#pragma unroll
-            for (int e = 0; e < 2 * DJ; ++e) Og[g][e] = 0.0f;
-        }
-        for (uint32_t s0 = (uint32_t)warp; s0 < nact; s0 += 4u * B) {
-            float2 ml[B][G], ov[B][G][DJ];
-#pragma unroll
-            for (int c = 0; c < B; ++c) {
-                const uint32_t s = s0 + 4u * c;
-                const float *pb = base0 + (size_t)(s < nact ? s : nact - 1) * G * stride;
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    ml[c][g] = __ldcg((const float2 *)(pb + g * stride));
-#pragma unroll
-                    for (int jj = 0; jj < DJ; ++jj)
-                        ov[c][g][jj] = __ldcg((const float2 *)(pb + g * stride + 2 + 2 * lane + 64 * jj));
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < B; ++c) {
-                if (s0 + 4u * c >= nact) break;
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const float mx = fmaxf(Mg[g], ml[c][g].x);
-                    const float a = expf(Mg[g] - mx), wgt = expf(ml[c][g].x - mx);
-                    Lg[g] = fmaf(wgt, ml[c][g].y, Lg[g] * a);
-#pragma unroll
-                    for (int jj = 0; jj < DJ; ++jj) {
-                        Og[g][2 * jj] = fmaf(wgt, ov[c][g][jj].x, Og[g][2 * jj] * a);
-                        Og[g][2 * jj + 1] = fmaf(wgt, ov[c][g][jj].y, Og[g][2 * jj + 1] * a);
-                    }
-                    Mg[g] = mx;
-                }
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            if (lane == 0) {
-                mrg[warp][g][0] = Mg[g];
-                mrg[warp][g][1] = Lg[g];
-            }
-#pragma unroll
-            for (int jj = 0; jj < DJ; ++jj)
-                *(float2 *)&mrg[warp][g][2 + 2 * lane + 64 * jj] = make_float2(Og[g][2 * jj], Og[g][2 * jj + 1]);
-        }
-        __syncthreads();
-        for (uint32_t i = tid; i < G * HD; i += kFastThreads) {
-            const uint32_t g = i / HD, d = i % HD;
-            float M = -INFINITY;
-#pragma unroll
-            for (int w = 0; w < kFastThreads / 32; ++w) M = fmaxf(M, mrg[w][g][0]);
-            float L = 0.0f, O = 0.0f;
-#pragma unroll
-            for (int w = 0; w < kFastThreads / 32; ++w) {
-                const float f = expf(mrg[w][g][0] - M);  // a warp that took no split: exp(-inf) = 0
-                L = fmaf(f, mrg[w][g][1], L);
-                O = fmaf(f, mrg[w][g][2 + d], O);
-            }
-            out[((size_t)kvh * G + g) * HD + d] = O / L;
-        }
-    }
-    if (tid == 0) *count = 0u;  // ready for the next launch on this stream
-}
-
-template <int G, int HD>
-void launch_decode_fast(tm_cuda_ctx *ctx, const float *q, const float *k, const float *v, const float *qn,
-                        const float *kn, const float *inv_freq, __half *kc, __half *vc, float *out, float *scratch,
-                        const uint32_t *pos, uint32_t *status, uint32_t kvh, uint32_t n_rot, uint32_t cap,
-                        uint32_t window, float eps, float scale, uint32_t n_seq = 1,
-                        const decode_seq_strides seqs = decode_seq_strides()) {
-    tm_launch_pdl(ctx, attention_decode_fast_kernel<G, HD>, dim3(kvh, (cap + kFastSplit - 1) / kFastSplit, n_seq),
-                  dim3(kFastThreads), 0, q, k, v, qn, kn, inv_freq, kc, vc, out, scratch, pos, status, kvh, n_rot, cap,
-                  window, eps, scale, seqs);
-}
-
-inline bool attn_fast_ok(uint32_t heads, uint32_t kv_heads, uint32_t hd, uint32_t n_rot) {
-    const uint32_t g = heads / kv_heads;
-    return (hd == 128 || hd == 256) && n_rot == hd && (g == 1 || g == 2 || g == 4);
-}
-
 // Launch helpers: G heads per warp (the group size, in chunks of at most 4) and
 // DPL = head_dim / 32 value dims per lane are compile-time.
 template <int G, int DPL>
@@ -1528,19 +1123,9 @@ int tm_cuda_attention_decode_dev(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_bu
         return tm_step_record_attention(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, sp, pp, stp, heads, kv_heads, head_dim,
                                         n_rot, cap, window, eps, scale, exact, err, err_cap);
     TM_OP_BEGIN("attention_decode");
-    if (!exact && attn_fast_ok(heads, kv_heads, head_dim, n_rot)) {
-#define TM_FAST(G, HD)                                                                                       \
-    launch_decode_fast<G, HD>(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, sp, pp, stp, kv_heads, n_rot, cap, window, \
-                              eps, scale)
-        switch ((heads / kv_heads) * 1000 + head_dim) {
-            case 1128: TM_FAST(1, 128); break;
-            case 2128: TM_FAST(2, 128); break;
-            case 4128: TM_FAST(4, 128); break;
-            case 1256: TM_FAST(1, 256); break;
-            case 2256: TM_FAST(2, 256); break;
-            default: TM_FAST(4, 256); break;
-        }
-#undef TM_FAST
+    if (!exact && tm_attention_decode_fast_ok(heads, kv_heads, head_dim, n_rot)) {
+        TM_CUDA_TRY(tm_attention_decode_fast_launch(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, pp, stp, heads, kv_heads,
+                                                    head_dim, cap, window, eps, scale, 1, 0, 0, 0, 0));
         TM_OP_END(1);
     }
 #define TM_DECODE(DPL)                                                                                        \
@@ -1612,26 +1197,17 @@ int tm_cuda_attention_decode_batch_dev(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_c
     // sequences is bound by the K/V bytes it reads).  TM_CUDA_DECODE_MMA=0 keeps the latency form.
     static const bool mma_off = [] { const char *e = getenv("TM_CUDA_DECODE_MMA"); return e && e[0] == '0'; }();
     if (!exact && n_seq > 1 && !mma_off && tm_attention_decode_mma_ok(heads, kv_heads, head_dim, n_rot)) {
-        const size_t nsplit64 = (cap + kFastSplit - 1) / kFastSplit;
+        const size_t nsplit64 = (cap + 63) / 64;
         const uint32_t count_off = (uint32_t)((size_t)kv_heads * nsplit64 * (heads / kv_heads) * (head_dim + 2));
         TM_CUDA_TRY(tm_attention_decode_mma_launch(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, sp, pp, stp, heads, kv_heads,
                                                    head_dim, cap, window, eps, scale, n_seq, st.q, st.k, st.out, st.cache,
                                                    st.scratch, count_off));
         TM_OP_END(1);
     }
-    if (!exact && attn_fast_ok(heads, kv_heads, head_dim, n_rot)) {
-#define TM_FAST(G, HD)                                                                                       \
-    launch_decode_fast<G, HD>(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, sp, pp, stp, kv_heads, n_rot, cap, window, \
-                              eps, scale, n_seq, st)
-        switch ((heads / kv_heads) * 1000 + head_dim) {
-            case 1128: TM_FAST(1, 128); break;
-            case 2128: TM_FAST(2, 128); break;
-            case 4128: TM_FAST(4, 128); break;
-            case 1256: TM_FAST(1, 256); break;
-            case 2256: TM_FAST(2, 256); break;
-            default: TM_FAST(4, 256); break;
-        }
-#undef TM_FAST
+    if (!exact && tm_attention_decode_fast_ok(heads, kv_heads, head_dim, n_rot)) {
+        TM_CUDA_TRY(tm_attention_decode_fast_launch(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, pp, stp, heads, kv_heads,
+                                                    head_dim, cap, window, eps, scale, n_seq, st.q, st.k, st.out,
+                                                    st.cache));
         TM_OP_END(1);
     }
 #define TM_DECODE(DPL)                                                                                        \
@@ -1710,9 +1286,8 @@ int tm_cuda_attention_decode_dev_static(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_
         g_static_decode_scratch_ptr[ctx->device].store(p, std::memory_order_release);
     }
     float *sp = (float *)g_static_decode_scratch_ptr[ctx->device].load(std::memory_order_acquire);
-    // The array keeps whatever the previous call left: the arrival counters (the
-    // tail of the region this geometry uses) must start at zero.  Both kernels
-    // keep their counters inside the last `heads` words of `need`.
+    // The array keeps whatever the previous call left: the arrival counters of the exact
+    // form (the last `heads` words of `need`) must start at zero.
     TM_CUDA_TRY(cudaMemsetAsync((unsigned char *)sp + need - (size_t)heads * 4, 0, (size_t)heads * 4, ctx->stream));
     const float *qp = (const float *)q->dev, *kp = (const float *)k->dev, *vp = (const float *)v->dev;
     const float *qn = (const float *)q_norm->dev, *kn = (const float *)k_norm->dev, *fq = (const float *)inv_freq->dev;
@@ -1720,23 +1295,9 @@ int tm_cuda_attention_decode_dev_static(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_
     float *op = (float *)out->dev;
     const uint32_t *pp = (const uint32_t *)pos_buf->dev + pos_index;
     uint32_t *stp = (uint32_t *)status->dev;
-    if (!exact && attn_fast_ok(heads, kv_heads, head_dim, n_rot)) {
-        // the fast kernel keeps kv_heads counters right after its partials; clear those too
-        const size_t nsplit = (cap + kFastSplit - 1) / kFastSplit;
-        const size_t off = (size_t)heads * nsplit * (head_dim + 2) * 4;
-        TM_CUDA_TRY(cudaMemsetAsync((unsigned char *)sp + off, 0, (size_t)kv_heads * 4, ctx->stream));
-#define TM_FAST(G, HD)                                                                                       \
-    launch_decode_fast<G, HD>(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, sp, pp, stp, kv_heads, n_rot, cap, window, \
-                              eps, scale)
-        switch ((heads / kv_heads) * 1000 + head_dim) {
-            case 1128: TM_FAST(1, 128); break;
-            case 2128: TM_FAST(2, 128); break;
-            case 4128: TM_FAST(4, 128); break;
-            case 1256: TM_FAST(1, 256); break;
-            case 2256: TM_FAST(2, 256); break;
-            default: TM_FAST(4, 256); break;
-        }
-#undef TM_FAST
+    if (!exact && tm_attention_decode_fast_ok(heads, kv_heads, head_dim, n_rot)) {
+        TM_CUDA_TRY(tm_attention_decode_fast_launch(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, pp, stp, heads, kv_heads,
+                                                    head_dim, cap, window, eps, scale, 1, 0, 0, 0, 0));
     } else {
 #define TM_DECODE(DPL)                                                                                        \
     launch_decode<DPL>(ctx, qp, kp, vp, qn, kn, fq, kcp, vcp, op, sp, pp, stp, heads, kv_heads, head_dim, n_rot, \
