@@ -174,6 +174,10 @@ mod ffi {
         pub fn tm_cuda_attention_decode_dev(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k: *mut TmCudaBuffer, v: *mut TmCudaBuffer, q_norm: *mut TmCudaBuffer, k_norm: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, out: *mut TmCudaBuffer, scratch: *mut TmCudaBuffer, pos_buf: *mut TmCudaBuffer, pos_index: u32, status: *mut TmCudaBuffer, heads: u32, kv_heads: u32, head_dim: u32, n_rot: u32, cap: u32, window: u32, eps: f32, scale: f32, exact: c_int, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_attention_decode_static_max_scratch() -> usize;
         pub fn tm_cuda_attention_decode_dev_static(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k: *mut TmCudaBuffer, v: *mut TmCudaBuffer, q_norm: *mut TmCudaBuffer, k_norm: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, out: *mut TmCudaBuffer, pos_buf: *mut TmCudaBuffer, pos_index: u32, status: *mut TmCudaBuffer, heads: u32, kv_heads: u32, head_dim: u32, n_rot: u32, cap: u32, window: u32, eps: f32, scale: f32, exact: c_int, err: *mut c_char, err_cap: usize) -> c_int;
+        pub fn tm_cuda_decode_attn_block_supported(hidden: u32, heads: u32, kv_heads: u32, head_dim: u32, n_rot: u32) -> c_int;
+        pub fn tm_cuda_decode_ffn_block_supported(hidden: u32, width: u32) -> c_int;
+        pub fn tm_cuda_decode_attn_block(ctx: *mut TmCudaCtx, x: *mut TmCudaBuffer, slots_in: *mut TmCudaBuffer, n_slots: u32, add_w: *mut TmCudaBuffer, norm_w: *mut TmCudaBuffer, x_out: *mut TmCudaBuffer, qkv: *mut TmCudaBuffer, o: *mut TmCudaBuffer, q_norm: *mut TmCudaBuffer, k_norm: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, pos_buf: *mut TmCudaBuffer, pos_index: u32, status: *mut TmCudaBuffer, slots_out: *mut TmCudaBuffer, hidden: u32, heads: u32, kv_heads: u32, head_dim: u32, cap: u32, window: u32, eps: f32, scale: f32, err: *mut c_char, err_cap: usize) -> c_int;
+        pub fn tm_cuda_decode_ffn_block(ctx: *mut TmCudaCtx, x: *mut TmCudaBuffer, slots_in: *mut TmCudaBuffer, n_slots: u32, add_w: *mut TmCudaBuffer, norm_w: *mut TmCudaBuffer, x_out: *mut TmCudaBuffer, gate_up: *mut TmCudaBuffer, down: *mut TmCudaBuffer, slots_out: *mut TmCudaBuffer, hidden: u32, width: u32, gelu: c_int, eps: f32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_attention_decode_batch_dev(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k: *mut TmCudaBuffer, v: *mut TmCudaBuffer, q_norm: *mut TmCudaBuffer, k_norm: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, out: *mut TmCudaBuffer, scratch: *mut TmCudaBuffer, pos_buf: *mut TmCudaBuffer, status: *mut TmCudaBuffer, n_seq: u32, q_stride: u32, kv_stride: u32, heads: u32, kv_heads: u32, head_dim: u32, n_rot: u32, cap: u32, window: u32, eps: f32, scale: f32, exact: c_int, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_rows_indirect_seq_f32_dev(ctx: *mut TmCudaCtx, w: *mut TmCudaBuffer, rows: u32, cols: u32, ids: *mut TmCudaBuffer, ids_stride: u32, pos_buf: *mut TmCudaBuffer, n_seq: u32, bias: i32, scale: f32, out: *mut TmCudaBuffer, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_argmax_rows_f32_dev(ctx: *mut TmCudaCtx, x: *mut TmCudaBuffer, n_rows: u32, n: u32, partial: *mut TmCudaBuffer, out: *mut TmCudaBuffer, out_stride: u32, base: u32, pos_buf: *mut TmCudaBuffer, out_cap: u32, mirror: *mut TmCudaBuffer, err: *mut c_char, err_cap: usize) -> c_int;

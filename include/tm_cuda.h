@@ -532,6 +532,30 @@ int tm_cuda_attention_decode_dev_static(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_
                                         uint32_t heads, uint32_t kv_heads, uint32_t head_dim, uint32_t n_rot,
                                         uint32_t cap, uint32_t window, float eps, float scale, int exact,
                                         char *err, size_t err_cap);
+
+/* No counterpart: a decode token's layer as two launches (tolerance-qualified like the GEMV; one sequence, one
+ * device).  x is the residual stream [hidden].  First, x_out = x + sum of slots_in[0..n_slots) in order -- or, with
+ * add_w, + rmsnorm(that sum) * add_w (a layer's output norm); x_out is a buffer other than x.  Then
+ *   attention block:    slots_out[h] = the columns of KV head h's query heads of  o * attention(rmsnorm(x_out) * norm_w),
+ *                       with q / k norm, RoPE, the f16 KV store and attention at pos_buf[pos_index] folded in
+ *                       (tm_cuda_attention_decode_dev); kv_heads slots;
+ *   feed-forward block: slots_out[c] = the c-th eighth of  down * (act(gate x') * up x'), x' = rmsnorm(x_out) * norm_w;
+ *                       gate_up holds width gate rows above width up rows; TM_CUDA_DECODE_SLOTS slots.
+ * The slots are for the next block's slots_in (or tm_cuda_reduce_ranks_add_f32). */
+#define TM_CUDA_DECODE_SLOTS 8
+int tm_cuda_decode_attn_block_supported(uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t head_dim, uint32_t n_rot);
+int tm_cuda_decode_ffn_block_supported(uint32_t hidden, uint32_t width);
+int tm_cuda_decode_attn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffer *slots_in, uint32_t n_slots,
+                              tm_cuda_buffer *add_w, tm_cuda_buffer *norm_w, tm_cuda_buffer *x_out, tm_cuda_buffer *qkv,
+                              tm_cuda_buffer *o, tm_cuda_buffer *q_norm, tm_cuda_buffer *k_norm, tm_cuda_buffer *inv_freq,
+                              tm_cuda_buffer *k_cache, tm_cuda_buffer *v_cache, tm_cuda_buffer *pos_buf, uint32_t pos_index,
+                              tm_cuda_buffer *status, tm_cuda_buffer *slots_out, uint32_t hidden, uint32_t heads,
+                              uint32_t kv_heads, uint32_t head_dim, uint32_t cap, uint32_t window, float eps, float scale,
+                              char *err, size_t err_cap);
+int tm_cuda_decode_ffn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffer *slots_in, uint32_t n_slots,
+                             tm_cuda_buffer *add_w, tm_cuda_buffer *norm_w, tm_cuda_buffer *x_out, tm_cuda_buffer *gate_up,
+                             tm_cuda_buffer *down, tm_cuda_buffer *slots_out, uint32_t hidden, uint32_t width, int gelu,
+                             float eps, char *err, size_t err_cap);
 /* No counterpart: decode steps of SEVERAL sequences in one recorded graph (the reference serves one
  * request at a time, crates/supervisor/src/queue.rs:1-4).  A step of n_seq sequences is a batch of
  * n_seq rows through the batched projections (tm_cuda_q8_0_gemm / _gemm_mma), with these operators

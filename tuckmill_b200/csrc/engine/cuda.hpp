@@ -405,6 +405,25 @@ public:
     }
 
     // x += sum of the ranks' partial products (then an optional output norm), include/tm_cuda.h.
+    // A decode token's layer in two launches; `slots_in` / `add_w` may be null (include/tm_cuda.h).
+    void decode_attn_block(const CudaBuffer &x, const CudaBuffer *slots_in, uint32_t n_slots, const CudaBuffer *add_w,
+                           const CudaBuffer &norm_w, const CudaBuffer &x_out, const CudaBuffer &qkv, const CudaBuffer &o,
+                           const CudaBuffer &q_norm, const CudaBuffer &k_norm, const CudaBuffer &inv_freq,
+                           const CudaBuffer &k_cache, const CudaBuffer &v_cache, const CudaBuffer &pos, const CudaBuffer &status,
+                           const CudaBuffer &slots_out, uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t head_dim,
+                           uint32_t cap, uint32_t window, float eps, float scale) const {
+        TM_CALL(tm_cuda_decode_attn_block, x.raw(), slots_in ? slots_in->raw() : nullptr, n_slots,
+                add_w ? add_w->raw() : nullptr, norm_w.raw(), x_out.raw(), qkv.raw(), o.raw(), q_norm.raw(), k_norm.raw(),
+                inv_freq.raw(), k_cache.raw(), v_cache.raw(), pos.raw(), 0, status.raw(), slots_out.raw(), hidden, heads,
+                kv_heads, head_dim, cap, window, eps, scale);
+    }
+    void decode_ffn_block(const CudaBuffer &x, const CudaBuffer *slots_in, uint32_t n_slots, const CudaBuffer *add_w,
+                          const CudaBuffer &norm_w, const CudaBuffer &x_out, const CudaBuffer &gate_up, const CudaBuffer &down,
+                          const CudaBuffer &slots_out, uint32_t hidden, uint32_t width, bool gelu, float eps) const {
+        TM_CALL(tm_cuda_decode_ffn_block, x.raw(), slots_in ? slots_in->raw() : nullptr, n_slots,
+                add_w ? add_w->raw() : nullptr, norm_w.raw(), x_out.raw(), gate_up.raw(), down.raw(), slots_out.raw(), hidden,
+                width, gelu ? 1 : 0, eps);
+    }
     void reduce_ranks_add(const CudaBuffer &slots, const CudaBuffer &x, const CudaBuffer *weight, uint32_t world,
                           uint32_t n_rows, uint32_t cols, float eps) const {
         TM_CALL(tm_cuda_reduce_ranks_add_f32, slots.raw(), x.raw(), weight ? weight->raw() : nullptr, world, n_rows, cols,

@@ -396,6 +396,28 @@ struct Residual {
     }
 };
 
+// The residual stream of a step whose blocks leave partial products ("slots") for their successor to add: the stream
+// alternates between two buffers, `pend` are the slots still to be added (with their norm weight, if any).
+struct SlotResidual {
+    const CudaBuffer *cur = nullptr, *alt = nullptr;
+    const CudaBuffer *pend = nullptr, *pend_w = nullptr;
+    uint32_t n = 0;
+    // A block has read cur + pend, written the sum to alt and left `slots`.
+    void left(const CudaBuffer &slots, uint32_t count, const CudaBuffer &out_norm) {
+        std::swap(cur, alt);
+        pend = &slots;
+        n = count;
+        pend_w = out_norm ? &out_norm : nullptr;
+    }
+    // Adds what is pending, for a consumer that takes the plain stream.
+    void settle(const CudaContext &ctx, size_t hidden, float eps) {
+        if (!n) return;
+        ctx.reduce_ranks_add(*pend, *cur, pend_w, n, 1, (uint32_t)hidden, eps);
+        pend = pend_w = nullptr;
+        n = 0;
+    }
+};
+
 // What the n rows of a batched pass are: n consecutive positions of sequence `seq` (a prefill chunk),
 // or -- with `pos_buf` set -- one decode row per sequence, sequence s at the device position pos_buf[s].
 struct RowsAre {
@@ -782,6 +804,40 @@ struct Layer {
         R.pend_p = &ffn.out;
         R.pend_w = &ffn.out_norm;
     }
+    // A one-token step's halves as one launch each (include/tm_cuda.h), where the shape allows it.
+    bool attn_block_applies(size_t hidden) const {
+        const AttentionSpec &m = mixer.spec;
+        return slices_apply() && tm_cuda_decode_attn_block_supported((uint32_t)hidden, (uint32_t)m.heads, (uint32_t)m.kv_heads,
+                                                                     (uint32_t)m.head_dim, (uint32_t)m.rope_dims);
+    }
+    bool ffn_block_applies(size_t hidden) const {
+        return slices_apply() && tm_cuda_decode_ffn_block_supported((uint32_t)hidden, (uint32_t)ffn.width);
+    }
+    void decode_blocks(const CudaContext &ctx, SlotResidual &R, const CudaBuffer &slots_a, const CudaBuffer &slots_f,
+                       const CudaBuffer &pos_buf, const CudaBuffer &status, size_t hidden, float eps, bool attn_block) const {
+        const AttentionSpec &m = mixer.spec;
+        if (attn_block) {
+            ctx.decode_attn_block(*R.cur, R.pend, R.n, R.pend_w, pre_norm, *R.alt, mixer.qkv.buf, mixer.o.buf, mixer.q_norm,
+                                  mixer.k_norm, mixer.inv_freq, mixer.k_cache, mixer.v_cache, pos_buf, status, slots_a,
+                                  (uint32_t)hidden, (uint32_t)m.heads, (uint32_t)m.kv_heads, (uint32_t)m.head_dim,
+                                  (uint32_t)mixer.cap, (uint32_t)m.window, eps, mixer.scale());
+            R.left(slots_a, (uint32_t)m.kv_heads, mixer_out_norm);
+        } else {
+            R.settle(ctx, hidden, eps);
+            mixer.decode(ctx, *R.cur, pre_norm, pos_buf, status, false);
+            if (mixer_out_norm) {  // one slot: the o projection itself
+                mixer.o.gemv(ctx, mixer.attn, proj);
+                R.pend = &proj;
+                R.n = 1;
+                R.pend_w = &mixer_out_norm;
+            } else {
+                mixer.o.gemv_fused(ctx, mixer.attn, *R.cur, TM_CUDA_PRO_NONE, nullptr, 0.0f, TM_CUDA_EPI_ADD);
+            }
+        }
+        ctx.decode_ffn_block(*R.cur, R.pend, R.n, R.pend_w, post_norm, *R.alt, ffn.gate_up.buf, ffn.down.buf, slots_f,
+                             (uint32_t)hidden, (uint32_t)ffn.width, ffn.act != GluActivation::Silu, eps);
+        R.left(slots_f, TM_CUDA_DECODE_SLOTS, ffn.out_norm);
+    }
     // Every matrix Q8_0 on one device: the batched fused GEMV forms apply.
     bool slices_apply() const {
         return mixer.sh.world == 1 && mixer.qkv.type == 8 && mixer.o.type == 8 && ffn.gate_up.type == 8 &&
@@ -884,6 +940,9 @@ struct EngineModel::Impl {
     CudaBuffer tied_view;  // row split of a tied head: this rank's rows of the (replicated) embedding
     uint32_t head_rows = 0;  // rows of the head this rank multiplies (vocab / world)
     CudaBuffer final_norm, x, x2, logits, partial, tokens, tokens_mirror, pos_buf, status;
+    CudaBuffer slots_a, slots_f;  // partial products of a step's attention / feed-forward blocks
+    // A one-sequence step's feed-forward / attention halves run as one launch each (Layer::decode_blocks).
+    bool ffn_blocks = false, attn_blocks = false;
     bool fold_norms = false;  // every layer's output norms ride into the next projection (Residual)
     CudaBuffer logits_full, pairs;  // row split only
     std::vector<Layer> layers;
@@ -900,13 +959,14 @@ struct EngineModel::Impl {
     const Matrix &head() const { return tied ? embedding : head_own; }  // single device only
     uint32_t head_cols() const { return embedding.cols; }
     uint32_t head_type() const { return tied ? embedding.type : head_own.type; }
-    // Final norm folded into the vocabulary projection of the one row in `x`.
-    void project_head(const CudaContext &c, float eps) const {
+    // Final norm folded into the vocabulary projection of one row (the one in `x`).
+    void project_head(const CudaContext &c, float eps) const { project_head(c, x, eps); }
+    void project_head(const CudaContext &c, const CudaBuffer &row, float eps) const {
         if (head_type() == 1)
-            c.f16_gemv_fused(head_buf(), x, logits, head_rows, head_cols(), TM_CUDA_PRO_RMSNORM, &final_norm, eps,
+            c.f16_gemv_fused(head_buf(), row, logits, head_rows, head_cols(), TM_CUDA_PRO_RMSNORM, &final_norm, eps,
                              TM_CUDA_EPI_STORE);
         else
-            c.q8_0_gemv_fused(head_buf(), x, logits, head_rows, head_cols(), TM_CUDA_PRO_RMSNORM, &final_norm, eps,
+            c.q8_0_gemv_fused(head_buf(), row, logits, head_rows, head_cols(), TM_CUDA_PRO_RMSNORM, &final_norm, eps,
                               TM_CUDA_EPI_STORE);
     }
 };
@@ -992,6 +1052,7 @@ GpuAllocPlan alloc_plan_with(const ModelGraph &graph, const WeightSource &src, s
     if (graph.head != graph.embedding) p.weights += Matrix::plan(src, {graph.head}, sh);
     p.weights_f32(vector_len(src, graph.final_norm));
     p.scratch_f32(graph.hidden);              // x
+    for (int i = 0; i < 2; ++i) p.scratch_f32(TM_CUDA_DECODE_SLOTS * graph.hidden);  // slots of the decode blocks
     p.scratch_f32(graph.hidden);              // x2: the other buffer of a residual stream that alternates
     p.scratch_f32(graph.vocab / sh.world * seqs);  // logits (this rank's slice), a row per sequence
     p.scratch_bytes(kArgmaxPartialBytes * seqs);   // argmax partials
@@ -1068,6 +1129,8 @@ std::unique_ptr<EngineModel> EngineModel::load_with(std::shared_ptr<CudaContext>
         throw TuckmillError(ErrorCode::UnsupportedArchitecture, "embedding / head shapes do not match the graph");
     I.final_norm = vector(c, src, graph.final_norm);
     I.x = zeros_f32(c, graph.hidden);
+    I.slots_a = zeros_f32(c, TM_CUDA_DECODE_SLOTS * graph.hidden);
+    I.slots_f = zeros_f32(c, TM_CUDA_DECODE_SLOTS * graph.hidden);
     I.x2 = zeros_f32(c, graph.hidden);
     I.logits = zeros_f32(c, (size_t)I.head_rows * I.seqs);
     if (sh.world > 1) {
@@ -1104,13 +1167,17 @@ std::unique_ptr<EngineModel> EngineModel::load_with(std::shared_ptr<CudaContext>
                 per_layer += Matrix::bytes_of(mx->type, mx->rows, mx->cols);
         size_t ahead = per_layer > (20u << 20) && per_layer <= (40u << 20) ? 1 : 0;
         if (const char *e = std::getenv("TM_ENGINE_L2_AHEAD")) ahead = (size_t)std::max(0, std::min(8, std::atoi(e)));
-        if (opts.shard_world > 1 || I.persistent) ahead = 0;
+        const char *fold = std::getenv("TM_ENGINE_FOLD_NORMS");
+        I.ffn_blocks = !(fold && fold[0] == '1') && !opts.exact && !I.persistent && opts.shard_world == 1 && !I.layers.empty();
+        for (const Layer &L : I.layers) I.ffn_blocks = I.ffn_blocks && L.ffn_block_applies(g.hidden);
+        I.attn_blocks = I.ffn_blocks;
+        for (const Layer &L : I.layers) I.attn_blocks = I.attn_blocks && L.attn_block_applies(g.hidden);
+        if (opts.shard_world > 1 || I.persistent || I.ffn_blocks) ahead = 0;  // (the blocks bring their own weights ahead)
         I.l2_ahead = ahead;
         // Folding the output norms into the next projection (Layer::decode_folded) saves two launches per
         // layer and is bit-identical, but measured slower on the Gemma-3-1B shape (1344 against 1299 us per
         // token: every CTA of the wide gate|up projection repeats a second reduction and two more vector
         // loads, which costs more than the small kernel it replaces): off unless TM_ENGINE_FOLD_NORMS=1.
-        const char *fold = std::getenv("TM_ENGINE_FOLD_NORMS");
         I.fold_norms = fold && fold[0] == '1' && !I.persistent && opts.shard_world == 1 && I.head_type() == 8 &&
                        !I.layers.empty();
         for (const Layer &L : I.layers) I.fold_norms = I.fold_norms && L.norms_fold(g.hidden);
@@ -1176,7 +1243,15 @@ void EngineModel::encode_decode_step() {
         c.prefetch_l2({&P.mixer.qkv.buf, &P.mixer.o.buf, &P.ffn.gate_up.buf, &P.ffn.down.buf});
     };
     for (size_t l = 0; l < ahead; ++l) prefetch(l);
-    if (I.fold_norms) {
+    if (I.ffn_blocks) {
+        SlotResidual R;
+        R.cur = &I.x;
+        R.alt = &I.x2;
+        for (const Layer &L : I.layers)
+            L.decode_blocks(c, R, I.slots_a, I.slots_f, I.pos_buf, I.status, g.hidden, g.eps, I.attn_blocks);
+        R.settle(c, g.hidden, g.eps);
+        I.project_head(c, *R.cur, g.eps);
+    } else if (I.fold_norms) {
         Residual R;
         R.cur = &I.x;
         R.alt = &I.x2;

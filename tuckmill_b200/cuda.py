@@ -111,6 +111,8 @@ _OPS = {
     "qk_prep_chunk": [_P] * 9 + [_U32] * 7 + [_F],
     "attention_chunk_mma": [_P, _P, _P, _P, _P, _U32, _U32, _U32, _U32, _U32, _F, _U32, _U32],
     "attention_decode_dev": [_P] * 12 + [_U32, _P] + [_U32] * 6 + [_F, _F, _I],
+    "decode_attn_block": [_P, _P, _P, _U32] + [_P] * 11 + [_U32, _P, _P] + [_U32] * 6 + [_F, _F],
+    "decode_ffn_block": [_P, _P, _P, _U32] + [_P] * 6 + [_U32, _U32, _I, _F],
     "attention_decode_dev_static": [_P] * 11 + [_U32, _P] + [_U32] * 6 + [_F, _F, _I],
 }
 
@@ -437,6 +439,19 @@ class CudaContext:
 
     def f16_rows_indirect(self, w, rows, cols, ids, first, n, scale, out):
         self._call("f16_rows_indirect_f32", w.handle, rows, cols, ids.handle, first, n, scale, out.handle)
+
+    # a decode token's layer in two launches (include/tm_cuda.h)
+    def decode_attn_block(self, x, slots_in, n_slots, add_w, norm_w, x_out, qkv, o, q_norm, k_norm, inv_freq, k_cache,
+                          v_cache, pos_buf, pos_index, status, slots_out, hidden, heads, kv_heads, head_dim, cap, window,
+                          eps, scale):
+        self._call("decode_attn_block", x.handle, self._h(slots_in), n_slots, self._h(add_w), norm_w.handle, x_out.handle,
+                   qkv.handle, o.handle, q_norm.handle, k_norm.handle, inv_freq.handle, k_cache.handle, v_cache.handle,
+                   pos_buf.handle, pos_index, status.handle, slots_out.handle, hidden, heads, kv_heads, head_dim, cap,
+                   window, eps, scale)
+
+    def decode_ffn_block(self, x, slots_in, n_slots, add_w, norm_w, x_out, gate_up, down, slots_out, hidden, width, gelu, eps):
+        self._call("decode_ffn_block", x.handle, self._h(slots_in), n_slots, self._h(add_w), norm_w.handle, x_out.handle,
+                   gate_up.handle, down.handle, slots_out.handle, hidden, width, int(gelu), eps)
 
     # decode steps of several sequences (include/tm_cuda.h)
     def q8_0_gemv_addnorm(self, w, x, add_p, add_w, x_out, norm_w, y, rows, cols, eps):
