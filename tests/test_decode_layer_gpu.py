@@ -37,3 +37,75 @@ def test_cluster_attention_equals_the_exact_form(ctx, oracle, heads, kvh, hd, wi
     for a, b in zip(*caches):
         assert np.max(np.abs(a - b)) <= 2e-3 * max(1.0, float(np.max(np.abs(a))))  # one f16 step of the fresh row
     assert int(status.download(0, 4, np.uint32)[0]) == 0
+
+
+def f64_layer(x, slots, add_w, norm_w, eps):
+    p = slots.astype(np.float64).sum(axis=0) if slots is not None else 0.0
+    if add_w is not None:
+        p = p / np.sqrt((p ** 2).mean() + eps) * add_w
+    x = x + p
+    return x, x / np.sqrt((x ** 2).mean() + eps) * norm_w
+
+
+# widths that cut evenly over clusters and CTAs, that leave remainders, and the narrowest there is
+@pytest.mark.parametrize("hidden,width,n_slots,normed", [(1024, 3072, 8, False), (64, 512, 0, False), (320, 576, 1, True),
+                                                         (1088, 1024, 3, True), (1024, 2112, 8, True)])
+@pytest.mark.parametrize("gelu", [False, True])
+def test_feed_forward_block(ctx, hidden, width, n_slots, normed, gelu):
+    eps = 1e-6
+    raw_gu, raw_dn = T.q8_0_matrix(3, 1, 2 * width, hidden), T.q8_0_matrix(3, 2, hidden, width)
+    x, nw = T.activations(3, 3, hidden), (1 + 0.1 * T.activations(3, 4, hidden)).astype(np.float32)
+    slots = T.activations(3, 5, n_slots * hidden).reshape(n_slots, hidden) if n_slots else None
+    aw = (1 + 0.1 * T.activations(3, 6, hidden)).astype(np.float32) if normed else None
+    want_x, h = f64_layer(x, slots, aw, nw, eps)
+    g, u = np.split(T.q8_0_dequant(raw_gu).astype(np.float64) @ h, 2)
+    act = (0.5 * g * (1 + np.tanh(0.7978845608028654 * (g + 0.044715 * g ** 3))) if gelu else g / (1 + np.exp(-g))) * u
+    want = T.q8_0_dequant(raw_dn).astype(np.float64) @ act
+    xo, so = ctx.buffer(hidden * 4), ctx.buffer(8 * hidden * 4)
+    ctx.decode_ffn_block(ctx.floats(x), ctx.floats(slots) if n_slots else None, n_slots, ctx.floats(aw) if normed else None,
+                         ctx.floats(nw), xo, ctx.q8_0_matrix(raw_gu, 2 * width, hidden), ctx.q8_0_matrix(raw_dn, hidden, width),
+                         so, hidden, width, gelu, eps)
+    assert rel_err(xo.download(0, hidden * 4, np.float32), want_x) <= 2e-6
+    assert rel_err(so.download(0, 8 * hidden * 4, np.float32).reshape(8, hidden).astype(np.float64).sum(axis=0), want) <= 2e-6
+
+
+@pytest.mark.parametrize("hidden,heads,kvh,hd,pos,window", [(1024, 16, 8, 128, 700, 0), (256, 4, 2, 128, 0, 0), (64, 3, 3, 128, 129, 50),
+                                                            (128, 4, 1, 256, 1030, 40), (1088, 8, 8, 128, 15, 0)])
+def test_attention_block_equals_the_operators_it_replaces(ctx, oracle, hidden, heads, kvh, hd, pos, window):
+    eps, cap, scale, n_slots = 1e-6, 1100, 1.0 / np.sqrt(np.float32(hd)), 4
+    rows = (heads + 2 * kvh) * hd
+    qkv = ctx.q8_0_matrix(T.q8_0_matrix(4, 1, rows, hidden), rows, hidden)
+    o = ctx.q8_0_matrix(T.q8_0_matrix(4, 2, hidden, heads * hd), hidden, heads * hd)
+    x, nw = T.activations(4, 3, hidden), (1 + 0.1 * T.activations(4, 4, hidden)).astype(np.float32)
+    slots = T.activations(4, 5, n_slots * hidden).reshape(n_slots, hidden)
+    qn, kn = (ctx.floats((1 + 0.1 * T.activations(4, t, hd)).astype(np.float32)) for t in (20, 21))
+    inv, pb = ctx.floats(oracle.rope_inv_freq(hd, 1e6)), ctx.from_array(np.array([pos], np.uint32))
+    kfill, vfill = (T.activations(4, t, kvh * cap * hd).astype(np.float16) for t in (30, 31))
+    status = ctx.buffer(4, shared=True)
+    status.zero()
+    want_x = f64_layer(x, slots, None, nw, eps)[0].astype(np.float32)
+    # the operators: norm + q|k|v, exact attention, o
+    xb, y, att, out = ctx.floats(want_x), ctx.buffer(rows * 4), ctx.buffer(heads * hd * 4), ctx.buffer(hidden * 4)
+    ctx.q8_0_gemv_fused(qkv, xb, y, rows, hidden, cuda.PRO_RMSNORM, ctx.floats(nw), eps)
+    scratch = ctx.buffer(cuda.decode_attention_scratch_bytes(heads, kvh, hd, cap))
+    scratch.zero()
+    kc, vc = ctx.from_array(kfill), ctx.from_array(vfill)
+    ctx.attention_decode_dev(y.view(0, heads * hd * 4), y.view(heads * hd * 4, kvh * hd * 4),
+                             y.view((heads + kvh) * hd * 4, kvh * hd * 4), qn, kn, inv, kc, vc, att, scratch, pb, 0, status,
+                             heads, kvh, hd, hd, cap, window, eps, scale, True)
+    ctx.q8_0_gemv(o, att, out, hidden, heads * hd)
+    # the block
+    kc2, vc2, xo, so = ctx.from_array(kfill), ctx.from_array(vfill), ctx.buffer(hidden * 4), ctx.buffer(8 * hidden * 4)
+    ctx.decode_attn_block(ctx.floats(x), ctx.floats(slots), n_slots, None, ctx.floats(nw), xo, qkv, o, qn, kn, inv, kc2, vc2, pb,
+                          0, status, so, hidden, heads, kvh, hd, cap, window, eps, scale)
+    assert rel_err(xo.download(0, hidden * 4, np.float32), want_x) <= 2e-6
+    got = so.download(0, kvh * hidden * 4, np.float32).reshape(kvh, hidden).astype(np.float64).sum(axis=0)
+    assert rel_err(got, out.download(0, hidden * 4, np.float32)) <= 1e-4
+    for a, b in ((kc, kc2), (vc, vc2)):
+        d = np.abs(a.download(0, kfill.nbytes, np.float16).astype(np.float32) - b.download(0, kfill.nbytes, np.float16).astype(np.float32))
+        assert float(np.max(d)) <= 4e-3  # one f16 step of the fresh row
+    # a position past the capacity is flagged, not stored
+    pb.upload(0, np.array([cap], np.uint32))
+    ctx.decode_attn_block(ctx.floats(x), None, 0, None, ctx.floats(nw), xo, qkv, o, qn, kn, inv, kc2, vc2, pb, 0, status, so,
+                          hidden, heads, kvh, hd, cap, window, eps, scale)
+    assert int(status.download(0, 4, np.uint32)[0]) == 1

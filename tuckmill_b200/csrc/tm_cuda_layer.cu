@@ -10,9 +10,10 @@
 //     columns of down.  Both end in one full-width partial product per cluster, a "slot";
 //   * the slots are added (in order) to the residual stream by whoever reads it next, as the first thing its CTAs do
 //     anyway; one cluster also stores the sum.  A layer's output norm is applied there too;
-//   * weights never wait for activations: every warp streams its own sequence of 16-row x 64-column pieces, both
-//     projections of the block in turn, through a ring in shared memory, starting before the dependency wait; both
-//     blocks' CTAs fit on an SM together, so a block's weights arrive while the block before it computes.
+//   * weights never wait for activations: every warp copies its own 16-row x 64-column pieces of both projections to
+//     shared memory before the dependency wait; both blocks' CTAs fit on an SM together, so a block's weights arrive
+//     while the block before it computes.  (Only 7 of the 8 GPCs have the 16 SMs of a cluster: a block that fills more
+//     than half an SM's shared memory runs its eighth cluster after the others, 20 us a layer instead of 11.)
 // Products are the decode GEMV's (tm_cuda_q8.cu): int8 tensor-core MMAs on activations split into four 7-bit digits,
 // exact sums per 32-column block.  How a row's columns are cut over warps, CTAs and clusters depends on the shape
 // alone, and every sum has a fixed order.
@@ -26,13 +27,15 @@ constexpr int kWarps = kT / 32;
 constexpr uint32_t kSlotBytes = 1024u + 64u;  // 16 rows x 64 quants, 16 rows x 2 scales
 constexpr uint32_t kC = 16;                   // CTAs per cluster
 constexpr uint32_t kSlots = TM_CUDA_DECODE_SLOTS;
-constexpr uint32_t kResident = 12;            // pieces a warp's ring holds
+constexpr uint32_t kResident = 12;            // most pieces a warp keeps in shared memory
 
 __host__ __device__ inline uint32_t plane_bytes(uint32_t cols) {  // 64 mod 128: the four digit planes hit distinct banks
     const uint32_t pad = (cols + 63u) & ~63u;
     return pad % 128u == 0u ? pad + 64u : pad;
 }
 __host__ __device__ inline uint32_t digit_bytes(uint32_t cols) { return (4u * plane_bytes(cols) + cols / 32u * 16u + 15u) & ~15u; }
+
+__host__ __device__ inline uint32_t max_of(uint32_t a, uint32_t b) { return a > b ? a : b; }
 
 struct residual_in {
     const float *x;       // [hidden]
@@ -186,14 +189,12 @@ struct matrix_part {
     __device__ __forceinline__ uint32_t first(uint32_t warp) const { return tiles * chunks * warp / kWarps; }
 };
 
-// A warp's weight stream through D slots of shared memory: its items of the first projection, then those of the
-// second.  Every lane copies, and later reads back, its own 16 bytes of rows g and g + 8 of a piece; the 32 block
-// scales ride along as 4-byte copies.  RES: all of them fit the slots, so the copies of a projection are one group and
-// one wait, and every piece leaves its own partial sum -- no bookkeeping between pieces (a commit, a wait and a running
-// sum per piece cost more than 400 cycles each in a chain that multiplies six).  Otherwise two pieces are consumed and
-// two requested per trip, and a warp adds the pieces of a tile before it leaves the sum.
-template <int D, bool RES, class RowOf1, class RowOf2>
-struct weight_ring {
+// A warp's weight pieces in shared memory: its items of the first projection, then those of the second, each one copy
+// group with one wait.  Every lane copies, and later reads back, its own 16 bytes of rows g and g + 8 of a piece; the 32
+// block scales ride along as 4-byte copies.  Every piece leaves its own partial sum: no bookkeeping between pieces (a
+// commit, a wait and a running sum per piece cost more than 400 cycles each in a chain that multiplies six).
+template <class RowOf1, class RowOf2>
+struct weight_pieces {
     matrix_part m1, m2;
     RowOf1 row1;  // (tile, r): the weight row of row r of a tile
     RowOf2 row2;
@@ -237,9 +238,7 @@ struct weight_ring {
             pa += 64;
             pb += 64;
             ps += 2;
-            if (--left == 0u) {
-                if (!RES && !second) open(true);
-            } else if (--left_tile == 0u) {
+            if (--left != 0u && --left_tile == 0u) {
                 ++tile;
                 open_tile(0u);
             }
@@ -250,24 +249,14 @@ struct weight_ring {
         base = ring;
         slot = 0;
         open(false);
-        if constexpr (RES) {
 #pragma unroll 1
-            while (left) issue(slot++);
-            commit();
-            open(true);
+        while (left) issue(slot++);
+        commit();
+        open(true);
 #pragma unroll 1
-            while (left) issue(slot++);
-            commit();
-            slot = 0;
-        } else {
-            if (left == 0u) open(true);
-#pragma unroll 1
-            for (int i = 0; i < D; i += 2) {  // groups of two
-                issue(i);
-                issue(i + 1);
-                commit();
-            }
-        }
+        while (left) issue(slot++);
+        commit();
+        slot = 0;
     }
     // One piece: this lane's digits' share of rows g (x) and g + 8 (y).
     __device__ __forceinline__ float2 piece(uint32_t at, const unsigned char *dig, uint32_t plane, uint32_t ch) const {
@@ -287,14 +276,8 @@ struct weight_ring {
         return make_float2(__half2float(__ushort_as_half(sa)) * fmaf((float)dd[1], cx.y, (float)dd[0] * cx.x),
                            __half2float(__ushort_as_half(sb)) * fmaf((float)dd[3], cx.y, (float)dd[2] * cx.x));
     }
-    // This warp's pieces of one projection.  Partial sums: part[piece][16 rows] (RES), or part[warp][tile][16 rows]
-    // with zeros where the warp has none.
+    // This warp's pieces of one projection: piece i leaves its sums in part[i][16 rows].
     __device__ __forceinline__ void multiply(const matrix_part &m, bool sec, const unsigned char *dig, uint32_t plane, float *part) {
-        if constexpr (RES) multiply_resident(m, sec, dig, plane, part);
-        else multiply_stream(m, dig, plane, part);
-    }
-    __device__ __forceinline__ void multiply_resident(const matrix_part &m, bool sec, const unsigned char *dig, uint32_t plane,
-                                                      float *part) {
         const uint32_t l = lane(), g = l >> 2, t4 = l & 3u, i0 = m.first(warp()), end = m.first(warp() + 1u);
         uint32_t ch = i0 % m.chunks;
         if (sec) asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -323,85 +306,22 @@ struct weight_ring {
             }
         }
     }
-    __device__ __forceinline__ void multiply_stream(const matrix_part &m, const unsigned char *dig, uint32_t plane, float *part) {
-        const uint32_t l = lane(), g = l >> 2, t4 = l & 3u;
-        uint32_t i = m.first(warp());
-        const uint32_t end = m.first(warp() + 1u);
-        float *mine = part + warp() * m.tiles * 16u;
-        for (uint32_t z = l; z < m.tiles * 16u; z += 32u) mine[z] = 0.0f;
-        __syncwarp();
-        uint32_t t = i / m.chunks, ch = i - t * m.chunks;
-        float2 acc = make_float2(0.0f, 0.0f);
-        auto add = [&](float2 v, bool last) {
-            acc.x += v.x;
-            acc.y += v.y;
-            if (++ch == m.chunks || last) {
-                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 1);
-                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 1);
-                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 2);
-                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 2);
-                if (t4 == 0u) {
-                    mine[t * 16u + g] = acc.x;
-                    mine[t * 16u + g + 8u] = acc.y;
-                }
-                acc = make_float2(0.0f, 0.0f);
-                ch = 0;
-                ++t;
-            }
-        };
-        // Pieces of one trip: two, but the first projection's last trip takes one when its count is odd (the second
-        // projection then starts at the group's other slot, which has landed too).
-#pragma unroll 1
-        while (i < end) {
-            const bool odd = (slot & 1u) != 0u, two = !odd && i + 1u < end;
-            asm volatile("cp.async.wait_group %0;" ::"n"(D / 2 - 1) : "memory");
-            __syncwarp();  // scales were copied by other lanes
-            const float2 v0 = piece(slot, dig, plane, ch);
-            float2 v1 = make_float2(0.0f, 0.0f);
-            if (two) v1 = piece(slot + 1u, dig, plane, ch + 1u == m.chunks ? 0u : ch + 1u);
-            if (two || odd) {
-                __syncwarp();  // every lane has read the slots before they are refilled
-                const uint32_t s0 = slot & ~1u;
-                issue(s0);
-                issue(s0 + 1u);
-                commit();
-                slot = s0 + 2u == (uint32_t)D ? 0u : s0 + 2u;
-            } else {
-                ++slot;
-            }
-            add(v0, i + 1u == end);
-            if (two) add(v1, i + 2u == end);
-            i += two ? 2u : 1u;
-        }
-    }
 };
 
-// Row r of tile t: the sum of its partial sums -- the tile's pieces (RES) or the warps' shares -- by one thread
-// (row_sum) or by the 16 lanes of half a warp, which all receive it (half_sum).
-template <bool RES>
-__device__ __forceinline__ float part_term(const float *part, const matrix_part &m, uint32_t t, uint32_t r, uint32_t k) {
-    return RES ? part[(t * m.chunks + k) * 16u + r] : part[(k * m.tiles + t) * 16u + r];
-}
-template <bool RES>
+// Row r of tile t: the sum over the tile's pieces, by one thread (row_sum) or by the 16 lanes of half a warp, which all
+// receive it (half_sum).
 __device__ __forceinline__ float row_sum(const float *part, const matrix_part &m, uint32_t t, uint32_t r) {
-    const uint32_t n = RES ? m.chunks : (uint32_t)kWarps;
     float v = 0.0f;
 #pragma unroll 4
-    for (uint32_t k = 0; k < n; ++k) v += part_term<RES>(part, m, t, r, k);
+    for (uint32_t k = 0; k < m.chunks; ++k) v += part[(t * m.chunks + k) * 16u + r];
     return v;
 }
-template <bool RES>
 __device__ __forceinline__ float half_sum(const float *part, const matrix_part &m, uint32_t t, uint32_t r) {
-    const uint32_t n = RES ? m.chunks : (uint32_t)kWarps, k = threadIdx.x & 15u;
-    float v = k < n ? part_term<RES>(part, m, t, r, k) : 0.0f;
-    for (uint32_t j = k + 16u; j < n; j += 16u) v += part_term<RES>(part, m, t, r, j);
+    float v = 0.0f;
+    for (uint32_t k = threadIdx.x & 15u; k < m.chunks; k += 16u) v += part[(t * m.chunks + k) * 16u + r];
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-__host__ __device__ inline uint32_t part_bytes(bool res, uint32_t items1, uint32_t items2, uint32_t tiles1, uint32_t tiles2) {
-    const uint32_t a = res ? items1 : kWarps * tiles1, b = res ? items2 : kWarps * tiles2;
-    return 64u * (a > b ? a : b);
 }
 
 // ---------------- feed-forward block ----------------
@@ -417,19 +337,18 @@ struct ffn_args {
 struct ffn_smem {
     uint32_t dig2, acts, part, red, ring, bytes;
 };
-__host__ __device__ inline ffn_smem ffn_layout(uint32_t hidden, uint32_t acts, uint32_t tiles1, uint32_t tiles2, bool res,
-                                               uint32_t slots) {
+__host__ __device__ inline ffn_smem ffn_layout(uint32_t hidden, uint32_t acts, uint32_t tiles1, uint32_t tiles2, uint32_t slots) {
     ffn_smem s;
     s.dig2 = digit_bytes(hidden);
     s.acts = s.dig2 + digit_bytes(acts);
     s.part = s.acts + acts * 4u;
-    s.red = s.part + part_bytes(res, tiles1 * (hidden / 64u), tiles2 * (acts / 64u), tiles1, tiles2);
+    s.red = s.part + 64u * max_of(tiles1 * (hidden / 64u), tiles2 * (acts / 64u));
     s.ring = s.red + 64u;
     s.bytes = s.ring + kWarps * slots * kSlotBytes;
     return s;
 }
 
-template <bool RES, int NB>
+template <int NB>
 __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint32_t ring_slots) {
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t rank = cluster_rank(), cluster = blockIdx.x / kC, n_clusters = gridDim.x / kC;
@@ -438,7 +357,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
     const uint32_t groups = nfc * 8u;                  // of 8 gate rows and the 8 up rows they gate: one tile
     const uint32_t g0 = groups * rank / kC, n1 = groups * (rank + 1u) / kC - g0;
     const uint32_t row_tiles = H / 16u, t0 = row_tiles * rank / kC, n2 = row_tiles * (rank + 1u) / kC - t0;
-    const ffn_smem L = ffn_layout(H, a.acts, a.tiles1, a.tiles2, RES, ring_slots);
+    const ffn_smem L = ffn_layout(H, a.acts, a.tiles1, a.tiles2, ring_slots);
     unsigned char *dig1 = smem, *dig2 = smem + L.dig2;
     float *acts = (float *)(smem + L.acts), *part = (float *)(smem + L.part), *red = (float *)(smem + L.red);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -447,7 +366,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
         return fc0 * 64u + (g0 + tile) * 8u + (r & 7u) + (r & 8u ? F : 0u);
     };
     auto row2 = [=](uint32_t tile, uint32_t r) -> size_t { return (t0 + tile) * 16u + r; };
-    weight_ring<(int)kResident, RES, decltype(row1), decltype(row2)> W = {
+    weight_pieces<decltype(row1), decltype(row2)> W = {
         {a.gu_q, a.gu_d, H, 0u, n1, H / 64u}, {a.dn_q, a.dn_d, F, fc0, n2, nfc}, row1, row2};
     W.start(smem_addr(smem + L.ring) + warp * ring_slots * kSlotBytes);
     tmdev::pdl_trigger();
@@ -459,7 +378,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
     cluster_wait();  // every CTA of the cluster has started
     // A warp finishes an activation: gate in its lower half, up in its upper; lane c of the lower half sends it to CTA c.
     for (uint32_t i = warp; i < n1 * 8u; i += kWarps) {
-        const float sum = half_sum<RES>(part, W.m1, i >> 3, (i & 7u) + (lane & 16u) / 2u);
+        const float sum = half_sum(part, W.m1, i >> 3, (i & 7u) + (lane & 16u) / 2u);
         const float up = __shfl_down_sync(0xffffffffu, sum, 16);
         const float v = (a.gelu ? tmdev::gelu_tanh_f(sum) : tmdev::silu_f(sum)) * up;
         if (lane < kC) st_cluster(smem_addr(acts + g0 * 8u + i), lane, v);
@@ -476,7 +395,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
     W.multiply(W.m2, true, dig2, plane_bytes(a.acts), part);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < n2 * 16u; i += kT)
-        a.slots_out[(size_t)cluster * H + t0 * 16u + i] = row_sum<RES>(part, W.m2, i >> 4, i & 15u);
+        a.slots_out[(size_t)cluster * H + t0 * 16u + i] = row_sum(part, W.m2, i >> 4, i & 15u);
 }
 
 // ---------------- attention block ----------------
@@ -506,7 +425,7 @@ __host__ __device__ inline attn_smem attn_layout(uint32_t hidden, uint32_t tiles
     s.recv_ml = s.recv + kC * G * HD * 4u;
     s.wgt = s.recv_ml + kC * G * 2u * 4u;
     s.part = s.wgt + kC * G * 4u;
-    s.red = s.part + part_bytes(true, tiles1 * (hidden / 64u), tiles2 * (G * HD / 64u), tiles1, tiles2);
+    s.red = s.part + 64u * max_of(tiles1 * (hidden / 64u), tiles2 * (G * HD / 64u));
     s.ring = s.red + 64u;
     s.bytes = s.ring + kWarps * slots * kSlotBytes;
     return s;
@@ -536,7 +455,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                                   : kvw * (G + 1) + kvh * HD + (i - (G + 1) * HD);
     };
     auto row2 = [=](uint32_t tile, uint32_t r) -> size_t { return (t0 + tile) * 16u + r; };
-    weight_ring<(int)kResident, true, decltype(row1), decltype(row2)> W = {
+    weight_pieces<decltype(row1), decltype(row2)> W = {
         {a.qkv_q, a.qkv_d, H, 0u, n1, H / 64u}, {a.o_q, a.o_d, kvw * G, kvh * (G * HD / 64u), n2, G * HD / 64u}, row1, row2};
     W.start(smem_addr(smem + L.ring) + warp * ring_slots * kSlotBytes);
     __half *kp = a.kc + (size_t)kvh * cap * HD, *vp = a.vc + (size_t)kvh * cap * HD;
@@ -546,7 +465,8 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
     tmdev::pdl_wait();
     tmdev::pdl_trigger();  // only now: see tm_cuda_attn_core.cuh
     const uint32_t pos = *pos_p;
-    if (pos >= cap) {  // uniform over the cluster; the ring's copies land before the CTA's memory goes away
+    stage_residual<NB>(a.in, kvh == 0u, rank, dig1, red);
+    if (pos >= cap) {  // uniform over the cluster; the pieces's copies land before the CTA's memory goes away
         if (tid == 0 && rank == 0) atomicOr(a.status, 1u);
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
@@ -562,14 +482,13 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
         for (int r = 0; r < EPL; ++r) nw[r] = __ldg(src + lane + 32 * r);
         rot.set(a.inv_freq, pos);
     }
-    stage_residual<NB>(a.in, kvh == 0u, rank, dig1, red);
     __syncthreads();
     W.multiply(W.m1, false, dig1, plane_bytes(H), part);
     __syncthreads();
     cluster_wait();  // every CTA of the cluster has started
     // Half a warp finishes a row; its lane c sends it to CTA c.
     for (uint32_t i = warp * 2u + (lane >> 4); i < n1 * 16u; i += 2u * kWarps)
-        st_cluster(smem_addr(qkv + u0 * 16u + i), lane & 15u, half_sum<true>(part, W.m1, i >> 4, i & 15u));
+        st_cluster(smem_addr(qkv + u0 * 16u + i), lane & 15u, half_sum(part, W.m1, i >> 4, i & 15u));
     cluster_arrive();
     cluster_wait();
     // ---- every CTA has the head's q, k and v ----
@@ -642,7 +561,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
     W.multiply(W.m2, true, dig2, plane_bytes(G * HD), part);
     __syncthreads();
     for (uint32_t i = tid; i < n2 * 16u; i += kT)
-        a.slots_out[(size_t)kvh * H + t0 * 16u + i] = row_sum<true>(part, W.m2, i >> 4, i & 15u);
+        a.slots_out[(size_t)kvh * H + t0 * 16u + i] = row_sum(part, W.m2, i >> 4, i & 15u);
 }
 
 // ---------------- launches ----------------
@@ -674,11 +593,11 @@ cudaError_t launch_clusters(tm_cuda_ctx *ctx, Kernel kernel, std::atomic<bool> *
     return cudaLaunchKernelEx(&cfg, kernel, a, ring_slots);
 }
 
-template <bool RES, int NB>
+template <int NB>
 cudaError_t launch_ffn(tm_cuda_ctx *ctx, const ffn_args &a, uint32_t slots) {
     static std::atomic<bool> attr_set[64] = {};  // per device; contexts of a process share it
-    return launch_clusters(ctx, ffn_block_kernel<RES, NB>, attr_set, kSlots,
-                           ffn_layout(a.in.hidden, a.acts, a.tiles1, a.tiles2, RES, slots).bytes, a, slots);
+    return launch_clusters(ctx, ffn_block_kernel<NB>, attr_set, kSlots,
+                           ffn_layout(a.in.hidden, a.acts, a.tiles1, a.tiles2, slots).bytes, a, slots);
 }
 template <int G, int HD, int NB>
 cudaError_t launch_attn(tm_cuda_ctx *ctx, const attn_block_args &a, uint32_t slots) {
@@ -700,9 +619,10 @@ cudaError_t launch_attn_any(tm_cuda_ctx *ctx, attn_block_args a) {
     return H <= 1024u ? launch_attn<G, HD, 1>(ctx, a, items) : launch_attn<G, HD, 2>(ctx, a, items);
 }
 
-// The attention block serves layers whose q|k|v and o pieces all stay in shared memory (0.6B shape: 6 a warp).  One
-// that has to stream them has no reason to: a cluster per KV head leaves most of the machine without work then
-// (1B shape, one KV head: 26 us against 18 as three launches; 8B shape: 34 against 30).
+// A block serves layers whose weights' pieces all stay in shared memory (0.6B shape: 6 and 9 a warp).  A layer that has
+// to stream them is bound by bytes, and eight warps on 128 SMs do not pull them fast enough (8B shape: feed-forward
+// block 79 us against 49 as two launches, attention block 34 against 30; 1B shape: 24 against 21), or has few KV heads
+// and leaves most of the machine without work (1B shape, one KV head: 26 us against 18).
 bool attn_shape(uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t hd) {
     const uint32_t g = kv_heads ? heads / kv_heads : 0u;
     return hidden >= 64u && hidden % 64u == 0u && hidden <= 2048u && (hd == 128u || hd == 256u) && kv_heads >= 1u &&
@@ -721,8 +641,6 @@ ffn_args ffn_shape(uint32_t hidden, uint32_t width) {
 uint32_t ffn_items(const ffn_args &a) {
     return ceil_div(a.tiles1 * (a.in.hidden / 64u), kWarps) + ceil_div(a.tiles2 * (a.acts / 64u), kWarps);
 }
-// The feed-forward block: up to about twice its ring (1B shape: 25 pieces a warp).  Longer streams are bound by bytes,
-// and eight warps an SM do not pull them fast enough (8B shape: 79 us against 49 as two launches).
 bool ffn_shape_ok(uint32_t hidden, uint32_t width) {
     return hidden >= 64u && hidden % 64u == 0u && hidden <= 2048u && width % 64u == 0u && width / 64u >= kSlots &&
            ffn_items(ffn_shape(hidden, width)) <= kResident;
@@ -837,8 +755,7 @@ int tm_cuda_decode_ffn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffer
     a.gelu = gelu ? 1u : 0u;
     const uint32_t items = ffn_items(a);
     TM_OP_BEGIN("decode_ffn_block");
-    TM_CUDA_TRY(items > kResident ? (hidden <= 1024u ? launch_ffn<false, 1>(ctx, a, kResident) : launch_ffn<false, 2>(ctx, a, kResident))
-                                  : (hidden <= 1024u ? launch_ffn<true, 1>(ctx, a, items) : launch_ffn<true, 2>(ctx, a, items)));
+    TM_CUDA_TRY(hidden <= 1024u ? launch_ffn<1>(ctx, a, items) : launch_ffn<2>(ctx, a, items));
     TM_OP_END(1);
 }
 
