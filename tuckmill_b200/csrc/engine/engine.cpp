@@ -1172,7 +1172,8 @@ std::unique_ptr<EngineModel> EngineModel::load_with(std::shared_ptr<CudaContext>
         for (const Layer &L : I.layers) I.ffn_blocks = I.ffn_blocks && L.ffn_block_applies(g.hidden);
         I.attn_blocks = I.ffn_blocks;
         for (const Layer &L : I.layers) I.attn_blocks = I.attn_blocks && L.attn_block_applies(g.hidden);
-        if (opts.shard_world > 1 || I.persistent || I.ffn_blocks) ahead = 0;  // (the blocks bring their own weights ahead)
+        if (opts.shard_world > 1 || I.persistent || I.ffn_blocks || I.head_type() == 1) ahead = 0;  // (the blocks and the F16 kernel
+        // ask for their own weights before their inputs are ready; a second reader in between only delays them)
         I.l2_ahead = ahead;
         // Folding the output norms into the next projection (Layer::decode_folded) saves two launches per
         // layer and is bit-identical, but measured slower on the Gemma-3-1B shape (1344 against 1299 us per

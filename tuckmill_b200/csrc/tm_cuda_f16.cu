@@ -8,9 +8,8 @@
 // on how many tokens share the launch, so batch 1 is bit-identical to the GEMV, the contract of
 // tm_metal.h:160-164) and the fused forms the decode step uses (the elementwise prologue of the
 // Q8_0 GEMV: RMS norm with the same canonical sum of squares, silu/gelu * up; store or accumulate).
-// A warp owns a row: lane l adds columns 2l, 2l+1, 2l+64, ... in that order, the lanes are added
-// with a xor butterfly.  The hot path of this library is Q8_0; this kernel is sized for
-// correctness on fixtures (coalesced 4-byte loads, activations staged once per CTA), not tuned.
+// Lane l of a warp adds columns 8l .. 8l+7, 8l+256, ... of its rows in that order, the lanes are added with a xor
+// butterfly.
 #include "tm_cuda_internal.cuh"
 #include "tm_cuda_device.cuh"
 
@@ -29,81 +28,161 @@ struct f16_args {
     int prologue, epilogue;
 };
 
-template <int M>
-__global__ void __launch_bounds__(kThreads) f16_gemv_kernel(const f16_args a) {
-    extern __shared__ __align__(16) float xs[];  // [M][cols]
+// A warp takes R rows at a time, lane l the eight columns 8l..8l+7 of every 256: one 16-byte load per row and trip, the
+// trip's activations read from shared memory once for all R rows and M tokens.  Which columns a lane adds, and in which
+// order, depends on neither R nor M, so a (row, token) result is the same bits in every batch.
+//   * one token: bound by bytes.  The first trip's weights are requested before the dependency wait and the next trip's
+//     while one is multiplied (16 MB projection of a 0.6B decoder, 2-byte loads of 64 columns: 1.0 TB/s; now 3.4);
+//   * several: bound by FMAs and the shared-memory reads that feed them, R x M products for M reads.
+// Activations lie as two planes of half-octets, so that lanes read consecutive 16-byte words.
+template <int M, int R>
+__global__ void __launch_bounds__(kThreads) f16_gemv_kernel(const f16_args args) {
+    f16_args a = args;
+    if constexpr (M > 1) {  // a grid row per slice of M tokens
+        const size_t t0 = (size_t)blockIdx.y * M;
+        a.x += t0 * a.cols;
+        a.y += t0 * a.rows;
+        if (a.prologue == TM_CUDA_PRO_SILU_MUL || a.prologue == TM_CUDA_PRO_GELU_MUL) a.pro += t0 * a.cols;
+    }
+    extern __shared__ __align__(16) float xs[];  // [M][2][octets][4]
     __shared__ float red[kWarps];
-    const uint32_t cols = a.cols, rows = a.rows;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int U = M == 1 ? (R == 1 ? 4 : 2) : 1;  // 256-column trips requested together
+    const uint32_t cols = a.cols, rows = a.rows, octets = (cols + 7u) / 8u;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool vec = (cols & 7u) == 0u && (((size_t)a.w) & 15u) == 0u;
+    auto load = [&](uint32_t row, uint32_t o) -> int4 {
+        if (o >= octets || row >= rows) return make_int4(0, 0, 0, 0);
+        const __half *p = a.w + (size_t)row * cols + o * 8u;
+        if (vec) return __ldg((const int4 *)p);
+        __half h[8];
+#pragma unroll
+        for (uint32_t e = 0; e < 8u; ++e) h[e] = o * 8u + e < cols ? p[e] : __float2half_rn(0.0f);
+        return *(const int4 *)h;
+    };
+    uint32_t row0 = (blockIdx.x * kWarps + warp) * R;
+    int4 cur[U][R];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int r = 0; r < R; ++r) cur[u][r] = load(row0 + r, lane + 32u * u);
     tmdev::pdl_trigger();
     tmdev::pdl_wait();
 #pragma unroll 1
     for (int m = 0; m < M; ++m) {
         const float *xm = a.x + (size_t)m * cols;
+        float *xd = xs + (size_t)m * octets * 8u;
         float inv_rms = 0.0f;
         if (a.prologue == TM_CUDA_PRO_RMSNORM) {
             const float ss = tmdev::block_sumsq(xm, cols, red);
             inv_rms = 1.0f / sqrtf(ss / (float)cols + a.eps);
         }
-        for (uint32_t c = threadIdx.x; c < cols; c += kThreads) {
-            float v = xm[c];
-            if (a.prologue == TM_CUDA_PRO_RMSNORM) v = v * inv_rms * a.pro[c];
-            else if (a.prologue == TM_CUDA_PRO_SILU_MUL) v = tmdev::silu_f(v) * a.pro[(size_t)m * cols + c];
-            else if (a.prologue == TM_CUDA_PRO_GELU_MUL) v = tmdev::gelu_tanh_f(v) * a.pro[(size_t)m * cols + c];
-            xs[(size_t)m * cols + c] = v;
+        for (uint32_t c = threadIdx.x; c < octets * 8u; c += kThreads) {
+            float v = c < cols ? xm[c] : 0.0f;
+            if (c < cols) {
+                if (a.prologue == TM_CUDA_PRO_RMSNORM) v = v * inv_rms * a.pro[c];
+                else if (a.prologue == TM_CUDA_PRO_SILU_MUL) v = tmdev::silu_f(v) * a.pro[(size_t)m * cols + c];
+                else if (a.prologue == TM_CUDA_PRO_GELU_MUL) v = tmdev::gelu_tanh_f(v) * a.pro[(size_t)m * cols + c];
+            }
+            xd[((c & 4u) ? octets * 4u : 0u) + (c >> 3) * 4u + (c & 3u)] = v;
         }
     }
     __syncthreads();
-    for (uint32_t row = blockIdx.x * kWarps + warp; row < rows; row += gridDim.x * kWarps) {
-        const __half *wr = a.w + (size_t)row * cols;
-        float acc[M];
+    const uint32_t stride = gridDim.x * kWarps * R;
+    for (; row0 < rows; row0 += stride) {
+        float acc[R][M];
 #pragma unroll
-        for (int m = 0; m < M; ++m) acc[m] = 0.0f;
-        if ((cols & 1u) == 0u && (((size_t)wr) & 3u) == 0u) {
-            for (uint32_t c = 2u * lane; c < cols; c += 64u) {
-                const float2 wv = __half22float2(*(const __half2 *)(wr + c));
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    acc[m] = fmaf(wv.x, xs[(size_t)m * cols + c], acc[m]);
-                    acc[m] = fmaf(wv.y, xs[(size_t)m * cols + c + 1], acc[m]);
+            for (int m = 0; m < M; ++m) acc[r][m] = 0.0f;
+#pragma unroll 1
+        for (uint32_t o = lane; o - lane < octets; o += 32u * U) {
+            int4 nxt[U][R];
+            const bool more = o - lane + 32u * U < octets;  // else the next rows' first trip
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    nxt[u][r] = more ? load(row0 + r, o + 32u * (U + u)) : load(row0 + stride + r, lane + 32u * u);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t oc = o + 32u * u;
+                if (oc < octets) {
+                    float wf[R][8];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const __half2 *h = (const __half2 *)&cur[u][r];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float2 f = __half22float2(h[e]);
+                            wf[r][2 * e] = f.x;
+                            wf[r][2 * e + 1] = f.y;
+                        }
+                    }
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        const float *xd = xs + (size_t)m * octets * 8u + oc * 4u;
+                        const float4 x0 = *(const float4 *)xd, x1 = *(const float4 *)(xd + octets * 4u);
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            float t = acc[r][m];
+                            t = fmaf(wf[r][0], x0.x, t);
+                            t = fmaf(wf[r][1], x0.y, t);
+                            t = fmaf(wf[r][2], x0.z, t);
+                            t = fmaf(wf[r][3], x0.w, t);
+                            t = fmaf(wf[r][4], x1.x, t);
+                            t = fmaf(wf[r][5], x1.y, t);
+                            t = fmaf(wf[r][6], x1.z, t);
+                            acc[r][m] = fmaf(wf[r][7], x1.w, t);
+                        }
+                    }
                 }
             }
-        } else {  // odd widths / unaligned rows: the same columns per lane, one value at a time
-            for (uint32_t c = 2u * lane; c < cols; c += 64u) {
 #pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    acc[m] = fmaf(__half2float(wr[c]), xs[(size_t)m * cols + c], acc[m]);
-                    if (c + 1 < cols) acc[m] = fmaf(__half2float(wr[c + 1]), xs[(size_t)m * cols + c + 1], acc[m]);
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int r = 0; r < R; ++r) cur[u][r] = nxt[u][r];
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                float v = acc[r][m];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0 && row0 + r < rows) {
+                    float *yp = a.y + (size_t)m * rows + row0 + r;
+                    *yp = a.epilogue == TM_CUDA_EPI_ADD ? *yp + v : v;
                 }
             }
-        }
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-            float v = acc[m];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) {
-                float *yp = a.y + (size_t)m * rows + row;
-                *yp = a.epilogue == TM_CUDA_EPI_ADD ? *yp + v : v;
-            }
-        }
     }
 }
 
-template <int M>
-cudaError_t launch_f16(tm_cuda_ctx *ctx, const f16_args &a, size_t smem) {
+template <int M, int R>
+cudaError_t launch_f16_rows(tm_cuda_ctx *ctx, const f16_args &a, size_t smem, uint32_t slices) {
     static std::atomic<bool> attr_set[64] = {};
     const int dev = ctx->device;
-    if (smem > 48u * 1024u && (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire))) {
-        cudaError_t e = cudaFuncSetAttribute(f16_gemv_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    // (the kernel's own shared array counts towards the 48 KB that need no attribute)
+    if (smem + 1024u > 48u * 1024u && (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire))) {
+        cudaError_t e = cudaFuncSetAttribute(f16_gemv_kernel<M, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)ctx->smem_optin - 4096);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    uint32_t grid = (a.rows + kWarps - 1) / kWarps;
-    const uint32_t cap = (uint32_t)ctx->sm_count * 8u;
-    if (grid > cap) grid = cap;
-    return tm_launch_pdl(ctx, f16_gemv_kernel<M>, dim3(grid), dim3(kThreads), smem, a);
+    // One resident wave: every CTA stages the activations once and walks its share of the rows.
+    uint32_t per_sm = (uint32_t)(ctx->smem_optin / (smem + 2048u));
+    per_sm = per_sm < 1u ? 1u : per_sm > (M == 1 ? 4u : 2u) ? (M == 1 ? 4u : 2u) : per_sm;
+    uint32_t grid = (a.rows + kWarps * R - 1) / (kWarps * R);
+    const uint32_t wave = (uint32_t)ctx->sm_count * per_sm / slices;
+    if (grid > wave) grid = wave < 1u ? 1u : wave;
+    return tm_launch_pdl(ctx, f16_gemv_kernel<M, R>, dim3(grid, slices), dim3(kThreads), smem, a);
+}
+// Rows per warp: as many as leave every SM a CTA (a 1024-row projection of one token keeps one row a warp).
+template <int M>
+cudaError_t launch_f16(tm_cuda_ctx *ctx, const f16_args &a, size_t smem, uint32_t slices) {
+    const uint64_t warps = (uint64_t)ctx->sm_count * kWarps, rows = (uint64_t)a.rows * slices;
+    if (rows >= 4u * warps || (M > 2 && rows >= 2u * warps)) return launch_f16_rows<M, 4>(ctx, a, smem, slices);
+    if (rows >= 2u * warps || M > 2) return launch_f16_rows<M, 2>(ctx, a, smem, slices);
+    return launch_f16_rows<M, 1>(ctx, a, smem, slices);
 }
 
 // out[c] = f32(w[row][c]) (* scale when non-zero); row < 0 writes zeros.
@@ -162,7 +241,7 @@ int f16_common(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, tm_cuda_b
     if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_BUF(pro, (size_t)cols * 4, "norm weight");
     if (prologue == TM_CUDA_PRO_SILU_MUL || prologue == TM_CUDA_PRO_GELU_MUL)
         TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate multiplicand");
-    const size_t per_token = (size_t)cols * 4, budget = ctx->smem_optin - 4096;
+    const size_t per_token = ((size_t)cols + 7u) / 8u * 32u, budget = ctx->smem_optin - 4096;
     if (per_token > budget)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "cols %u exceeds the activation stage of one CTA", cols);
     if (ctx->program)
@@ -185,14 +264,15 @@ int f16_common(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, tm_cuda_b
         a.prologue = prologue;
         a.epilogue = epilogue;
         const size_t smem = (size_t)m * per_token;
-        cudaError_t e = m == 8   ? launch_f16<8>(ctx, a, smem)
-                        : m == 4 ? launch_f16<4>(ctx, a, smem)
-                        : m == 2 ? launch_f16<2>(ctx, a, smem)
-                                 : launch_f16<1>(ctx, a, smem);
+        const uint32_t slices = m > 1 ? (batch - done) / (uint32_t)m : 1u;
+        cudaError_t e = m == 8   ? launch_f16<8>(ctx, a, smem, slices)
+                        : m == 4 ? launch_f16<4>(ctx, a, smem, slices)
+                        : m == 2 ? launch_f16<2>(ctx, a, smem, slices)
+                                 : launch_f16<1>(ctx, a, smem, 1u);
         if (e != cudaSuccess)
             return tm_fail(err, err_cap, TM_CUDA_ERR_INTERNAL, "F16 GEMV launch failed: %s", cudaGetErrorString(e));
         kernels += 1;
-        done += (uint32_t)m;
+        done += (uint32_t)m * slices;
     }
     TM_OP_END(kernels);
 }
