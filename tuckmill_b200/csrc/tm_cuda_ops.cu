@@ -315,11 +315,45 @@ __device__ __forceinline__ uint32_t attn_dim(int lane, int i) {
 // Partial attention of G query heads (shared memory qs[G][hd]) over the keys
 // [lo, hi) of the 32-key block starting at j0.  Slot i of o[g] holds value dim
 // attn_dim(lane, i).  Per head the arithmetic does not depend on G.
+// `ahead` (nullptr: none) holds the lane's first key trip and the first VB value rows, loaded by attend_ahead.
+template <int DPL>
+struct attend_loads {
+    static constexpr int KB = DPL * 4 < 16 ? DPL * 4 : 16;  // 16-byte key loads in flight (hd/8, at most 16)
+    static constexpr int VB = DPL <= 4 ? 16 : 8;            // value rows in flight
+    int4 k[KB];
+    __half v[VB][DPL];
+};
+template <int DPL>
+__device__ __forceinline__ void attend_value_row(const __half *vr, int lane, __half (&v)[DPL]) {
+    if constexpr (DPL % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < DPL; i += 2) *(__half2 *)&v[i] = *(const __half2 *)(vr + attn_dim<DPL>(lane, i));
+    } else {
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) v[i] = vr[attn_dim<DPL>(lane, i)];
+    }
+}
+template <int DPL>
+__device__ __forceinline__ void attend_ahead(attend_loads<DPL> &a, const __half *kc, const __half *vc, uint32_t hd,
+                                             uint32_t j0, uint32_t lo, uint32_t hi, int lane) {
+    using L = attend_loads<DPL>;
+    const uint32_t j = j0 + lane;
+    if (j >= lo && j < hi) {
+#pragma unroll
+        for (int c = 0; c < L::KB; ++c) a.k[c] = *(const int4 *)(kc + (size_t)j * hd + c * 8);
+    }
+    const uint32_t first = lo > j0 ? lo : j0, end = hi < j0 + kAttnBlock ? hi : j0 + kAttnBlock;
+#pragma unroll
+    for (int c = 0; c < L::VB; ++c)
+        attend_value_row<DPL>(vc + (size_t)(first + c < end ? first + c : first) * hd, lane, a.v[c]);
+}
 template <int G, int DPL>
 __device__ __forceinline__ void attend_block(const float *qs, const __half *kc, const __half *vc, uint32_t hd,
                                              uint32_t j0, uint32_t lo, uint32_t hi, float scale,
                                              const __half *k_new, const __half *v_new, uint32_t pos_new,
-                                             int lane, float (&m)[G], float (&l)[G], float (&o)[G][DPL]) {
+                                             int lane, float (&m)[G], float (&l)[G], float (&o)[G][DPL],
+                                             const attend_loads<DPL> *ahead = nullptr) {
+    using Loads = attend_loads<DPL>;
     const uint32_t j = j0 + lane;
     const bool valid = j >= lo && j < hi;
     // Four interleaved partial sums per head (chunk c of 8 dims goes to sum
@@ -329,11 +363,12 @@ __device__ __forceinline__ void attend_block(const float *qs, const __half *kc, 
     for (int g = 0; g < G; ++g) dot[g][0] = dot[g][1] = dot[g][2] = dot[g][3] = 0.0f;
     if (valid) {
         const __half *kr = (k_new && j == pos_new) ? k_new : kc + (size_t)j * hd;
-        constexpr int KB = DPL * 4 < 16 ? DPL * 4 : 16;  // 16-byte loads in flight (hd/8, at most 16)
+        constexpr int KB = Loads::KB;
         for (uint32_t d0 = 0; d0 < hd; d0 += KB * 8) {
             int4 raw[KB];
 #pragma unroll
-            for (int c = 0; c < KB; ++c) raw[c] = *(const int4 *)(kr + d0 + c * 8);
+            for (int c = 0; c < KB; ++c)
+                raw[c] = ahead && d0 == 0 && !(k_new && j == pos_new) ? ahead->k[c] : *(const int4 *)(kr + d0 + c * 8);
 #pragma unroll
             for (int c = 0; c < KB; ++c) {
                 const uint32_t d = d0 + c * 8;
@@ -375,7 +410,7 @@ __device__ __forceinline__ void attend_block(const float *qs, const __half *kc, 
     }
     const uint32_t jj0 = lo > j0 ? lo - j0 : 0, jj1 = (hi < j0 + kAttnBlock ? hi : j0 + kAttnBlock) - j0;
     // Keys in increasing order; the value rows of VB keys are loaded before use.
-    constexpr int VB = DPL <= 4 ? 16 : 8;
+    constexpr int VB = Loads::VB;
     for (uint32_t jb = jj0; jb < jj1; jb += VB) {
         float vf[VB][DPL];
 #pragma unroll
@@ -383,17 +418,15 @@ __device__ __forceinline__ void attend_block(const float *qs, const __half *kc, 
             const uint32_t jk = j0 + jb + c;
             const bool ok = jb + c < jj1;
             const __half *vr = (v_new && jk == pos_new) ? v_new : vc + (size_t)(ok ? jk : j0 + jj0) * hd;
-            if (DPL % 2 == 0) {
+            __half vh[DPL];
+            if (ahead && jb == jj0 && !(v_new && jk == pos_new)) {
 #pragma unroll
-                for (int i = 0; i < DPL; i += 2) {
-                    const float2 f = __half22float2(*(const __half2 *)(vr + attn_dim<DPL>(lane, i)));
-                    vf[c][i] = f.x;
-                    vf[c][i + 1] = f.y;
-                }
+                for (int i = 0; i < DPL; ++i) vh[i] = ahead->v[c][i];
             } else {
-#pragma unroll
-                for (int i = 0; i < DPL; ++i) vf[c][i] = __half2float(vr[attn_dim<DPL>(lane, i)]);
+                attend_value_row<DPL>(vr, lane, vh);
             }
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) vf[c][i] = __half2float(vh[i]);
         }
 #pragma unroll
         for (int c = 0; c < VB; ++c) {
@@ -461,7 +494,7 @@ __global__ void __launch_bounds__(32) attention_chunk_kernel(const float *q, con
         for (int i = 0; i < DPL; ++i) orow[g * hd + attn_dim<DPL>(lane, i)] = O[g][i] / L[g];
 }
 
-// Decode: grid (heads, ceil(cap/32)), one warp per (query head, key block).
+// Decode: grid (heads, ceil(cap/128)), one warp per (query head, key block), four consecutive blocks a CTA.
 // Every warp norms and rotates its query head (cheap, avoids a dependency); the
 // warps whose block holds the new position also norm, rotate and round the new
 // K/V row (the first head of each group stores it), each warp writes its block
@@ -487,19 +520,24 @@ struct decode_seq_strides {
         pos_p += sq_;                                \
     }
 
+// Bound by its chain of dependent steps, and by starting and retiring the CTAs of blocks past the position: with one
+// warp a CTA (2048 of them at 4096 positions of a 0.6B decoder, each fetching all small inputs before it looked at the
+// position, and the key loads only after the norm) a layer's call took 15.8 us at 150 positions, now 10.4.
+constexpr int kDecodeWarps = 4;
 template <int DPL>
-__global__ void __launch_bounds__(32) attention_decode_kernel(
+__global__ void __launch_bounds__(32 * kDecodeWarps) attention_decode_kernel(
     const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm,
     const float *inv_freq, __half *kc, __half *vc, float *out, float *scratch, const uint32_t *pos_p,
     uint32_t *status, uint32_t heads, uint32_t kv_heads, uint32_t hd, uint32_t n_rot, uint32_t cap,
     uint32_t window, float eps, float scale, const decode_seq_strides seqs) {
     TM_DECODE_SEQ_OFFSETS(seqs)
-    __shared__ __align__(16) float qs[32 * DPL];
-    __shared__ __align__(16) float ks[32 * DPL];
+    __shared__ __align__(16) float qs_all[kDecodeWarps][32 * DPL];
+    __shared__ __align__(16) float ks[32 * DPL];  // (one block holds the new position)
     __shared__ __align__(16) __half kh[32 * DPL];
     __shared__ __align__(16) __half vh[32 * DPL];
-    const int lane = threadIdx.x;
-    const uint32_t head = blockIdx.x, blk = blockIdx.y, group = heads / kv_heads, kvh = head / group;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *qs = qs_all[warp];
+    const uint32_t head = blockIdx.x, blk = blockIdx.y * kDecodeWarps + warp, group = heads / kv_heads, kvh = head / group;
     const uint32_t nblk = (cap + kAttnBlock - 1) / kAttnBlock;
     const __half *kp = kc + (size_t)kvh * cap * hd, *vp = vc + (size_t)kvh * cap * hd;
     // The cache rows of this block do not depend on the predecessor's output
@@ -507,7 +545,11 @@ __global__ void __launch_bounds__(32) attention_decode_kernel(
     // Only as far as L2, which is coherent: a kernel two places back in a chain of
     // programmatic launches (the previous token's attention) may still be storing
     // its row, and a copy of that line taken into L1 now would be read stale later.
-    {
+    // The position read now only says which blocks are worth it: asking for every row of the capacity cost more
+    // (33 MB a layer at 4096 positions of a 0.6B decoder) than the attention itself.
+    const uint32_t hint = *(const volatile uint32_t *)pos_p;
+    const bool likely = blk < nblk && blk * kAttnBlock <= hint;
+    if (likely) {
         const uint32_t j = min(blk * kAttnBlock + lane, cap - 1u);
         for (uint32_t off = 0; off < hd * 2u; off += 128u) {
             asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)(kp + (size_t)j * hd) + off));
@@ -520,6 +562,7 @@ __global__ void __launch_bounds__(32) attention_decode_kernel(
     // attention call could read cache rows early that a call several places back is still storing.
     // This way only the call directly before can still be running: the row it stores is read again below.
     tmdev::pdl_trigger();
+    if (!likely && blk * kAttnBlock > *pos_p && !(blk == 0)) return;
     // Every small input is fetched in one trip, before the position is needed.
     // Lane l holds quads l and l + 32 of a row.
     constexpr int QW = DPL > 4 ? 2 : 1;
@@ -548,6 +591,9 @@ __global__ void __launch_bounds__(32) attention_decode_kernel(
     const uint32_t seq = pos + 1u, start = attn_start(seq, window);
     const uint32_t first = start / kAttnBlock, last = pos / kAttnBlock;
     if (blk < first || blk > last) return;
+    // The cached keys and values travel while the heads are normed and rotated (the new row's are not read).
+    attend_loads<DPL> ahead;
+    attend_ahead<DPL>(ahead, kp, vp, hd, blk * kAttnBlock, start, pos, lane);
     float rc[RP], rs[RP];
 #pragma unroll
     for (int r = 0; r < RP; ++r) {
@@ -619,7 +665,7 @@ __global__ void __launch_bounds__(32) attention_decode_kernel(
     __syncwarp();
     float m[1], l[1], o[1][DPL];
     attend_block<1, DPL>(qs, kp, vp, hd, blk * kAttnBlock, start, seq, scale, owns_new ? kh : nullptr,
-                         owns_new ? vh : nullptr, pos, lane, m, l, o);
+                         owns_new ? vh : nullptr, pos, lane, m, l, o, &ahead);
     float *orow = out + (size_t)head * hd;
     if (first == last) {  // a single block: merge it into the empty state and finish
         float M = -INFINITY, L = 0.0f, O[DPL];
@@ -688,8 +734,9 @@ void launch_decode(tm_cuda_ctx *ctx, const float *q, const float *k, const float
                    uint32_t *status, uint32_t heads, uint32_t kvh, uint32_t hd, uint32_t n_rot, uint32_t cap,
                    uint32_t window, float eps, float scale, uint32_t n_seq = 1,
                    const decode_seq_strides seqs = decode_seq_strides()) {
-    tm_launch_pdl(ctx, attention_decode_kernel<DPL>, dim3(heads, (cap + kAttnBlock - 1) / kAttnBlock, n_seq), dim3(32),
-                  0, q, k, v, qn, kn, inv_freq, kc, vc, out, scratch, pos, status, heads, kvh, hd, n_rot, cap, window,
+    tm_launch_pdl(ctx, attention_decode_kernel<DPL>, 
+                  dim3(heads, (cap + kAttnBlock * kDecodeWarps - 1) / (kAttnBlock * kDecodeWarps), n_seq),
+                  dim3(32 * kDecodeWarps), 0, q, k, v, qn, kn, inv_freq, kc, vc, out, scratch, pos, status, heads, kvh, hd, n_rot, cap, window,
                   eps, scale, seqs);
 }
 

@@ -82,7 +82,14 @@ __host__ __device__ inline size_t token_smem(uint32_t cols, uint32_t plane) {
  * bit-identical between the GEMV and any batched call.
  */
 template <int M, int kSlots, int H, bool kAdd = false>
-__global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args a) {
+__global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args) {
+    gemv_args a = args;
+    if constexpr (M > 1) {  // a grid row per slice of M tokens
+        const size_t t0 = (size_t)blockIdx.y * M;
+        a.x += t0 * a.cols;
+        a.y += t0 * a.y_stride;
+        if (a.prologue == TM_CUDA_PRO_SILU_MUL || a.prologue == TM_CUDA_PRO_GELU_MUL) a.pro += t0 * a.cols;
+    }
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float red[kWarps];
     __shared__ float partial[kWarps][M][16];
@@ -479,7 +486,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args a) {
 }
 
 template <int M, int kSlots, int H, bool kAdd>
-cudaError_t launch_gemv_form(tm_cuda_ctx *ctx, const gemv_args &a, int grid, size_t smem) {
+cudaError_t launch_gemv_form(tm_cuda_ctx *ctx, const gemv_args &a, dim3 grid, size_t smem) {
     static std::atomic<bool> attr_set[64] = {};  // per device; contexts of a process share it
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
@@ -489,10 +496,10 @@ cudaError_t launch_gemv_form(tm_cuda_ctx *ctx, const gemv_args &a, int grid, siz
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    return tm_launch_pdl(ctx, q8_gemv_kernel<M, kSlots, H, kAdd>, dim3(grid), dim3(kThreads), smem, a);
+    return tm_launch_pdl(ctx, q8_gemv_kernel<M, kSlots, H, kAdd>, grid, dim3(kThreads), smem, a);
 }
 template <int M, int kSlots, int H>
-cudaError_t launch_gemv(tm_cuda_ctx *ctx, const gemv_args &a, int grid, size_t smem) {
+cudaError_t launch_gemv(tm_cuda_ctx *ctx, const gemv_args &a, dim3 grid, size_t smem) {
     if constexpr (M == 1)
         if (a.add_p) return launch_gemv_form<M, kSlots, H, true>(ctx, a, grid, smem);
     return launch_gemv_form<M, kSlots, H, false>(ctx, a, grid, smem);
@@ -515,9 +522,9 @@ uint32_t resident_ctas_per_sm(const tm_cuda_ctx *ctx, uint32_t cols, int m) {
     return (uint32_t)(fit > 4u ? 4u : fit < 1u ? 1u : fit);
 }
 
-// One launch for `m` tokens (m in {1,2,4,8}) over a.rows rows.  The column split comes from the
+// One launch for `slices` slices of `m` tokens (m in {1,2,4,8}) over a.rows rows.  The column split comes from the
 // matrix shape alone, so small projections still fill the machine.
-cudaError_t gemv_part(tm_cuda_ctx *ctx, gemv_args a, int m) {
+cudaError_t gemv_part(tm_cuda_ctx *ctx, gemv_args a, int m, uint32_t slices) {
     a.plane = digit_plane_bytes(a.cols);
     const size_t smem = (size_t)m * token_smem(a.cols, a.plane);
     const uint32_t n_tiles = (a.rows + 15u) / 16u;
@@ -538,14 +545,17 @@ cudaError_t gemv_part(tm_cuda_ctx *ctx, gemv_args a, int m) {
         // Several tokens: staging them (norm, digit split) costs a CTA far more than streaming one row
         // tile's weights, so the grid is one resident wave and every warp walks its share of the tiles
         // with the activations staged once.  (Which CTA multiplies a tile does not change its sums.)
+        // Slices of a larger batch share the wave: a 1024-row projection is 64 CTAs, and one slice after the other
+        // (15 us each on the 0.6B shape) left most of the machine without work.
         const size_t fit = (size_t)ctx->smem_optin / (smem + 1024u);
-        const uint32_t wave = (uint32_t)ctx->sm_count * (uint32_t)(fit >= 2u ? 2u : 1u);
+        uint32_t wave = (uint32_t)ctx->sm_count * (uint32_t)(fit >= 2u ? 2u : 1u) / slices;
+        if (wave < 1u) wave = 1u;
         if (ctas > wave) ctas = wave;
     }
     switch (m) {
-        case 8: return launch_gemv<8, 2, 2>(ctx, a, (int)ctas, smem);
-        case 4: return launch_gemv<4, 2, 2>(ctx, a, (int)ctas, smem);
-        case 2: return launch_gemv<2, 2, 2>(ctx, a, (int)ctas, smem);
+        case 8: return launch_gemv<8, 2, 2>(ctx, a, dim3(ctas, slices), smem);
+        case 4: return launch_gemv<4, 2, 2>(ctx, a, dim3(ctas, slices), smem);
+        case 2: return launch_gemv<2, 2, 2>(ctx, a, dim3(ctas, slices), smem);
         default:
             // Measured on the 8B-scale shapes and both lm_heads (same-box A/B): wherever a warp streams at
             // least six chunks per tile the shared-memory ring of eight chunks wins (64 registers, three
@@ -560,24 +570,24 @@ cudaError_t gemv_part(tm_cuda_ctx *ctx, gemv_args a, int m) {
                 auto ring_bytes = [&](int depth) { return base + (size_t)kWarps * (size_t)depth * 1088u; };
                 if (a.cols % 64u == 0u && ring_bytes(8) <= budget) {
                     if (ctas <= (uint32_t)ctx->sm_count && n_chunks / ks >= 24u && ring_bytes(24) <= budget)
-                        return launch_gemv<1, 0, 24>(ctx, a, (int)ctas, ring_bytes(24));
+                        return launch_gemv<1, 0, 24>(ctx, a, dim3(ctas), ring_bytes(24));
                     if (ctas <= (uint32_t)ctx->sm_count && n_chunks / ks >= 16u && ring_bytes(16) <= budget)
-                        return launch_gemv<1, 0, 16>(ctx, a, (int)ctas, ring_bytes(16));
-                    return launch_gemv<1, 0, 8>(ctx, a, (int)ctas, ring_bytes(8));
+                        return launch_gemv<1, 0, 16>(ctx, a, dim3(ctas), ring_bytes(16));
+                    return launch_gemv<1, 0, 8>(ctx, a, dim3(ctas), ring_bytes(8));
                 }
-                return launch_gemv<1, 1, 6>(ctx, a, (int)ctas, smem);
+                return launch_gemv<1, 1, 6>(ctx, a, dim3(ctas, slices), smem);
             }
-            return launch_gemv<1, 3, 2>(ctx, a, (int)ctas, smem);
+            return launch_gemv<1, 3, 2>(ctx, a, dim3(ctas, slices), smem);
     }
 }
 
-// `m` tokens over the whole matrix.  A very tall matrix whose CTAs (8 row tiles each, no column
+// `slices` slices of `m` tokens over the whole matrix.  A very tall matrix whose CTAs (8 row tiles each, no column
 // split) do not fill a whole number of resident waves would spend up to a full CTA time on a nearly
 // empty last wave (151936 rows: 4.01 waves).  Its rows are cut instead: the bulk that fills whole
 // waves keeps ks = 1, the remaining rows go to a second launch that takes its own, much wider
 // column split and slots into the SMs the bulk's last wave frees.  The cut depends on the shape
 // only, so a (row, token) result is still the same for every batch size.
-cudaError_t gemv_slice(tm_cuda_ctx *ctx, gemv_args a, int m) {
+cudaError_t gemv_slice(tm_cuda_ctx *ctx, gemv_args a, int m, uint32_t slices) {
     a.y_stride = a.rows;
     const uint32_t per_sm = resident_ctas_per_sm(ctx, a.cols, 1);  // shape only, like the column split
     const uint32_t slots = (uint32_t)ctx->sm_count * per_sm;   // resident CTAs
@@ -588,15 +598,15 @@ cudaError_t gemv_slice(tm_cuda_ctx *ctx, gemv_args a, int m) {
         const uint32_t bulk_rows = (ctas - rem) * rows_per_cta;
         gemv_args bulk = a, rest = a;
         bulk.rows = bulk.shape_rows = bulk_rows;
-        cudaError_t e = gemv_part(ctx, bulk, m);
+        cudaError_t e = gemv_part(ctx, bulk, m, slices);
         if (e != cudaSuccess) return e;
         rest.q = a.q + (size_t)bulk_rows * a.cols;
         rest.d = a.d + (size_t)bulk_rows * (a.cols / 32u);
         rest.y = a.y + bulk_rows;
         rest.rows = rest.shape_rows = a.rows - bulk_rows;
-        return gemv_part(ctx, rest, m);
+        return gemv_part(ctx, rest, m, slices);
     }
-    return gemv_part(ctx, a, m);
+    return gemv_part(ctx, a, m, slices);
 }
 
 // Whole batch in slices of 8/4/2/1 tokens that fit shared memory.
@@ -616,12 +626,13 @@ int gemv_batch(tm_cuda_ctx *ctx, gemv_args a, uint32_t batch, uint64_t *kernels,
         s.y = a.y + (size_t)done * a.rows;
         if (a.prologue == TM_CUDA_PRO_SILU_MUL || a.prologue == TM_CUDA_PRO_GELU_MUL)
             s.pro = a.pro + (size_t)done * a.cols;
-        cudaError_t e = gemv_slice(ctx, s, m);
+        const uint32_t slices = m > 1 ? (batch - done) / (uint32_t)m : 1u;
+        cudaError_t e = gemv_slice(ctx, s, m, slices);
         if (e != cudaSuccess)
             return tm_fail(err, err_cap, TM_CUDA_ERR_INTERNAL, "Q8_0 GEMV launch failed: %s",
                            cudaGetErrorString(e));
         *kernels += 1;
-        done += (uint32_t)m;
+        done += (uint32_t)m * slices;
     }
     return TM_CUDA_OK;
 }
