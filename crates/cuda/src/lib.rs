@@ -170,6 +170,7 @@ mod ffi {
         pub fn tm_cuda_qk_prep_chunk(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k: *mut TmCudaBuffer, v: *mut TmCudaBuffer, q_norm: *mut TmCudaBuffer, k_norm: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, heads: u32, kv_heads: u32, head_dim: u32, n_rot: u32, pos0: u32, cap: u32, n: u32, eps: f32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_attention_chunk_mma_supported(head_dim: u32) -> c_int;
         pub fn tm_cuda_attention_chunk_mma(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, out: *mut TmCudaBuffer, heads: u32, pos0: u32, cap: u32, head_dim: u32, group: u32, scale: f32, n: u32, window: u32, err: *mut c_char, err_cap: usize) -> c_int;
+        pub fn tm_cuda_attention_prefill(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k: *mut TmCudaBuffer, v: *mut TmCudaBuffer, q_norm: *mut TmCudaBuffer, k_norm: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, out: *mut TmCudaBuffer, heads: u32, kv_heads: u32, head_dim: u32, n_rot: u32, cap: u32, window: u32, eps: f32, scale: f32, out_f16: c_int, n_segments: u32, segments: *const u32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_attention_decode_scratch_bytes(heads: u32, kv_heads: u32, head_dim: u32, cap: u32) -> usize;
         pub fn tm_cuda_attention_decode_dev(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k: *mut TmCudaBuffer, v: *mut TmCudaBuffer, q_norm: *mut TmCudaBuffer, k_norm: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, out: *mut TmCudaBuffer, scratch: *mut TmCudaBuffer, pos_buf: *mut TmCudaBuffer, pos_index: u32, status: *mut TmCudaBuffer, heads: u32, kv_heads: u32, head_dim: u32, n_rot: u32, cap: u32, window: u32, eps: f32, scale: f32, exact: c_int, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_attention_decode_static_max_scratch() -> usize;

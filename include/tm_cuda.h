@@ -251,7 +251,7 @@ int tm_cuda_rows_indirect_f32(tm_cuda_ctx *ctx, tm_cuda_buffer *w, uint32_t rows
  *   epilogue: 0 y = Wx  | 1 y += Wx */
 enum { TM_CUDA_PRO_NONE = 0, TM_CUDA_PRO_RMSNORM = 1, TM_CUDA_PRO_SILU_MUL = 2,
        TM_CUDA_PRO_GELU_MUL = 3,
-       TM_CUDA_PRO_F16 = 4 }; /* tm_cuda_q8_0_gemm_rows: x holds binary16 values */
+       TM_CUDA_PRO_F16 = 4 }; /* tm_cuda_q8_0_gemm_rows, _gemm_mma_fused: x holds binary16 values */
 enum { TM_CUDA_EPI_STORE = 0, TM_CUDA_EPI_ADD = 1,
        TM_CUDA_EPI_SILU_MUL_F16 = 2, TM_CUDA_EPI_GELU_MUL_F16 = 3 }; /* tm_cuda_q8_0_gemm_rows */
 int tm_cuda_q8_0_gemv_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x,
@@ -468,6 +468,19 @@ int tm_cuda_attention_chunk_mma(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buf
                                 tm_cuda_buffer *v_cache, tm_cuda_buffer *out, uint32_t heads,
                                 uint32_t pos0, uint32_t cap, uint32_t head_dim, uint32_t group,
                                 float scale, uint32_t n, uint32_t window, char *err, size_t err_cap);
+
+/* tm_cuda_qk_prep_chunk and tm_cuda_attention_chunk_mma over several runs of consecutive positions, each of one
+ * sequence, in two launches: segments holds (sequence, first position, rows) per run, at most
+ * TM_CUDA_PREFILL_SEGMENTS; the runs' rows lie one after the other in q / k / v [rows][heads][head_dim] (raw
+ * projections, left as they are) and out (f32, or binary16 with out_f16: the rounding the next multiply would do).
+ * The caches hold the sequences one after the other, [sequences][kv_heads][cap][head_dim]. */
+enum { TM_CUDA_PREFILL_SEGMENTS = 64 };
+int tm_cuda_attention_prefill(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffer *k, tm_cuda_buffer *v,
+                              tm_cuda_buffer *q_norm, tm_cuda_buffer *k_norm, tm_cuda_buffer *inv_freq,
+                              tm_cuda_buffer *k_cache, tm_cuda_buffer *v_cache, tm_cuda_buffer *out, uint32_t heads,
+                              uint32_t kv_heads, uint32_t head_dim, uint32_t n_rot, uint32_t cap, uint32_t window,
+                              float eps, float scale, int out_f16, uint32_t n_segments, const uint32_t *segments,
+                              char *err, size_t err_cap);
 
 /* No counterpart: the per-token attention core with the position read from
  * device memory (u32 pos_buf[pos_index]), so one recorded decode graph serves

@@ -9,6 +9,7 @@
 #include <memory>
 #include <string>
 #include <utility>
+#include <array>
 #include <vector>
 
 #include "error.hpp"
@@ -328,6 +329,16 @@ public:
                              uint32_t n, uint32_t window) const {
         TM_CALL(tm_cuda_attention_chunk_mma, q.raw(), kc.raw(), vc.raw(), out.raw(), heads, pos0, cap, hd, group, scale,
                 n, window);
+    }
+    // `runs`: (sequence, first position, rows) of each run
+    void attention_prefill(const CudaBuffer &q, const CudaBuffer &k, const CudaBuffer &v, const CudaBuffer &qn,
+                           const CudaBuffer &kn, const CudaBuffer &inv_freq, const CudaBuffer &kc, const CudaBuffer &vc,
+                           const CudaBuffer &out, uint32_t heads, uint32_t kvh, uint32_t hd, uint32_t n_rot, uint32_t cap,
+                           uint32_t window, float eps, float scale, bool out_f16,
+                           const std::vector<std::array<uint32_t, 3>> &runs) const {
+        TM_CALL(tm_cuda_attention_prefill, q.raw(), k.raw(), v.raw(), qn.raw(), kn.raw(), inv_freq.raw(), kc.raw(),
+                vc.raw(), out.raw(), heads, kvh, hd, n_rot, cap, window, eps, scale, out_f16, (uint32_t)runs.size(),
+                runs.empty() ? nullptr : runs[0].data());
     }
     void attention_decode_dev(const CudaBuffer &q, const CudaBuffer &k, const CudaBuffer &v, const CudaBuffer &qn,
                               const CudaBuffer &kn, const CudaBuffer &inv_freq, const CudaBuffer &kc,

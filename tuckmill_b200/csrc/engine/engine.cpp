@@ -420,9 +420,11 @@ struct SlotResidual {
 
 // What the n rows of a batched pass are: n consecutive positions of sequence `seq` (a prefill chunk),
 // or -- with `pos_buf` set -- one decode row per sequence, sequence s at the device position pos_buf[s].
+// (fused form) several runs of consecutive positions, each of one sequence.
 struct RowsAre {
     size_t seq = 0;
     const CudaBuffer *pos_buf = nullptr, *status = nullptr;
+    std::vector<std::array<uint32_t, 3>> runs;  // (sequence, first position, rows); empty: one chunk
 };
 
 // Gated FFN: down(act(gate x) * up x), optional RMS norm on the output before
@@ -689,8 +691,9 @@ struct AttentionBlock {
                qkv.part_rows[1] % 128 == 0 && tm_cuda_attention_chunk_mma_supported((uint32_t)spec.head_dim);
     }
     bool fusable() const { return sh.world == 1 && fusable_rows(); }
+    // Leaves the heads' output in s.e, binary16 when `out_f16` (a prefill whose next multiply rounds it anyway).
     void prefill_fused(const CudaContext &ctx, const PrefillScratch &s, size_t n, uint32_t pos0,
-                       const CudaBuffer &pre_norm, const RowsAre &rows) const {
+                       const CudaBuffer &pre_norm, const RowsAre &rows, bool out_f16) const {
         const uint32_t nn = (uint32_t)n, heads = (uint32_t)heads_l, kv = (uint32_t)kv_l, hd = (uint32_t)spec.head_dim;
         qkv.gemm_f16(ctx, s.x, nn, {&s.a, &s.b, &s.c}, {qkv.part_rows[0], qkv.part_rows[1], qkv.part_rows[2]},
                      TM_CUDA_PRO_RMSNORM, &pre_norm, eps, TM_CUDA_EPI_STORE);
@@ -698,10 +701,10 @@ struct AttentionBlock {
             attend_batch(ctx, s.a, s.b, s.c, 0, 0, s.e, n, *rows.pos_buf, *rows.status, false);
             return;
         }
-        ctx.qk_prep_chunk(s.a, s.b, s.c, q_norm, k_norm, inv_freq, kc(rows.seq), vc(rows.seq), heads, kv, hd,
-                          (uint32_t)spec.rope_dims, pos0, (uint32_t)cap, nn, eps);
-        ctx.attention_chunk_mma(s.a, kc(rows.seq), vc(rows.seq), s.e, heads, pos0, (uint32_t)cap, hd, heads / kv,
-                                scale(), nn, (uint32_t)spec.window);
+        const std::vector<std::array<uint32_t, 3>> one{{(uint32_t)rows.seq, pos0, nn}};
+        ctx.attention_prefill(s.a, s.b, s.c, q_norm, k_norm, inv_freq, k_cache, v_cache, s.e, heads, kv, hd,
+                              (uint32_t)spec.rope_dims, (uint32_t)cap, (uint32_t)spec.window, eps, scale(), out_f16,
+                              rows.runs.empty() ? one : rows.runs);
     }
     // Chunk core over n queries at pos0.. (engine/metal.rs:1170-1233): every
     // chunk K/V row is stored before any chunk query attends.
@@ -881,17 +884,19 @@ struct Layer {
                  bool exact, const RowsAre &rows = RowsAre()) const {
         const uint32_t nn = (uint32_t)n;
         if (!exact && mixer.fusable() && ffn.fusable()) {
-            mixer.prefill_fused(ctx, s, n, pos0, pre_norm, rows);
+            // (a handful of rows of a narrow matrix keep the exact GEMV: tm_cuda_q8_0_gemm_mma)
+            const bool by_f16 = !mixer_out_norm || (nn >= 3 && (nn >= 9 || mixer.o.cols >= 2048));
+            const bool e_f16 = by_f16 && !rows.pos_buf;
+            const int pro = e_f16 ? TM_CUDA_PRO_F16 : TM_CUDA_PRO_NONE;
+            mixer.prefill_fused(ctx, s, n, pos0, pre_norm, rows, e_f16);
             if (mixer_out_norm) {
-                // (a handful of rows of a narrow matrix keep the exact GEMV: tm_cuda_q8_0_gemm_mma)
-                if (Matrix::few_rows(mixer.o, nn) && nn >= 3 && (nn >= 9 || mixer.o.cols >= 2048))
-                    mixer.o.gemm_f16(ctx, s.e, nn, {&s.proj}, {mixer.o.rows}, TM_CUDA_PRO_NONE, nullptr, 0.0f,
-                                     TM_CUDA_EPI_STORE);
+                if (by_f16)
+                    mixer.o.gemm_f16(ctx, s.e, nn, {&s.proj}, {mixer.o.rows}, pro, nullptr, 0.0f, TM_CUDA_EPI_STORE);
                 else
                     mixer.o.gemm_all(ctx, s.e, s.proj, nn, false);
                 ctx.rmsnorm_add(s.proj, mixer_out_norm, s.x, nn, (uint32_t)hidden, eps);
             } else {
-                mixer.o.gemm_f16(ctx, s.e, nn, {&s.x}, {mixer.o.rows}, TM_CUDA_PRO_NONE, nullptr, 0.0f, TM_CUDA_EPI_ADD);
+                mixer.o.gemm_f16(ctx, s.e, nn, {&s.x}, {mixer.o.rows}, pro, nullptr, 0.0f, TM_CUDA_EPI_ADD);
             }
             ffn.prefill_fused(ctx, s, n, post_norm, hidden);
             return;
@@ -900,9 +905,9 @@ struct Layer {
             // Split model, tolerance mode: q|k|v and gate|up as one fused launch each over this rank's
             // rows, attention on the rank's heads, o and down over this rank's columns (4 GEMM calls and
             // 2 exchanges per layer).
-            mixer.prefill_fused(ctx, s, n, pos0, pre_norm, rows);
+            mixer.prefill_fused(ctx, s, n, pos0, pre_norm, rows, !rows.pos_buf);
             ctx.q8_0_gemm_mma_fused(mixer.o.buf, s.e, mixer.o.rows, mixer.o.cols, nn, {&s.h}, {mixer.o.rows},
-                                    TM_CUDA_PRO_NONE, nullptr, 0.0f, TM_CUDA_EPI_STORE);
+                                    rows.pos_buf ? TM_CUDA_PRO_NONE : TM_CUDA_PRO_F16, nullptr, 0.0f, TM_CUDA_EPI_STORE);
             ctx.push_rows(s.h, s.proj, 1, (uint32_t)(n * hidden));
             ctx.reduce_ranks_add(s.proj, s.x, mixer_out_norm ? &mixer_out_norm : nullptr, mixer.sh.world, nn,
                                  (uint32_t)hidden, eps);
@@ -1396,20 +1401,25 @@ size_t EngineModel::position_of(size_t seq) const { return seq < impl_->seqs ? i
 
 void EngineModel::prefill(const uint32_t *tokens, size_t n, bool want_token) { prefill_seq(0, tokens, n, want_token); }
 
-void EngineModel::prefill_seq(size_t seq, const uint32_t *tokens, size_t n, bool want_token) {
+void EngineModel::check_prompt(size_t seq, const uint32_t *tokens, size_t n) const {
     if (seq >= impl_->seqs)
         throw TuckmillError(ErrorCode::InvalidRequest, "sequence " + std::to_string(seq) + " outside the " +
                                                            std::to_string(impl_->seqs) + " the engine holds");
-    const size_t pos_ = impl_->pos_b[seq];  // this sequence's position (shadows the member: sequence 0's)
+    const size_t pos = impl_->pos_b[seq];
     if (n == 0) throw TuckmillError(ErrorCode::InvalidRequest, "prefill of zero tokens");
-    if (pos_ + n > capacity_)
-        throw TuckmillError(ErrorCode::ContextExceedsBudget, "position " + std::to_string(pos_ + n - 1) +
+    if (pos + n > capacity_)
+        throw TuckmillError(ErrorCode::ContextExceedsBudget, "position " + std::to_string(pos + n - 1) +
                                                                  " exceeds KV capacity " + std::to_string(capacity_));
     for (size_t i = 0; i < n; ++i)
         if (tokens[i] >= graph_.vocab)
             throw TuckmillError(ErrorCode::InvalidRequest, "token id " + std::to_string(tokens[i]) +
                                                                " is outside the vocabulary (0.." +
                                                                std::to_string(graph_.vocab) + ")");
+}
+
+void EngineModel::prefill_seq(size_t seq, const uint32_t *tokens, size_t n, bool want_token) {
+    check_prompt(seq, tokens, n);
+    const size_t pos_ = impl_->pos_b[seq];  // this sequence's position (shadows the member: sequence 0's)
     Impl &I = *impl_;
     const CudaContext &c = *ctx_;
     const size_t log0 = seq * I.log_stride;  // this sequence's token log
@@ -1450,6 +1460,79 @@ void EngineModel::prefill_seq(size_t seq, const uint32_t *tokens, size_t n, bool
     }
     I.pos_b[seq] = pos_ + n;
     if (seq == 0) this->pos_ = I.pos_b[0];
+}
+
+// Whether prompts of several sequences may share a pass: the layers' fused form, which takes runs of several
+// sequences, on one rank.
+bool EngineModel::packs_prompts() const {
+    const Impl &I = *impl_;
+    bool ok = !opts_.exact && I.sh.world == 1 && I.seqs > 1 && I.embedding.type == 8 && I.head_type() == 8;
+    for (const Layer &L : I.layers) ok = ok && L.mixer.fusable() && L.ffn.fusable();
+    return ok;
+}
+
+// The prompts of all sequences, one after the other in passes of a full prefill chunk.  A pass per prompt leaves a
+// prompt of 200 tokens with multiplies that cost nearly as much as those of 512 (27 against 23 us for a 1024 x 3072
+// projection, 27 launches a layer against 8): 32 prompts of 100 to 400 tokens
+// and 64 tokens each on the 0.6B shape took 178 ms, now 129; on 8 layers of the 8B shape 107, now 73.
+// A prompt of under nine tokens whose pass multiplies in the exact form (Layer::prefill with output norms) keeps it.
+void EngineModel::prefill_packed(const std::vector<std::vector<uint32_t>> &prompts) {
+    Impl &I = *impl_;
+    const CudaContext &c = *ctx_;
+    const size_t R = prompts.size(), hidden = graph_.hidden, batch = std::min<size_t>(opts_.prefill_batch, capacity_);
+    size_t own_pass = 1;  // prompts shorter than this keep a pass of their own
+    for (const Layer &L : I.layers)
+        if (L.mixer_out_norm) own_pass = 9;
+    for (size_t s = 0; s < R; ++s) check_prompt(s, prompts[s].data(), prompts[s].size());
+    const CudaBuffer &last = I.scratch.h;  // [sequence][hidden]: the row of each prompt's last token (unused by the fused form)
+    size_t s = 0, t0 = 0;                  // the next token: t0 of prompt s
+    while (s < R) {
+        if (t0 == 0 && prompts[s].size() < own_pass) {
+            const size_t n = prompts[s].size();
+            prefill_seq(s, prompts[s].data(), n, false);
+            I.pos_b[s] -= n;  // (all positions advance together below)
+            c.copy_f32(I.scratch.x, (uint32_t)((n - 1) % batch * hidden), last, (uint32_t)(s * hidden), (uint32_t)hidden);
+            ++s;
+            continue;
+        }
+        RowsAre rows;
+        size_t n = 0;
+        std::vector<std::pair<size_t, size_t>> ends;  // (row, sequence) of the prompts that end in this pass
+        c.burst([&] {
+            while (s < R && n < batch && rows.runs.size() < TM_CUDA_PREFILL_SEGMENTS &&
+                   (t0 > 0 || prompts[s].size() >= own_pass)) {
+                const size_t k = std::min(batch - n, prompts[s].size() - t0), at = I.pos_b[s] + t0;
+                const uint32_t slot = (uint32_t)(s * I.log_stride + at);
+                I.tokens.store_u32(slot, prompts[s].data() + t0, k);
+                c.rows_indirect(I.embedding.buf, I.embedding.rows, I.embedding.cols, I.tokens, slot, (uint32_t)k,
+                                graph_.embedding_scale, I.scratch.x.view(n * hidden * 4, k * hidden * 4));
+                rows.runs.push_back({(uint32_t)s, (uint32_t)at, (uint32_t)k});
+                n += k;
+                t0 += k;
+                if (t0 == prompts[s].size()) {
+                    ends.emplace_back(n - 1, s);
+                    I.kv_rows = std::max(I.kv_rows, I.pos_b[s] + t0);
+                    ++s;
+                    t0 = 0;
+                }
+            }
+            for (const Layer &L : I.layers) L.prefill(c, I.scratch, n, 0, hidden, graph_.eps, false, rows);
+            for (const auto &e : ends)
+                c.copy_f32(I.scratch.x, (uint32_t)(e.first * hidden), last, (uint32_t)(e.second * hidden), (uint32_t)hidden);
+        });
+    }
+    c.burst([&] {
+        std::vector<uint32_t> pos(R);
+        for (size_t i = 0; i < R; ++i) pos[i] = (uint32_t)(I.pos_b[i] += prompts[i].size());
+        I.pos_buf.store_u32(0u, pos.data(), R);
+        const size_t vocab = graph_.vocab;
+        for (size_t i = 0; i < R; ++i)
+            c.q8_0_gemv_fused(I.head_buf(), last.view(i * hidden * 4, hidden * 4), I.logits.view(i * vocab * 4, vocab * 4),
+                              I.head_rows, I.head_cols(), TM_CUDA_PRO_RMSNORM, &I.final_norm, graph_.eps, TM_CUDA_EPI_STORE);
+        c.argmax_rows_dev(I.logits, (uint32_t)R, (uint32_t)vocab, I.partial, I.tokens, (uint32_t)I.log_stride, 0, I.pos_buf,
+                          (uint32_t)capacity_ + 1, &I.tokens_mirror);
+    });
+    pos_ = I.pos_b[0];
 }
 
 uint32_t EngineModel::prefill_token() { return prefill_token_of(0); }
@@ -1516,9 +1599,11 @@ std::vector<std::vector<uint32_t>> EngineModel::generate_batch(const std::vector
     const uint64_t t_start = now_ns();
     reset();
     uint64_t n_prompt = 0;
-    for (size_t s = 0; s < R; ++s) {
-        prefill_seq(s, prompts[s].data(), prompts[s].size(), true);
-        n_prompt += prompts[s].size();
+    for (const auto &p : prompts) n_prompt += p.size();
+    if (packs_prompts()) {
+        prefill_packed(prompts);
+    } else {
+        for (size_t s = 0; s < R; ++s) prefill_seq(s, prompts[s].data(), prompts[s].size(), true);
     }
     auto is_stop = [&](uint32_t t) {
         return t == 0xFFFFFFFFu || (!ignore_eos && graph_.has_eos && t == graph_.eos_token_id);

@@ -10,13 +10,15 @@
 // bit-identical form.  Attention is not the Q8_0 hot path: this kernel exists
 // because a 512-token prefill otherwise spends half its time here.
 //
-// One CTA of 4 warps serves 64 queries of one head (16 per warp) and, when the
-// head dim exceeds 128, one 128-wide half of the value dims (grid.z).
+// A CTA of 8 warps serves 64 or 128 queries of one head: a warp takes 32 of them and every second or fourth block of
+// 32 keys, and the warps that share queries add their results at the end.  When the head dim exceeds 128 a CTA makes
+// one 128-wide half of the value dims (grid.y).
 #include "tm_cuda_internal.cuh"
+#include "tm_cuda_device.cuh"
 
 namespace {
 
-constexpr int kBQ = 64, kBKV = 64, kThreads = 128;
+constexpr int kBKV = 64, kThreads = 128;  // of the decode kernel
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -53,193 +55,376 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     return *(const uint32_t *)&h;
 }
 
+// The rows of one launch: up to 64 runs of consecutive positions, each of one sequence (of one prompt's chunk there is
+// one run).  Runs lie one after the other in the row-major operands.
+struct attn_segs {
+    uint32_t n;
+    uint32_t row0[TM_CUDA_PREFILL_SEGMENTS + 1];  // first row; [n]: all rows
+    uint32_t pos0[TM_CUDA_PREFILL_SEGMENTS], seq[TM_CUDA_PREFILL_SEGMENTS];
+};
+
 struct attn_args {
-    const float *q;    // [n][heads][HD]
-    const __half *kc;  // [kv_heads][cap][HD]
+    const float *q;  // [rows][heads][HD]
+    const float *q_norm, *inv_freq;  // q_norm null: q is normed and rotated already
+    const __half *kc;  // [sequences][kv_heads][cap][HD]
     const __half *vc;
-    float *out;        // [n][heads][HD]
-    uint32_t heads, group, pos0, cap, n, window;
-    float scale_log2e;
+    void *out;  // [rows][heads][HD], f32 or binary16
+    size_t seq_stride;
+    uint32_t heads, group, cap, window, n_rot, out_f16;
+    float scale_log2e, eps;
+    attn_segs segs;
 };
 
-template <int HD>
+// RMS norm and split-half RoPE of one HD-vector by one warp; element lane + 32 r in x[r].
+template <int R>
+__device__ __forceinline__ void norm_rope_row(float (&x)[R], const float *nw, const float *inv_freq, uint32_t n_rot,
+                                              uint32_t pos, float eps, uint32_t lane) {
+    float ss = 0.0f;
+#pragma unroll
+    for (int r = 0; r < R; ++r) ss = fmaf(x[r], x[r], ss);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    const float inv = 1.0f / sqrtf(ss / (float)(32 * R) + eps);
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = x[r] * inv * nw[lane + 32u * r];
+    const uint32_t half = n_rot / 2u;
+    if (R > 1 && n_rot == 32u * R) {  // partners are R/2 registers apart in the same lane
+#pragma unroll
+        for (int r = 0; r < R / 2; ++r) {
+            float sn, cs;
+            sincosf((float)pos * inv_freq[lane + 32u * r], &sn, &cs);
+            const float a = x[r], b = x[r + R / 2];
+            x[r] = a * cs - b * sn;
+            x[r + R / 2] = a * sn + b * cs;
+        }
+        return;
+    }
+    float y[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t e = lane + 32u * r;
+        const bool first = e < half, second = e >= half && e < n_rot;
+        const uint32_t pe = first ? e + half : e - half;
+        float partner = 0.0f;
+#pragma unroll
+        for (int rr = 0; rr < R; ++rr) {
+            const float cand = __shfl_sync(0xffffffffu, x[rr], (int)(pe & 31u));
+            if ((first || second) && (uint32_t)rr == (pe >> 5)) partner = cand;
+        }
+        y[r] = x[r];
+        if (first || second) {
+            float sn, cs;
+            sincosf((float)pos * inv_freq[first ? e : e - half], &sn, &cs);
+            y[r] = first ? x[r] * cs - partner * sn : partner * sn + x[r] * cs;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = y[r];
+}
+
+// RW warps of 32 queries, 8 / RW of them to a set of queries: warp (rw, sp) takes the 32-key block sp of every round.
+//   * 32 queries a warp: an ldmatrix of keys or values serves two MMAs.  With 16 the shared-memory reads took as long
+//     as the MMAs (256 of 270 cycles for 16 queries x 64 keys on an SM);
+//   * keys split between warps: a 512-token chunk of 16 heads is 128 CTAs of 64 queries.  Four warps of 16 queries and
+//     all keys were one warp per scheduler, each alone with its chain of product, maximum, exponential, product.
+template <int HD, int RW>
 struct attn_cfg {
-    static constexpr int kDV = HD > 128 ? 128 : HD;      // value dims per CTA
-    static constexpr int kQPitch = HD * 2, kVPitch = kDV * 2;
-    static constexpr uint32_t kQBytes = kBQ * kQPitch, kKBytes = kBKV * kQPitch, kVBytes = kBKV * kVPitch;
+    static constexpr int kSP = 8 / RW, kBQ = 32 * RW, kRound = 32 * kSP;
+    static constexpr int kDV = HD > 128 ? 128 : HD;  // value dims per CTA
+    static constexpr int kQPitch = HD * 2, kVPitch = kDV * 2, kOPitch = kDV + 8;
+    static constexpr uint32_t kQBytes = kBQ * kQPitch, kKBytes = kRound * kQPitch, kVBytes = kRound * kVPitch;
     static constexpr uint32_t kStage = kKBytes + kVBytes;
-    static constexpr uint32_t kBytes = kQBytes + 2 * kStage;
+    static constexpr uint32_t kMerge = kBQ * kOPitch * 4 + 2 * kSP * kBQ * 4;  // after the loop, over the stages
+    static constexpr uint32_t kLoop = 2 * kStage > kMerge ? 2 * kStage : kMerge;
+    static constexpr uint32_t kBytes = kQBytes + kLoop;
 };
+constexpr int kChunkThreads = 256;
 
-template <int HD>
-__global__ void __launch_bounds__(kThreads) attention_chunk_mma_kernel(const attn_args a) {
-    using C = attn_cfg<HD>;
-    constexpr int DV = C::kDV;
+template <int HD, int RW>
+__global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(const __grid_constant__ attn_args a) {
+    using C = attn_cfg<HD, RW>;
+    constexpr int DV = C::kDV, SP = C::kSP, BQ = C::kBQ, KR = C::kRound;
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *sQ = smem, *sKV = smem + C::kQBytes;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t head = blockIdx.y, kvh = head / a.group;
-    const uint32_t q0 = blockIdx.x * kBQ;        // first query (chunk row) of this CTA
-    const uint32_t dv0 = blockIdx.z * DV;        // first value dim of this CTA
-    const uint32_t q_last = min(q0 + kBQ, a.n) - 1u;
+    const int rw = warp % RW, sp = warp / RW;
+    // Tiles of queries from the last one down (the last of a chunk sees the most keys), heads next to one another.
+    const uint32_t head = blockIdx.x % a.heads, kvh = head / a.group;
+    const uint32_t dv0 = blockIdx.y * DV;
+    uint32_t seg = 0, q0 = (gridDim.x - 1u - blockIdx.x) / a.heads;
+    for (; seg + 1u < a.segs.n; ++seg) {
+        const uint32_t tiles = (a.segs.row0[seg + 1] - a.segs.row0[seg] + BQ - 1) / BQ;
+        if (q0 < tiles) break;
+        q0 -= tiles;
+    }
+    q0 *= BQ;  // first query of this CTA, of the run's n at pos0
+    const uint32_t row0 = a.segs.row0[seg], n = a.segs.row0[seg + 1] - row0, pos0 = a.segs.pos0[seg];
+    const uint32_t q_last = min(q0 + BQ, n) - 1u;
     // Keys any query of the block may see: from the first query's window start to the last query's position.
-    const uint32_t seq_first = a.pos0 + q0 + 1u;
+    const uint32_t seq_first = pos0 + q0 + 1u;
     const uint32_t kv_lo = (a.window != 0u && seq_first > a.window) ? seq_first - a.window : 0u;
-    const uint32_t kv_hi = a.pos0 + q_last;  // inclusive
-    const uint32_t tile_lo = kv_lo / kBKV, tile_hi = kv_hi / kBKV;
-    const __half *kp = a.kc + (size_t)kvh * a.cap * HD, *vp = a.vc + (size_t)kvh * a.cap * HD;
+    const uint32_t kv_hi = pos0 + q_last;  // inclusive
+    const uint32_t round_lo = kv_lo / KR, round_hi = kv_hi / KR;
+    const size_t plane = (size_t)a.segs.seq[seg] * a.seq_stride + (size_t)kvh * a.cap * HD;
+    const __half *kp = a.kc + plane, *vp = a.vc + plane;
+    tmdev::pdl_wait();
+    tmdev::pdl_trigger();
 
-    auto load_tile = [&](uint32_t tile, int stage) {
-        unsigned char *sK = sKV + stage * C::kStage, *sV = sK + C::kKBytes;
-        const uint32_t j0 = tile * kBKV;
+    auto load_round = [&](uint32_t round) {
+        unsigned char *sK = sKV + (round & 1u) * C::kStage, *sV = sK + C::kKBytes;
+        const uint32_t j0 = round * KR;
         constexpr int KCH = HD / 8, VCH = DV / 8;  // 16-byte chunks per row
-        for (int i = tid; i < kBKV * KCH; i += kThreads) {
+        for (int i = tid; i < KR * KCH; i += kChunkThreads) {
             const uint32_t r = i / KCH, c = i % KCH;
             const uint32_t j = min(j0 + r, kv_hi);  // rows past the last visible key repeat it (they are masked)
             cp_async16(smem_u32(sK) + sw<C::kQPitch>(r, c), kp + (size_t)j * HD + c * 8);
         }
-        for (int i = tid; i < kBKV * VCH; i += kThreads) {
+        for (int i = tid; i < KR * VCH; i += kChunkThreads) {
             const uint32_t r = i / VCH, c = i % VCH;
             const uint32_t j = min(j0 + r, kv_hi);
             cp_async16(smem_u32(sV) + sw<C::kVPitch>(r, c), vp + (size_t)j * HD + dv0 + c * 8);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    load_round(round_lo);
 
-    load_tile(tile_lo, 0);
-    // Q: f32 -> f16 into the swizzled tile (rows past the chunk are zero).
-    for (int i = tid; i < kBQ * (HD / 8); i += kThreads) {
-        const uint32_t r = i / (HD / 8), c = i % (HD / 8);
-        uint4 w = make_uint4(0, 0, 0, 0);
-        if (q0 + r < a.n) {
-            const float *src = a.q + ((size_t)(q0 + r) * a.heads + head) * HD + c * 8;
-            const float4 f0 = *(const float4 *)src, f1 = *(const float4 *)(src + 4);
-            w = make_uint4(pack_h2(f0.x, f0.y), pack_h2(f0.z, f0.w), pack_h2(f1.x, f1.y), pack_h2(f1.z, f1.w));
+    // Q: f32 -> f16 into the swizzled tile (rows past the run are zero).
+    if (a.q_norm) {
+        constexpr int R = HD / 32;
+#pragma unroll 2
+        for (uint32_t r = warp; r < BQ; r += 8) {
+            float x[R];
+            const bool in = q0 + r < n;
+            const float *src = a.q + ((size_t)(row0 + (in ? q0 + r : q0)) * a.heads + head) * HD;
+#pragma unroll
+            for (int i = 0; i < R; ++i) x[i] = src[lane + 32 * i];
+            norm_rope_row<R>(x, a.q_norm, a.inv_freq, a.n_rot, pos0 + q0 + r, a.eps, lane);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const uint32_t e = lane + 32u * i;
+                *(__half *)(sQ + sw<C::kQPitch>(r, e >> 3) + (e & 7u) * 2u) = __float2half_rn(in ? x[i] : 0.0f);
+            }
         }
-        *(uint4 *)(sQ + sw<C::kQPitch>(r, c)) = w;
+    } else {
+        for (int i = tid; i < BQ * (HD / 8); i += kChunkThreads) {
+            const uint32_t r = i / (HD / 8), c = i % (HD / 8);
+            uint4 w = make_uint4(0, 0, 0, 0);
+            if (q0 + r < n) {
+                const float *src = a.q + ((size_t)(row0 + q0 + r) * a.heads + head) * HD + c * 8;
+                const float4 f0 = *(const float4 *)src, f1 = *(const float4 *)(src + 4);
+                w = make_uint4(pack_h2(f0.x, f0.y), pack_h2(f0.z, f0.w), pack_h2(f1.x, f1.y), pack_h2(f1.z, f1.w));
+            }
+            *(uint4 *)(sQ + sw<C::kQPitch>(r, c)) = w;
+        }
     }
 
-    float o[DV / 8][4];
+    float o[2][DV / 8][4];
 #pragma unroll
-    for (int i = 0; i < DV / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
-    // Query rows of this thread: warp*16 + g and + 8; their positions and window starts.
-    uint32_t qpos[2], qstart[2];
+    for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t qi = q0 + warp * 16 + g + 8 * h;
-        qpos[h] = a.pos0 + qi;
-        const uint32_t seq = qpos[h] + 1u;
-        qstart[h] = (a.window != 0u && seq > a.window) ? seq - a.window : 0u;
-        if (qi >= a.n) qstart[h] = 0xffffffffu;  // a row past the chunk sees nothing
-    }
+        for (int i = 0; i < DV / 8; ++i) o[mt][i][0] = o[mt][i][1] = o[mt][i][2] = o[mt][i][3] = 0.0f;
+    float m_run[2][2], l_run[2][2];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) m_run[mt][h] = -INFINITY, l_run[mt][h] = 0.0f;
+    // Query rows of this thread: rw*32 + 16 mt + 8 h + g.
+    const uint32_t w_first = pos0 + q0 + rw * 32, w_last = w_first + 31u;
+    const bool idle = q0 + rw * 32 >= n;  // every query of this warp is past the run
 
-    for (uint32_t tile = tile_lo; tile <= tile_hi; ++tile) {
-        const int stage = (int)((tile - tile_lo) & 1u);
-        if (tile < tile_hi) {
-            load_tile(tile + 1, stage ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const uint32_t sK = smem_u32(sKV + stage * C::kStage), sV = sK + C::kKBytes;
+    for (uint32_t round = round_lo; round <= round_hi; ++round) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // this round has landed, and every warp is done with the stage the next one goes to
+        if (round < round_hi) load_round(round + 1);
+        const uint32_t j0 = round * KR + sp * 32;
+        if (idle || j0 > w_last || (a.window != 0u && j0 + 31u + a.window <= w_first)) continue;  // nothing visible
+        const uint32_t sK = smem_u32(sKV + (round & 1u) * C::kStage), sV = sK + C::kKBytes;
 
-        // ---- S = Q K^T for 16 queries x 64 keys ----
-        float s[kBKV / 8][4];
+        // ---- S = Q K^T for 32 queries x 32 keys ----
+        float s[2][4][4];
 #pragma unroll
-        for (int i = 0; i < kBKV / 8; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.0f;
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[mt][i][0] = s[mt][i][1] = s[mt][i][2] = s[mt][i][3] = 0.0f;
+        const uint32_t m = lane >> 3;
 #pragma unroll
         for (int kt = 0; kt < HD / 16; ++kt) {
-            uint32_t a0, a1, a2, a3;
-            {
-                const uint32_t m = lane >> 3;
-                const uint32_t row = warp * 16 + (m & 1u) * 8 + (lane & 7), chunk = kt * 2 + (m >> 1);
-                ldsm_x4(smem_u32(sQ) + sw<C::kQPitch>(row, chunk), a0, a1, a2, a3);
+            uint32_t q[2][4];
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                const uint32_t row = rw * 32 + mt * 16 + (m & 1u) * 8 + (lane & 7), chunk = kt * 2 + (m >> 1);
+                ldsm_x4(smem_u32(sQ) + sw<C::kQPitch>(row, chunk), q[mt][0], q[mt][1], q[mt][2], q[mt][3]);
             }
 #pragma unroll
-            for (int np = 0; np < kBKV / 16; ++np) {  // two key n-tiles per ldmatrix
+            for (int np = 0; np < 2; ++np) {  // two key n-tiles per ldmatrix
                 uint32_t b0, b1, b2, b3;
-                const uint32_t m = lane >> 3;
-                const uint32_t row = np * 16 + (m >> 1) * 8 + (lane & 7), chunk = kt * 2 + (m & 1u);
+                const uint32_t row = sp * 32 + np * 16 + (m >> 1) * 8 + (lane & 7), chunk = kt * 2 + (m & 1u);
                 ldsm_x4(sK + sw<C::kQPitch>(row, chunk), b0, b1, b2, b3);
-                mma_f16(s[2 * np], a0, a1, a2, a3, b0, b1);
-                mma_f16(s[2 * np + 1], a0, a1, a2, a3, b2, b3);
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt) {
+                    mma_f16(s[mt][2 * np], q[mt][0], q[mt][1], q[mt][2], q[mt][3], b0, b1);
+                    mma_f16(s[mt][2 * np + 1], q[mt][0], q[mt][1], q[mt][2], q[mt][3], b2, b3);
+                }
             }
         }
-        // ---- mask, running maximum, exponentials ----
-        const uint32_t j0 = tile * kBKV;
-        float mx[2] = {-INFINITY, -INFINITY};
+        // ---- mask (only blocks that the diagonal or the window's edge cuts), running maximum, exponentials ----
+        if (j0 + 31u > w_first || (a.window != 0u && j0 + a.window <= w_last)) {
 #pragma unroll
-        for (int i = 0; i < kBKV / 8; ++i)
+            for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int h = e >> 1;
-                const uint32_t j = j0 + i * 8 + 2 * t + (e & 1);
-                const bool vis = j <= qpos[h] && j >= qstart[h] && qstart[h] != 0xffffffffu;
-                s[i][e] = vis ? s[i][e] * a.scale_log2e : -INFINITY;
-                mx[h] = fmaxf(mx[h], s[i][e]);
+                for (int e = 0; e < 4; ++e) {
+                    const uint32_t qpos = w_first + mt * 16 + (e >> 1) * 8 + g;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t j = j0 + i * 8 + 2 * t + (e & 1);
+                        if (j > qpos || (a.window != 0u && j + a.window <= qpos)) s[mt][i][e] = -INFINITY;
+                    }
+                }
+        }
+        uint32_t pa[2][2][4];  // the weights as A fragments of the second product
+        bool moved = false;
+        float alpha[2][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float mx = s[mt][0][2 * h];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mx = fmaxf(mx, fmaxf(s[mt][i][2 * h], s[mt][i][2 * h + 1]));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                const float m_new = fmaxf(m_run[mt][h], mx * a.scale_log2e);
+                const float m_use = m_new == -INFINITY ? 0.0f : m_new;  // nothing visible yet: every weight is 0
+                alpha[mt][h] = exp2f(m_run[mt][h] - m_use);             // m_run = -inf gives 0
+                moved = moved || m_new != m_run[mt][h];
+                m_run[mt][h] = m_new;
+                float rs = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float p0 = exp2f(fmaf(s[mt][i][2 * h], a.scale_log2e, -m_use));
+                    const float p1 = exp2f(fmaf(s[mt][i][2 * h + 1], a.scale_log2e, -m_use));
+                    rs += p0 + p1;
+                    pa[mt][i >> 1][(i & 1) * 2 + h] = pack_h2(p0, p1);
+                }
+                l_run[mt][h] = l_run[mt][h] * alpha[mt][h] + rs;  // (this thread's keys; the quad is added at the end)
             }
-        float alpha[2], m_use[2];
+        if (__any_sync(0xffffffffu, moved)) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-            const float m_new = fmaxf(m_run[h], mx[h]);
-            m_use[h] = m_new == -INFINITY ? 0.0f : m_new;  // nothing visible yet: every weight is exp2(-inf) = 0
-            alpha[h] = exp2f(m_run[h] - m_use[h]);         // m_run = -inf gives 0
-            m_run[h] = m_new;
-        }
-        float rs[2] = {0.0f, 0.0f};
-        uint32_t pa[kBKV / 16][4];  // the weights as A fragments of the second product
+            for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-        for (int i = 0; i < kBKV / 8; ++i) {
-            const float p0 = exp2f(s[i][0] - m_use[0]), p1 = exp2f(s[i][1] - m_use[0]);
-            const float p2 = exp2f(s[i][2] - m_use[1]), p3 = exp2f(s[i][3] - m_use[1]);
-            rs[0] += p0 + p1;
-            rs[1] += p2 + p3;
-            pa[i >> 1][(i & 1) * 2] = pack_h2(p0, p1);      // rows g:   a0a1 (keys 0-7) / a4a5 (keys 8-15)
-            pa[i >> 1][(i & 1) * 2 + 1] = pack_h2(p2, p3);  // rows g+8: a2a3 / a6a7
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            rs[h] += __shfl_xor_sync(0xffffffffu, rs[h], 1);
-            rs[h] += __shfl_xor_sync(0xffffffffu, rs[h], 2);
-            l_run[h] = l_run[h] * alpha[h] + rs[h];
-        }
-#pragma unroll
-        for (int i = 0; i < DV / 8; ++i) {
-            o[i][0] *= alpha[0];
-            o[i][1] *= alpha[0];
-            o[i][2] *= alpha[1];
-            o[i][3] *= alpha[1];
+                for (int i = 0; i < DV / 8; ++i) {
+                    o[mt][i][0] *= alpha[mt][0];
+                    o[mt][i][1] *= alpha[mt][0];
+                    o[mt][i][2] *= alpha[mt][1];
+                    o[mt][i][3] *= alpha[mt][1];
+                }
         }
         // ---- O += P V ----
 #pragma unroll
-        for (int kk = 0; kk < kBKV / 16; ++kk) {
+        for (int kk = 0; kk < 2; ++kk) {
 #pragma unroll
             for (int dp = 0; dp < DV / 16; ++dp) {  // two dim n-tiles per ldmatrix
                 uint32_t b0, b1, b2, b3;
-                const uint32_t m = lane >> 3;
-                const uint32_t row = kk * 16 + (m & 1u) * 8 + (lane & 7), chunk = dp * 2 + (m >> 1);
+                const uint32_t row = sp * 32 + kk * 16 + (m & 1u) * 8 + (lane & 7), chunk = dp * 2 + (m >> 1);
                 ldsm_x4_t(sV + sw<C::kVPitch>(row, chunk), b0, b1, b2, b3);
-                mma_f16(o[2 * dp], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b0, b1);
-                mma_f16(o[2 * dp + 1], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b2, b3);
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt) {
+                    mma_f16(o[mt][2 * dp], pa[mt][kk][0], pa[mt][kk][1], pa[mt][kk][2], pa[mt][kk][3], b0, b1);
+                    mma_f16(o[mt][2 * dp + 1], pa[mt][kk][0], pa[mt][kk][1], pa[mt][kk][2], pa[mt][kk][3], b2, b3);
+                }
             }
         }
-        __syncthreads();  // the stage is refilled by the next iteration's prefetch
     }
-    // ---- normalise and store ----
+    // ---- the splits' results, brought to one maximum and added in order; normalise and store ----
+    __syncthreads();
+    float *sO = (float *)sKV, *sM = sO + BQ * C::kOPitch, *sL = sM + SP * BQ;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t qi = q0 + warp * 16 + g + 8 * h;
-        if (qi >= a.n) continue;
-        const float inv = 1.0f / l_run[h];
-        float *dst = a.out + ((size_t)qi * a.heads + head) * HD + dv0 + 2 * t;
+    for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-        for (int i = 0; i < DV / 8; ++i)
-            *(float2 *)(dst + i * 8) = make_float2(o[i][2 * h] * inv, o[i][2 * h + 1] * inv);
+        for (int h = 0; h < 2; ++h) {
+            float l = l_run[mt][h];
+            l += __shfl_xor_sync(0xffffffffu, l, 1);
+            l += __shfl_xor_sync(0xffffffffu, l, 2);
+            const int row = rw * 32 + mt * 16 + h * 8 + g;
+            if (t == 0) {
+                sM[sp * BQ + row] = m_run[mt][h];
+                sL[sp * BQ + row] = l;
+            }
+        }
+    __syncthreads();
+    float inv[2][2];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = rw * 32 + mt * 16 + h * 8 + g;
+            float mx = -INFINITY, l = 0.0f;
+#pragma unroll
+            for (int p = 0; p < SP; ++p) mx = fmaxf(mx, sM[p * BQ + row]);
+            if (mx == -INFINITY) mx = 0.0f;  // (a row past the run)
+#pragma unroll
+            for (int p = 0; p < SP; ++p) l += sL[p * BQ + row] * exp2f(sM[p * BQ + row] - mx);
+            inv[mt][h] = exp2f(m_run[mt][h] - mx) / l;
+        }
+    for (int p = 0; p < SP; ++p) {
+        if (sp == p) {
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float *dst = sO + (rw * 32 + mt * 16 + h * 8 + g) * C::kOPitch + 2 * t;
+#pragma unroll
+                    for (int i = 0; i < DV / 8; ++i) {
+                        float2 v = make_float2(o[mt][i][2 * h] * inv[mt][h], o[mt][i][2 * h + 1] * inv[mt][h]);
+                        if (p > 0) {
+                            const float2 w = *(const float2 *)(dst + i * 8);
+                            v.x += w.x;
+                            v.y += w.y;
+                        }
+                        *(float2 *)(dst + i * 8) = v;
+                    }
+                }
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < BQ * (DV / 4); i += kChunkThreads) {
+        const uint32_t r = i / (DV / 4), c = i % (DV / 4);
+        if (q0 + r >= n) break;
+        const float4 v = *(const float4 *)(sO + r * C::kOPitch + c * 4);
+        const size_t at = ((size_t)(row0 + q0 + r) * a.heads + head) * HD + dv0 + c * 4;
+        if (a.out_f16) *(uint2 *)((__half *)a.out + at) = make_uint2(pack_h2(v.x, v.y), pack_h2(v.z, v.w));
+        else *(float4 *)((float *)a.out + at) = v;
+    }
+}
+
+// The cache rows of a launch's runs: k normed, rotated and rounded, v rounded.  One warp per (row, KV head).
+template <int HD>
+__global__ void __launch_bounds__(256) kv_store_rows_kernel(const float *k, const float *v, const float *k_norm,
+                                                            const float *inv_freq, __half *kc, __half *vc, size_t seq_stride,
+                                                            uint32_t kvh, uint32_t n_rot, uint32_t cap, float eps,
+                                                            const __grid_constant__ attn_segs segs) {
+    constexpr int R = HD / 32;
+    const uint32_t lane = threadIdx.x & 31u, vec = blockIdx.x * 8u + (threadIdx.x >> 5);
+    tmdev::pdl_wait();
+    tmdev::pdl_trigger();
+    if (vec >= segs.row0[segs.n] * kvh) return;
+    const uint32_t row = vec / kvh, kh = vec % kvh;
+    uint32_t seg = 0;
+    while (seg + 1u < segs.n && row >= segs.row0[seg + 1]) ++seg;
+    const uint32_t pos = segs.pos0[seg] + row - segs.row0[seg];
+    float x[R], y[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        x[r] = k[(size_t)vec * HD + lane + 32 * r];
+        y[r] = v[(size_t)vec * HD + lane + 32 * r];
+    }
+    norm_rope_row<R>(x, k_norm, inv_freq, n_rot, pos, eps, lane);
+    const size_t dst = (size_t)segs.seq[seg] * seq_stride + ((size_t)kh * cap + pos) * HD + lane;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        kc[dst + 32 * r] = __float2half_rn(x[r]);
+        vc[dst + 32 * r] = __float2half_rn(y[r]);
     }
 }
 
@@ -622,19 +807,42 @@ cudaError_t launch_decode_mma(tm_cuda_ctx *ctx, const decode_mma_args &a, uint32
     return tm_launch_pdl(ctx, attention_decode_mma_kernel<G, HD>, grid, dim3(kThreads), kBytes, a);
 }
 
-template <int HD>
-cudaError_t launch_attn(const attn_args &a, int device, cudaStream_t stream) {
-    using C = attn_cfg<HD>;
+attn_segs attn_segments(uint32_t pos0, uint32_t n) {
+    attn_segs s;
+    s.n = 1;
+    s.row0[0] = 0;
+    s.row0[1] = n;
+    s.pos0[0] = pos0;
+    s.seq[0] = 0;
+    return s;
+}
+
+template <int HD, int RW>
+cudaError_t launch_attn_rows(tm_cuda_ctx *ctx, const attn_args &a, uint32_t tiles) {
+    using C = attn_cfg<HD, RW>;
+    const int device = ctx->device;
     static std::atomic<bool> attr_done[64] = {};  // per device; contexts of a process share it
     if (device < 0 || device >= 64 || !attr_done[device].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(attention_chunk_mma_kernel<HD>,
+        const cudaError_t e = cudaFuncSetAttribute(attention_chunk_mma_kernel<HD, RW>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kBytes);
         if (e != cudaSuccess) return e;
         if (device >= 0 && device < 64) attr_done[device].store(true, std::memory_order_release);
     }
-    const dim3 grid((a.n + kBQ - 1) / kBQ, a.heads, HD / C::kDV);
-    attention_chunk_mma_kernel<HD><<<grid, kThreads, C::kBytes, stream>>>(a);
-    return cudaGetLastError();
+    return tm_launch_pdl(ctx, attention_chunk_mma_kernel<HD, RW>, dim3(tiles * a.heads, HD / C::kDV), dim3(kChunkThreads),
+                         C::kBytes, a);
+}
+// 128 queries a CTA (half the key and value traffic from L2) where that leaves every SM two CTAs, else 64.
+template <int HD>
+cudaError_t launch_attn(tm_cuda_ctx *ctx, const attn_args &a) {
+    uint32_t t64 = 0, t128 = 0;
+    for (uint32_t i = 0; i < a.segs.n; ++i) {
+        const uint32_t n = a.segs.row0[i + 1] - a.segs.row0[i];
+        t64 += (n + 63u) / 64u;
+        t128 += (n + 127u) / 128u;
+    }
+    if ((uint64_t)t128 * a.heads * (HD / attn_cfg<HD, 4>::kDV) >= 2u * (uint64_t)ctx->sm_count)
+        return launch_attn_rows<HD, 4>(ctx, a, t128);
+    return launch_attn_rows<HD, 2>(ctx, a, t64);
 }
 
 }  // namespace
@@ -728,23 +936,100 @@ int tm_cuda_attention_chunk_mma(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buf
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "tensor-core chunk attention needs 16-byte aligned buffers");
     attn_args a;
     a.q = (const float *)q->dev;
+    a.q_norm = nullptr;  // the queries are normed and rotated already
     a.kc = (const __half *)k_cache->dev;
     a.vc = (const __half *)v_cache->dev;
-    a.out = (float *)out->dev;
+    a.out = out->dev;
+    a.out_f16 = 0;
     a.heads = heads;
     a.group = group;
-    a.pos0 = pos0;
     a.cap = cap;
-    a.n = n;
     a.window = window;
+    a.seq_stride = 0;
     a.scale_log2e = scale * 1.4426950408889634f;
+    a.segs = attn_segments(pos0, n);
     TM_OP_BEGIN("attention_chunk_mma");
-    cudaError_t e = head_dim == 32    ? launch_attn<32>(a, ctx->device, ctx->stream)
-                    : head_dim == 64  ? launch_attn<64>(a, ctx->device, ctx->stream)
-                    : head_dim == 128 ? launch_attn<128>(a, ctx->device, ctx->stream)
-                                      : launch_attn<256>(a, ctx->device, ctx->stream);
+    cudaError_t e = head_dim == 32    ? launch_attn<32>(ctx, a)
+                    : head_dim == 64  ? launch_attn<64>(ctx, a)
+                    : head_dim == 128 ? launch_attn<128>(ctx, a)
+                                      : launch_attn<256>(ctx, a);
     TM_CUDA_TRY(e);
     TM_OP_END(1);
+}
+
+int tm_cuda_attention_prefill(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffer *k, tm_cuda_buffer *v,
+                              tm_cuda_buffer *q_norm, tm_cuda_buffer *k_norm, tm_cuda_buffer *inv_freq,
+                              tm_cuda_buffer *k_cache, tm_cuda_buffer *v_cache, tm_cuda_buffer *out, uint32_t heads,
+                              uint32_t kv_heads, uint32_t head_dim, uint32_t n_rot, uint32_t cap, uint32_t window,
+                              float eps, float scale, int out_f16, uint32_t n_segments, const uint32_t *segments,
+                              char *err, size_t err_cap) {
+    TM_ENTER();
+    if (!tm_cuda_attention_chunk_mma_supported(head_dim) || heads == 0 || kv_heads == 0 || heads % kv_heads != 0 ||
+        n_rot == 0 || n_rot > head_dim || n_rot % 2 != 0 || cap == 0 || n_segments == 0 ||
+        n_segments > TM_CUDA_PREFILL_SEGMENTS || !segments)
+        return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS,
+                       "prefill attention: heads %u/%u, head_dim %u (32, 64, 128 or 256), n_rot %u, capacity %u, %u runs "
+                       "(1 .. %u)", heads, kv_heads, head_dim, n_rot, cap, n_segments, (unsigned)TM_CUDA_PREFILL_SEGMENTS);
+    attn_args a;
+    a.segs.n = n_segments;
+    uint32_t seqs = 0;
+    size_t rows = 0;
+    for (uint32_t i = 0; i < n_segments; ++i) {
+        const uint32_t *s = segments + 3 * (size_t)i;
+        if (s[2] == 0 || (size_t)s[1] + s[2] > cap || s[0] > 0xfffffffeu)
+            return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "run %u: rows %u..%zu of capacity %u", i, s[1],
+                           (size_t)s[1] + s[2], cap);
+        a.segs.row0[i] = (uint32_t)rows;
+        a.segs.seq[i] = s[0];
+        a.segs.pos0[i] = s[1];
+        rows += s[2];
+        if (s[0] >= seqs) seqs = s[0] + 1u;
+    }
+    if (rows * (heads + kv_heads) > 0x7fffffffu)
+        return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "prefill attention: %zu rows", rows);
+    a.segs.row0[n_segments] = (uint32_t)rows;
+    a.seq_stride = (size_t)kv_heads * cap * head_dim;
+    TM_CHECK_BUF(q, rows * heads * head_dim * 4, "q");
+    TM_CHECK_BUF(k, rows * kv_heads * head_dim * 4, "k");
+    TM_CHECK_BUF(v, rows * kv_heads * head_dim * 4, "v");
+    TM_CHECK_BUF(q_norm, (size_t)head_dim * 4, "q norm");
+    TM_CHECK_BUF(k_norm, (size_t)head_dim * 4, "k norm");
+    TM_CHECK_BUF(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
+    TM_CHECK_BUF(out, rows * heads * head_dim * (out_f16 ? 2 : 4), "attention output");
+    TM_CHECK_BUF(k_cache, (size_t)seqs * a.seq_stride * 2, "K cache");
+    TM_CHECK_BUF(v_cache, (size_t)seqs * a.seq_stride * 2, "V cache");
+    if (((size_t)out->dev | (size_t)k_cache->dev | (size_t)v_cache->dev) & 15u)
+        return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "prefill attention needs 16-byte aligned buffers");
+    a.q = (const float *)q->dev;
+    a.q_norm = (const float *)q_norm->dev;
+    a.inv_freq = (const float *)inv_freq->dev;
+    a.kc = (const __half *)k_cache->dev;
+    a.vc = (const __half *)v_cache->dev;
+    a.out = out->dev;
+    a.out_f16 = out_f16 ? 1u : 0u;
+    a.heads = heads;
+    a.group = heads / kv_heads;
+    a.cap = cap;
+    a.window = window;
+    a.n_rot = n_rot;
+    a.eps = eps;
+    a.scale_log2e = scale * 1.4426950408889634f;
+    TM_OP_BEGIN("attention_prefill");
+    const dim3 grid(((uint32_t)rows * kv_heads + 7u) / 8u);
+    auto store = [&](auto kernel) {
+        return tm_launch_pdl(ctx, kernel, grid, dim3(256), 0, (const float *)k->dev, (const float *)v->dev,
+                             (const float *)k_norm->dev, a.inv_freq, (__half *)k_cache->dev, (__half *)v_cache->dev,
+                             a.seq_stride, kv_heads, n_rot, cap, eps, a.segs);
+    };
+    TM_CUDA_TRY(head_dim == 32    ? store(kv_store_rows_kernel<32>)
+                : head_dim == 64  ? store(kv_store_rows_kernel<64>)
+                : head_dim == 128 ? store(kv_store_rows_kernel<128>)
+                                  : store(kv_store_rows_kernel<256>));
+    TM_CUDA_TRY(head_dim == 32    ? launch_attn<32>(ctx, a)
+                : head_dim == 64  ? launch_attn<64>(ctx, a)
+                : head_dim == 128 ? launch_attn<128>(ctx, a)
+                                  : launch_attn<256>(ctx, a));
+    TM_OP_END(2);
 }
 
 }  // extern "C"

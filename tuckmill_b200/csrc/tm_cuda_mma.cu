@@ -814,11 +814,11 @@ struct mma_push {
 
 static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, uint32_t cols, uint32_t batch,
                       float *const y[3], const uint32_t part_end[3], int accumulate, char *err, size_t err_cap,
-                      const mma_push &push = mma_push()) {
+                      const mma_push &push = mma_push(), const __half *x_f16 = nullptr) {
     encode_tiled_fn encode = get_encode_tiled();
     if (!encode)
         return tm_fail(err, err_cap, TM_CUDA_ERR_INTERNAL, "the driver does not export cuTensorMapEncodeTiled");
-    __half *xh = (__half *)ctx->mma_scratch;
+    const __half *xh = x_f16 ? x_f16 : (const __half *)ctx->mma_scratch;
     uint32_t *abort_flag = (uint32_t *)ctx->mma_abort;
     // Sub-tile width BN (a tile is 128 rows x 2*BN tokens): the one whose rounds of the persistent
     // grid cost the fewest cycles.  Fitted to measurements: a K step takes the larger of the
@@ -971,7 +971,7 @@ int tm_cuda_q8_0_gemm_mma_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buf
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "batch %u outside 1..%u", batch, TM_CUDA_GEMM_MMA_MAX_BATCH);
     if (n_parts < 1 || n_parts > 3 || !y_parts || !part_rows)
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "1 to 3 output parts, got %u", n_parts);
-    if (prologue < TM_CUDA_PRO_NONE || prologue > TM_CUDA_PRO_GELU_MUL ||
+    if (prologue < TM_CUDA_PRO_NONE || prologue > TM_CUDA_PRO_F16 ||
         (epilogue != TM_CUDA_EPI_STORE && epilogue != TM_CUDA_EPI_ADD))
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "unknown prologue %d / epilogue %d", prologue, epilogue);
     float *ys[3] = {nullptr, nullptr, nullptr};
@@ -986,15 +986,20 @@ int tm_cuda_q8_0_gemm_mma_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buf
         ends[p] = sum;
     }
     if (sum != rows) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "parts cover %u of %u rows", sum, rows);
-    TM_CHECK_BUF(x, (size_t)batch * cols * 4, "activation");
+    const bool f16 = prologue == TM_CUDA_PRO_F16;
+    TM_CHECK_BUF(x, (size_t)batch * cols * (f16 ? 2 : 4), "activation");
+    if (f16 && (((size_t)x->dev & 15u) || cols % 8u))
+        return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "binary16 activations must be 16-byte aligned rows");
     if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_BUF(pro, (size_t)cols * 4, "norm weight");
-    else if (prologue != TM_CUDA_PRO_NONE) TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate operand");
+    else if (prologue != TM_CUDA_PRO_NONE && !f16) TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate operand");
     TM_OP_BEGIN("q8_0_gemm_mma_fused");
-    TM_CUDA_TRY(tm_x_prep_launch(ctx, prologue, (const float *)x->dev, pro ? (const float *)pro->dev : nullptr, cols, batch,
-                                 eps));
-    rc = mma_launch(ctx, w, rows, cols, batch, ys, ends, epilogue == TM_CUDA_EPI_ADD, err, err_cap);
+    if (!f16)
+        TM_CUDA_TRY(tm_x_prep_launch(ctx, prologue, (const float *)x->dev, pro ? (const float *)pro->dev : nullptr, cols,
+                                     batch, eps));
+    rc = mma_launch(ctx, w, rows, cols, batch, ys, ends, epilogue == TM_CUDA_EPI_ADD, err, err_cap, mma_push(),
+                    f16 ? (const __half *)x->dev : nullptr);
     if (rc != TM_CUDA_OK) return rc;
-    TM_OP_END(2);
+    TM_OP_END(f16 ? 1 : 2);
 }
 
 int tm_cuda_q8_0_gemm_mma_push(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, tm_cuda_buffer *dst,

@@ -110,6 +110,7 @@ _OPS = {
     "q8_0_gemm_rows": [_P, _P, _P, _U32, _U32, _U32, _U32, C.POINTER(C.c_void_p), C.POINTER(C.c_uint32), _I, _P, _F, _I],
     "qk_prep_chunk": [_P] * 9 + [_U32] * 7 + [_F],
     "attention_chunk_mma": [_P, _P, _P, _P, _P, _U32, _U32, _U32, _U32, _U32, _F, _U32, _U32],
+    "attention_prefill": [_P] * 10 + [_U32] * 6 + [_F, _F, _I, _U32, C.POINTER(C.c_uint32)],
     "attention_decode_dev": [_P] * 12 + [_U32, _P] + [_U32] * 6 + [_F, _F, _I],
     "decode_attn_block": [_P, _P, _P, _U32] + [_P] * 11 + [_U32, _P, _P] + [_U32] * 6 + [_F, _F],
     "decode_ffn_block": [_P, _P, _P, _U32] + [_P] * 6 + [_U32, _U32, _I, _F],
@@ -531,6 +532,14 @@ class CudaContext:
 
     def attention_chunk_mma(self, q, k_cache, v_cache, out, heads, pos0, cap, head_dim, group, scale, n, window):
         self._call("attention_chunk_mma", q.handle, k_cache.handle, v_cache.handle, out.handle, heads, pos0, cap, head_dim, group, scale, n, window)
+
+    def attention_prefill(self, q, k, v, q_norm, k_norm, inv_freq, k_cache, v_cache, out, heads, kv_heads, head_dim,
+                          n_rot, cap, window, eps, scale, runs, out_f16=False):
+        """`runs`: (sequence, first position, rows) of each run of rows."""
+        flat = [int(u) for r in runs for u in r]
+        self._call("attention_prefill", q.handle, k.handle, v.handle, q_norm.handle, k_norm.handle, inv_freq.handle,
+                   k_cache.handle, v_cache.handle, out.handle, heads, kv_heads, head_dim, n_rot, cap, window, eps, scale,
+                   int(out_f16), len(runs), (C.c_uint32 * len(flat))(*flat))
 
     def qwen35_attention_chunk(self, q, k_cache, v_cache, out, scratch, heads, pos0, cap, head_dim, group, scale, n, window):
         self._call("qwen35_attention_f16_chunk", q.handle, k_cache.handle, v_cache.handle, out.handle, scratch.handle, heads, pos0, cap, head_dim, group, scale, n, window)
