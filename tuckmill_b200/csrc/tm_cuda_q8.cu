@@ -38,6 +38,8 @@ __device__ __forceinline__ void mma_s8(int (&d)[4], int a0, int a1, int a2, int 
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+constexpr uint32_t kPairSplit = 32;
+
 struct gemv_args {
     const signed char *q;   // [rows][cols]
     const __half *d;        // [rows][cols/32]
@@ -49,7 +51,7 @@ struct gemv_args {
     float eps;
     int prologue, epilogue;
     uint32_t plane;         // bytes between digit planes (== 64 mod 128)
-    uint32_t ks;            // column splits per row tile (1, 2, 4 or 8)
+    uint32_t ks;            // column splits per row tile (1, 2, 4, 8, or 32 = kPairSplit: see q8_gemv_cluster_kernel)
     uint32_t shape_rows;    // host only: rows of the matrix the column split is chosen for (a row view: its parent's)
     // kAdd forms only: x' = x + rmsnorm(add_p, add_w, eps) is formed first (a layer's output norm and
     // residual add, folded into the projection that consumes the result), multiplied after the prologue's
@@ -61,6 +63,54 @@ struct gemv_args {
 // Bytes of shared memory one token's staged activations take.
 __host__ __device__ inline size_t token_smem(uint32_t cols, uint32_t plane) {
     return 4u * (size_t)plane + (size_t)(cols / 32u) * 16u;
+}
+
+// Four consecutive values of a thread as digits (at `dst` of each plane; nullptr: past the row); eight adjacent lanes own
+// a 32-column block, whose four coefficients 2^(e - 7k) go to `coef`.  Whole warps call it.
+__device__ __forceinline__ void digitise_quad(const float (&v)[4], signed char *dst, uint32_t plane, float *coef, uint32_t lane) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)  // a non-finite value poisons its block (amax = inf -> NaN coefficient)
+        amax = fmaxf(amax, fabsf(v[j]) <= 3.402823466e38f ? fabsf(v[j]) : INFINITY);
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    if (!dst) return;
+    const bool bad = !(amax <= 3.402823466e38f);
+    int e = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 127 - 5;
+    e = e < -100 ? -100 : e > 122 ? 122 : e;  // blocks below 2^-94 digitise to (near) zero
+    const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    // t = v * 2^-e (|t| < 64, exact) is rounded once to a multiple of 2^-21
+    // and split into balanced base-128 digits with integer arithmetic:
+    // T = a0 2^21 + a1 2^14 + a2 2^7 + a3, a1..a3 in [-64, 63].
+    const float inv21 = inv * 2097152.0f;
+    uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        int T = __float2int_rn(v[j] * inv21);
+        const int a3 = (int)((uint32_t)T << 25) >> 25;
+        T = (T - a3) >> 7;
+        const int a2 = (int)((uint32_t)T << 25) >> 25;
+        T = (T - a2) >> 7;
+        const int a1 = (int)((uint32_t)T << 25) >> 25;
+        const int a0 = (T - a1) >> 7;
+        w0 |= ((uint32_t)a0 & 0xffu) << (8 * j);
+        w1 |= ((uint32_t)a1 & 0xffu) << (8 * j);
+        w2 |= ((uint32_t)a2 & 0xffu) << (8 * j);
+        w3 |= ((uint32_t)a3 & 0xffu) << (8 * j);
+    }
+    *(uint32_t *)dst = w0;
+    *(uint32_t *)(dst + plane) = w1;
+    *(uint32_t *)(dst + 2u * plane) = w2;
+    *(uint32_t *)(dst + 3u * plane) = w3;
+    const uint32_t k = lane & 7u;
+    if (k < 4u) {
+        const int ex = 127 + e - 7 * (int)k;  // 2^(e - 7k); below the normal range -> 0
+        float sc = ex > 0 ? __uint_as_float((uint32_t)ex << 23) : 0.0f;
+        if (amax == 0.0f) sc = 0.0f;
+        if (bad) sc = __uint_as_float(0x7fc00000u);
+        coef[k] = sc;
+    }
 }
 
 /*
@@ -81,7 +131,7 @@ __host__ __device__ inline size_t token_smem(uint32_t cols, uint32_t plane) {
  * matrix shape, never on the batch, which keeps a (row, token) result
  * bit-identical between the GEMV and any batched call.
  */
-template <int M, int kSlots, int H, bool kAdd = false>
+template <int M, int kSlots, int H, bool kAdd = false, bool kPaired = false>
 __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args) {
     gemv_args a = args;
     if constexpr (M > 1) {  // a grid row per slice of M tokens
@@ -98,7 +148,9 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t4 = lane & 3;
 
-    const uint32_t ks = a.ks, tiles_per_cta = kWarps / ks;
+    // Paired split (ks = 32): split v takes the chunk pairs v, v + 32, ...; a warp has the four splits 8 s + warp.
+    constexpr bool paired = kPaired;
+    const uint32_t ks = paired ? (uint32_t)kWarps : a.ks, tiles_per_cta = kWarps / ks;
     const uint32_t my_ks = warp % ks, my_tile = warp / ks;
     const uint32_t n_tiles = (rows + 15u) / 16u;
     const uint32_t n_chunks = (cols + kChunkCols - 1u) / kChunkCols;
@@ -124,6 +176,8 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
     unsigned short ha[U], hb[U];
     const uint32_t tile_stride = gridDim.x * tiles_per_cta;
     uint32_t ld_tile = blockIdx.x * tiles_per_cta + my_tile, ld_ch = my_ks;  // next group to request
+    uint32_t ld_sub = 0;
+    if (paired) ld_ch = warp;
     auto load_half = [&](auto half_c) {
         constexpr int half = decltype(half_c)::value;
         if (ld_tile >= n_tiles) return;
@@ -134,7 +188,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
         const unsigned short *sb = (const unsigned short *)a.d + (size_t)row_b * nb + (t4 >> 1);
 #pragma unroll
         for (int u = 0; u < H; ++u) {
-            const uint32_t ch = ld_ch + u * ks;
+            const uint32_t ch = paired ? 2u * ld_ch + u : ld_ch + u * ks;
             const bool inb = ch < n_chunks && ch * kChunkCols + t4 * 16u < cols;
             wa[half * H + u] = wb[half * H + u] = make_int4(0, 0, 0, 0);
             ha[half * H + u] = hb[half * H + u] = 0;
@@ -144,6 +198,15 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
                 ha[half * H + u] = __ldg(sa + ch * 2u);
                 hb[half * H + u] = __ldg(sb + ch * 2u);
             }
+        }
+        if (paired) {
+            ld_ch += kPairSplit;
+            if (2u * ld_ch >= n_chunks) {
+                ld_sub = (ld_sub + 1u) & 3u;
+                ld_ch = 8u * ld_sub + warp;
+                if (ld_sub == 0u) ld_tile += tile_stride;
+            }
+            return;
         }
         ld_ch += H * ks;
         if (ld_ch >= n_chunks) {
@@ -188,7 +251,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
         if constexpr (kSlots > 1) load_half(half1{});
         if constexpr (kSlots > 2) load_half(half2{});
     }
-    if (ld_tile < n_tiles) {  // the groups after those: towards L2
+    if (ld_tile < n_tiles && !paired) {  // the groups after those: towards L2
         const uint32_t row_a = min(ld_tile * 16u + g, rows - 1u), row_b = min(ld_tile * 16u + g + 8u, rows - 1u);
 #pragma unroll
         for (uint32_t j = 0; j < 4; ++j) {
@@ -294,55 +357,13 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
                 if (cb + (i * kThreads + (threadIdx.x & ~31u)) * 4u >= cols) break;
                 float v[4] = {vs[i].x, vs[i].y, vs[i].z, vs[i].w};
                 const float pw[4] = {ps[i].x, ps[i].y, ps[i].z, ps[i].w};
-                float amax = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (a.prologue == TM_CUDA_PRO_RMSNORM) v[j] = v[j] * inv_rms * pw[j];
                     else if (a.prologue == TM_CUDA_PRO_SILU_MUL) v[j] = silu_f(v[j]) * pw[j];
                     else if (a.prologue == TM_CUDA_PRO_GELU_MUL) v[j] = gelu_tanh_f(v[j]) * pw[j];
-                    // a non-finite value poisons its block (amax = inf -> NaN coefficient)
-                    amax = fmaxf(amax, fabsf(v[j]) <= 3.402823466e38f ? fabsf(v[j]) : INFINITY);
                 }
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-                if (c < cols) {
-                    const bool bad = !(amax <= 3.402823466e38f);
-                    int e = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 127 - 5;
-                    e = e < -100 ? -100 : e > 122 ? 122 : e;  // blocks below 2^-94 digitise to (near) zero
-                    const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
-                    // t = v * 2^-e (|t| < 64, exact) is rounded once to a multiple of 2^-21
-                    // and split into balanced base-128 digits with integer arithmetic:
-                    // T = a0 2^21 + a1 2^14 + a2 2^7 + a3, a1..a3 in [-64, 63].
-                    const float inv21 = inv * 2097152.0f;
-                    uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        int T = __float2int_rn(v[j] * inv21);
-                        const int a3 = (int)((uint32_t)T << 25) >> 25;
-                        T = (T - a3) >> 7;
-                        const int a2 = (int)((uint32_t)T << 25) >> 25;
-                        T = (T - a2) >> 7;
-                        const int a1 = (int)((uint32_t)T << 25) >> 25;
-                        const int a0 = (T - a1) >> 7;
-                        w0 |= ((uint32_t)a0 & 0xffu) << (8 * j);
-                        w1 |= ((uint32_t)a1 & 0xffu) << (8 * j);
-                        w2 |= ((uint32_t)a2 & 0xffu) << (8 * j);
-                        w3 |= ((uint32_t)a3 & 0xffu) << (8 * j);
-                    }
-                    *(uint32_t *)(dig + c) = w0;
-                    *(uint32_t *)(dig + plane + c) = w1;
-                    *(uint32_t *)(dig + 2u * plane + c) = w2;
-                    *(uint32_t *)(dig + 3u * plane + c) = w3;
-                    const int k = lane & 7;
-                    if (k < 4) {
-                        const int ex = 127 + e - 7 * k;  // 2^(e - 7k); below the normal range -> 0
-                        float sc = ex > 0 ? __uint_as_float((uint32_t)ex << 23) : 0.0f;
-                        if (amax == 0.0f) sc = 0.0f;
-                        if (bad) sc = __uint_as_float(0x7fc00000u);
-                        coef[(c >> 5) * 4u + k] = sc;
-                    }
-                }
+                digitise_quad(v, c < cols ? dig + c : nullptr, plane, coef + (c >> 5) * 4u, lane);
             }
         }
     }
@@ -355,7 +376,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
         constexpr int half = decltype(half_c)::value;
 #pragma unroll
         for (int u = 0; u < H; ++u) {
-            const uint32_t ch = ch0 + u * ks;
+            const uint32_t ch = paired ? 2u * ch0 + u : ch0 + u * ks;
             const uint32_t c0 = ch * kChunkCols + t4 * 16u;
             const bool inb = ch < n_chunks && c0 < cols;
             if (ch >= n_chunks) break;
@@ -390,6 +411,45 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
 #pragma unroll
         for (int m = 0; m < M; ++m) acc[m][0] = acc[m][1] = 0.0f;
 
+        if constexpr (paired) {
+            float total = 0.0f, run = 0.0f;
+#pragma unroll 1
+            for (uint32_t s = 0; s < 4u; ++s) {
+#pragma unroll
+                for (int m = 0; m < M; ++m) acc[m][0] = acc[m][1] = 0.0f;
+#pragma unroll 1
+                for (uint32_t pr = 8u * s + warp; 2u * pr < n_chunks; pr += kPairSplit) {
+                    if (cur_half == 0) multiply_half(half0{}, pr, acc);
+                    else if (cur_half == 1 || kSlots == 2) multiply_half(half1{}, pr, acc);
+                    else if constexpr (kSlots > 2) multiply_half(half2{}, pr, acc);
+                    cur_half = cur_half == (uint32_t)(kSlots - 1) ? 0u : cur_half + 1u;
+                }
+                __syncthreads();  // the previous sums' readers are done with `partial`
+#pragma unroll
+                for (int m = 0; m < M; ++m)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float v = acc[m][h];
+                        v += __shfl_xor_sync(0xffffffffu, v, 1);
+                        v += __shfl_xor_sync(0xffffffffu, v, 2);
+                        if (t4 == 0) partial[warp][m][g + 8 * h] = v;
+                    }
+                __syncthreads();
+                if (threadIdx.x < M * 16u) {
+                    // splits 0 .. 15 in order, 16 .. 31 in order, the two sums
+#pragma unroll
+                    for (int k = 0; k < kWarps; ++k) run += partial[k][threadIdx.x >> 4][threadIdx.x & 15u];
+                    if (s == 1u) total = run, run = 0.0f;
+                    if (s == 3u) total += run;
+                }
+            }
+            const uint32_t row = tile * 16u + (threadIdx.x & 15u);
+            if (threadIdx.x < M * 16u && row < rows) {
+                float *yp = a.y + (size_t)(threadIdx.x >> 4) * a.y_stride + row;
+                *yp = a.epilogue == TM_CUDA_EPI_ADD ? *yp + total : total;
+            }
+            continue;
+        }
         if constexpr (kAsync) {
             if (tile_ok) {
 #pragma unroll 1
@@ -485,29 +545,251 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
     }
 }
 
-template <int M, int kSlots, int H, bool kAdd>
+uint32_t digit_plane_bytes(uint32_t cols) {
+    const uint32_t pad = (uint32_t)tm_round_up(cols, kChunkCols);
+    return pad % 128u == 0 ? pad + 64u : pad;
+}
+
+/*
+ * One token, wide matrices (paired_split): clusters of two CTAs, one CTA on every SM, walk the row tiles; the 32 warps of
+ * a cluster share a tile's columns.  Warp w of CTA r is split v = 16 r + w and takes the pairs of chunks v, v + 32, ...:
+ * 128 contiguous bytes of each of 16 rows.  Bound by the weights' bytes, and by what comes before them:
+ *   * a grid of warps with whole row tiles is uneven (24576 x 4096: 192 CTAs of 128 rows on 296 places; 4096 x 12288:
+ *     128 CTAs).  A tile of a cluster is half a tile of work for an SM;
+ *   * a CTA stages the half of the activations its warps multiply, not all of them;
+ *   * nothing waits between tiles: a warp leaves its sums in shared memory and goes on; they are added once, at the end.
+ * Clusters of four found only 132 SMs.  Two CTAs to an SM (or room for the next launch's beside this one's) were slower
+ * in a decode step: a launch that starts while another still holds some SMs puts two of its CTAs on the others.
+ * One token, norm or activation before it, weights from HBM: 24576 x 4096 28 -> 23 us (fixed cost of a launch 4, then 5.9
+ * TB/s), 4096 x 12288 20 -> 15, 6144 x 4096 10.6 -> 8.7, 4096 x 4096 7.9 -> 7.1, 1152 x 6912 8.6 -> 6.3.
+ */
+constexpr uint32_t kClusterCtas = 2, kClusterThreads = 512, kClusterWarps = 16, kRingChunk = 1024u + 64u;
+constexpr int kRing = 4;  // chunks of a warp
+
+__host__ __device__ inline uint32_t cluster_local_cols(uint32_t cols) {  // of one CTA: half of every 4096
+    return (cols + 4095u) / 4096u * 2048u;
+}
+
+__global__ void __launch_bounds__(kClusterThreads, 2) q8_gemv_cluster_kernel(const gemv_args a, const uint32_t tiles_max) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ float red[kWarps];
+    const uint32_t cols = a.cols, rows = a.rows, nb = cols / 32u, plane = a.plane;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, t4 = lane & 3u;
+    const uint32_t rank = blockIdx.x & (kClusterCtas - 1u), cluster = blockIdx.x / kClusterCtas;
+    const uint32_t clusters = gridDim.x / kClusterCtas, n_tiles = (rows + 15u) / 16u, n_chunks = cols / kChunkCols;
+    const uint32_t v = kClusterWarps * rank + warp;
+    signed char *dig = (signed char *)smem;
+    float *coef = (float *)(smem + 4u * (size_t)plane);
+    const uint32_t staged = (uint32_t)token_smem(cluster_local_cols(cols), plane);
+    float *partial = (float *)(smem + staged);                    // [tiles_max][16 warps][16]
+    float *gather = partial + (size_t)tiles_max * kClusterWarps * 16u;  // [2 CTAs][owned tiles][16]
+    const uint32_t owned_max = (tiles_max + kClusterCtas - 1u) / kClusterCtas;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(gather + (size_t)kClusterCtas * owned_max * 16u) +
+                          warp * (kRing * kRingChunk);
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // (waited for before the first remote store)
+
+    uint32_t ld_tile = cluster, ld_ch = 2u * v;
+    auto issue = [&](uint32_t slot) {  // the warp's next chunk; an empty group past the end
+        if (ld_tile < n_tiles) {
+            const uint32_t row_a = min(ld_tile * 16u + g, rows - 1u), row_b = min(ld_tile * 16u + g + 8u, rows - 1u);
+            const uint32_t dst = ring + slot * kRingChunk;
+            const size_t col = (size_t)ld_ch * kChunkCols + t4 * 16u;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + lane * 16u),
+                         "l"(a.q + (size_t)row_a * cols + col) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512u + lane * 16u),
+                         "l"(a.q + (size_t)row_b * cols + col) : "memory");
+            if (t4 < 2u) {  // the chunk's two block scales of row g (t4 = 0) / g + 8 (t4 = 1)
+                const unsigned short *sp = (const unsigned short *)a.d + (size_t)(t4 == 0u ? row_a : row_b) * nb + ld_ch * 2u;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 1024u + (g + 8u * t4) * 4u), "l"(sp) : "memory");
+            }
+            ld_ch += ld_ch & 1u ? 2u * kPairSplit - 1u : 1u;
+            if (ld_ch >= n_chunks) {
+                ld_ch = 2u * v;
+                ld_tile += clusters;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (uint32_t i = 0; i < kRing; ++i) issue(i);
+    tmdev::pdl_trigger();
+    tmdev::pdl_wait();
+
+    // ---- stage this CTA's activations: thread (warp, lane) has columns 4 lane .. of pair 32 q + 16 rank + warp ----
+    float inv_rms = 0.0f;
+    if (a.prologue == TM_CUDA_PRO_RMSNORM) {  // the sum of squares of the 256-thread kernels
+        const bool vec = tmdev::quads_vectorizable(a.x, cols);
+        float ss = 0.0f;
+        if (tid < (uint32_t)kThreads)
+            for (uint32_t q = tid; q < cols / 4u; q += kThreads) ss = tmdev::sumsq_quad(ss, tmdev::load_quad(a.x, cols, q, vec));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0u && warp < (uint32_t)kWarps) red[warp] = ss;
+        __syncthreads();
+        float sum = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) sum += red[w];
+        inv_rms = 1.0f / sqrtf(sum / (float)cols + a.eps);
+    }
+    const bool vec_ok = (((size_t)a.x | (size_t)a.pro) & 15u) == 0;
+    const bool has_pro = a.prologue != TM_CUDA_PRO_NONE;
+    const uint32_t segs = (cols + 4095u) / 4096u;
+#pragma unroll 4
+    for (uint32_t q = 0; q < segs; ++q) {
+        const uint32_t c = (kPairSplit * q + v) * 128u + lane * 4u, lc = q * 2048u + tid * 4u;
+        if (c - lane * 4u >= cols) break;  // (whole pairs of warps: cols may end with half a pair, whose lanes stay as zeros)
+        float x[4] = {0.f, 0.f, 0.f, 0.f}, pw[4] = {1.f, 1.f, 1.f, 1.f};
+        if (c < cols) {
+            if (vec_ok) {
+                *(float4 *)x = *(const float4 *)(a.x + c);
+                if (has_pro) *(float4 *)pw = *(const float4 *)(a.pro + c);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    x[j] = a.x[c + j];
+                    if (has_pro) pw[j] = a.pro[c + j];
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (a.prologue == TM_CUDA_PRO_RMSNORM) x[j] = x[j] * inv_rms * pw[j];
+            else if (a.prologue == TM_CUDA_PRO_SILU_MUL) x[j] = silu_f(x[j]) * pw[j];
+            else if (a.prologue == TM_CUDA_PRO_GELU_MUL) x[j] = gelu_tanh_f(x[j]) * pw[j];
+        }
+        digitise_quad(x, dig + lc, plane, coef + (lc >> 5) * 4u, lane);
+    }
+    __syncthreads();
+
+    const bool b_live = (t4 >> 1) == (g >> 2);
+    uint32_t slot = 0;
+    uint32_t tl = 0;
+#pragma unroll 1
+    for (uint32_t tile = cluster; tile < n_tiles; tile += clusters, ++tl) {
+        float acc_a = 0.0f, acc_b = 0.0f;
+        uint32_t lc = warp * 128u + t4 * 16u;
+#pragma unroll 1
+        for (uint32_t ch = 2u * v; ch < n_chunks;) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
+            __syncwarp();  // the scale pairs were copied by other lanes
+            const uint32_t src = ring + slot * kRingChunk;
+            int4 qa, qb;
+            unsigned short sa16, sb16;
+            asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(qa.x), "=r"(qa.y), "=r"(qa.z), "=r"(qa.w) : "r"(src + lane * 16u));
+            asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(qb.x), "=r"(qb.y), "=r"(qb.z), "=r"(qb.w) : "r"(src + 512u + lane * 16u));
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sa16) : "r"(src + 1024u + g * 4u + (t4 >> 1) * 2u));
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb16) : "r"(src + 1024u + (g + 8u) * 4u + (t4 >> 1) * 2u));
+            __syncwarp();  // every lane has read the slot before it is refilled
+            issue(slot);
+            slot = (slot + 1u) % kRing;
+            int4 bx = make_int4(0, 0, 0, 0);
+            if (b_live) bx = *(const int4 *)(dig + (size_t)(g & 3u) * plane + lc);
+            int dd[4] = {0, 0, 0, 0};
+            mma_s8(dd, qa.x, qb.x, qa.y, qb.y, bx.x, bx.y);
+            mma_s8(dd, qa.z, qb.z, qa.w, qb.w, bx.z, bx.w);
+            const float2 cx = *(const float2 *)(coef + (lc >> 5) * 4u + 2u * (t4 & 1u));
+            const float va = fmaf((float)dd[1], cx.y, (float)dd[0] * cx.x);
+            const float vb = fmaf((float)dd[3], cx.y, (float)dd[2] * cx.x);
+            acc_a = fmaf(__half2float(__ushort_as_half(sa16)), va, acc_a);
+            acc_b = fmaf(__half2float(__ushort_as_half(sb16)), vb, acc_b);
+            lc += ch & 1u ? 2048u - 64u : 64u;
+            ch += ch & 1u ? 2u * kPairSplit - 1u : 1u;
+        }
+        acc_a += __shfl_xor_sync(0xffffffffu, acc_a, 1);
+        acc_a += __shfl_xor_sync(0xffffffffu, acc_a, 2);
+        acc_b += __shfl_xor_sync(0xffffffffu, acc_b, 1);
+        acc_b += __shfl_xor_sync(0xffffffffu, acc_b, 2);
+        if (t4 == 0u) {
+            partial[(tl * kClusterWarps + warp) * 16u + g] = acc_a;
+            partial[(tl * kClusterWarps + warp) * 16u + g + 8u] = acc_b;
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // the peers have started
+    __syncthreads();
+    // ---- this CTA's warps in order, to the CTA that owns the tile; there the two CTAs in order ----
+    const uint32_t outs = tl * 16u;
+    for (uint32_t o = tid; o < outs; o += kClusterThreads) {
+        const uint32_t t = o >> 4, r16 = o & 15u;
+        float sum = 0.0f;
+#pragma unroll
+        for (uint32_t w = 0; w < kClusterWarps; ++w) sum += partial[(t * kClusterWarps + w) * 16u + r16];
+        uint32_t dst = (uint32_t)__cvta_generic_to_shared(gather + (rank * owned_max + t / kClusterCtas) * 16u + r16);
+        asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(dst) : "r"(t % kClusterCtas));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(sum) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (uint32_t o = tid; o < (tl + kClusterCtas - 1u - rank) / kClusterCtas * 16u; o += kClusterThreads) {
+        const uint32_t t = (o >> 4) * kClusterCtas + rank, row = (cluster + t * clusters) * 16u + (o & 15u);
+        if (row >= rows) continue;
+        float sum = gather[o];
+#pragma unroll
+        for (uint32_t r = 1; r < kClusterCtas; ++r) sum += gather[r * owned_max * 16u + o];
+        a.y[row] = a.epilogue == TM_CUDA_EPI_ADD ? a.y[row] + sum : sum;
+    }
+}
+
+cudaError_t launch_cluster(tm_cuda_ctx *ctx, gemv_args a) {
+    static std::atomic<int> clusters_of[64] = {};  // per device; contexts of a process share it
+    const int dev = ctx->device;
+    int clusters = dev >= 0 && dev < 64 ? clusters_of[dev].load(std::memory_order_acquire) : 0;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kClusterCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.attrs = at;
+    if (clusters == 0) {
+        const int most = (int)ctx->smem_optin - 4096;
+        cudaError_t e = cudaFuncSetAttribute(q8_gemv_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return e;
+        cfg.gridDim = dim3((unsigned)ctx->sm_count / kClusterCtas * kClusterCtas);
+        cfg.dynamicSmemBytes = (size_t)most;  // one CTA on an SM
+        cfg.numAttrs = 1;
+        e = cudaOccupancyMaxActiveClusters(&clusters, q8_gemv_cluster_kernel, &cfg);
+        if (e != cudaSuccess) return e;
+        if (clusters < 1) return cudaErrorInvalidConfiguration;
+        if (dev >= 0 && dev < 64) clusters_of[dev].store(clusters, std::memory_order_release);
+    }
+    const uint32_t n_tiles = (a.rows + 15u) / 16u, local = cluster_local_cols(a.cols);
+    a.plane = digit_plane_bytes(local);
+    a.ks = kPairSplit;
+    const uint32_t used = n_tiles < (uint32_t)clusters ? n_tiles : (uint32_t)clusters;
+    const uint32_t tiles_max = (n_tiles + used - 1u) / used, owned = (tiles_max + kClusterCtas - 1u) / kClusterCtas;
+    const size_t smem = token_smem(local, a.plane) + (size_t)tiles_max * kClusterWarps * 64u + (size_t)kClusterCtas * owned * 64u +
+                        (size_t)kClusterWarps * kRing * kRingChunk;
+    cfg.gridDim = dim3(used * kClusterCtas);
+    cfg.dynamicSmemBytes = smem < 120u * 1024u ? 120u * 1024u : smem;  // one CTA on an SM
+    cfg.stream = ctx->stream;
+    cfg.numAttrs = ctx->pdl ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, q8_gemv_cluster_kernel, a, tiles_max);
+}
+
+template <int M, int kSlots, int H, bool kAdd, bool kPaired>
 cudaError_t launch_gemv_form(tm_cuda_ctx *ctx, const gemv_args &a, dim3 grid, size_t smem) {
     static std::atomic<bool> attr_set[64] = {};  // per device; contexts of a process share it
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(q8_gemv_kernel<M, kSlots, H, kAdd>,
+        cudaError_t e = cudaFuncSetAttribute(q8_gemv_kernel<M, kSlots, H, kAdd, kPaired>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)ctx->smem_optin - 8192);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    return tm_launch_pdl(ctx, q8_gemv_kernel<M, kSlots, H, kAdd>, grid, dim3(kThreads), smem, a);
+    return tm_launch_pdl(ctx, q8_gemv_kernel<M, kSlots, H, kAdd, kPaired>, grid, dim3(kThreads), smem, a);
 }
 template <int M, int kSlots, int H>
 cudaError_t launch_gemv(tm_cuda_ctx *ctx, const gemv_args &a, dim3 grid, size_t smem) {
+    if constexpr (H == 2 && kSlots == (M == 1 ? 3 : 2))
+        if (a.ks == kPairSplit)  // (one token without an add is q8_gemv_cluster_kernel's)
+            return launch_gemv_form<M, kSlots, H, M == 1, true>(ctx, a, grid, smem);
     if constexpr (M == 1)
-        if (a.add_p) return launch_gemv_form<M, kSlots, H, true>(ctx, a, grid, smem);
-    return launch_gemv_form<M, kSlots, H, false>(ctx, a, grid, smem);
-}
-
-uint32_t digit_plane_bytes(uint32_t cols) {
-    const uint32_t pad = (uint32_t)tm_round_up(cols, kChunkCols);
-    return pad % 128u == 0 ? pad + 64u : pad;
+        if (a.add_p) return launch_gemv_form<M, kSlots, H, true, false>(ctx, a, grid, smem);
+    return launch_gemv_form<M, kSlots, H, false, false>(ctx, a, grid, smem);
 }
 
 // Resident CTAs per SM of the form the launcher picks for long column ranges: the register forms
@@ -521,6 +803,10 @@ uint32_t resident_ctas_per_sm(const tm_cuda_ctx *ctx, uint32_t cols, int m) {
     const size_t fit = (228u * 1024u) / cta;
     return (uint32_t)(fit > 4u ? 4u : fit < 1u ? 1u : fit);
 }
+
+// Matrices whose column split is that of q8_gemv_cluster_kernel: from 4096 columns on each of its 32 warps has a pair
+// of chunks of every tile; the partial sums of its tiles (512 bytes each) have to fit beside the ring.
+bool paired_split(uint32_t rows, uint32_t cols) { return cols >= 4096u && cols % 64u == 0u && rows <= 32768u; }
 
 // One launch for `slices` slices of `m` tokens (m in {1,2,4,8}) over a.rows rows.  The column split comes from the
 // matrix shape alone, so small projections still fill the machine.
@@ -536,9 +822,11 @@ cudaError_t gemv_part(tm_cuda_ctx *ctx, gemv_args a, int m, uint32_t slices) {
     // in the same order whether the whole matrix or a part of it is multiplied.
     const uint32_t shape_tiles = ((a.shape_rows ? a.shape_rows : a.rows) + 15u) / 16u;
     uint32_t ks = 1;
-    while (ks < (uint32_t)kWarps && shape_tiles * ks * 2u <= want && ks * 2u <= n_chunks) ks <<= 1;
-    a.ks = ks;
-    const uint32_t tiles_per_cta = kWarps / ks;
+    const bool paired = paired_split(a.shape_rows ? a.shape_rows : a.rows, a.cols);
+    if (paired && m == 1 && !a.add_p) return launch_cluster(ctx, a);
+    while (!paired && ks < (uint32_t)kWarps && shape_tiles * ks * 2u <= want && ks * 2u <= n_chunks) ks <<= 1;
+    a.ks = paired ? kPairSplit : ks;
+    const uint32_t tiles_per_cta = paired ? 1u : kWarps / ks;
     uint32_t ctas = (n_tiles + tiles_per_cta - 1u) / tiles_per_cta;
     if (ctas > 1u << 20) ctas = 1u << 20;  // the kernel strides over any remainder
     if (m > 1) {
@@ -562,17 +850,10 @@ cudaError_t gemv_part(tm_cuda_ctx *ctx, gemv_args a, int m, uint32_t slices) {
             // CTAs per SM, 192 KB of loads in flight per SM); it needs whole 64-column chunks, otherwise
             // one register slot of six chunks is next best; short column ranges do best with three
             // slots of two.
-            if (n_chunks / ks >= 6u) {
-                // Ring depth: 8 chunks per warp leaves room for three CTAs per SM; a grid that puts at
-                // most one CTA on an SM anyway (the mid-size projections) takes the deepest ring that
-                // fits instead, so that its few warps still keep enough bytes in flight.
+            if (!paired && n_chunks / ks >= 6u) {
                 const size_t base = (smem + 15u) & ~(size_t)15u, budget = ctx->smem_optin - 8192u;
                 auto ring_bytes = [&](int depth) { return base + (size_t)kWarps * (size_t)depth * 1088u; };
                 if (a.cols % 64u == 0u && ring_bytes(8) <= budget) {
-                    if (ctas <= (uint32_t)ctx->sm_count && n_chunks / ks >= 24u && ring_bytes(24) <= budget)
-                        return launch_gemv<1, 0, 24>(ctx, a, dim3(ctas), ring_bytes(24));
-                    if (ctas <= (uint32_t)ctx->sm_count && n_chunks / ks >= 16u && ring_bytes(16) <= budget)
-                        return launch_gemv<1, 0, 16>(ctx, a, dim3(ctas), ring_bytes(16));
                     return launch_gemv<1, 0, 8>(ctx, a, dim3(ctas), ring_bytes(8));
                 }
                 return launch_gemv<1, 1, 6>(ctx, a, dim3(ctas, slices), smem);
