@@ -1160,25 +1160,18 @@ std::unique_ptr<EngineModel> EngineModel::load_with(std::shared_ptr<CudaContext>
     // model allows it the step becomes one persistent kernel, else a graph of kernels.
     I.persistent = persistent_decode_applies(g, src, opts);
     {
-        // Bytes of one layer's four matrices.  Measured on this part: a decoder whose projections are
-        // 2-6 MB (17 MB per layer) gains nothing -- its launches are bound by the dependency chain, not by
-        // the DRAM round trip, and the side branch costs a microsecond per layer (827 -> 857 us per token) --
-        // while 20-40 MB layers (the 1B-class shape, 7-15 MB projections) gain 2 % with one layer ahead;
-        // wider models stream long enough per launch to be bandwidth-bound and do not fit anyway.
-        uint64_t per_layer = 0;
-        if (!I.layers.empty())
-            for (const Matrix *mx : {&I.layers[0].mixer.qkv, &I.layers[0].mixer.o, &I.layers[0].ffn.gate_up,
-                                     &I.layers[0].ffn.down})
-                per_layer += Matrix::bytes_of(mx->type, mx->rows, mx->cols);
-        size_t ahead = per_layer > (20u << 20) && per_layer <= (40u << 20) ? 1 : 0;
+        // Layers whose weights a side branch asks into L2 ahead of use: off unless TM_ENGINE_L2_AHEAD asks for it.  The
+        // multiplies ask for their own first weights before their inputs are ready, and a second reader beside them
+        // delays them: the 1B-class shape, the last that gained from a layer ahead, 81.4 ms with it for 700 + 64 tokens,
+        // 78.3 without; F16 layers 5-7 us per projection.
+        size_t ahead = 0;
         if (const char *e = std::getenv("TM_ENGINE_L2_AHEAD")) ahead = (size_t)std::max(0, std::min(8, std::atoi(e)));
         const char *fold = std::getenv("TM_ENGINE_FOLD_NORMS");
         I.ffn_blocks = !(fold && fold[0] == '1') && !opts.exact && !I.persistent && opts.shard_world == 1 && !I.layers.empty();
         for (const Layer &L : I.layers) I.ffn_blocks = I.ffn_blocks && L.ffn_block_applies(g.hidden);
         I.attn_blocks = I.ffn_blocks;
         for (const Layer &L : I.layers) I.attn_blocks = I.attn_blocks && L.attn_block_applies(g.hidden);
-        if (opts.shard_world > 1 || I.persistent || I.ffn_blocks || I.head_type() == 1) ahead = 0;  // (the blocks and the F16 kernel
-        // ask for their own weights before their inputs are ready; a second reader in between only delays them)
+        if (opts.shard_world > 1 || I.persistent || I.ffn_blocks || I.head_type() == 1) ahead = 0;
         I.l2_ahead = ahead;
         // Folding the output norms into the next projection (Layer::decode_folded) saves two launches per
         // layer and is bit-identical, but measured slower on the Gemma-3-1B shape (1344 against 1299 us per
