@@ -9,6 +9,9 @@
 // replaces met through a scratch buffer in HBM (store, fence, atomic, reload: three dependent memory trips) and
 // launched a CTA per 64 positions of CAPACITY, each reading its rows before it knew whether they exist: 16.8 MB a
 // layer at capacity 4096 and 8.9 us of the step at position 700, against 6.
+// Code that runs once per launch comes from a cold instruction cache, so it is kept short and, where it can be, done
+// before the dependency wait (rotation angles, later rows towards L2): 4 heads of 256 dims 11.5 -> 6.3 us after the
+// wait, 4 of 128 at position 2060 11.4 -> 9, 2 of 128 4.9 -> 3.5.
 #include "tm_cuda_attn_core.cuh"
 
 namespace {
@@ -42,7 +45,10 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
     __half *kp = a.kc + seq_i * a.scache + (size_t)kvh * cap * HD, *vp = a.vc + seq_i * a.scache + (size_t)kvh * cap * HD;
     const volatile uint32_t *pos_p = a.pos + seq_i;
     keys<G, HD> K;
-    K.early(kp, vp, min(*pos_p, cap - 1u), a.window, C, rank);
+    const uint32_t hint = min(*pos_p, cap - 1u);
+    K.early(kp, vp, hint, a.window, C, rank);
+    rotation<HD> rot;  // as if the position stood already
+    rot.set(a.inv_freq, hint);
     tmdev::pdl_wait();
     tmdev::pdl_trigger();
     // Warp g < G normalises and rotates query head g, warp G the new key; the loads go out with the position's.
@@ -65,8 +71,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
     }
     K.late(pos, a.window, C, rank);
     if (warp < G || (is_k && K.lo <= pos && pos < K.hi)) {
-        rotation<HD> rot;
-        rot.set(a.inv_freq, pos);
+        if (pos != hint) rot.set(a.inv_freq, pos);
         norm_rope<HD>(x, w, rot, a.eps);
 #pragma unroll
         for (int r = 0; r < EPL; ++r) {
@@ -87,34 +92,53 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
     __syncthreads();
     cluster_wait();  // every CTA of the cluster has started
     // ---- value i (head i / HD, dim i % HD) is finished by CTA i / E: push it there, and everyone the max and sum ----
-    const uint32_t E = G * HD / C;
+    const uint32_t logc = 31u - (uint32_t)__clz((int)C), E = (uint32_t)(G * HD) >> logc;  // C, E: powers of two
+    keys<G, HD>::combine(sh);
 #pragma unroll
     for (int r = 0; r < PER; ++r) {
         const uint32_t i = tid + r * kT;
-        if (i < G * HD) st_cluster(smem_addr(&recv[rank * E + i % E]), i / E, keys<G, HD>::value(sh, i));
+        if (i < G * HD) st_cluster(smem_addr(&recv[rank * E + (i & (E - 1u))]), (i << logc) / (G * HD), keys<G, HD>::value(sh, i));
     }
     for (uint32_t i = tid; i < C * G * 2u; i += kT) {
-        const uint32_t g = (i >> 1) % G, to = i / (2u * G);
-        const float2 ml = keys<G, HD>::max_sum(sh, g);
-        st_cluster(smem_addr(&recv_ml[rank][g][i & 1u]), to, (i & 1u) ? ml.y : ml.x);
+        const uint32_t g = (i >> 1) % G;
+        st_cluster(smem_addr(&recv_ml[rank][g][i & 1u]), i / (2u * G), sh.l[g][i & 1u]);
     }
     cluster_arrive();
     cluster_wait();
     // ---- C lanes per value: source s's share, added over the lanes ----
-    const uint32_t src = tid % C;
-    for (uint32_t e = tid / C; e < E; e += kT / C) {
-        const uint32_t i = rank * E + e, g = i / HD;
-        const float m = recv_ml[src][g][0];
-        float M = m;
-        for (uint32_t off = C >> 1; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
-        const float f = expf(m - M);  // a CTA without keys: exp(-inf) = 0
-        float L = f * recv_ml[src][g][1], O = f * recv[src * E + e];
-        for (uint32_t off = C >> 1; off > 0; off >>= 1) {
-            L += __shfl_xor_sync(0xffffffffu, L, off);
-            O += __shfl_xor_sync(0xffffffffu, O, off);
-        }
-        if (src == 0) a.out[seq_i * a.so + (size_t)kvh * G * HD + i] = O / L;
+    const uint32_t src = tid & (C - 1u);
+    float O[PER], L[PER], M[PER];
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+        const uint32_t e = (tid + r * kT) >> logc, g = min(rank * E + e, G * HD - 1u) / HD;
+        M[r] = recv_ml[src][g][0];
+        L[r] = recv_ml[src][g][1];
+        O[r] = e < E ? recv[src * E + e] : 0.0f;
     }
+    float top[PER];
+#pragma unroll
+    for (int r = 0; r < PER; ++r) top[r] = M[r];
+    for (uint32_t off = C >> 1; off > 0; off >>= 1)
+#pragma unroll
+        for (int r = 0; r < PER; ++r) top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], off));
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+        const float f = expf(M[r] - top[r]);  // a CTA without keys: exp(-inf) = 0
+        L[r] *= f;
+        O[r] *= f;
+    }
+    for (uint32_t off = C >> 1; off > 0; off >>= 1)
+#pragma unroll
+        for (int r = 0; r < PER; ++r) {
+            L[r] += __shfl_xor_sync(0xffffffffu, L[r], off);
+            O[r] += __shfl_xor_sync(0xffffffffu, O[r], off);
+        }
+    if (src == 0)
+#pragma unroll
+        for (int r = 0; r < PER; ++r) {
+            const uint32_t e = (tid + r * kT) >> logc;
+            if (e < E) a.out[seq_i * a.so + (size_t)kvh * G * HD + rank * E + e] = O[r] / L[r];
+        }
 }
 
 // The widest cluster this device can hold of the kernel (16 needs the non-portable size).

@@ -514,6 +514,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
     __syncthreads();
     K.attend(sh, pos, a.scale);
     __syncthreads();
+    keys<G, HD>::combine(sh);
     // ---- this CTA's (max, sum, output) to every CTA: each needs all of the head's output for its rows of o ----
     for (uint32_t i = tid; i < G * HD; i += kT) {
         const float o = keys<G, HD>::value(sh, i);
@@ -523,8 +524,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
     }
     for (uint32_t i = tid; i < kC * G * 2u; i += kT) {
         const uint32_t e = i % (2u * G);
-        const float2 ml = keys<G, HD>::max_sum(sh, e % G);
-        st_cluster(smem_addr(recv_ml + rank * 2u * G + e), i / (2u * G), e < G ? ml.x : ml.y);
+        st_cluster(smem_addr(recv_ml + rank * 2u * G + e), i / (2u * G), sh.l[e % G][e / G]);
     }
     cluster_arrive();
     cluster_wait();
