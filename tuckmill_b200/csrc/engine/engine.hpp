@@ -158,6 +158,7 @@ private:
     EngineModel() = default;
     void encode_decode_step();
     void encode_batch_step();
+    void download_logits(float *out, size_t n) const;
     void check_prompt(size_t seq, const uint32_t *tokens, size_t n) const;
     bool packs_prompts() const;
     void prefill_packed(const std::vector<std::vector<uint32_t>> &prompts);
