@@ -76,14 +76,40 @@ __global__ void __launch_bounds__(kThreads) f16_gemv_kernel(const f16_args args)
             const float ss = tmdev::block_sumsq(xm, cols, red);
             inv_rms = 1.0f / sqrtf(ss / (float)cols + a.eps);
         }
-        for (uint32_t c = threadIdx.x; c < octets * 8u; c += kThreads) {
-            float v = c < cols ? xm[c] : 0.0f;
-            if (c < cols) {
-                if (a.prologue == TM_CUDA_PRO_RMSNORM) v = v * inv_rms * a.pro[c];
-                else if (a.prologue == TM_CUDA_PRO_SILU_MUL) v = tmdev::silu_f(v) * a.pro[(size_t)m * cols + c];
-                else if (a.prologue == TM_CUDA_PRO_GELU_MUL) v = tmdev::gelu_tanh_f(v) * a.pro[(size_t)m * cols + c];
+        const float *pm = a.prologue == TM_CUDA_PRO_NONE ? nullptr : a.prologue == TM_CUDA_PRO_RMSNORM ? a.pro : a.pro + (size_t)m * cols;
+        const bool quads = (cols & 3u) == 0u && (((size_t)xm | (size_t)pm) & 15u) == 0u;
+        // A thread's 16 columns are loaded before any is computed: one column after the other, silu * up of 3072 columns
+        // took half of a 12 us call.
+        constexpr int B = 4;
+#pragma unroll 1
+        for (uint32_t cb = threadIdx.x * 4u; cb < octets * 8u; cb += kThreads * 4u * B) {
+            float v[B][4], p[B][4];
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                const uint32_t c = cb + i * kThreads * 4u;
+                if (quads && c < cols) {
+                    *(float4 *)v[i] = *(const float4 *)(xm + c);
+                    *(float4 *)p[i] = pm ? *(const float4 *)(pm + c) : make_float4(1.f, 1.f, 1.f, 1.f);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        v[i][j] = c + j < cols ? xm[c + j] : 0.0f;
+                        p[i][j] = pm && c + j < cols ? pm[c + j] : 1.0f;
+                    }
+                }
             }
-            xd[((c & 4u) ? octets * 4u : 0u) + (c >> 3) * 4u + (c & 3u)] = v;
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                const uint32_t c = cb + i * kThreads * 4u;
+                if (c >= octets * 8u) break;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (a.prologue == TM_CUDA_PRO_RMSNORM) v[i][j] = v[i][j] * inv_rms * p[i][j];
+                    else if (a.prologue == TM_CUDA_PRO_SILU_MUL) v[i][j] = tmdev::silu_f(v[i][j]) * p[i][j];
+                    else if (a.prologue == TM_CUDA_PRO_GELU_MUL) v[i][j] = tmdev::gelu_tanh_f(v[i][j]) * p[i][j];
+                }
+                *(float4 *)(xd + ((c & 4u) ? octets * 4u : 0u) + (c >> 3) * 4u) = *(const float4 *)v[i];
+            }
         }
     }
     __syncthreads();
