@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(kThreads) f16_gemv_kernel(const f16_args args)
         const float *xm = a.x + (size_t)m * cols;
         float *xd = xs + (size_t)m * octets * 8u;
         float inv_rms = 0.0f;
-        if (a.prologue == TM_CUDA_PRO_RMSNORM) {
+        const bool one_pass = octets * 8u <= kThreads * 16u;  // the norm's sum from the registers that hold the row
+        if (a.prologue == TM_CUDA_PRO_RMSNORM && !one_pass) {
             const float ss = tmdev::block_sumsq(xm, cols, red);
             inv_rms = 1.0f / sqrtf(ss / (float)cols + a.eps);
         }
@@ -82,7 +83,8 @@ __global__ void __launch_bounds__(kThreads) f16_gemv_kernel(const f16_args args)
         // took half of a 12 us call.
         constexpr int B = 4;
 #pragma unroll 1
-        for (uint32_t cb = threadIdx.x * 4u; cb < octets * 8u; cb += kThreads * 4u * B) {
+        for (uint32_t c0 = 0; c0 < octets * 8u; c0 += kThreads * 4u * B) {
+            const uint32_t cb = c0 + threadIdx.x * 4u;
             float v[B][4], p[B][4];
 #pragma unroll
             for (int i = 0; i < B; ++i) {
@@ -97,6 +99,12 @@ __global__ void __launch_bounds__(kThreads) f16_gemv_kernel(const f16_args args)
                         p[i][j] = pm && c + j < cols ? pm[c + j] : 1.0f;
                     }
                 }
+            }
+            if (a.prologue == TM_CUDA_PRO_RMSNORM && one_pass) {
+                float ss = 0.0f;
+#pragma unroll
+                for (int i = 0; i < B; ++i) ss = tmdev::sumsq_quad(ss, make_float4(v[i][0], v[i][1], v[i][2], v[i][3]));
+                inv_rms = 1.0f / sqrtf(tmdev::block_reduce_sumsq(ss, red) / (float)cols + a.eps);
             }
 #pragma unroll
             for (int i = 0; i < B; ++i) {
