@@ -1,0 +1,32 @@
+"""Split-K sums of the tcgen05 multiply taken by groups of 32 tokens: fewer groups than parts and more, a last group of one
+token, a second token tile with one group, row tiles that end inside the matrix; repeated calls leave the counters at
+zero, so the results are the same bits, and the residual form adds to them."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from tuckmill_b200 import cuda, testing as T
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,cols,batch", [(1000, 2048, 33), (1024, 3072, 65), (1024, 2048, 97), (900, 3072, 129),
+                                             (1024, 2048, 161), (2048, 4096, 257), (1024, 3072, 512)])
+def test_groups_of_a_split_sum(ctx, oracle, rows, cols, batch):
+    raw = T.q8_0_matrix(3, 1, rows, cols)
+    x = T.activations(3, 2, batch * cols).reshape(batch, cols)
+    w, xb, y = ctx.q8_0_matrix(raw, rows, cols), ctx.floats(x), ctx.buffer(batch * rows * 4)
+    runs = []
+    for _ in range(3):
+        y.zero()
+        ctx.q8_0_gemm_mma(w, xb, y, rows, cols, batch)
+        runs.append(y.download(0, batch * rows * 4, np.float32).reshape(batch, rows))
+    assert ctx.mma_last_split() > 1 and not ctx.mma_aborted()
+    np.testing.assert_array_equal(runs[1], runs[0])
+    np.testing.assert_array_equal(runs[2], runs[0])
+    some = sorted({0, 31, 32, batch // 2, batch - 1})
+    assert rel_err(runs[0][some], oracle.matmul_q8_0(raw, rows, cols, x[some])) <= 1e-3
+    base = T.activations(3, 4, batch * rows).reshape(batch, rows)
+    acc = ctx.floats(base)
+    ctx.q8_0_gemm_mma_fused(w, xb, rows, cols, batch, [acc], [rows], cuda.PRO_NONE, None, 0.0, cuda.EPI_ADD)
+    np.testing.assert_array_equal(acc.download(0, batch * rows * 4, np.float32).reshape(batch, rows), base + runs[0])

@@ -54,7 +54,8 @@ constexpr uint32_t kSpinLimit = 1u << 20;  // a healthy wait is microseconds; th
 // more (output tile, part) slots into the same bytes.  Arrival counters: 4 row quarters per output tile.
 constexpr uint32_t kSplitSlots = 148;
 constexpr uint32_t kSplitSlotFloats = 128u * 256u;
-constexpr size_t kSplitCountBytes = 4096;                   // up to 256 output tiles x 4 x u32
+constexpr uint32_t kSplitTiles = 256;                       // output tiles with arrival counters, 4 x 8 x u32 each
+constexpr size_t kSplitCountBytes = kSplitTiles * 4u * 8u * 4u;
 constexpr size_t kSplitBytes = (size_t)kSplitSlots * kSplitSlotFloats * 4 + kSplitCountBytes;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -163,6 +164,40 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[32]) { tmem_ld32(taddr, v); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// W tokens from t0 on of one row: Y[t0 + j] (+)= v[j] for the tokens below `batch`.
+template <int W>
+__device__ __forceinline__ void store_tokens(float *p, size_t stride, bool add, uint32_t t0, uint32_t batch, const float (&v)[W]) {
+    if (add) {
+        // all loads first: a load after a store to the same array cannot be hoisted by
+        // the compiler, and W dependent round trips cost more than the tile's main loop
+        float old[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) old[j] = t0 + (uint32_t)j < batch ? __ldcg(p + (size_t)j * stride) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+            if (t0 + (uint32_t)j < batch) p[(size_t)j * stride] = old[j] + v[j];
+    } else if (t0 + W <= batch) {
+#pragma unroll
+        for (int j = 0; j < W; ++j) p[(size_t)j * stride] = v[j];
+    } else {
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+            if (t0 + (uint32_t)j < batch) p[(size_t)j * stride] = v[j];
+    }
+}
+
 struct mma_args {
     const __half *d;       // [rows][cols/32] block scales
     // The rows may be cut into up to three consecutive parts (q | k | v, gate | up), each with its own
@@ -174,7 +209,7 @@ struct mma_args {
     uint32_t ksplit;       // K parts per output tile (1: none)
     float *kpart;          // [slot][token][128 rows] partial accumulators, slot = output tile * ksplit + part
     uint32_t kslot;        // floats per slot: 128 rows x the tokens of a tile (rounded up to 32)
-    uint32_t *kcount;      // [output tile][4 row quarters] arrivals (left at zero)
+    uint32_t *kcount;      // [output tile][4 row quarters][8 groups of 32 tokens] arrivals (left at zero)
     // Row split: the epilogue stores this rank's rows straight into EVERY rank's gathered
     // Y[t][rank * rows + r] (peer memory, plain stores over NVLink), so the all-gather overlaps the
     // MMAs of later tiles; the last CTA ends the exchange (tm_symm_finish).  push_world = 0: off.
@@ -422,115 +457,127 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
         for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
           const uint32_t ot = tile / ksplit, part = tile % ksplit;
           const uint32_t acc0 = (it % kAccs) * (uint32_t)kIssuers;  // this tile's accumulators
-          // Split K, pass 0: the accumulators go to this part's workspace slot; pass 1 (only the warp that
-          // arrived last for this tile's row quarter): the parts are added in order and stored.
-          for (uint32_t pass = 0; pass < (ksplit > 1u ? 2u : 1u) && ok; ++pass) {
-          if (pass == 1u) {
-              __threadfence();
-              __syncwarp();
-              uint32_t last = 0u;
-              if (lane == 0) last = atomicAdd(a.kcount + ot * 4u + quarter, 1u) == ksplit - 1u ? 1u : 0u;
-              last = __shfl_sync(0xffffffffu, last, 0);
-              if (!last) break;
-              __threadfence();
-              if (lane == 0) a.kcount[ot * 4u + quarter] = 0u;  // ready for the next launch
-          }
-          for (uint32_t sub = 0; sub < (uint32_t)L::kSubs && ok; ++sub) {
-            const uint32_t tile_row0 = (ot % row_tiles) * kBM;
-            const uint32_t rr = tile_row0 + quarter * 32u + (uint32_t)lane;
-            const uint32_t tok0 = (ot / row_tiles) * kTB + sub * BN;
-            // (selects, not indexing: the arrays are kernel parameters)
-            const bool p0 = tile_row0 < a.part_end[0], p1 = tile_row0 < a.part_end[1];
-            const uint32_t part_row0 = p0 ? 0u : p1 ? a.part_end[0] : a.part_end[1];
-            const uint32_t part_row1 = p0 ? a.part_end[0] : p1 ? a.part_end[1] : a.part_end[2];
-            const size_t stride = part_row1 - part_row0;  // rows of this part = token stride of its output
-            float *ybase = (p0 ? a.y[0] : p1 ? a.y[1] : a.y[2]) + (rr - part_row0);
-            if (pass == 0u) {
-                if (ok) ok = mbar_wait(&acc_full[acc0 + sub], (it / kAccs) & 1u, abort_s);
-                for (uint32_t i = 1; kTurns && i < (uint32_t)kIssuers; ++i)
-                    if (ok) ok = mbar_wait(&acc_full[acc0 + i], (it / kAccs) & 1u, abort_s);
-                ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads below are warp-collective
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
+          const uint32_t tile_row0 = (ot % row_tiles) * kBM, tile_tok0 = (ot / row_tiles) * kTB;
+          const uint32_t rr = tile_row0 + quarter * 32u + (uint32_t)lane;
+          // (selects, not indexing: the arrays are kernel parameters)
+          const bool p0 = tile_row0 < a.part_end[0], p1 = tile_row0 < a.part_end[1];
+          const uint32_t part_row0 = p0 ? 0u : p1 ? a.part_end[0] : a.part_end[1];
+          const uint32_t part_row1 = p0 ? a.part_end[0] : p1 ? a.part_end[1] : a.part_end[2];
+          const size_t stride = part_row1 - part_row0;  // rows of this part = token stride of its output
+          float *ybase = (p0 ? a.y[0] : p1 ? a.y[1] : a.y[2]) + (rr - part_row0);
+          auto wait_acc = [&](uint32_t sub) {
+              if (ok) ok = mbar_wait(&acc_full[acc0 + sub], (it / kAccs) & 1u, abort_s);
+              for (uint32_t i = 1; kTurns && i < (uint32_t)kIssuers; ++i)
+                  if (ok) ok = mbar_wait(&acc_full[acc0 + i], (it / kAccs) & 1u, abort_s);
+              ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads are warp-collective
+              if (ok) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          };
+          const uint32_t groups = (min((uint32_t)kTB, a.batch - tile_tok0) + 31u) / 32u;  // of 32 tokens
+          // Split K: every part leaves its groups in the workspace, from group part * groups / ksplit on, and counts
+          // itself in at each; whoever came last at a group adds its parts in order.  The parts run side
+          // by side, so with the groups taken in turns each adds about its share of the tile.  (All groups left to the
+          // last part of a tile: 16 rounds of loads at the end of it; 512 tokens by 1024 x 2048 20 us, now 14.)
+          uint32_t *count = a.kcount + (ot * 4u + quarter) * 8u;
+          constexpr int W = SETS > 2 ? 16 : 32;  // tokens at a time: what the registers of a thread hold twice
+          uint32_t mine = 0;  // groups this warp came last at
+          uint32_t c = part * groups / ksplit, waited = 0;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                const uint32_t t0 = tok0 + (uint32_t)c0;
-                if (t0 >= a.batch) break;  // uniform: the rest of the sub-tile is past the batch
-                uint32_t v[32];
-                if (pass == 1u) {
-                    // this row's 32 tokens of every part, part 0 first
-                    const size_t at = ((size_t)(sub * BN + (uint32_t)c0)) * 128u + quarter * 32u + (uint32_t)lane;
+          for (uint32_t k = 0; k < groups; ++k, c = c + 1u == groups ? 0u : c + 1u) {
+              const uint32_t sub = c * 32u / BN;
+              if (!(waited >> sub & 1u)) {
+                  wait_acc(sub);
+                  if (!ok) break;
+                  waited |= 1u << sub;
+              }
+#pragma unroll 1
+              for (uint32_t h = 0; h < 32u; h += W) {
+                  const uint32_t c0 = (c * 32u + h) % BN, t0 = tile_tok0 + c * 32u + h;
+                  uint32_t u[W];
+                  float v[W];
+                  tmem_ld(tmem_base + ((quarter * 32u) << 16) + (acc0 + sub) * BN + c0, u);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = 0u;
-                    for (uint32_t pp = 0; pp < ksplit; ++pp) {
-                        const float *src = a.kpart + (size_t)(ot * ksplit + pp) * a.kslot + at;
-                        float f[32];
+                  for (int j = 0; j < W; ++j) v[j] = __uint_as_float(u[j]);
+                  if (kTurns) {
+                      // the other issuers' accumulators, in order (a tile of fewer K steps than issuers skips some)
+                      for (uint32_t i = 1; i < (uint32_t)kIssuers; ++i) {
+                          const uint32_t g0 = it * nkb, first = (i + (uint32_t)kIssuers - g0 % kIssuers) % kIssuers;
+                          if (nkb < (uint32_t)kIssuers && first >= nkb) continue;
+                          tmem_ld(tmem_base + ((quarter * 32u) << 16) + (acc0 + i) * BN + c0, u);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) f[j] = __ldcg(src + (size_t)j * 128u);
+                          for (int j = 0; j < W; ++j) v[j] += __uint_as_float(u[j]);
+                      }
+                  }
+                  if (ksplit > 1u) {
+                      float *dst = a.kpart + (size_t)tile * a.kslot + (size_t)(c * 32u + h) * 128u + quarter * 32u + (uint32_t)lane;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(pp == 0u ? f[j] : __uint_as_float(v[j]) + f[j]);
-                    }
-                } else {
-                tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (acc0 + sub) * BN + (uint32_t)c0, v);
-                if (kTurns) {
-                    // the other issuers' accumulators, in order (a tile of fewer K steps than issuers skips some)
-                    for (uint32_t i = 1; i < (uint32_t)kIssuers; ++i) {
-                        const uint32_t g0 = it * nkb, first = (i + (uint32_t)kIssuers - g0 % kIssuers) % kIssuers;
-                        if (nkb < (uint32_t)kIssuers && first >= nkb) continue;
-                        uint32_t f[32];
-                        tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (acc0 + i) * BN + (uint32_t)c0, f);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(f[j]));
-                    }
-                }
-                }
-                if (ksplit > 1u && pass == 0u) {
-                    float *dst = a.kpart + (size_t)(ot * ksplit + part) * a.kslot +
-                                 ((size_t)(sub * BN + (uint32_t)c0)) * 128u + quarter * 32u + (uint32_t)lane;
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) dst[(size_t)j * 128u] = __uint_as_float(v[j]);
-                } else if (rr < a.rows) {
-                    // Lane = row: for a fixed token the warp writes 128 contiguous bytes; the addresses
-                    // are independent (no add chain between the stores).
-                    float *p = ybase + (size_t)t0 * stride;
-                    if (a.push_world) {
-                        const size_t wide = (size_t)a.push_world * a.rows;  // token stride of the gathered Y
-                        const size_t at = a.push_off + (size_t)t0 * wide + (size_t)a.push_rank * a.rows + rr;
-                        for (uint32_t pr = 0; pr < a.push_world; ++pr) {
-                            float *q = a.peer[pr] + at;
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (t0 + (uint32_t)j < a.batch) q[(size_t)j * wide] = __uint_as_float(v[j]);
-                        }
-                    } else if (a.accumulate) {
-                        // all 32 loads first: a load after a store to the same array cannot be hoisted by
-                        // the compiler, and 32 dependent round trips cost more than the tile's main loop
-                        float old[32];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            old[j] = t0 + (uint32_t)j < a.batch ? __ldcg(p + (size_t)j * stride) : 0.0f;
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (t0 + (uint32_t)j < a.batch) p[(size_t)j * stride] = old[j] + __uint_as_float(v[j]);
-                    } else if (t0 + 32u <= a.batch) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) p[(size_t)j * stride] = __uint_as_float(v[j]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (t0 + (uint32_t)j < a.batch) p[(size_t)j * stride] = __uint_as_float(v[j]);
-                    }
-                }
-            }
+                      for (int j = 0; j < W; ++j) dst[(size_t)j * 128u] = v[j];
+                  } else if (rr < a.rows && t0 < a.batch) {
+                      // Lane = row: for a fixed token the warp writes 128 contiguous bytes; the addresses
+                      // are independent (no add chain between the stores).
+                      if (a.push_world) {
+                          const size_t wide = (size_t)a.push_world * a.rows;  // token stride of the gathered Y
+                          const size_t at = a.push_off + (size_t)t0 * wide + (size_t)a.push_rank * a.rows + rr;
+                          for (uint32_t pr = 0; pr < a.push_world; ++pr)
+                              store_tokens<W>(a.peer[pr] + at, wide, false, t0, a.batch, v);
+                      } else {
+                          store_tokens<W>(ybase + (size_t)t0 * stride, stride, a.accumulate != 0u, t0, a.batch, v);
+                      }
+                  }
+              }
+              if (ksplit > 1u) {
+                  __threadfence();
+                  __syncwarp();
+                  uint32_t before = 0;
+                  if (lane == 0) before = atomicAdd(count + c, 1u);
+                  mine |= (before == ksplit - 1u ? 1u : 0u) << c;  // (lane 0's)
+              }
           }
-            if (!ok) break;
-            if (pass == 0u) {
-                // The accumulator may be overwritten once every warp has its values in registers.
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[it % kAccs]);
-            }
+          for (uint32_t sub = 0; sub < (uint32_t)L::kSubs && ok; ++sub)  // (a sub-tile past the batch is committed, too)
+              if (!(waited >> sub & 1u)) wait_acc(sub);
+          if (!ok) break;
+          // The accumulator may be overwritten once every warp has its values in registers.
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[it % kAccs]);
+          if (ksplit > 1u) {
+              mine = __shfl_sync(0xffffffffu, mine, 0);
+              if (mine) __threadfence();
+#pragma unroll 1
+              for (; mine; mine &= mine - 1u) {
+                  const uint32_t cc = (uint32_t)__ffs((int)mine) - 1u;
+                  if (lane == 0) count[cc] = 0u;  // ready for the next launch
+#pragma unroll 1
+                  for (uint32_t h = 0; h < 32u; h += W) {
+                      const float *src = a.kpart + (size_t)ot * ksplit * a.kslot + (size_t)(cc * 32u + h) * 128u + quarter * 32u + (uint32_t)lane;
+                      float v[W], f[W], g[W];
+#pragma unroll
+                      for (int j = 0; j < W; ++j) v[j] = __ldcg(src + (size_t)j * 128u);
+#pragma unroll
+                      for (int j = 0; j < W; ++j) f[j] = __ldcg(src + a.kslot + (size_t)j * 128u);
+#pragma unroll
+                      for (int j = 0; j < W; ++j) v[j] += f[j];
+#pragma unroll 1
+                      for (uint32_t pp = 2; pp < ksplit; pp += 2) {
+                          src += 2u * (size_t)a.kslot;
+                          const bool two = pp + 1u < ksplit;
+#pragma unroll
+                          for (int j = 0; j < W; ++j) f[j] = __ldcg(src + (size_t)j * 128u);
+                          if (two) {
+#pragma unroll
+                              for (int j = 0; j < W; ++j) g[j] = __ldcg(src + a.kslot + (size_t)j * 128u);
+                          }
+#pragma unroll
+                          for (int j = 0; j < W; ++j) v[j] += f[j];
+                          if (two) {
+#pragma unroll
+                              for (int j = 0; j < W; ++j) v[j] += g[j];
+                          }
+                      }
+                      const uint32_t t0 = tile_tok0 + cc * 32u + h;
+                      if (rr < a.rows && t0 < a.batch)
+                          store_tokens<W>(ybase + (size_t)t0 * stride, stride, a.accumulate != 0u, t0, a.batch, v);
+                  }
+              }
           }
             if (!ok) break;
         }
@@ -891,7 +938,7 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     {
         const uint32_t out_tiles = row_tiles * ((batch + 2 * bn - 1) / (2 * bn)), nkb = (cols + kBK - 1) / kBK;
         static const bool off = [] { const char *e = getenv("TM_CUDA_MMA_SPLITK"); return e && e[0] == '0'; }();
-        if (!off && push.world == 0 && bn <= 128 && cols % kBK == 0 && out_tiles * 16 <= kSplitCountBytes &&
+        if (!off && push.world == 0 && bn <= 128 && cols % kBK == 0 && out_tiles <= kSplitTiles &&
             ctx->mma_scratch_bytes >= kSplitBytes) {
             const uint64_t whole = (uint64_t)((out_tiles + sms - 1) / sms) * (nkb + 4);
             uint64_t best = whole;
