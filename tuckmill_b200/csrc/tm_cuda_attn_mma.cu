@@ -522,8 +522,8 @@ __global__ void __launch_bounds__(256) qk_prep_chunk_kernel(float *q, const floa
 // row per sequence, throughput form: when tens of sequences decode together the step reads every
 // sequence's K and V rows and is bandwidth-bound, which the latency-optimised kernel (scalar dot
 // products, two threads per key) cannot feed.  Here one CTA of 4 warps serves ONE (sequence, KV head,
-// split of `tiles` 64-key tiles): the G query heads of the group are the rows of a 16-row MMA tile,
-// K/V tiles arrive by cp.async (double-buffered), warp w owns keys 16w..16w+15 of every tile with its
+// equal run of 64-key tiles): the G query heads of the group are the rows of a 16-row MMA tile,
+// K/V tiles arrive by cp.async (a ring of two or three), warp w owns keys 16w..16w+15 of every tile with its
 // own running (max, sum, output), the four are merged through shared memory, and the splits of a
 // (sequence, KV head) by last arrival through `scratch` (no waiting).  Same mathematics as the other
 // decode kernels, f16 Q and softmax weights, base-2 exponentials: tolerance-qualified.
@@ -535,12 +535,12 @@ struct decode_mma_args {
     float *out, *scratch;
     const uint32_t *pos;
     uint32_t *status;
-    uint32_t kv_heads, cap, window, tiles, count_off;  // count_off: floats from a sequence's scratch to its counters
+    uint32_t kv_heads, cap, window, splits, count_off;  // count_off: floats from a sequence's scratch to its counters
     float eps, scale_log2e;
     size_t sq, sk, sv, so, scache, sscratch;  // element strides between sequences
 };
 
-template <int G, int HD>
+template <int G, int HD, uint32_t kDecodeStages>
 __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const decode_mma_args a) {
     constexpr int PITCH = HD * 2, EPL = HD / 32;
     constexpr uint32_t kQBytes = 16 * PITCH, kTile = kBKV * PITCH, kStage = 2 * kTile;
@@ -557,19 +557,58 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
     const float *q = a.q + sidx * a.sq, *k = a.k + sidx * a.sk, *v = a.v + sidx * a.sv;
     __half *kc = a.kc + sidx * a.scache + (size_t)kvh * a.cap * HD, *vc = a.vc + sidx * a.scache + (size_t)kvh * a.cap * HD;
     float *out = a.out + sidx * a.so, *scratch = a.scratch + sidx * a.sscratch;
+    // The tiles of a sequence at position p that this split takes: equal runs.
+    uint32_t start, last_tile, tile_lo, tile_hi, nact;
+    auto take = [&](uint32_t p) {
+        const uint32_t n = p + 1u;
+        start = (a.window != 0u && n > a.window) ? n - a.window : 0u;
+        last_tile = p / kBKV;
+        const uint32_t first_tile = start / kBKV, used = last_tile - first_tile + 1u;
+        const uint32_t per = (used + gridDim.y - 1u) / gridDim.y;
+        nact = (used + per - 1u) / per;  // splits of this (sequence, KV head) with work
+        tile_lo = first_tile + split * per;
+        tile_hi = min(tile_lo + per - 1u, last_tile);
+    };
+    // Before the wait, as if the position stood already: cached rows towards L2 (never closer: an earlier step's call
+    // may still be storing one), the rotation's angles, the padding rows of Q.
+    const uint32_t hint = min(*(const volatile uint32_t *)(a.pos + sidx), a.cap - 1u);
+    take(hint);
+    if (tile_lo <= last_tile)
+        for (uint32_t j = tile_lo * kBKV + tid / 2; j < min((tile_hi + 1u) * kBKV, hint); j += kThreads / 2)
+#pragma unroll
+            for (uint32_t c = 0; c < PITCH; c += 128u)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)((tid & 1 ? vc : kc) + (size_t)j * HD) + c));
+    float sn[EPL / 2], cs[EPL / 2];
+    auto angles = [&](uint32_t p) {
+#pragma unroll
+        for (int r = 0; r < EPL / 2; ++r) sincosf((float)p * a.inv_freq[lane + 32 * r], &sn[r], &cs[r]);
+    };
+    angles(hint);
+    for (int i = tid; i < 16 * (HD / 8); i += kThreads) *(uint4 *)(sQ + i * 16) = make_uint4(0, 0, 0, 0);
+    __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
+    float x[EPL], nw[EPL];  // warp w < G: head w; warp G: the new key
+    auto fetch = [&](int vec) {
+        const float *src = vec == G ? k + (size_t)kvh * HD : q + ((size_t)kvh * G + vec) * HD;
+        const float *wsrc = vec == G ? a.k_norm : a.q_norm;
+#pragma unroll
+        for (int r = 0; r < EPL; ++r) {
+            x[r] = src[lane + 32 * r];
+            nw[r] = wsrc[lane + 32 * r];
+        }
+    };
+    if (warp <= G) fetch(warp);  // (with the position's own trip)
     const uint32_t pos = a.pos[sidx];
     if (pos >= a.cap) {
         if (tid == 0 && split == 0 && kvh == 0) atomicOr(a.status, 1u);
         return;
     }
-    const uint32_t seq = pos + 1u, start = (a.window != 0u && seq > a.window) ? seq - a.window : 0u;
-    const uint32_t first_tile = start / kBKV, last_tile = pos / kBKV;
-    const uint32_t tile_lo = first_tile + split * a.tiles;
+    if (pos != hint) {
+        take(pos);
+        angles(pos);
+    }
     if (tile_lo > last_tile) return;
-    const uint32_t tile_hi = min(tile_lo + a.tiles - 1u, last_tile);
-    const uint32_t nact = (last_tile - first_tile) / a.tiles + 1u;  // splits of this (sequence, KV head)
     const bool owns_new = tile_hi == last_tile;
 
     auto load_tile = [&](uint32_t tile, int stage) {
@@ -584,35 +623,29 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    load_tile(tile_lo, 0);
+#pragma unroll
+    for (uint32_t i = 0; i < kDecodeStages - 1; ++i)
+        if (tile_lo + i <= tile_hi) load_tile(tile_lo + i, (int)i);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
 
     // ---- q_0..q_{G-1} (and k, v for the split that holds the position): RMS norm + RoPE, a warp each ----
-    for (int i = tid; i < 16 * (HD / 8); i += kThreads) *(uint4 *)(sQ + i * 16) = make_uint4(0, 0, 0, 0);
-    __syncthreads();
     for (int vec = warp; vec < G + (owns_new ? 1 : 0); vec += kThreads / 32) {
         const bool is_k = vec == G;
-        const float *src = is_k ? k + (size_t)kvh * HD : q + ((size_t)kvh * G + vec) * HD;
-        const float *nw = is_k ? a.k_norm : a.q_norm;
-        float x[EPL];
+        if (vec != warp) fetch(vec);
         float ss = 0.0f;
 #pragma unroll
-        for (int r = 0; r < EPL; ++r) {
-            x[r] = src[lane + 32 * r];
-            ss = fmaf(x[r], x[r], ss);
-        }
+        for (int r = 0; r < EPL; ++r) ss = fmaf(x[r], x[r], ss);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
         const float inv = 1.0f / sqrtf(ss / (float)HD + a.eps);
 #pragma unroll
-        for (int r = 0; r < EPL; ++r) x[r] = x[r] * inv * nw[lane + 32 * r];
+        for (int r = 0; r < EPL; ++r) x[r] = x[r] * inv * nw[r];
         // full rotation: pair (i, i + HD/2), i = lane + 32 r, has both members in this lane
 #pragma unroll
         for (int r = 0; r < EPL / 2; ++r) {
-            float sn, cs;
-            sincosf((float)pos * a.inv_freq[lane + 32 * r], &sn, &cs);
             const float a0 = x[r], b0 = x[r + EPL / 2];
-            x[r] = a0 * cs - b0 * sn;
-            x[r + EPL / 2] = a0 * sn + b0 * cs;
+            x[r] = a0 * cs[r] - b0 * sn[r];
+            x[r + EPL / 2] = a0 * sn[r] + b0 * cs[r];
         }
         if (is_k) {
             const float *vsrc = v + (size_t)kvh * HD;
@@ -642,14 +675,11 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
     const bool row_live = g < G;
 
     for (uint32_t tile = tile_lo; tile <= tile_hi; ++tile) {
-        const int stage = (int)((tile - tile_lo) & 1u);
-        if (tile < tile_hi) {
-            load_tile(tile + 1, stage ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();  // the tile has landed (and, first time round, Q and the new row are written)
+        const int stage = (int)((tile - tile_lo) % kDecodeStages);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kDecodeStages - 2) : "memory");
+        __syncthreads();  // the tile has landed, the one before it is done (first time round: Q and the new row are written)
+        if (tile + kDecodeStages - 1 <= tile_hi) load_tile(tile + kDecodeStages - 1, (int)((tile - tile_lo + kDecodeStages - 1) % kDecodeStages));
+        else asm volatile("cp.async.commit_group;" ::: "memory");
         const uint32_t j0 = tile * kBKV;
         if (tile == last_tile) {  // the position's own row comes from this step, not from the cache
             const uint32_t r = pos - j0;
@@ -710,8 +740,8 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
             mma_f16(o[2 * dp], pa0, 0u, pa2, 0u, b0, b1);
             mma_f16(o[2 * dp + 1], pa0, 0u, pa2, 0u, b2, b3);
         }
-        __syncthreads();  // the stage is refilled by the next iteration's prefetch
     }
+    __syncthreads();
 
     // ---- the four warps' (m, l, o) -> this split's; the K/V stages are free now ----
     float *wo = (float *)sKV;  // [4][G][HD]
@@ -791,20 +821,19 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
     if (tid == 0) *count = 0u;  // ready for the next launch on this stream
 }
 
-template <int G, int HD>
+template <int G, int HD, uint32_t kDecodeStages>
 cudaError_t launch_decode_mma(tm_cuda_ctx *ctx, const decode_mma_args &a, uint32_t n_seq) {
-    constexpr uint32_t kBytes = 16 * HD * 2 + 2 * 2 * kBKV * HD * 2;
+    constexpr uint32_t kBytes = 16 * HD * 2 + kDecodeStages * 2 * kBKV * HD * 2;
     static std::atomic<bool> attr_done[64] = {};
     const int device = ctx->device;
     if (device < 0 || device >= 64 || !attr_done[device].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(attention_decode_mma_kernel<G, HD>,
+        const cudaError_t e = cudaFuncSetAttribute(attention_decode_mma_kernel<G, HD, kDecodeStages>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBytes);
         if (e != cudaSuccess) return e;
         if (device >= 0 && device < 64) attr_done[device].store(true, std::memory_order_release);
     }
-    const uint32_t n_tiles = (a.cap + kBKV - 1) / kBKV;
-    const dim3 grid(a.kv_heads, (n_tiles + a.tiles - 1) / a.tiles, n_seq);
-    return tm_launch_pdl(ctx, attention_decode_mma_kernel<G, HD>, grid, dim3(kThreads), kBytes, a);
+    const dim3 grid(a.kv_heads, a.splits, n_seq);
+    return tm_launch_pdl(ctx, attention_decode_mma_kernel<G, HD, kDecodeStages>, grid, dim3(kThreads), kBytes, a);
 }
 
 attn_segs attn_segments(uint32_t pos0, uint32_t n) {
@@ -869,16 +898,20 @@ cudaError_t tm_attention_decode_mma_launch(tm_cuda_ctx *ctx, const float *q, con
     a.eps = eps;
     a.scale_log2e = scale * 1.4426950408889634f;
     a.sq = sq; a.sk = a.sv = skv; a.so = so; a.scache = scache; a.sscratch = sscratch;
-    // Keys per CTA: enough CTAs to fill the machine a few times over, as few splits as that allows.
-    const uint32_t n_tiles = (cap + kBKV - 1) / kBKV;
-    uint32_t tiles = 8;
-    while (tiles > 1 && (uint64_t)n_seq * kv_heads * ((n_tiles + tiles - 1) / tiles) < 4ull * (uint64_t)ctx->sm_count) tiles >>= 1;
-    a.tiles = tiles;
+    // As many splits as find a place at once (two CTAs of three tiles in shared memory to an SM): the splits of a head
+    // meet through memory (store, fence, atomic, reload: 5 us), so many sequences are better off without any.  Three
+    // CTAs of two tiles where one CTA a head is more than that.  (By the capacity, 1024 CTAs of which half had nothing
+    // to do: 32 sequences at 100 to 460 of 1024 positions 13.9 us, now 12.1; 32 of 50 to 250, groups of four heads,
+    // 11.5, now 8.4; 4 at 200 to 620 16.2, now 12.8.)
+    const uint32_t n_tiles = (cap + kBKV - 1) / kBKV, heads_all = n_seq * kv_heads, places = 2u * (uint32_t)ctx->sm_count;
+    const uint32_t splits = places / heads_all;
+    a.splits = splits < 1u ? 1u : splits > n_tiles ? n_tiles : splits;
     (void)hd;
+    const bool deep = heads_all <= places;
     switch (heads / kv_heads) {
-        case 1: return launch_decode_mma<1, 128>(ctx, a, n_seq);
-        case 2: return launch_decode_mma<2, 128>(ctx, a, n_seq);
-        default: return launch_decode_mma<4, 128>(ctx, a, n_seq);
+        case 1: return deep ? launch_decode_mma<1, 128, 3>(ctx, a, n_seq) : launch_decode_mma<1, 128, 2>(ctx, a, n_seq);
+        case 2: return deep ? launch_decode_mma<2, 128, 3>(ctx, a, n_seq) : launch_decode_mma<2, 128, 2>(ctx, a, n_seq);
+        default: return deep ? launch_decode_mma<4, 128, 3>(ctx, a, n_seq) : launch_decode_mma<4, 128, 2>(ctx, a, n_seq);
     }
 }
 
