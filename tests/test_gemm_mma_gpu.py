@@ -116,6 +116,31 @@ def test_mma_gemm_split_k_is_deterministic_and_within_the_profile(ctx, oracle, r
         b.free()
 
 
+# Several tiles to a CTA (more row tiles than SMs) of fewer K steps than a form has issuers: were the issuers to take
+# them in turn, the accumulator of one without a step in a tile would still hold an older tile.
+@pytest.mark.parametrize("rows", [148 * 128 + 1, 20000, 4 * 148 * 128 + 129, 151936])
+@pytest.mark.parametrize("cols", [32, 64, 96, 128, 160, 192])
+def test_mma_gemm_many_tiles_of_few_k_steps(ctx, oracle, rows, cols):
+    base = T.q8_0_matrix(7, cols, 4096, cols)
+    raw = np.tile(base, ((rows + 4095) // 4096, 1, 1))[:rows]
+    w = ctx.q8_0_matrix(raw, rows, cols)
+    for batch in (9, 17, 32, 33, 64, 65, 128):
+        X = T.activations(7, batch, batch * cols).reshape(batch, cols)
+        xb, yb = ctx.floats(X), ctx.buffer(batch * rows * 4)
+        ctx.q8_0_gemm_mma(w, xb, yb, rows, cols, batch)
+        Y = yb.download(0, batch * rows * 4, np.float32).reshape(batch, rows)
+        assert not ctx.mma_aborted()
+        ref16, cpu = f16_profile_reference(base, X), oracle.matmul_q8_0(base[:256], 256, cols, X)
+        for r0 in range(0, rows, 4096):
+            got = Y[:, r0:r0 + 4096]
+            # f32 sums of at most 192 exact products in another order: 192 * 2^-24 of the summed magnitudes
+            assert rel_err(got, ref16[:, :got.shape[1]]) <= 2e-5, f"{batch} tokens, rows from {r0}"
+            assert float(np.max(np.abs(got[:, :256] - cpu[:, :got.shape[1]]))) <= 2e-2
+        for b in (xb, yb):
+            b.free()
+    w.free()
+
+
 def test_mma_gemm_row_view_and_larger_scales(ctx, oracle):
     """A projection stored inside a fused matrix (row view), scales up to ~1."""
     rows, cols, batch = 384, 512, 200

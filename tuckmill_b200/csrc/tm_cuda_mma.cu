@@ -498,10 +498,8 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
 #pragma unroll
                   for (int j = 0; j < W; ++j) v[j] = __uint_as_float(u[j]);
                   if (kTurns) {
-                      // the other issuers' accumulators, in order (a tile of fewer K steps than issuers skips some)
+                      // the other issuers' accumulators, in order: each has a K step in every tile (see the launcher)
                       for (uint32_t i = 1; i < (uint32_t)kIssuers; ++i) {
-                          const uint32_t g0 = it * nkb, first = (i + (uint32_t)kIssuers - g0 % kIssuers) % kIssuers;
-                          if (nkb < (uint32_t)kIssuers && first >= nkb) continue;
                           tmem_ld(tmem_base + ((quarter * 32u) << 16) + (acc0 + i) * BN + c0, u);
 #pragma unroll
                           for (int j = 0; j < W; ++j) v[j] += __uint_as_float(u[j]);
@@ -893,10 +891,15 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
         }
     }
     // Up to 128 tokens, the forms with four converter sets (one token tile, as with two 64-token sub-tiles, so the
-    // split below is the same): 24576 x 4096 46 -> 36 us at 32 tokens, 60 -> 50 us at 128.  From 65 tokens on they
+    // split below is the same): 24576 x 4096 46 -> 34 us at 32 tokens, 60 -> 48 us at 128.  From 65 tokens on they
     // pay only where an SM has at least eight K steps to stream (4096 x 1024 at 128: 19 us against 16).
-    const uint64_t sm_steps = (uint64_t)row_tiles * ((cols + kBK - 1) / kBK) / sms;
-    const int few = push.world ? 0 : batch <= 32u ? 32 : batch <= 64u ? 64 : batch <= 128u && sm_steps >= 8u ? 128 : 0;
+    // The issuers of these forms take K steps in turn over all tiles of a CTA, each into its own accumulator, and a tile's
+    // sum takes all of them: with fewer K steps than issuers one would have none in some tile (151936 x 64 at 32 tokens
+    // takes 18 us with the two-set form; a check per issuer and tile, in the sum, made that 20 and 24576 x 4096 at 128 51).
+    const uint32_t nk = (cols + kBK - 1) / kBK;
+    const uint64_t sm_steps = (uint64_t)row_tiles * nk / sms;
+    const int few = push.world ? 0 : batch <= 32u && nk >= 4u ? 32 : batch <= 64u && nk >= 2u ? 64
+                    : batch <= 128u && nk >= 2u && sm_steps >= 8u ? 128 : 0;
     CUtensorMap xmap, wmap;
     const cuuint32_t estr[2] = {1, 1};
     {
