@@ -156,6 +156,7 @@ mod ffi {
         pub fn tm_cuda_allocated_bytes(ctx: *const TmCudaCtx) -> u64;
         pub fn tm_cuda_in_flight_bytes(ctx: *const TmCudaCtx) -> u64;
         pub fn tm_cuda_kernel_launches(ctx: *const TmCudaCtx) -> u64;
+        pub fn tm_cuda_ordered_launches(ctx: *const TmCudaCtx) -> u64;
         pub fn tm_cuda_device_memory(ctx: *mut TmCudaCtx, free_bytes: *mut u64, total_bytes: *mut u64) -> c_int;
         pub fn tm_cuda_stream(ctx: *mut TmCudaCtx) -> *mut c_void;
         pub fn tm_cuda_qwen35_rope_partial(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, pos: u32, n_q_heads: u32, n_kv_heads: u32, head_dim: u32, n_rot: u32, err: *mut c_char, err_cap: usize) -> c_int;

@@ -15,6 +15,12 @@
  * positions, multi-GPU row split); a host that only knows the reference
  * surface can ignore them and still run every operator.
  *
+ * Operators take effect in the order of the calls, whatever they write: a kernel may overlap the
+ * tail of its predecessors and read weights or cached rows ahead of them only while nothing in
+ * flight writes those (tm_cuda_ordered_launches counts the launches that had to wait).  Storage
+ * written around the operators (tm_cuda_buffer_device_ptr, tm_cuda_buffer_contents) must be
+ * complete before the call that reads it.
+ *
  * There is no CPU fallback anywhere behind this interface: without a usable
  * CUDA device tm_cuda_create fails with TM_CUDA_ERR_NO_DEVICE.
  */
@@ -374,6 +380,9 @@ uint64_t tm_cuda_in_flight_bytes(const tm_cuda_ctx *ctx);
 /* No counterpart: kernels launched by this context so far (each operator
  * launch and each graph node counts one). */
 uint64_t tm_cuda_kernel_launches(const tm_cuda_ctx *ctx);
+/* No counterpart: launches that waited for all work before them because an operand that the kernel
+ * reads ahead (a matrix, a norm weight, a rotation table, a KV cache) had just been written. */
+uint64_t tm_cuda_ordered_launches(const tm_cuda_ctx *ctx);
 /* No counterpart: free and total bytes of the context's device (the budget B
  * the planner admits against when the caller names none). */
 int tm_cuda_device_memory(tm_cuda_ctx *ctx, uint64_t *free_bytes, uint64_t *total_bytes);

@@ -9,7 +9,9 @@
 // Cached rows are read before the predecessor kernel finishes.  The position read at that moment only says which
 // rows to ask for; it is read again afterwards, and a changed one reloads them.  Row pos - 1 is always read after the
 // wait: the attention call of the previous token may still be storing it.  Calls further back have finished, because
-// a kernel that stores KV rows lets its successor start only after its own predecessor is complete.
+// a kernel that stores KV rows lets its successor start only after its own predecessor is complete.  Where another
+// operator has written the cache or the table of frequencies, or the call before took its position from another word,
+// the launch does not overlap what is before it (tm_read_cache_ahead).
 #pragma once
 #include "tm_cuda_internal.cuh"
 #include "tm_cuda_device.cuh"

@@ -173,19 +173,7 @@ cudaError_t launch(tm_cuda_ctx *ctx, const attn_args &a, uint32_t kv_heads, uint
     // As many CTAs per KV head as keep the launch within two resident waves, a power of two.
     uint32_t c = max_cluster<G, HD>(ctx->device);
     while (c > 1u && (uint64_t)c * kv_heads * n_seq > 2ull * (uint32_t)ctx->sm_count) c >>= 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(c * kv_heads, 1, n_seq);
-    cfg.blockDim = dim3(kT);
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = c;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = ctx->pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, attention_decode_cluster_kernel<G, HD>, a);
+    return tm_launch_cluster_pdl(ctx, c, attention_decode_cluster_kernel<G, HD>, dim3(c * kv_heads, 1, n_seq), dim3(kT), 0, a);
 }
 
 }  // namespace

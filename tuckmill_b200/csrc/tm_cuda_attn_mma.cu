@@ -936,9 +936,9 @@ int tm_cuda_qk_prep_chunk(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffer *k
     TM_CHECK_BUF(q, (size_t)n * heads * head_dim * 4, "q");
     TM_CHECK_BUF(k, (size_t)n * kv_heads * head_dim * 4, "k");
     TM_CHECK_BUF(v, (size_t)n * kv_heads * head_dim * 4, "v");
-    TM_CHECK_BUF(q_norm, (size_t)head_dim * 4, "q norm");
-    TM_CHECK_BUF(k_norm, (size_t)head_dim * 4, "k norm");
-    TM_CHECK_BUF(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
+    TM_CHECK_IN(q_norm, (size_t)head_dim * 4, "q norm");
+    TM_CHECK_IN(k_norm, (size_t)head_dim * 4, "k norm");
+    TM_CHECK_IN(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
     TM_CHECK_BUF(k_cache, plane, "K cache");
     TM_CHECK_BUF(v_cache, plane, "V cache");
     TM_OP_BEGIN("qk_prep_chunk");
@@ -961,10 +961,10 @@ int tm_cuda_attention_chunk_mma(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buf
                        "%u..%u of capacity %u", heads, group, head_dim, pos0, pos0 + n, cap);
     const uint32_t kv_heads = heads / group;
     const size_t plane = (size_t)kv_heads * cap * head_dim * 2;
-    TM_CHECK_BUF(q, (size_t)n * heads * head_dim * 4, "q");
+    TM_CHECK_IN(q, (size_t)n * heads * head_dim * 4, "q");
     TM_CHECK_BUF(out, (size_t)n * heads * head_dim * 4, "attention output");
-    TM_CHECK_BUF(k_cache, plane, "K cache");
-    TM_CHECK_BUF(v_cache, plane, "V cache");
+    TM_CHECK_IN(k_cache, plane, "K cache");
+    TM_CHECK_IN(v_cache, plane, "V cache");
     if (((size_t)q->dev | (size_t)out->dev | (size_t)k_cache->dev | (size_t)v_cache->dev) & 15u)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "tensor-core chunk attention needs 16-byte aligned buffers");
     attn_args a;
@@ -1025,9 +1025,9 @@ int tm_cuda_attention_prefill(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffe
     TM_CHECK_BUF(q, rows * heads * head_dim * 4, "q");
     TM_CHECK_BUF(k, rows * kv_heads * head_dim * 4, "k");
     TM_CHECK_BUF(v, rows * kv_heads * head_dim * 4, "v");
-    TM_CHECK_BUF(q_norm, (size_t)head_dim * 4, "q norm");
-    TM_CHECK_BUF(k_norm, (size_t)head_dim * 4, "k norm");
-    TM_CHECK_BUF(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
+    TM_CHECK_IN(q_norm, (size_t)head_dim * 4, "q norm");
+    TM_CHECK_IN(k_norm, (size_t)head_dim * 4, "k norm");
+    TM_CHECK_IN(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
     TM_CHECK_BUF(out, rows * heads * head_dim * (out_f16 ? 2 : 4), "attention output");
     TM_CHECK_BUF(k_cache, (size_t)seqs * a.seq_stride * 2, "K cache");
     TM_CHECK_BUF(v_cache, (size_t)seqs * a.seq_stride * 2, "V cache");

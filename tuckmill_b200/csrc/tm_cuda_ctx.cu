@@ -111,6 +111,7 @@ int tm_check_packed(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, ui
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED,
                        "weight buffer is not a packed %u x %u Q8_0 matrix (pack it with "
                        "tm_cuda_q8_0_pack first)", rows, cols);
+    tm_read_ahead(ctx, w);
     return TM_CUDA_OK;
 }
 
@@ -315,6 +316,7 @@ int tm_cuda_buffer_zero(tm_cuda_ctx *ctx, tm_cuda_buffer *buffer, size_t off, si
     TM_CHECK_BUF(buffer, off + len, "zero target");
     TM_OP_BEGIN("buffer_zero");
     TM_CUDA_TRY(cudaMemsetAsync(buffer->dev + off, 0, len, ctx->stream));
+    tm_settle(ctx);
     TM_OP_END(1);
 }
 
@@ -326,6 +328,7 @@ int tm_cuda_buffer_zero_2d(tm_cuda_ctx *ctx, tm_cuda_buffer *buffer, size_t off,
     TM_CHECK_BUF(buffer, off + (height - 1) * pitch + width, "zero target");
     TM_OP_BEGIN("buffer_zero_2d");
     TM_CUDA_TRY(cudaMemset2DAsync(buffer->dev + off, pitch, 0, width, height, ctx->stream));
+    tm_settle(ctx);
     TM_OP_END(1);
 }
 
@@ -371,9 +374,10 @@ int tm_cuda_upload(tm_cuda_ctx *ctx, tm_cuda_buffer *dst, size_t off, const void
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "upload with a dispatch group open");
     if (!src || len == 0 || off > SIZE_MAX - len)
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "upload range is empty or overflows");
-    TM_CHECK_BUF(dst, off + len, "upload target");
+    TM_CHECK_IN(dst, off + len, "upload target");  // (complete before the call returns)
     TM_CUDA_TRY(cudaMemcpyAsync(dst->dev + off, src, len, cudaMemcpyDefault, ctx->stream));
     TM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    ctx->settled = ctx->op;
     poll_locked(ctx, false);
     return TM_CUDA_OK;
 }
@@ -385,9 +389,10 @@ int tm_cuda_download(tm_cuda_ctx *ctx, tm_cuda_buffer *src, size_t off, void *ds
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "download with a dispatch group open");
     if (!dst || len == 0 || off > SIZE_MAX - len)
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "download range is empty or overflows");
-    TM_CHECK_BUF(src, off + len, "download source");
+    TM_CHECK_IN(src, off + len, "download source");
     TM_CUDA_TRY(cudaMemcpyAsync(dst, src->dev + off, len, cudaMemcpyDefault, ctx->stream));
     TM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    ctx->settled = ctx->op;
     poll_locked(ctx, false);
     return TM_CUDA_OK;
 }
@@ -397,7 +402,7 @@ int tm_cuda_download_after(tm_cuda_ctx *ctx, tm_cuda_buffer *src, size_t off, vo
     TM_ENTER();
     if (!dst || len == 0 || off > SIZE_MAX - len)
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "download range is empty or overflows");
-    TM_CHECK_BUF(src, off + len, "download source");
+    TM_CHECK_IN(src, off + len, "download source");
     if (!src->shared)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED,
                        "download_after reads a shared buffer; this one is device-private");
@@ -464,6 +469,9 @@ int tm_cuda_begin_group(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
     TM_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
     ctx->group_open = true;
     ctx->group_kernels = 0;
+    // A graph starts after everything before its launch; the stream itself has not reached a boundary here.
+    ctx->settled_outside = ctx->settled;
+    ctx->settled = ctx->op;
     return TM_CUDA_OK;
 }
 
@@ -478,6 +486,7 @@ static int end_capture(tm_cuda_ctx *ctx, cudaGraphExec_t *exec, char *err, size_
     cudaGraph_t graph = nullptr;
     join_side(ctx);
     ctx->group_open = false;
+    ctx->settled = ctx->settled_outside;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
     if (e != cudaSuccess || !graph) {
         cudaGetLastError();
@@ -504,6 +513,7 @@ static int launch_exec(tm_cuda_ctx *ctx, cudaGraphExec_t exec, uint64_t kernels,
     int rc = commit_begin(ctx, &c, label, err, err_cap);
     if (rc != TM_CUDA_OK) return rc;
     TM_CUDA_TRY(cudaGraphLaunch(exec, ctx->stream));
+    ctx->settled = 0;  // whatever an operator ever wrote, the graph may be writing
     ctx->launches.fetch_add(kernels);
     return commit_end(ctx, &c, err, err_cap);
 }
@@ -582,6 +592,7 @@ int tm_cuda_graph_launch(tm_cuda_ctx *ctx, tm_cuda_graph *graph, char *err, size
         if (rc != TM_CUDA_OK) return rc;
         rc = tm_step_launch(ctx, graph->program, err, err_cap);
         if (rc != TM_CUDA_OK) return rc;
+        ctx->settled = 0;  // (as after a graph)
         ctx->launches.fetch_add(1);
         return commit_end(ctx, &c, err, err_cap);
     }
@@ -608,6 +619,7 @@ int tm_cuda_fence(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
     if (ctx->group_open || ctx->burst_open)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "fence with a dispatch group open");
     TM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    ctx->settled = ctx->op;
     poll_locked(ctx, true);
     return TM_CUDA_OK;
 }
@@ -671,6 +683,7 @@ int tm_cuda_device_memory(tm_cuda_ctx *ctx, uint64_t *free_bytes, uint64_t *tota
     if (total_bytes) *total_bytes = t;
     return TM_CUDA_OK;
 }
+uint64_t tm_cuda_ordered_launches(const tm_cuda_ctx *ctx) { return ctx ? ctx->ordered_launches.load() : 0; }
 void *tm_cuda_stream(tm_cuda_ctx *ctx) { return ctx ? (void *)ctx->stream : nullptr; }
 
 }  // extern "C"

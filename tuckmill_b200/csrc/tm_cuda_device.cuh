@@ -61,8 +61,9 @@ static __device__ float block_sumsq(const float *x, uint32_t n, float *red /* [k
 // Programmatic dependent launch: a kernel launched with the stream-serialization
 // attribute may start while its predecessor still runs.  `pdl_wait` blocks until
 // the predecessor has completed and its writes are visible (a no-op for an
-// ordinary launch); `pdl_trigger` lets the successor start launching.  Work that
-// touches only constants (weights) goes before the wait.
+// ordinary launch); `pdl_trigger` lets the successor start launching.  Before the
+// wait a kernel reads only operands that nothing in flight writes: its entry point
+// says which (TM_CHECK_AHEAD in tm_cuda_internal.cuh).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 

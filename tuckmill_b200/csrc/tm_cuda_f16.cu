@@ -266,13 +266,13 @@ int f16_common(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, tm_cuda_b
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "F16 geometry %u x %u", rows, cols);
     if (batch == 0 || batch > TM_CUDA_GEMM_MAX_BATCH)
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "batch %u outside 1..%u", batch, TM_CUDA_GEMM_MAX_BATCH);
-    TM_CHECK_BUF(w, (size_t)rows * cols * 2, "F16 weights");
+    TM_CHECK_AHEAD(w, (size_t)rows * cols * 2, "F16 weights");
     TM_CHECK_BUF(x, ((size_t)x_off + (size_t)batch * cols) * 4, "activation");
     TM_CHECK_BUF(y, ((size_t)y_off + (size_t)batch * rows) * 4, "output");
     if (prologue < TM_CUDA_PRO_NONE || prologue > TM_CUDA_PRO_GELU_MUL ||
         (epilogue != TM_CUDA_EPI_STORE && epilogue != TM_CUDA_EPI_ADD))
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "unknown prologue/epilogue");
-    if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_BUF(pro, (size_t)cols * 4, "norm weight");
+    if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_IN(pro, (size_t)cols * 4, "norm weight");
     if (prologue == TM_CUDA_PRO_SILU_MUL || prologue == TM_CUDA_PRO_GELU_MUL)
         TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate multiplicand");
     const size_t per_token = ((size_t)cols + 7u) / 8u * 32u, budget = ctx->smem_optin - 4096;
@@ -340,7 +340,7 @@ int tm_cuda_f16_row_f32(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *out
                         uint32_t out_off, char *err, size_t err_cap) {
     TM_ENTER();
     if (cols == 0) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "F16 row of zero columns");
-    TM_CHECK_BUF(w, ((size_t)row + 1) * cols * 2, "F16 weights");
+    TM_CHECK_IN(w, ((size_t)row + 1) * cols * 2, "F16 weights");
     TM_CHECK_BUF(out, ((size_t)out_off + cols) * 4, "row output");
     TM_OP_BEGIN("f16_row");
     f16_row_kernel<<<(cols + 255) / 256, 256, 0, ctx->stream>>>((const __half *)w->dev, cols, row,
@@ -353,7 +353,7 @@ int tm_cuda_f16_row_indirect_f32_dev(tm_cuda_ctx *ctx, tm_cuda_buffer *w, uint32
                                      tm_cuda_buffer *out, char *err, size_t err_cap) {
     TM_ENTER();
     if (rows == 0 || cols == 0) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "F16 geometry %u x %u", rows, cols);
-    TM_CHECK_BUF(w, (size_t)rows * cols * 2, "F16 weights");
+    TM_CHECK_IN(w, (size_t)rows * cols * 2, "F16 weights");
     TM_CHECK_BUF(ids, ((size_t)base + 1) * 4, "token ids");
     TM_CHECK_BUF(out, (size_t)cols * 4, "row output");
     const uint32_t *pos = nullptr;
@@ -373,7 +373,7 @@ int tm_cuda_f16_rows_indirect_f32(tm_cuda_ctx *ctx, tm_cuda_buffer *w, uint32_t 
     TM_ENTER();
     if (rows == 0 || cols == 0) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "F16 geometry %u x %u", rows, cols);
     if (n == 0 || n > 65535u) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "row count %u outside 1..65535", n);
-    TM_CHECK_BUF(w, (size_t)rows * cols * 2, "F16 weights");
+    TM_CHECK_IN(w, (size_t)rows * cols * 2, "F16 weights");
     TM_CHECK_BUF(ids, ((size_t)first + n) * 4, "token ids");
     TM_CHECK_BUF(out, (size_t)n * cols * 4, "rows output");
     TM_OP_BEGIN("f16_rows_indirect");

@@ -32,6 +32,10 @@ struct tm_cuda_buffer {
     const unsigned char *qp = nullptr; // packed: int8 quant plane of row 0
     const unsigned char *dp = nullptr; // packed: f16 scale plane of row 0
     void *symm = nullptr;              // peer mappings of a symmetric exchange buffer (tm_cuda_comm.cu)
+    // Operands that kernels read ahead (see tm_read_ahead): the last operator that may have written the storage (kept
+    // at the buffer that owns it), and the position word of the last decode attention over this cache.
+    uint64_t written = 0;
+    const void *kv_pos = nullptr;
 };
 
 // Closes the peer mappings of a symmetric buffer (no-op for ordinary buffers).
@@ -81,6 +85,11 @@ struct tm_cuda_ctx {
     uint64_t group_kernels = 0;
     bool profiling = false;
     bool pdl = true;                     // chain kernels with programmatic dependent launch
+    // Operators are numbered; what operators up to `settled` wrote is complete before any later launch starts.
+    // `ordered`: the operator being encoded reads ahead something younger, so its first launch waits for all before it.
+    uint64_t op = 0, settled = 0, settled_outside = 0;
+    bool ordered = false;
+    std::atomic<uint64_t> ordered_launches{0};
     std::deque<tm_commit> pending;       // committed, completion not yet observed
     tm_commit open_commit;               // the ungrouped dispatch being encoded
     std::vector<cudaEvent_t> event_pool;
@@ -130,10 +139,47 @@ inline int tm_check(tm_cuda_ctx *ctx, const tm_cuda_buffer *b, size_t need, cons
     return TM_CUDA_OK;
 }
 
-#define TM_CHECK_BUF(buf, need, what)                                        \
+// Operands read ahead.  A kernel launched to overlap its predecessors (tm_launch_pdl) may read weights, a rotation
+// table or cached rows before its dependency wait, or through the read-only path, which the compiler may move there.
+// Nothing orders such a read after a predecessor's write, and a predecessor that lets its successor start at once
+// leaves its own predecessors running too.  So every operand that an operator may write is marked with the operator's
+// number, and an operator that reads ahead an operand younger than the last full boundary of the stream is launched
+// without the overlap, which is such a boundary itself.
+//   TM_CHECK_BUF   any other operand: marked as written
+//   TM_CHECK_IN    an operand that the operator only reads, after its wait
+//   TM_CHECK_AHEAD an operand that it reads ahead.  (Decode attention takes its caches this way although it adds a row:
+//                  the next call reads that row after its wait, see tm_cuda_attn_core.cuh.)
+inline tm_cuda_buffer *tm_root(const tm_cuda_buffer *b) {
+    while (b->parent) b = b->parent;
+    return const_cast<tm_cuda_buffer *>(b);
+}
+inline void tm_read_ahead(tm_cuda_ctx *ctx, const tm_cuda_buffer *b) {
+    if (tm_root(b)->written > ctx->settled) ctx->ordered = true;
+}
+// Cached rows are also younger where the call before took its position from another word: the one row that is read
+// late is then not the one that call stores.
+inline void tm_read_cache_ahead(tm_cuda_ctx *ctx, tm_cuda_buffer *b, const void *pos) {
+    if (b->kv_pos && b->kv_pos != pos) ctx->ordered = true;
+    b->kv_pos = pos;
+    tm_read_ahead(ctx, b);
+}
+// Everything encoded before the current operator is complete before what follows starts.
+inline void tm_settle(tm_cuda_ctx *ctx) { ctx->settled = ctx->op - 1; }
+
+#define TM_CHECK_IN(buf, need, what)                                         \
     do {                                                                     \
         int rc_ = tm_check(ctx, (buf), (need), (what), err, err_cap);        \
         if (rc_ != TM_CUDA_OK) return rc_;                                   \
+    } while (0)
+#define TM_CHECK_BUF(buf, need, what)                                        \
+    do {                                                                     \
+        TM_CHECK_IN(buf, need, what);                                        \
+        tm_root(buf)->written = ctx->op;                                     \
+    } while (0)
+#define TM_CHECK_AHEAD(buf, need, what)                                      \
+    do {                                                                     \
+        TM_CHECK_IN(buf, need, what);                                        \
+        tm_read_ahead(ctx, (buf));                                           \
     } while (0)
 
 // Every operator entry point opens with this: context present, device current,
@@ -141,6 +187,8 @@ inline int tm_check(tm_cuda_ctx *ctx, const tm_cuda_buffer *b, size_t need, cons
 #define TM_ENTER()                                                                          \
     if (!ctx) return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "null context");        \
     std::lock_guard<std::mutex> lock_(ctx->mu);                                             \
+    ctx->op += 1;                                                                           \
+    ctx->ordered = false;                                                                   \
     TM_CUDA_TRY(cudaSetDevice(ctx->device))
 
 // Book-keeping around one operator launch (ungrouped: one dispatch per op with
@@ -171,23 +219,44 @@ inline size_t tm_q8_qplane_bytes(uint32_t rows, uint32_t cols) {
 int tm_check_packed(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, uint32_t cols,
                     char *err, size_t err_cap);
 
-// Launch on the context's stream, allowing the kernel to overlap the tail of
-// its predecessor (the kernel itself orders its dependent reads with
-// griddepcontrol.wait).
+// Launch on the context's stream, allowing the kernel to overlap the tail of its predecessor (the kernel itself orders
+// its dependent reads with griddepcontrol.wait) unless the operator reads ahead what a predecessor may be writing.
+// Clusters of `cluster` CTAs along x where it is not 0.
 template <class... KArgs, class... Args>
-inline cudaError_t tm_launch_pdl(tm_cuda_ctx *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                 Args... args) {
+inline cudaError_t tm_launch_cluster_pdl(tm_cuda_ctx *ctx, uint32_t cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                                         size_t smem, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    const bool ordered = ctx->ordered;
+    if (ctx->pdl && !ordered) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = ctx->pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+    cfg.numAttrs = n;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+    if (e == cudaSuccess && ordered) {
+        ctx->ordered = false;
+        ctx->ordered_launches.fetch_add(1);
+        tm_settle(ctx);
+    }
+    return e;
+}
+template <class... KArgs, class... Args>
+inline cudaError_t tm_launch_pdl(tm_cuda_ctx *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                 Args... args) {
+    return tm_launch_cluster_pdl(ctx, 0, kernel, grid, block, smem, args...);
 }
 
 // Tensor-core decode attention for several sequences in one launch (tm_cuda_attn_mma.cu).

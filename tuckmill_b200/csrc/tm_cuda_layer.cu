@@ -577,20 +577,7 @@ cudaError_t launch_clusters(tm_cuda_ctx *ctx, Kernel kernel, std::atomic<bool> *
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(clusters * kC);
-    cfg.blockDim = dim3(kT);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kC;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = ctx->pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a, ring_slots);
+    return tm_launch_cluster_pdl(ctx, kC, kernel, dim3(clusters * kC), dim3(kT), smem, a, ring_slots);
 }
 
 template <int NB>
@@ -651,10 +638,10 @@ int check_residual(tm_cuda_ctx *ctx, residual_in &r, tm_cuda_buffer *x, tm_cuda_
                    char *err, size_t err_cap) {
     TM_CHECK_BUF(x, (size_t)hidden * 4, "x");
     TM_CHECK_BUF(x_out, (size_t)hidden * 4, "x output");
-    TM_CHECK_BUF(norm_w, (size_t)hidden * 4, "norm weight");
+    TM_CHECK_AHEAD(norm_w, (size_t)hidden * 4, "norm weight");
     if (n_slots > kSlots) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "%u slots, at most %u", n_slots, kSlots);
     if (n_slots) TM_CHECK_BUF(slots, (size_t)n_slots * hidden * 4, "slots");
-    if (add_w) TM_CHECK_BUF(add_w, (size_t)hidden * 4, "output norm weight");
+    if (add_w) TM_CHECK_AHEAD(add_w, (size_t)hidden * 4, "output norm weight");
     if (x_out->dev == x->dev)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "x_out must be a buffer other than x (every cluster reads x)");
     if (((size_t)x->dev | (size_t)x_out->dev | (size_t)norm_w->dev | (n_slots ? (size_t)slots->dev : 0) | (add_w ? (size_t)add_w->dev : 0)) & 15u)
@@ -696,13 +683,15 @@ int tm_cuda_decode_attn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffe
     if (rc == TM_CUDA_OK) rc = check_residual(ctx, a.in, x, slots_in, n_slots, add_w, norm_w, x_out, hidden, eps, err, err_cap);
     if (rc != TM_CUDA_OK) return rc;
     const size_t plane = (size_t)kv_heads * cap * head_dim * 2;
-    TM_CHECK_BUF(q_norm, (size_t)head_dim * 4, "q norm");
-    TM_CHECK_BUF(k_norm, (size_t)head_dim * 4, "k norm");
-    TM_CHECK_BUF(inv_freq, (size_t)(head_dim / 2) * 4, "inv_freq");
-    TM_CHECK_BUF(k_cache, plane, "k cache");
-    TM_CHECK_BUF(v_cache, plane, "v cache");
+    TM_CHECK_AHEAD(q_norm, (size_t)head_dim * 4, "q norm");
+    TM_CHECK_AHEAD(k_norm, (size_t)head_dim * 4, "k norm");
+    TM_CHECK_AHEAD(inv_freq, (size_t)(head_dim / 2) * 4, "inv_freq");
+    TM_CHECK_IN(k_cache, plane, "k cache");
+    TM_CHECK_IN(v_cache, plane, "v cache");
     TM_CHECK_BUF(pos_buf, ((size_t)pos_index + 1) * 4, "position");
     TM_CHECK_BUF(status, 4, "status");
+    tm_read_cache_ahead(ctx, k_cache, (const uint32_t *)pos_buf->dev + pos_index);
+    tm_read_cache_ahead(ctx, v_cache, (const uint32_t *)pos_buf->dev + pos_index);
     TM_CHECK_BUF(slots_out, (size_t)kv_heads * hidden * 4, "slots output");
     a.qkv_q = (const signed char *)qkv->qp;
     a.qkv_d = (const unsigned short *)qkv->dp;

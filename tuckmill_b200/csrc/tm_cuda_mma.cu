@@ -1046,7 +1046,7 @@ int tm_cuda_q8_0_gemm_mma_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buf
     TM_CHECK_BUF(x, (size_t)batch * cols * (f16 ? 2 : 4), "activation");
     if (f16 && (((size_t)x->dev & 15u) || cols % 8u))
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "binary16 activations must be 16-byte aligned rows");
-    if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_BUF(pro, (size_t)cols * 4, "norm weight");
+    if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_IN(pro, (size_t)cols * 4, "norm weight");
     else if (prologue != TM_CUDA_PRO_NONE && !f16) TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate operand");
     TM_OP_BEGIN("q8_0_gemm_mma_fused");
     if (!f16)

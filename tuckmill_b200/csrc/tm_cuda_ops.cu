@@ -913,7 +913,7 @@ int tm_cuda_reduce_ranks_add_f32(tm_cuda_ctx *ctx, tm_cuda_buffer *slots, tm_cud
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "reduction geometry %u x %u x %u", world, n_rows, cols);
     TM_CHECK_BUF(slots, (size_t)world * n_rows * cols * 4, "rank slots");
     TM_CHECK_BUF(x, (size_t)n_rows * cols * 4, "x");
-    if (weight) TM_CHECK_BUF(weight, (size_t)cols * 4, "norm weight");
+    if (weight) TM_CHECK_IN(weight, (size_t)cols * 4, "norm weight");
     if (ctx->program)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "operator reduce_ranks_add cannot be recorded into a persistent program");
     TM_OP_BEGIN("reduce_ranks_add");
@@ -974,7 +974,7 @@ int tm_cuda_rmsnorm_f32(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffer *wei
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "rmsnorm geometry %u x %u", rows, cols);
     TM_CHECK_BUF(x, (size_t)rows * cols * 4, "x");
     TM_CHECK_BUF(y, (size_t)rows * cols * 4, "y");
-    TM_CHECK_BUF(weight, (size_t)cols * 4, "norm weight");
+    TM_CHECK_IN(weight, (size_t)cols * 4, "norm weight");
     TM_OP_BEGIN("rmsnorm");
     TM_CUDA_TRY(tm_launch_pdl(ctx, rmsnorm_kernel, dim3(rows), dim3(kThreads), 0, (const float *)x->dev,
                               (const float *)weight->dev, (float *)y->dev, cols, eps));
@@ -988,7 +988,7 @@ int tm_cuda_rmsnorm_add_f32(tm_cuda_ctx *ctx, tm_cuda_buffer *p, tm_cuda_buffer 
         return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "rmsnorm geometry %u x %u", rows, cols);
     TM_CHECK_BUF(p, (size_t)rows * cols * 4, "p");
     TM_CHECK_BUF(x, (size_t)rows * cols * 4, "x");
-    TM_CHECK_BUF(weight, (size_t)cols * 4, "norm weight");
+    TM_CHECK_AHEAD(weight, (size_t)cols * 4, "norm weight");
     if (p == x) return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "rmsnorm_add in place");
     if (ctx->program)
         return tm_step_record_norm_add(ctx, (const float *)p->dev, (const float *)weight->dev, (float *)x->dev, rows,
@@ -1048,7 +1048,7 @@ static int rope_common(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffer *k,
                        n_rot, n);
     TM_CHECK_BUF(q, (size_t)n * n_q * hd * 4, "q");
     TM_CHECK_BUF(k, (size_t)n * n_kv * hd * 4, "k");
-    TM_CHECK_BUF(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
+    TM_CHECK_IN(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
     TM_OP_BEGIN("rope");
     const int threads = n_rot / 2 >= 128 ? 128 : n_rot / 2 >= 64 ? 64 : 32;
     rope_kernel<<<dim3(n_q + n_kv, n), threads, 0, ctx->stream>>>(
@@ -1119,10 +1119,10 @@ static int attention_common(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffer 
                        "at position %u, capacity %u", heads, group, hd, n, pos0, cap);
     const uint32_t kvh = heads / group;
     const size_t plane = (size_t)kvh * cap * hd * 2;
-    TM_CHECK_BUF(q, (size_t)n * heads * hd * 4, "q");
+    TM_CHECK_IN(q, (size_t)n * heads * hd * 4, "q");
     TM_CHECK_BUF(out, (size_t)n * heads * hd * 4, "attention output");
-    TM_CHECK_BUF(k_cache, plane, "k cache");
-    TM_CHECK_BUF(v_cache, plane, "v cache");
+    TM_CHECK_IN(k_cache, plane, "k cache");
+    TM_CHECK_IN(v_cache, plane, "v cache");
     // The reference sizes a score scratch of n*heads*cap f32; this kernel keeps
     // its state in registers and only checks that a buffer was passed.
     TM_CHECK_BUF(scratch, 4, "attention scratch");
@@ -1186,16 +1186,18 @@ int tm_cuda_attention_decode_dev(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_bu
     TM_CHECK_BUF(q, (size_t)heads * head_dim * 4, "q");
     TM_CHECK_BUF(k, (size_t)kv_heads * head_dim * 4, "k");
     TM_CHECK_BUF(v, (size_t)kv_heads * head_dim * 4, "v");
-    TM_CHECK_BUF(q_norm, (size_t)head_dim * 4, "q norm");
-    TM_CHECK_BUF(k_norm, (size_t)head_dim * 4, "k norm");
-    TM_CHECK_BUF(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
-    TM_CHECK_BUF(k_cache, plane, "k cache");
-    TM_CHECK_BUF(v_cache, plane, "v cache");
+    TM_CHECK_IN(q_norm, (size_t)head_dim * 4, "q norm");
+    TM_CHECK_IN(k_norm, (size_t)head_dim * 4, "k norm");
+    TM_CHECK_AHEAD(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
+    TM_CHECK_IN(k_cache, plane, "k cache");
+    TM_CHECK_IN(v_cache, plane, "v cache");
     TM_CHECK_BUF(out, (size_t)heads * head_dim * 4, "attention output");
     TM_CHECK_BUF(scratch, tm_cuda_attention_decode_scratch_bytes(heads, kv_heads, head_dim, cap),
                  "decode attention scratch");
     TM_CHECK_BUF(pos_buf, ((size_t)pos_index + 1) * 4, "position");
     TM_CHECK_BUF(status, 4, "status");
+    tm_read_cache_ahead(ctx, k_cache, (const uint32_t *)pos_buf->dev + pos_index);
+    tm_read_cache_ahead(ctx, v_cache, (const uint32_t *)pos_buf->dev + pos_index);
     const float *qp = (const float *)q->dev, *kp = (const float *)k->dev, *vp = (const float *)v->dev;
     const float *qn = (const float *)q_norm->dev, *kn = (const float *)k_norm->dev, *fq = (const float *)inv_freq->dev;
     __half *kcp = (__half *)k_cache->dev, *vcp = (__half *)v_cache->dev;
@@ -1252,15 +1254,17 @@ int tm_cuda_attention_decode_batch_dev(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_c
     TM_CHECK_BUF(q, ((size_t)(n_seq - 1) * q_stride + (size_t)heads * head_dim) * 4, "q");
     TM_CHECK_BUF(k, ((size_t)(n_seq - 1) * kv_stride + (size_t)kv_heads * head_dim) * 4, "k");
     TM_CHECK_BUF(v, ((size_t)(n_seq - 1) * kv_stride + (size_t)kv_heads * head_dim) * 4, "v");
-    TM_CHECK_BUF(q_norm, (size_t)head_dim * 4, "q norm");
-    TM_CHECK_BUF(k_norm, (size_t)head_dim * 4, "k norm");
-    TM_CHECK_BUF(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
-    TM_CHECK_BUF(k_cache, (size_t)n_seq * plane, "k caches");
-    TM_CHECK_BUF(v_cache, (size_t)n_seq * plane, "v caches");
+    TM_CHECK_IN(q_norm, (size_t)head_dim * 4, "q norm");
+    TM_CHECK_IN(k_norm, (size_t)head_dim * 4, "k norm");
+    TM_CHECK_AHEAD(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
+    TM_CHECK_IN(k_cache, (size_t)n_seq * plane, "k caches");
+    TM_CHECK_IN(v_cache, (size_t)n_seq * plane, "v caches");
     TM_CHECK_BUF(out, (size_t)n_seq * heads * head_dim * 4, "attention output");
     TM_CHECK_BUF(scratch, (size_t)n_seq * per_seq, "decode attention scratch");
     TM_CHECK_BUF(pos_buf, (size_t)n_seq * 4, "positions");
     TM_CHECK_BUF(status, 4, "status");
+    tm_read_cache_ahead(ctx, k_cache, (const uint32_t *)pos_buf->dev);
+    tm_read_cache_ahead(ctx, v_cache, (const uint32_t *)pos_buf->dev);
     if (ctx->program)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "operator attention_decode_batch cannot be recorded into a persistent program");
     const float *qp = (const float *)q->dev, *kp = (const float *)k->dev, *vp = (const float *)v->dev;
@@ -1349,14 +1353,16 @@ int tm_cuda_attention_decode_dev_static(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_
     TM_CHECK_BUF(q, (size_t)heads * head_dim * 4, "q");
     TM_CHECK_BUF(k, (size_t)kv_heads * head_dim * 4, "k");
     TM_CHECK_BUF(v, (size_t)kv_heads * head_dim * 4, "v");
-    TM_CHECK_BUF(q_norm, (size_t)head_dim * 4, "q norm");
-    TM_CHECK_BUF(k_norm, (size_t)head_dim * 4, "k norm");
-    TM_CHECK_BUF(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
-    TM_CHECK_BUF(k_cache, plane, "k cache");
-    TM_CHECK_BUF(v_cache, plane, "v cache");
+    TM_CHECK_IN(q_norm, (size_t)head_dim * 4, "q norm");
+    TM_CHECK_IN(k_norm, (size_t)head_dim * 4, "k norm");
+    TM_CHECK_AHEAD(inv_freq, (size_t)(n_rot / 2) * 4, "inv_freq");
+    TM_CHECK_IN(k_cache, plane, "k cache");
+    TM_CHECK_IN(v_cache, plane, "v cache");
     TM_CHECK_BUF(out, (size_t)heads * head_dim * 4, "attention output");
     TM_CHECK_BUF(pos_buf, ((size_t)pos_index + 1) * 4, "position");
     TM_CHECK_BUF(status, 4, "status");
+    tm_read_cache_ahead(ctx, k_cache, (const uint32_t *)pos_buf->dev + pos_index);
+    tm_read_cache_ahead(ctx, v_cache, (const uint32_t *)pos_buf->dev + pos_index);
     // Set-up, once per device, with that device current (TM_ENTER made it so).
     if (!g_static_decode_scratch_ptr[ctx->device].load(std::memory_order_acquire)) {
         unsigned char *p = nullptr;

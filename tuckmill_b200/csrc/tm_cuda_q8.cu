@@ -734,19 +734,17 @@ cudaError_t launch_cluster(tm_cuda_ctx *ctx, gemv_args a) {
     static std::atomic<int> clusters_of[64] = {};  // per device; contexts of a process share it
     const int dev = ctx->device;
     int clusters = dev >= 0 && dev < 64 ? clusters_of[dev].load(std::memory_order_acquire) : 0;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kClusterCtas;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.blockDim = dim3(kClusterThreads);
-    cfg.attrs = at;
     if (clusters == 0) {
         const int most = (int)ctx->smem_optin - 4096;
         cudaError_t e = cudaFuncSetAttribute(q8_gemv_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kClusterCtas;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.blockDim = dim3(kClusterThreads);
         cfg.gridDim = dim3((unsigned)ctx->sm_count / kClusterCtas * kClusterCtas);
         cfg.dynamicSmemBytes = (size_t)most;  // one CTA on an SM
         cfg.numAttrs = 1;
@@ -762,11 +760,9 @@ cudaError_t launch_cluster(tm_cuda_ctx *ctx, gemv_args a) {
     const uint32_t tiles_max = (n_tiles + used - 1u) / used, owned = (tiles_max + kClusterCtas - 1u) / kClusterCtas;
     const size_t smem = token_smem(local, a.plane) + (size_t)tiles_max * kClusterWarps * 64u + (size_t)kClusterCtas * owned * 64u +
                         (size_t)kClusterWarps * kRing * kRingChunk;
-    cfg.gridDim = dim3(used * kClusterCtas);
-    cfg.dynamicSmemBytes = smem < 120u * 1024u ? 120u * 1024u : smem;  // one CTA on an SM
-    cfg.stream = ctx->stream;
-    cfg.numAttrs = ctx->pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, q8_gemv_cluster_kernel, a, tiles_max);
+    return tm_launch_cluster_pdl(ctx, kClusterCtas, q8_gemv_cluster_kernel, dim3(used * kClusterCtas), dim3(kClusterThreads),
+                                 smem < 120u * 1024u ? 120u * 1024u : smem,  // one CTA on an SM
+                                 a, tiles_max);
 }
 
 template <int M, int kSlots, int H, bool kAdd, bool kPaired>
@@ -1122,7 +1118,7 @@ static int gemv_common(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, t
     if (prologue < TM_CUDA_PRO_NONE || prologue > TM_CUDA_PRO_GELU_MUL ||
         (epilogue != TM_CUDA_EPI_STORE && epilogue != TM_CUDA_EPI_ADD))
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "unknown prologue/epilogue");
-    if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_BUF(pro, (size_t)cols * 4, "norm weight");
+    if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_IN(pro, (size_t)cols * 4, "norm weight");
     if (prologue == TM_CUDA_PRO_SILU_MUL || prologue == TM_CUDA_PRO_GELU_MUL)
         TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate multiplicand");
     gemv_args a;
@@ -1182,9 +1178,9 @@ int tm_cuda_q8_0_gemv_addnorm(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffe
                        kThreads * 16);
     TM_CHECK_BUF(x, (size_t)cols * 4, "x");
     TM_CHECK_BUF(add_p, (size_t)cols * 4, "vector to add");
-    TM_CHECK_BUF(add_w, (size_t)cols * 4, "its norm weight");
+    TM_CHECK_IN(add_w, (size_t)cols * 4, "its norm weight");
     TM_CHECK_BUF(x_out, (size_t)cols * 4, "x output");
-    TM_CHECK_BUF(norm_w, (size_t)cols * 4, "norm weight");
+    TM_CHECK_IN(norm_w, (size_t)cols * 4, "norm weight");
     TM_CHECK_BUF(y, (size_t)rows * 4, "output");
     if (x_out == x || x_out->dev == x->dev)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "x_out must be a buffer other than x (every CTA reads x)");

@@ -316,20 +316,7 @@ cudaError_t launch_rows(tm_cuda_ctx *ctx, const rows_args &args, const rows_plan
     const uint32_t per_sm = 2u * (smem + 1024u) <= 228u * 1024u ? 2u : 1u;
     uint32_t clusters = (uint32_t)ctx->sm_count * per_sm / pl.p;
     if (clusters > a.units) clusters = a.units;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(clusters * pl.p);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = pl.p;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = ctx->pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, q8_gemm_rows_kernel<NT>, a);
+    return tm_launch_cluster_pdl(ctx, pl.p, q8_gemm_rows_kernel<NT>, dim3(clusters * pl.p), dim3(kThreads), smem, a);
 }
 
 }  // namespace
@@ -403,7 +390,7 @@ int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *
         a.x = (const __half *)x->dev;
     } else {
         TM_CHECK_BUF(x, (size_t)batch * cols * 4, "activation");
-        if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_BUF(pro, (size_t)cols * 4, "norm weight");
+        if (prologue == TM_CUDA_PRO_RMSNORM) TM_CHECK_IN(pro, (size_t)cols * 4, "norm weight");
         else if (prologue != TM_CUDA_PRO_NONE) TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate operand");
         a.x = (const __half *)ctx->mma_scratch;
     }

@@ -171,7 +171,7 @@ def load_library() -> C.CDLL:
     L.tm_cuda_q8_0_packed_bytes.argtypes = [_U32, _U32]
     L.tm_cuda_graph_free.argtypes = [_P, _P]
     for name in ("committed_dispatches", "completed_dispatches", "gpu_nanos_total", "allocated_bytes",
-                 "in_flight_bytes", "kernel_launches"):
+                 "in_flight_bytes", "kernel_launches", "ordered_launches"):
         fn = getattr(L, "tm_cuda_" + name)
         fn.restype = C.c_uint64
         fn.argtypes = [_P]
@@ -637,6 +637,7 @@ class CudaContext:
     def allocated_bytes(self) -> int: return int(self._l.tm_cuda_allocated_bytes(self.handle))
     def in_flight_bytes(self) -> int: return int(self._l.tm_cuda_in_flight_bytes(self.handle))
     def kernel_launches(self) -> int: return int(self._l.tm_cuda_kernel_launches(self.handle))
+    def ordered_launches(self) -> int: return int(self._l.tm_cuda_ordered_launches(self.handle))
     def stream(self) -> int: return int(self._l.tm_cuda_stream(self.handle) or 0)
     def set_profiling(self, enabled: bool): self._l.tm_cuda_profile_set(self.handle, int(enabled))
 
