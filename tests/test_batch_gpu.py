@@ -312,6 +312,28 @@ def test_larger_batches_on_the_tensor_core_path_match_the_oracle(ctx, oracle, ar
                 assert int(np.argmax(rows[j][s])) == oracle.argmax(ref)
 
 
+# What is left of a prompt after its full chunks of 16: 1, 4 and 8 rows (multiplied apart from the other prompts where
+# layers end in output norms, as in the prompt's own passes), none, or a prompt that is nothing else.
+@pytest.mark.parametrize("first", [17, 20, 40, 32, 5])
+@pytest.mark.parametrize("second", [16, 3])
+def test_first_logits_of_a_packed_prompt_are_its_own_request(ctx, tmp_path_factory, first, second):
+    shape = T.DecoderShape("gemma3", 6, 128, 384, 4, 1, 256, 512, rope_base=1e6, window=40, tied_head=True, context=512)
+    path = tmp_path_factory.mktemp("gguf") / "fused_gemma3.gguf"
+    T.write_gguf(path, shape, seed=3, norm_jitter=0.1)
+    prompts = [T.token_ids(30 + i, n, shape.vocab) for i, n in enumerate((first, second))]
+    one = E.Engine(path, context=64, prefill_batch=16)
+    one.prefill(prompts[0])
+    want = one.logits()
+    tokens = [one.generate(p, 6)[0] for p in prompts]
+    one.close()
+    eng = E.Engine(path, context=64, prefill_batch=16, sequences=2)
+    eng.generate_batch(prompts, 1)
+    np.testing.assert_array_equal(eng.logits(), want)
+    for got, alone in zip(eng.generate_batch(prompts, 6)[0], tokens):
+        np.testing.assert_array_equal(got, alone)
+    eng.close()
+
+
 @pytest.mark.parametrize("exact", [True, False])
 def test_generate_batch_equals_one_request_at_a_time(ctx, artifact, exact):
     path, shape = artifact

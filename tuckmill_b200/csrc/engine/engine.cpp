@@ -1468,33 +1468,34 @@ bool EngineModel::packs_prompts() const {
 // prompt of 200 tokens with multiplies that cost nearly as much as those of 512 (27 against 23 us for a 1024 x 3072
 // projection, 27 launches a layer against 8): 32 prompts of 100 to 400 tokens
 // and 64 tokens each on the 0.6B shape took 178 ms, now 129; on 8 layers of the 8B shape 107, now 73.
-// A prompt of under nine tokens whose pass multiplies in the exact form (Layer::prefill with output norms) keeps it.
+// Under nine rows that a prompt's own passes would multiply in the exact form (Layer::prefill with output norms: a short
+// prompt, or what is left of one after its full chunks) keep a pass of their own: the first logits come from them.
 void EngineModel::prefill_packed(const std::vector<std::vector<uint32_t>> &prompts) {
     Impl &I = *impl_;
     const CudaContext &c = *ctx_;
     const size_t R = prompts.size(), hidden = graph_.hidden, batch = std::min<size_t>(opts_.prefill_batch, capacity_);
-    size_t own_pass = 1;  // prompts shorter than this keep a pass of their own
+    size_t own_pass = 1;  // fewer rows than this at the end of a prompt are not packed
     for (const Layer &L : I.layers)
         if (L.mixer_out_norm) own_pass = 9;
-    for (size_t s = 0; s < R; ++s) check_prompt(s, prompts[s].data(), prompts[s].size());
+    std::vector<size_t> packed(R);  // tokens of each prompt that share passes
+    for (size_t i = 0; i < R; ++i) {
+        const size_t n = prompts[i].size(), tail = n % batch;
+        check_prompt(i, prompts[i].data(), n);
+        packed[i] = n - (tail < own_pass ? tail : 0);
+        I.kv_rows = std::max(I.kv_rows, I.pos_b[i] + n);
+    }
     const CudaBuffer &last = I.scratch.h;  // [sequence][hidden]: the row of each prompt's last token (unused by the fused form)
     size_t s = 0, t0 = 0;                  // the next token: t0 of prompt s
-    while (s < R) {
-        if (t0 == 0 && prompts[s].size() < own_pass) {
-            const size_t n = prompts[s].size();
-            prefill_seq(s, prompts[s].data(), n, false);
-            I.pos_b[s] -= n;  // (all positions advance together below)
-            c.copy_f32(I.scratch.x, (uint32_t)((n - 1) % batch * hidden), last, (uint32_t)(s * hidden), (uint32_t)hidden);
-            ++s;
-            continue;
-        }
+    auto skip = [&] {
+        while (s < R && t0 == packed[s]) ++s, t0 = 0;
+    };
+    for (skip(); s < R;) {
         RowsAre rows;
         size_t n = 0;
         std::vector<std::pair<size_t, size_t>> ends;  // (row, sequence) of the prompts that end in this pass
         c.burst([&] {
-            while (s < R && n < batch && rows.runs.size() < TM_CUDA_PREFILL_SEGMENTS &&
-                   (t0 > 0 || prompts[s].size() >= own_pass)) {
-                const size_t k = std::min(batch - n, prompts[s].size() - t0), at = I.pos_b[s] + t0;
+            while (s < R && n < batch && rows.runs.size() < TM_CUDA_PREFILL_SEGMENTS) {
+                const size_t k = std::min(batch - n, packed[s] - t0), at = I.pos_b[s] + t0;
                 const uint32_t slot = (uint32_t)(s * I.log_stride + at);
                 I.tokens.store_u32(slot, prompts[s].data() + t0, k);
                 c.rows_indirect(I.embedding.buf, I.embedding.rows, I.embedding.cols, I.tokens, slot, (uint32_t)k,
@@ -1502,17 +1503,21 @@ void EngineModel::prefill_packed(const std::vector<std::vector<uint32_t>> &promp
                 rows.runs.push_back({(uint32_t)s, (uint32_t)at, (uint32_t)k});
                 n += k;
                 t0 += k;
-                if (t0 == prompts[s].size()) {
-                    ends.emplace_back(n - 1, s);
-                    I.kv_rows = std::max(I.kv_rows, I.pos_b[s] + t0);
-                    ++s;
-                    t0 = 0;
-                }
+                if (t0 == prompts[s].size()) ends.emplace_back(n - 1, s);
+                skip();
             }
             for (const Layer &L : I.layers) L.prefill(c, I.scratch, n, 0, hidden, graph_.eps, false, rows);
             for (const auto &e : ends)
                 c.copy_f32(I.scratch.x, (uint32_t)(e.first * hidden), last, (uint32_t)(e.second * hidden), (uint32_t)hidden);
         });
+    }
+    for (s = 0; s < R; ++s) {
+        const size_t at = packed[s], n = prompts[s].size() - at;
+        if (n == 0) continue;
+        I.pos_b[s] += at;
+        prefill_seq(s, prompts[s].data() + at, n, false);
+        I.pos_b[s] -= prompts[s].size();  // (all positions advance together below)
+        c.copy_f32(I.scratch.x, (uint32_t)((n - 1) * hidden), last, (uint32_t)(s * hidden), (uint32_t)hidden);
     }
     c.burst([&] {
         std::vector<uint32_t> pos(R);
