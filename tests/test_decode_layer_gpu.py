@@ -39,6 +39,49 @@ def test_cluster_attention_equals_the_exact_form(ctx, oracle, heads, kvh, hd, wi
     assert int(status.download(0, 4, np.uint32)[0]) == 0
 
 
+# A row whose sum of squares overflows is normed with 1 / infinity: zeros, in every form.
+@pytest.mark.parametrize("heads,kvh,hd", [(4, 2, 128), (4, 1, 256)])
+@pytest.mark.parametrize("big", ["q", "k"])
+def test_attention_of_a_row_beyond_the_range_of_its_norm(ctx, oracle, heads, kvh, hd, big):
+    cap, pos, eps, scale = 300, 200, 1e-6, 1.0 / np.sqrt(np.float32(hd))
+    qn = ctx.floats((1 + 0.1 * T.activations(0, 20, hd)).astype(np.float32))
+    inv, pb = ctx.floats(oracle.rope_inv_freq(hd, 1e6)), ctx.from_array(np.array([pos], np.uint32))
+    fill = [T.activations(1, t, kvh * cap * hd).astype(np.float16) for t in (1, 2)]
+    q, k, v = (T.activations(7, t, n * hd) * np.float32(1e25 if name == big else 1)
+               for name, t, n in (("q", 30, heads), ("k", 31, kvh), ("v", 32, kvh)))
+    status = ctx.buffer(4, shared=True)
+    status.zero()
+    scratch = ctx.buffer(cuda.decode_attention_scratch_bytes(heads, kvh, hd, cap))
+    outs = []
+    for exact in (True, False):
+        scratch.zero()
+        kc, vc, out = ctx.from_array(fill[0]), ctx.from_array(fill[1]), ctx.buffer(heads * hd * 4)
+        ctx.attention_decode_dev(ctx.floats(q), ctx.floats(k), ctx.floats(v), qn, qn, inv, kc, vc, out, scratch, pb, 0, status,
+                                 heads, kvh, hd, hd, cap, 0, eps, scale, exact)
+        outs.append(out.download(0, heads * hd * 4, np.float32))
+        new = kc.download(0, fill[0].nbytes, np.float16).reshape(kvh, cap, hd)[:, pos]
+        assert np.all(new == 0) if big == "k" else np.all(np.isfinite(new))
+    assert rel_err(outs[1], outs[0]) <= 2e-5  # (as for rows of an ordinary size, above)
+    if big == "q":  # every key weighs the same
+        vals = fill[1].astype(np.float64).reshape(kvh, cap, hd)[:, :pos]
+        mean = (vals.sum(axis=1) + v.reshape(kvh, hd).astype(np.float16)) / (pos + 1)
+        assert rel_err(outs[1].reshape(kvh, heads // kvh, hd), np.repeat(mean[:, None], heads // kvh, axis=1)) <= 2e-5
+
+
+def test_feed_forward_block_of_a_row_beyond_the_range_of_its_norm(ctx):
+    hidden, width = 1024, 3072
+    gu, dn = ctx.q8_0_matrix(T.q8_0_matrix(3, 1, 2 * width, hidden), 2 * width, hidden), ctx.q8_0_matrix(T.q8_0_matrix(3, 2, hidden, width), hidden, width)
+    one, xo, so = ctx.floats(np.ones(hidden)), ctx.buffer(hidden * 4), ctx.buffer(8 * hidden * 4)
+    x = T.activations(3, 3, hidden)
+    # the slots' sum under its output norm: adds nothing
+    ctx.decode_ffn_block(ctx.floats(x), ctx.floats(np.full(hidden, 1e25)), 1, one, one, xo, gu, dn, so, hidden, width, False, 1e-6)
+    np.testing.assert_array_equal(xo.download(0, hidden * 4, np.float32), x)
+    assert np.all(np.isfinite(so.download(0, 8 * hidden * 4, np.float32)))
+    # the stream itself under the block's input norm: the block adds nothing
+    ctx.decode_ffn_block(ctx.floats(x * np.float32(1e25)), None, 0, None, one, xo, gu, dn, so, hidden, width, False, 1e-6)
+    assert np.all(so.download(0, 8 * hidden * 4, np.float32) == 0)
+
+
 def f64_layer(x, slots, add_w, norm_w, eps):
     p = slots.astype(np.float64).sum(axis=0) if slots is not None else 0.0
     if add_w is not None:
