@@ -60,6 +60,34 @@ def test_runs_against_float32(ctx, heads, kv, hd, n_rot, window, runs):
         assert np.mean(have != want.numpy()) < 0.02
 
 
+# Any scale: zero (every visible key weighs the same) and negative ones, whose largest score is the smallest product.
+@pytest.mark.parametrize("scale", [0.0, -0.5, 0.5])
+@pytest.mark.parametrize("hd,window", [(128, 0), (128, 33), (256, 0), (64, 33)])
+def test_scales_of_any_sign(ctx, scale, hd, window):
+    heads, kv, cap, pos0, n = 4, 2, 128, 40, 70
+    g = torch.Generator().manual_seed(hd)
+    q, k, v = (torch.randn(n, m, hd, generator=g) for m in (heads, kv, kv))
+    one, freq = torch.ones(hd), 10000.0 ** (-torch.arange(hd // 2) * 2.0 / hd)
+    kc, vc = (torch.randn(1, kv, cap, hd, generator=g).half() for _ in range(2))
+    bufs = [ctx.from_array(t.numpy()) for t in (q, k, v, one, one, freq.float(), kc, vc)]
+    out = ctx.buffer(n * heads * hd * 4)
+    pos = torch.arange(pos0, pos0 + n)
+    ctx.attention_prefill(*bufs, out, heads, kv, hd, hd, cap, window, 1e-6, scale, [(0, pos0, n)], False)
+    got = [out.download(0, n * heads * hd * 4, np.float32).reshape(n, heads, hd)]
+    qq = norm_rope(q.clone(), one, freq, pos, hd, 1e-6)
+    ctx.attention_chunk_mma(ctx.floats(qq.numpy()), bufs[6], bufs[7], out, heads, pos0, cap, hd, heads // kv, scale, n, window)
+    got.append(out.download(0, n * heads * hd * 4, np.float32).reshape(n, heads, hd))
+    kc[0, :, pos0:pos0 + n] = norm_rope(k.clone(), one, freq, pos, hd, 1e-6).transpose(0, 1).half()
+    vc[0, :, pos0:pos0 + n] = v.transpose(0, 1).half()
+    keys, vals = (c[0, :, :pos0 + n].float().repeat_interleave(heads // kv, 0) for c in (kc, vc))
+    j = torch.arange(pos0 + n)
+    hidden = (j > pos[:, None]) | ((j + window <= pos[:, None]) if window else torch.zeros(1, 1, dtype=torch.bool))
+    p = (qq.transpose(0, 1) @ keys.transpose(1, 2) * scale).masked_fill(hidden, float("-inf")).softmax(-1)
+    want = (p @ vals).transpose(0, 1).numpy()
+    for have in got:  # scores to 2^-12 sqrt(hd) / 2 (binary16 queries), weights to 2^-11
+        assert np.abs(have - want).max() <= 4e-3 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("lengths", [[40, 3, 17], [1, 1, 1], [16, 16, 33], [7, 50, 9]])
 @pytest.mark.parametrize("shape", [T.SMALL_QWEN3, T.TINY_GEMMA3], ids=["qwen3", "gemma3"])
 def test_shared_passes_give_the_tokens_of_passes_of_their_own(tmp_path, shape, lengths):

@@ -71,7 +71,8 @@ struct attn_args {
     void *out;  // [rows][heads][HD], f32 or binary16
     size_t seq_stride;
     uint32_t heads, group, cap, window, n_rot, out_f16;
-    float scale_log2e, eps;
+    float scale_log2e, eps;  // the scale's magnitude: its sign multiplies the queries (attn_scale)
+    float q_sign;
     attn_segs segs;
 };
 
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 const uint32_t e = lane + 32u * i;
-                *(__half *)(sQ + sw<C::kQPitch>(r, e >> 3) + (e & 7u) * 2u) = __float2half_rn(in ? x[i] : 0.0f);
+                *(__half *)(sQ + sw<C::kQPitch>(r, e >> 3) + (e & 7u) * 2u) = __float2half_rn(in ? x[i] * a.q_sign : 0.0f);
             }
         }
     } else {
@@ -212,7 +213,9 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
             uint4 w = make_uint4(0, 0, 0, 0);
             if (q0 + r < n) {
                 const float *src = a.q + ((size_t)(row0 + q0 + r) * a.heads + head) * HD + c * 8;
-                const float4 f0 = *(const float4 *)src, f1 = *(const float4 *)(src + 4);
+                float4 f0 = *(const float4 *)src, f1 = *(const float4 *)(src + 4);
+                f0.x *= a.q_sign, f0.y *= a.q_sign, f0.z *= a.q_sign, f0.w *= a.q_sign;
+                f1.x *= a.q_sign, f1.y *= a.q_sign, f1.z *= a.q_sign, f1.w *= a.q_sign;
                 w = make_uint4(pack_h2(f0.x, f0.y), pack_h2(f0.z, f0.w), pack_h2(f1.x, f1.y), pack_h2(f1.z, f1.w));
             }
             *(uint4 *)(sQ + sw<C::kQPitch>(r, c)) = w;
@@ -836,6 +839,13 @@ cudaError_t launch_decode_mma(tm_cuda_ctx *ctx, const decode_mma_args &a, uint32
     return tm_launch_pdl(ctx, attention_decode_mma_kernel<G, HD, kDecodeStages>, grid, dim3(kThreads), kBytes, a);
 }
 
+// The kernel masks scores with -inf and takes their maximum before it scales them, which needs a positive factor: a
+// negative scale becomes its magnitude times negated queries, zero becomes any factor times zero queries.
+void attn_scale(attn_args &a, float scale) {
+    a.q_sign = scale < 0.0f ? -1.0f : scale == 0.0f ? 0.0f : 1.0f;
+    a.scale_log2e = (scale == 0.0f ? 1.0f : scale * a.q_sign) * 1.4426950408889634f;
+}
+
 attn_segs attn_segments(uint32_t pos0, uint32_t n) {
     attn_segs s;
     s.n = 1;
@@ -979,7 +989,7 @@ int tm_cuda_attention_chunk_mma(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buf
     a.cap = cap;
     a.window = window;
     a.seq_stride = 0;
-    a.scale_log2e = scale * 1.4426950408889634f;
+    attn_scale(a, scale);
     a.segs = attn_segments(pos0, n);
     TM_OP_BEGIN("attention_chunk_mma");
     cudaError_t e = head_dim == 32    ? launch_attn<32>(ctx, a)
@@ -1046,7 +1056,7 @@ int tm_cuda_attention_prefill(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffe
     a.window = window;
     a.n_rot = n_rot;
     a.eps = eps;
-    a.scale_log2e = scale * 1.4426950408889634f;
+    attn_scale(a, scale);
     TM_OP_BEGIN("attention_prefill");
     const dim3 grid(((uint32_t)rows * kv_heads + 7u) / 8u);
     auto store = [&](auto kernel) {
