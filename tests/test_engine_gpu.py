@@ -3,6 +3,8 @@ artifacts -- the policy of crates/tuckcore/src/executor.rs:2143-2321 (logits
 within 1e-2 * scale, equal top-1, equal greedy tokens) and the engine
 invariants of crates/tuckcore/src/engine/metal.rs:3682-3774 (prefill == decode,
 ledger == plan)."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -72,6 +74,32 @@ def test_greedy_generation_matches_oracle(ctx, oracle, artifact):
         bad = np.nonzero(got != ref)[0]
         assert bad.size == 0, f"first divergence at step {bad[0]} (oracle top-1 margin {margins[bad[0]]:.3g})"
         eng.close()
+
+
+@pytest.mark.parametrize("sequences", [1, 2])
+def test_a_request_that_ends_on_its_first_token_leaves_the_prompts_state(ctx, artifact, tmp_path, sequences):
+    path, shape = artifact
+    prompt = T.token_ids(13, 20, shape.vocab)
+    eng = E.Engine(path, context=64, prefill_batch=16)
+    eng.prefill(prompt)
+    want, eos = eng.logits(), eng.prefill_token()
+    after = eng.step(7)
+    tokens = eng.generate(prompt, 6)[0]
+    eng.close()
+    ends = tmp_path / "ends.gguf"
+    T.write_gguf(ends, dataclasses.replace(shape, extra_kv={"tokenizer.ggml.eos_token_id": eos}), seed=3, norm_jitter=0.1)
+    eng = E.Engine(ends, context=64, prefill_batch=16, sequences=sequences)
+    if sequences == 1:
+        got, stats = eng.generate(prompt, 6, ignore_eos=False)
+    else:
+        (got, other), stats = eng.generate_batch([prompt, prompt], 6, ignore_eos=False)
+        assert other.tolist() == [eos]
+    assert got.tolist() == [eos]
+    np.testing.assert_array_equal(eng.logits(), want)
+    if sequences == 1:
+        np.testing.assert_array_equal(eng.step(7), after)  # at the position behind the prompt
+        np.testing.assert_array_equal(eng.generate(prompt, 6)[0], tokens)
+    eng.close()
 
 
 def test_ledger_equals_plan_and_info(ctx, artifact):

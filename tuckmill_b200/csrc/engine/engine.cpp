@@ -1613,9 +1613,8 @@ std::vector<std::vector<uint32_t>> EngineModel::generate_batch(const std::vector
     } else {
         for (size_t s = 0; s < R; ++s) prefill_seq(s, prompts[s].data(), prompts[s].size(), true);
     }
-    auto is_stop = [&](uint32_t t) {
-        return t == 0xFFFFFFFFu || (!ignore_eos && graph_.has_eos && t == graph_.eos_token_id);
-    };
+    const bool may_stop = !ignore_eos && graph_.has_eos;
+    auto is_stop = [&](uint32_t t) { return t == 0xFFFFFFFFu || (may_stop && t == graph_.eos_token_id); };
     std::vector<char> done(R, 0);
     // A step advances every sequence on the device; the host follows the ones still wanted.  Step
     // i + 1 is submitted before step i is read (executor.rs:1080-1087), so a sequence that stops runs
@@ -1644,7 +1643,9 @@ std::vector<std::vector<uint32_t>> EngineModel::generate_batch(const std::vector
     };
     std::vector<Flight> inflight;
     const uint64_t prefilled = ctx_->committed();
-    if (I.sh.world <= 1 && any_wants()) inflight.push_back(submit());
+    // The first step needs no token read before it, unless every request may end on its first token: the step would
+    // then move the state past the prompts.
+    if (I.sh.world <= 1 && !may_stop && any_wants()) inflight.push_back(submit());
     for (size_t s = 0; s < R; ++s) {
         uint32_t tok = 0;
         const size_t at = s * I.log_stride + I.pos_b[s];
@@ -1748,8 +1749,9 @@ std::vector<uint32_t> EngineModel::generate(const uint32_t *prompt, size_t n_pro
     const uint64_t t_start = now_ns();
     reset();
     prefill(prompt, n_prompt, true);
-    // Step i+1 is submitted before step i is collected (executor.rs:1080-1087), the first one before the prompt's
-    // own token is read: the device already has token i in its log.
+    // Step i+1 is submitted before step i is collected (executor.rs:1080-1087): the device already has token i in its
+    // log.  So is the first one before the prompt's own token is read, unless the request may end on that token: its
+    // position and logits are then the prompt's.
     std::vector<Ticket> inflight;
     size_t submitted = 0;
     const size_t want = max_new - 1;
@@ -1757,17 +1759,17 @@ std::vector<uint32_t> EngineModel::generate(const uint32_t *prompt, size_t n_pro
     const size_t first_slot = pos_;
     const uint64_t first_dispatch = ctx_->committed();
     const uint32_t first_split = impl_->sh.world > 1 ? prefill_token() : 0u;  // a split model's prefill has no mirror
-    if (can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
+    const bool may_stop = !ignore_eos && graph_.has_eos;
+    if (!may_stop && can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
     uint32_t tok = impl_->sh.world > 1 ? first_split : collect_greedy(Ticket{first_dispatch, first_slot});
     const uint64_t t_first = now_ns();
     uint64_t t_last = t_first;
-    auto is_stop = [&](uint32_t t) {
-        return t == 0xFFFFFFFFu || (!ignore_eos && graph_.has_eos && t == graph_.eos_token_id);
-    };
+    auto is_stop = [&](uint32_t t) { return t == 0xFFFFFFFFu || (may_stop && t == graph_.eos_token_id); };
     out.push_back(tok);
     if (tok == 0xFFFFFFFFu)
         throw TuckmillError(ErrorCode::Internal, "every logit was NaN; refusing to guess a token");
     if (!is_stop(tok)) {
+        if (inflight.empty() && can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
         while (!inflight.empty()) {
             if (can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
             const Ticket t = inflight.front();
