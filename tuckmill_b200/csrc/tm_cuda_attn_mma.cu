@@ -198,13 +198,14 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
             float x[R];
             const bool in = q0 + r < n;
             const float *src = a.q + ((size_t)(row0 + (in ? q0 + r : q0)) * a.heads + head) * HD;
+            const float sign = in ? a.q_sign : 0.0f;
 #pragma unroll
             for (int i = 0; i < R; ++i) x[i] = src[lane + 32 * i];
             norm_rope_row<R>(x, a.q_norm, a.inv_freq, a.n_rot, pos0 + q0 + r, a.eps, lane);
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 const uint32_t e = lane + 32u * i;
-                *(__half *)(sQ + sw<C::kQPitch>(r, e >> 3) + (e & 7u) * 2u) = __float2half_rn(in ? x[i] * a.q_sign : 0.0f);
+                *(__half *)(sQ + sw<C::kQPitch>(r, e >> 3) + (e & 7u) * 2u) = __float2half_rn(x[i] * sign);
             }
         }
     } else {
