@@ -152,3 +152,30 @@ def test_attention_block_equals_the_operators_it_replaces(ctx, oracle, hidden, h
     ctx.decode_attn_block(ctx.floats(x), None, 0, None, ctx.floats(nw), xo, qkv, o, qn, kn, inv, kc2, vc2, pb, 0, status, so,
                           hidden, heads, kvh, hd, cap, window, eps, scale)
     assert int(status.download(0, 4, np.uint32)[0]) == 1
+
+
+@pytest.mark.parametrize("block", ["attention", "feed-forward"])
+def test_blocks_refuse_outputs_in_what_other_clusters_read(ctx, oracle, block):
+    hidden, width, heads, kvh, hd, cap = 256, 1024, 4, 2, 128, 64
+    vec = lambda: ctx.floats(np.ones(hidden))  # noqa: E731
+    x, nw, aw, xo, arena = vec(), vec(), vec(), vec(), ctx.floats(np.zeros(20 * hidden))
+    slots, out = arena.view(0, 8 * hidden * 4), arena.view(8 * hidden * 4, 8 * hidden * 4)
+    if block == "attention":
+        rows = (heads + 2 * kvh) * hd
+        qkv, o = ctx.q8_0_matrix(T.q8_0_matrix(4, 1, rows, hidden), rows, hidden), ctx.q8_0_matrix(T.q8_0_matrix(4, 2, hidden, heads * hd), hidden, heads * hd)
+        kc, vc, status = ctx.buffer(kvh * cap * hd * 2), ctx.buffer(kvh * cap * hd * 2), ctx.buffer(4, shared=True)
+        kc.zero(), vc.zero(), status.zero()
+        qn, inv, pb = ctx.floats(np.ones(hd)), ctx.floats(oracle.rope_inv_freq(hd, 1e6)), ctx.from_array(np.zeros(1, np.uint32))
+        call = lambda xo, so: ctx.decode_attn_block(x, slots, 2, aw, nw, xo, qkv, o, qn, qn, inv, kc, vc, pb, 0, status, so,  # noqa: E731
+                                                    hidden, heads, kvh, hd, cap, 0, 1e-6, hd ** -0.5)
+    else:
+        gu, dn = ctx.q8_0_matrix(T.q8_0_matrix(3, 1, 2 * width, hidden), 2 * width, hidden), ctx.q8_0_matrix(T.q8_0_matrix(3, 2, hidden, width), hidden, width)
+        call = lambda xo, so: ctx.decode_ffn_block(x, slots, 2, aw, nw, xo, gu, dn, so, hidden, width, False, 1e-6)  # noqa: E731
+    call(xo, out)
+    row = hidden * 4
+    for bad_xo, bad_so in ((x, out), (arena.view(row, row), out), (nw, out), (aw, out), (xo, slots), (xo, arena.view(row, 8 * row))):
+        with pytest.raises(cuda.CudaError) as e:
+            call(bad_xo, bad_so)
+        assert e.value.code == -5
+    call(xo, arena.view(2 * row, 8 * row))  # behind the two slots that are read
+    ctx.fence()

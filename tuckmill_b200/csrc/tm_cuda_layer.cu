@@ -634,16 +634,29 @@ bool ffn_shape_ok(uint32_t hidden, uint32_t width) {
 }
 
 int check_residual(tm_cuda_ctx *ctx, residual_in &r, tm_cuda_buffer *x, tm_cuda_buffer *slots, uint32_t n_slots,
-                   tm_cuda_buffer *add_w, tm_cuda_buffer *norm_w, tm_cuda_buffer *x_out, uint32_t hidden, float eps,
-                   char *err, size_t err_cap) {
+                   tm_cuda_buffer *add_w, tm_cuda_buffer *norm_w, tm_cuda_buffer *x_out, tm_cuda_buffer *slots_out,
+                   uint32_t n_slots_out, uint32_t hidden, float eps, char *err, size_t err_cap) {
+    const size_t slots_out_bytes = (size_t)n_slots_out * hidden * 4;
+    TM_CHECK_BUF(slots_out, slots_out_bytes, "slots output");
     TM_CHECK_BUF(x, (size_t)hidden * 4, "x");
     TM_CHECK_BUF(x_out, (size_t)hidden * 4, "x output");
     TM_CHECK_AHEAD(norm_w, (size_t)hidden * 4, "norm weight");
     if (n_slots > kSlots) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "%u slots, at most %u", n_slots, kSlots);
     if (n_slots) TM_CHECK_BUF(slots, (size_t)n_slots * hidden * 4, "slots");
     if (add_w) TM_CHECK_AHEAD(add_w, (size_t)hidden * 4, "output norm weight");
-    if (x_out->dev == x->dev)
-        return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "x_out must be a buffer other than x (every cluster reads x)");
+    // Every cluster reads the stream, the slots and the weights while others may have finished.
+    const size_t row = (size_t)hidden * 4;
+    const struct {
+        const tm_cuda_buffer *buf;
+        size_t bytes;
+        const char *name;
+    } in[4] = {{x, row, "x"}, {n_slots ? slots : nullptr, n_slots * row, "slots_in"}, {norm_w, row, "norm_w"}, {add_w, row, "add_w"}},
+      out[2] = {{x_out, row, "x_out"}, {slots_out, slots_out_bytes, "slots_out"}};
+    for (const auto &o : out)
+        for (const auto &i : in)
+            if (i.buf && o.buf->dev < i.buf->dev + i.bytes && i.buf->dev < o.buf->dev + o.bytes)
+                return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "%s must be a buffer other than %s (every cluster reads it)",
+                               o.name, i.name);
     if (((size_t)x->dev | (size_t)x_out->dev | (size_t)norm_w->dev | (n_slots ? (size_t)slots->dev : 0) | (add_w ? (size_t)add_w->dev : 0)) & 15u)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "residual operands are not 16-byte aligned");
     r.x = (const float *)x->dev;
@@ -680,7 +693,7 @@ int tm_cuda_decode_attn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffe
     int rc = tm_check_packed(ctx, qkv, (heads + 2 * kv_heads) * head_dim, hidden, err, err_cap);
     if (rc == TM_CUDA_OK) rc = tm_check_packed(ctx, o, hidden, heads * head_dim, err, err_cap);
     attn_block_args a = {};
-    if (rc == TM_CUDA_OK) rc = check_residual(ctx, a.in, x, slots_in, n_slots, add_w, norm_w, x_out, hidden, eps, err, err_cap);
+    if (rc == TM_CUDA_OK) rc = check_residual(ctx, a.in, x, slots_in, n_slots, add_w, norm_w, x_out, slots_out, kv_heads, hidden, eps, err, err_cap);
     if (rc != TM_CUDA_OK) return rc;
     const size_t plane = (size_t)kv_heads * cap * head_dim * 2;
     TM_CHECK_AHEAD(q_norm, (size_t)head_dim * 4, "q norm");
@@ -692,7 +705,6 @@ int tm_cuda_decode_attn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffe
     TM_CHECK_BUF(status, 4, "status");
     tm_read_cache_ahead(ctx, k_cache, (const uint32_t *)pos_buf->dev + pos_index);
     tm_read_cache_ahead(ctx, v_cache, (const uint32_t *)pos_buf->dev + pos_index);
-    TM_CHECK_BUF(slots_out, (size_t)kv_heads * hidden * 4, "slots output");
     a.qkv_q = (const signed char *)qkv->qp;
     a.qkv_d = (const unsigned short *)qkv->dp;
     a.o_q = (const signed char *)o->qp;
@@ -733,9 +745,8 @@ int tm_cuda_decode_ffn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffer
     int rc = tm_check_packed(ctx, gate_up, 2 * width, hidden, err, err_cap);
     if (rc == TM_CUDA_OK) rc = tm_check_packed(ctx, down, hidden, width, err, err_cap);
     ffn_args a = ffn_shape(hidden, width);
-    if (rc == TM_CUDA_OK) rc = check_residual(ctx, a.in, x, slots_in, n_slots, add_w, norm_w, x_out, hidden, eps, err, err_cap);
+    if (rc == TM_CUDA_OK) rc = check_residual(ctx, a.in, x, slots_in, n_slots, add_w, norm_w, x_out, slots_out, kSlots, hidden, eps, err, err_cap);
     if (rc != TM_CUDA_OK) return rc;
-    TM_CHECK_BUF(slots_out, (size_t)kSlots * hidden * 4, "slots output");
     a.gu_q = (const signed char *)gate_up->qp;
     a.gu_d = (const unsigned short *)gate_up->dp;
     a.dn_q = (const signed char *)down->qp;
