@@ -564,7 +564,8 @@ int tm_cuda_attention_decode_dev_static(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_
  *   feed-forward block: slots_out[c] = the c-th eighth of  down * (act(gate x') * up x'), x' = rmsnorm(x_out) * norm_w;
  *                       gate_up holds width gate rows above width up rows; TM_CUDA_DECODE_SLOTS slots.
  * The slots are for the next block's slots_in (or tm_cuda_reduce_ranks_add_f32).  x_out and slots_out share no storage
- * with x, slots_in or the norm weights: such a call is refused. */
+ * with x, slots_in or the norm weights: such a call is refused.  `supported`: whether the shape has these forms and the
+ * current device can hold their clusters. */
 #define TM_CUDA_DECODE_SLOTS 8
 int tm_cuda_decode_attn_block_supported(uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t head_dim, uint32_t n_rot);
 int tm_cuda_decode_ffn_block_supported(uint32_t hidden, uint32_t width);

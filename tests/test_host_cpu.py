@@ -109,6 +109,14 @@ def test_library_exports_every_declared_symbol():
     assert cuda.packed_bytes(3, 64) == 256 + 3 * 2 * 2 and cuda.packed_bytes(3, 48) == 0
 
 
+def test_decode_blocks_answer_for_a_shape_with_and_without_a_device():
+    lib = cuda.load_library()
+    assert lib.tm_cuda_decode_ffn_block_supported(1024, 3072) == 1 and lib.tm_cuda_decode_ffn_block_supported(4096, 12288) == 0
+    assert lib.tm_cuda_decode_attn_block_supported(1024, 16, 8, 128, 128) == 1
+    for shape in ((1024, 16, 8, 128, 64), (4096, 32, 8, 128, 128), (1024, 16, 0, 128, 128)):
+        assert lib.tm_cuda_decode_attn_block_supported(*shape) == 0
+
+
 def test_no_device_is_a_typed_refusal_not_a_fallback(tmp_path):
     if cuda.available() > 0:
         pytest.skip("a CUDA device is present")

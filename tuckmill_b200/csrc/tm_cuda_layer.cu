@@ -567,13 +567,44 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
 // ---------------- launches ----------------
 uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1u) / b; }
 
+template <class Kernel>
+cudaError_t allow_clusters(Kernel kernel, int smem_optin) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
+    return e == cudaSuccess ? cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : e;
+}
+
+// Whether the current device holds a cluster of the kernel with this much shared memory (16 CTAs are more than the
+// portable size); where there is no device, the shape alone decides.
+template <class Kernel>
+bool cluster_fits(Kernel kernel, size_t smem) {
+    int dev = 0, optin = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kC);
+    cfg.blockDim = dim3(kT);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kC;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const bool ok = smem <= (size_t)optin && allow_clusters(kernel, optin) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+    cudaGetLastError();
+    return ok;
+}
+
 template <class Kernel, class Args>
 cudaError_t launch_clusters(tm_cuda_ctx *ctx, Kernel kernel, std::atomic<bool> *attr_set, uint32_t clusters, size_t smem,
                             const Args &a, uint32_t ring_slots) {
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        const cudaError_t e = allow_clusters(kernel, (int)ctx->smem_optin);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
@@ -598,12 +629,23 @@ uint32_t attn_items(uint32_t hidden, uint32_t g, uint32_t hd) {
            ceil_div(ceil_div(hidden / 16u, kC) * (g * hd / 64u), kWarps);
 }
 template <int G, int HD>
+void attn_tiles(uint32_t hidden, uint32_t &tiles1, uint32_t &tiles2) {
+    tiles1 = ceil_div((G + 2) * HD / 16u, kC);
+    tiles2 = ceil_div(hidden / 16u, kC);
+}
+template <int G, int HD>
 cudaError_t launch_attn_any(tm_cuda_ctx *ctx, attn_block_args a) {
     const uint32_t H = a.in.hidden;
-    a.tiles1 = ceil_div((G + 2) * HD / 16u, kC);
-    a.tiles2 = ceil_div(H / 16u, kC);
+    attn_tiles<G, HD>(H, a.tiles1, a.tiles2);
     const uint32_t items = attn_items(H, G, HD);
     return H <= 1024u ? launch_attn<G, HD, 1>(ctx, a, items) : launch_attn<G, HD, 2>(ctx, a, items);
+}
+template <int G, int HD>
+bool attn_fits(uint32_t hidden) {
+    uint32_t t1, t2;
+    attn_tiles<G, HD>(hidden, t1, t2);
+    const size_t smem = attn_layout<G, HD>(hidden, t1, t2, attn_items(hidden, G, HD)).bytes;
+    return hidden <= 1024u ? cluster_fits(attn_block_kernel<G, HD, 1>, smem) : cluster_fits(attn_block_kernel<G, HD, 2>, smem);
 }
 
 // A block serves layers whose weights' pieces all stay in shared memory (0.6B shape: 6 and 9 a warp).  A layer that has
@@ -675,9 +717,22 @@ int check_residual(tm_cuda_ctx *ctx, residual_in &r, tm_cuda_buffer *x, tm_cuda_
 extern "C" {
 
 int tm_cuda_decode_attn_block_supported(uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t head_dim, uint32_t n_rot) {
-    return n_rot == head_dim && attn_shape(hidden, heads, kv_heads, head_dim);
+    if (n_rot != head_dim || !attn_shape(hidden, heads, kv_heads, head_dim)) return 0;
+    switch ((heads / kv_heads) * 1000 + head_dim) {
+        case 1128: return attn_fits<1, 128>(hidden);
+        case 2128: return attn_fits<2, 128>(hidden);
+        case 4128: return attn_fits<4, 128>(hidden);
+        case 1256: return attn_fits<1, 256>(hidden);
+        case 2256: return attn_fits<2, 256>(hidden);
+        default: return attn_fits<4, 256>(hidden);
+    }
 }
-int tm_cuda_decode_ffn_block_supported(uint32_t hidden, uint32_t width) { return ffn_shape_ok(hidden, width); }
+int tm_cuda_decode_ffn_block_supported(uint32_t hidden, uint32_t width) {
+    if (!ffn_shape_ok(hidden, width)) return 0;
+    const ffn_args a = ffn_shape(hidden, width);
+    const size_t smem = ffn_layout(hidden, a.acts, a.tiles1, a.tiles2, ffn_items(a)).bytes;
+    return hidden <= 1024u ? cluster_fits(ffn_block_kernel<1>, smem) : cluster_fits(ffn_block_kernel<2>, smem);
+}
 
 int tm_cuda_decode_attn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffer *slots_in, uint32_t n_slots,
                               tm_cuda_buffer *add_w, tm_cuda_buffer *norm_w, tm_cuda_buffer *x_out, tm_cuda_buffer *qkv,
