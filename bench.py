@@ -342,7 +342,8 @@ def gemm_rooflines(device, torch):
         tf = 2.0 * m * rows * cols / us / 1e6
         out.append({"bound": "tensor", "rows": rows, "cols": cols, "batch": m, "us_per_launch": us, "achieved": tf,
                     "peak": peak, "unit": "TFLOP/s", "frac": tf / peak, "traffic": None,
-                    "kernel": "x_to_f16_kernel + q8_gemm_mma_kernel<%d>" % ctx.mma_last_tile(),
+                    "kernel": "x_to_f16_kernel + q8_gemm_mma_kernel (token sub-tile %d, %d converter sets)" % (
+                        ctx.mma_last_tile(), ctx.mma_last_sets()),
                     "weights": "%d copies in turn (%.0f MB)" % (copies, copies * rows * cols * 1.0625 / 1e6),
                     "peak_source": "MEASURED_PEAKS.json bf16_tflops (%s), burst" % kind})
         for b in ws + [x, y]:

@@ -197,9 +197,11 @@ int tm_cuda_mma_workspace_reserve(tm_cuda_ctx *ctx, size_t bytes, char *err, siz
  * bounded pipeline waits (its output is then undefined); waits for the stream. */
 int tm_cuda_mma_aborted(tm_cuda_ctx *ctx);
 /* No counterpart: which instantiation of the tensor-core kernel the context's last GEMM
- * launch used, as its token sub-tile width (64, 128 or 192; 0 before the first launch).
+ * launch used, as its token sub-tile width (32, 64, 128 or 192) and its sets of converter
+ * warps (4: a form for few tokens; 2: the others); 0 before the first launch.
  * The launcher picks it from the shape; tests use this to prove each one is covered. */
 int tm_cuda_mma_last_tile(tm_cuda_ctx *ctx);
+int tm_cuda_mma_last_sets(tm_cuda_ctx *ctx);
 /* No counterpart: how many parts the last GEMM launch cut the K range of every output tile into
  * (1: none; 0 before the first launch).  A call with fewer output tiles than half the SMs (a batch of
  * decode rows, a narrow projection) is split so that the whole machine streams its weights; the

@@ -116,6 +116,29 @@ def test_mma_gemm_split_k_is_deterministic_and_within_the_profile(ctx, oracle, r
         b.free()
 
 
+# Either side of each line between the forms for few tokens and the others: tokens, K steps for every issuer, and K steps
+# of an SM (151552 rows x 1 step: 1184 tiles on 148 SMs).
+@pytest.mark.parametrize("rows,cols,batch,tile,sets", [
+    (256, 256, 32, 32, 4), (256, 256, 33, 64, 4), (256, 192, 32, 64, 4), (256, 224, 9, 32, 4), (256, 128, 64, 64, 4),
+    (256, 64, 64, 64, 2), (256, 96, 33, 64, 4), (8192, 1152, 65, 64, 2), (8192, 1184, 65, 128, 4),
+    (8192, 1216, 128, 128, 4), (8192, 1216, 129, 64, 2), (151552, 64, 128, 64, 2), (75776, 128, 128, 128, 4)])
+def test_mma_gemm_forms_for_few_tokens(ctx, rows, cols, batch, tile, sets):
+    base = T.q8_0_matrix(8, cols, min(rows, 4096), cols)
+    raw = np.tile(base, ((rows + 4095) // 4096, 1, 1))[:rows]
+    X = T.activations(8, batch, batch * cols).reshape(batch, cols)
+    w, xb, yb = ctx.q8_0_matrix(raw, rows, cols), ctx.floats(X), ctx.buffer(batch * rows * 4)
+    ctx.q8_0_gemm_mma(w, xb, yb, rows, cols, batch)
+    Y = yb.download(0, batch * rows * 4, np.float32).reshape(batch, rows)
+    assert not ctx.mma_aborted()
+    assert (ctx.mma_last_tile(), ctx.mma_last_sets()) == (tile, sets)
+    ref16 = f16_profile_reference(base, X)
+    for r0 in range(0, rows, 4096):
+        got = Y[:, r0:r0 + 4096]
+        assert rel_err(got, ref16[:, :got.shape[1]]) <= 2e-5, f"rows from {r0}"
+    for b in (w, xb, yb):
+        b.free()
+
+
 # Several tiles to a CTA (more row tiles than SMs) of fewer K steps than a form has issuers: were the issuers to take
 # them in turn, the accumulator of one without a step in a tile would still hold an older tile.
 @pytest.mark.parametrize("rows", [148 * 128 + 1, 20000, 4 * 148 * 128 + 129, 151936])

@@ -968,7 +968,8 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     a.cols = cols;
     a.batch = batch;
     a.abort_flag = abort_flag;
-    ctx->mma_last_bn = bn;
+    ctx->mma_last_bn = few ? few : bn;
+    ctx->mma_last_sets = few ? 4 : 2;
     ctx->mma_last_ksplit = (int)a.ksplit;
     const uint32_t n_tiles = row_tiles * ((batch + 2 * bn - 1) / (2 * bn)) * a.ksplit;
     const int grid = (int)(n_tiles < (uint32_t)ctx->sm_count ? n_tiles : (uint32_t)ctx->sm_count);
@@ -1095,11 +1096,17 @@ int tm_cuda_q8_0_gemm_mma_push(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buff
     TM_OP_END(2);
 }
 
-// Token sub-tile width (64, 128 or 192) of the kernel instantiation the last GEMM launch used.
+// Token sub-tile width (32, 64, 128 or 192) and converter sets of the kernel instantiation the last GEMM launch used.
 int tm_cuda_mma_last_tile(tm_cuda_ctx *ctx) {
     if (!ctx) return 0;
     std::lock_guard<std::mutex> lock(ctx->mu);
     return ctx->mma_last_bn;
+}
+
+int tm_cuda_mma_last_sets(tm_cuda_ctx *ctx) {
+    if (!ctx) return 0;
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return ctx->mma_last_sets;
 }
 
 // K parts per output tile of the last GEMM launch (1: no split).

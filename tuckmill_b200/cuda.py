@@ -159,6 +159,8 @@ def load_library() -> C.CDLL:
     L.tm_cuda_mma_aborted.argtypes = [_P]
     L.tm_cuda_mma_last_tile.restype = C.c_int
     L.tm_cuda_mma_last_tile.argtypes = [_P]
+    L.tm_cuda_mma_last_sets.restype = C.c_int
+    L.tm_cuda_mma_last_sets.argtypes = [_P]
     L.tm_cuda_mma_last_split.restype = C.c_int
     L.tm_cuda_mma_last_split.argtypes = [_P]
     L.tm_cuda_program_bytes.restype = _SZ
@@ -416,6 +418,7 @@ class CudaContext:
     def mma_workspace_reserve(self, nbytes: int): self._call("mma_workspace_reserve", nbytes)
     def mma_aborted(self) -> bool: return bool(self._l.tm_cuda_mma_aborted(self.handle))
     def mma_last_tile(self) -> int: return int(self._l.tm_cuda_mma_last_tile(self.handle))
+    def mma_last_sets(self) -> int: return int(self._l.tm_cuda_mma_last_sets(self.handle))
     def mma_last_split(self) -> int: return int(self._l.tm_cuda_mma_last_split(self.handle))
 
     def q8_0_gemv_fused(self, w, x, y, rows, cols, prologue=PRO_NONE, pro=None, eps=0.0, epilogue=EPI_STORE):
