@@ -323,13 +323,15 @@ cudaError_t launch_rows(tm_cuda_ctx *ctx, const rows_args &args, const rows_plan
 
 extern "C" {
 
-// Where the multiply for a few rows beats the tcgen05 GEMM (measured, us against us, with the f16 copy of X): up to 8
-// tokens everywhere (24576 x 4096: 32 / 36, 151936 x 1024: 49 / 47); the more tokens, the sooner its MMAs and token
-// fragments cost more than the other kernel's hand-overs: at 16 tokens 12288 x 4096 is 22 / 23 but 24576 x 4096
-// 38 / 36, at 24 tokens 4096 x 4096 14 / 15, at 32 tokens 6144 x 1024 8.7 / 10.4 but 13824 x 1152 14 / 13.
+// Where the multiply for a few rows beats the tcgen05 GEMM: the more tokens, the sooner its MMAs and token fragments cost
+// more than the other kernel's hand-overs.  Measured, us against us, both with the f16 copy of X, at either side of the
+// lines: 8 tokens 24576 x 4096 30.6 / 33.9, 151936 x 1024 48.4 / 45.8; 16 tokens 6144 x 4096 15.9 / 16.1, 12288 x 4096
+// 21.6 / 21.6, 4096 x 12288 33.5 / 21.5; 24 tokens 4096 x 4096 13.5 / 14.0, 6144 x 4096 17.1 / 16.3; 32 tokens 6144 x 1024
+// 8.5 / 9.9, 13824 x 1152 13.6 / 11.6.  (On the wrong side of them: 151936 x 4096 at 8 tokens, 140 / 152; 13824 x 1152 and
+// 1152 x 6912 at 24, 11.8 / 11.6 and 15.1 / 13.8.)
 int tm_cuda_q8_0_gemm_rows_pays(uint32_t rows, uint32_t cols, uint32_t batch, int gated) {
     if (!rows_ok(rows, cols, batch, gated != 0)) return 0;
-    const uint64_t weights = (uint64_t)rows * cols, limit[4] = {160u << 20, 32u << 20, 17u << 20, 7u << 20};
+    const uint64_t weights = (uint64_t)rows * cols, limit[4] = {128u << 20, 32u << 20, 17u << 20, 7u << 20};
     return weights <= limit[(batch - 1u) / 8u];
 }
 
