@@ -22,24 +22,12 @@ constexpr int kT = 256;     // threads per CTA
 constexpr int kTile = 64;   // keys at a time
 constexpr uint32_t kMaxCluster = 16;
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t v;
-    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v));
-    return v;
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t v;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
-    return v;
-}
+using tmdev::cluster_arrive;
+using tmdev::cluster_rank;
+using tmdev::cluster_size;
+using tmdev::cluster_wait;
+using tmdev::smem_addr;
+using tmdev::st_cluster;
 
 // CTA `rank` of C owns keys [lo, hi) of a step at position p: equal contiguous runs of whole eights.
 __device__ __forceinline__ void key_range(uint32_t p, uint32_t window, uint32_t C, uint32_t rank, uint32_t &lo, uint32_t &hi) {

@@ -73,5 +73,95 @@ __device__ __forceinline__ float gelu_tanh_f(float x) {
     return 0.5f * x * (1.0f + tanhf(inner));
 }
 
+// D += A(16x32 s8, row) * B(32x8 s8, col), s32 accumulate.
+__device__ __forceinline__ void mma_s8(int (&d)[4], int a0, int a1, int a2, int a3, int b0, int b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// D += A(16x16 f16, row) * B(16x8 f16, col), f32 accumulate.
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Four consecutive values of a thread as digits (at `dst` of each plane, unless the thread is past the row); eight
+// adjacent lanes own a 32-column block, whose four coefficients 2^(e - 7k) go to `coef`.  Whole warps call it.
+__device__ __forceinline__ void digitise_quad(const float (&v)[4], bool live, signed char *dst, uint32_t plane, float *coef, uint32_t lane) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)  // a non-finite value poisons its block (amax = inf -> NaN coefficient)
+        amax = fmaxf(amax, fabsf(v[j]) <= 3.402823466e38f ? fabsf(v[j]) : INFINITY);
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    if (!live) return;
+    const bool bad = !(amax <= 3.402823466e38f);
+    int e = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 127 - 5;
+    e = e < -100 ? -100 : e > 122 ? 122 : e;  // blocks below 2^-94 digitise to (near) zero
+    const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    // t = v * 2^-e (|t| < 64, exact) is rounded once to a multiple of 2^-21
+    // and split into balanced base-128 digits with integer arithmetic:
+    // T = a0 2^21 + a1 2^14 + a2 2^7 + a3, a1..a3 in [-64, 63].
+    const float inv21 = inv * 2097152.0f;
+    uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        int T = __float2int_rn(v[j] * inv21);
+#pragma unroll
+        for (int k = 3; k > 0; --k) {
+            const int d = (int)((uint32_t)T << 25) >> 25;
+            T = (T - d) >> 7;
+            w[k] |= ((uint32_t)d & 0xffu) << (8 * j);
+        }
+        w[0] |= ((uint32_t)T & 0xffu) << (8 * j);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) *(uint32_t *)(dst + k * plane) = w[k];
+    const uint32_t k = lane & 7u;
+    if (k < 4u) {
+        const int ex = 127 + e - 7 * (int)k;  // 2^(e - 7k); below the normal range -> 0
+        float sc = ex > 0 ? __uint_as_float((uint32_t)ex << 23) : 0.0f;
+        if (amax == 0.0f) sc = 0.0f;
+        if (bad) sc = __uint_as_float(0x7fc00000u);
+        coef[k] = sc;
+    }
+}
+
+// ---- thread-block clusters: the CTA's place, barriers, a peer's shared memory ----
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t v;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t v;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    cluster_arrive();
+    cluster_wait();
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote));
+    return v;
+}
 
 }  // namespace tmdev

@@ -47,50 +47,11 @@ struct residual_in {
     float eps;
 };
 
-__device__ __forceinline__ void mma_s8(int (&d)[4], int a0, int a1, int a2, int a3, int b0, int b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+using tmdev::mma_s8;
 
-// Four consecutive columns of a vector into the digit planes; eight adjacent lanes own one 32-column block and all
-// lanes of the warp take part (dead ones with zeros).
+// Four consecutive columns of a vector into the digit planes (tmdev::digitise_quad; dead lanes with zeros).
 __device__ __forceinline__ void digitise(const float (&v)[4], uint32_t c, bool live, unsigned char *dig, uint32_t plane) {
-    float amax = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)  // a non-finite value poisons its block (amax = inf -> NaN coefficient)
-        amax = fmaxf(amax, fabsf(v[j]) <= 3.402823466e38f ? fabsf(v[j]) : INFINITY);
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    if (!live) return;
-    const bool bad = !(amax <= 3.402823466e38f);
-    int e = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 127 - 5;
-    e = e < -100 ? -100 : e > 122 ? 122 : e;
-    const float inv21 = __uint_as_float((uint32_t)(127 - e) << 23) * 2097152.0f;
-    uint32_t w[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {  // v * 2^(21-e) rounded once, balanced base-128 digits
-        int T = __float2int_rn(v[j] * inv21);
-#pragma unroll
-        for (int k = 3; k > 0; --k) {
-            const int d = (int)((uint32_t)T << 25) >> 25;
-            T = (T - d) >> 7;
-            w[k] |= ((uint32_t)d & 0xffu) << (8 * j);
-        }
-        w[0] |= ((uint32_t)T & 0xffu) << (8 * j);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) *(uint32_t *)(dig + k * plane + c) = w[k];
-    const int k = threadIdx.x & 7;
-    if (k < 4) {
-        const int ex = 127 + e - 7 * k;  // 2^(e - 7k); below the normal range -> 0
-        float sc = ex > 0 ? __uint_as_float((uint32_t)ex << 23) : 0.0f;
-        if (amax == 0.0f) sc = 0.0f;
-        if (bad) sc = __uint_as_float(0x7fc00000u);
-        ((float *)(dig + 4u * plane))[(c >> 5) * 4u + k] = sc;
-    }
+    tmdev::digitise_quad(v, live, (signed char *)dig + c, plane, (float *)(dig + 4u * plane) + (c >> 5) * 4u, threadIdx.x);
 }
 
 // Sum of every thread's value: one barrier (`red` is 8 floats no other sum between two barriers uses).

@@ -19,6 +19,8 @@ constexpr int kWarps = tmdev::kWarps;
 using tmdev::block_sumsq;
 using tmdev::silu_f;
 using tmdev::gelu_tanh_f;
+using tmdev::digitise_quad;
+using tmdev::mma_s8;
 constexpr int kChunkCols = 64;  // columns one m16n8k32 pair covers (two Q8_0 blocks)
 
 __device__ __forceinline__ int4 ldg_stream(const int4 *p) {
@@ -27,15 +29,6 @@ __device__ __forceinline__ int4 ldg_stream(const int4 *p) {
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;
-}
-
-// D += A(16x32 s8, row) * B(32x8 s8, col), s32 accumulate.
-__device__ __forceinline__ void mma_s8(int (&d)[4], int a0, int a1, int a2, int a3, int b0, int b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};"
-        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 constexpr uint32_t kPairSplit = 32;
@@ -63,54 +56,6 @@ struct gemv_args {
 // Bytes of shared memory one token's staged activations take.
 __host__ __device__ inline size_t token_smem(uint32_t cols, uint32_t plane) {
     return 4u * (size_t)plane + (size_t)(cols / 32u) * 16u;
-}
-
-// Four consecutive values of a thread as digits (at `dst` of each plane; nullptr: past the row); eight adjacent lanes own
-// a 32-column block, whose four coefficients 2^(e - 7k) go to `coef`.  Whole warps call it.
-__device__ __forceinline__ void digitise_quad(const float (&v)[4], signed char *dst, uint32_t plane, float *coef, uint32_t lane) {
-    float amax = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)  // a non-finite value poisons its block (amax = inf -> NaN coefficient)
-        amax = fmaxf(amax, fabsf(v[j]) <= 3.402823466e38f ? fabsf(v[j]) : INFINITY);
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    if (!dst) return;
-    const bool bad = !(amax <= 3.402823466e38f);
-    int e = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 127 - 5;
-    e = e < -100 ? -100 : e > 122 ? 122 : e;  // blocks below 2^-94 digitise to (near) zero
-    const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
-    // t = v * 2^-e (|t| < 64, exact) is rounded once to a multiple of 2^-21
-    // and split into balanced base-128 digits with integer arithmetic:
-    // T = a0 2^21 + a1 2^14 + a2 2^7 + a3, a1..a3 in [-64, 63].
-    const float inv21 = inv * 2097152.0f;
-    uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        int T = __float2int_rn(v[j] * inv21);
-        const int a3 = (int)((uint32_t)T << 25) >> 25;
-        T = (T - a3) >> 7;
-        const int a2 = (int)((uint32_t)T << 25) >> 25;
-        T = (T - a2) >> 7;
-        const int a1 = (int)((uint32_t)T << 25) >> 25;
-        const int a0 = (T - a1) >> 7;
-        w0 |= ((uint32_t)a0 & 0xffu) << (8 * j);
-        w1 |= ((uint32_t)a1 & 0xffu) << (8 * j);
-        w2 |= ((uint32_t)a2 & 0xffu) << (8 * j);
-        w3 |= ((uint32_t)a3 & 0xffu) << (8 * j);
-    }
-    *(uint32_t *)dst = w0;
-    *(uint32_t *)(dst + plane) = w1;
-    *(uint32_t *)(dst + 2u * plane) = w2;
-    *(uint32_t *)(dst + 3u * plane) = w3;
-    const uint32_t k = lane & 7u;
-    if (k < 4u) {
-        const int ex = 127 + e - 7 * (int)k;  // 2^(e - 7k); below the normal range -> 0
-        float sc = ex > 0 ? __uint_as_float((uint32_t)ex << 23) : 0.0f;
-        if (amax == 0.0f) sc = 0.0f;
-        if (bad) sc = __uint_as_float(0x7fc00000u);
-        coef[k] = sc;
-    }
 }
 
 /*
@@ -363,7 +308,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
                     else if (a.prologue == TM_CUDA_PRO_SILU_MUL) v[j] = silu_f(v[j]) * pw[j];
                     else if (a.prologue == TM_CUDA_PRO_GELU_MUL) v[j] = gelu_tanh_f(v[j]) * pw[j];
                 }
-                digitise_quad(v, c < cols ? dig + c : nullptr, plane, coef + (c >> 5) * 4u, lane);
+                digitise_quad(v, c < cols, dig + c, plane, coef + (c >> 5) * 4u, lane);
             }
         }
     }
@@ -657,7 +602,7 @@ __global__ void __launch_bounds__(kClusterThreads, 2) q8_gemv_cluster_kernel(con
             else if (a.prologue == TM_CUDA_PRO_SILU_MUL) x[j] = silu_f(x[j]) * pw[j];
             else if (a.prologue == TM_CUDA_PRO_GELU_MUL) x[j] = gelu_tanh_f(x[j]) * pw[j];
         }
-        digitise_quad(x, dig + lc, plane, coef + (lc >> 5) * 4u, lane);
+        digitise_quad(x, true, dig + lc, plane, coef + (lc >> 5) * 4u, lane);
     }
     __syncthreads();
 

@@ -36,13 +36,11 @@ struct rows_args {
     uint32_t rows, cols, batch, units, accumulate, mode, ring;
 };
 
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                        uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+using tmdev::cluster_rank;
+using tmdev::cluster_size;
+using tmdev::cluster_sync;
+using tmdev::ld_cluster;
+using tmdev::mma_f16;
 
 // Four quants -> two half2 of RN(d * q): bytes become f16 1024 + (q + 128) by permutes, minus 1152, times d.
 __device__ __forceinline__ void dequant4(uint32_t w, __half2 d2, uint32_t &lo, uint32_t &hi) {
@@ -53,27 +51,6 @@ __device__ __forceinline__ void dequant4(uint32_t w, __half2 d2, uint32_t &lo, u
     const __half2 b = __hmul2(__hsub2(*(const __half2 *)&s, bias), d2);
     lo = *(const uint32_t *)&a;
     hi = *(const uint32_t *)&b;
-}
-
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t v;
-    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v));
-    return v;
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t v;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
-    return v;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {
-    uint32_t remote;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote));
-    return v;
 }
 
 template <int NT>
