@@ -251,13 +251,6 @@ public:
         TM_CALL(tm_cuda_q8_0_gemm_rows, w.raw(), x.raw(), rows, cols, batch, n, yp, pr, prologue,
                 pro ? pro->raw() : nullptr, eps, epilogue);
     }
-    void qk_prep_chunk(const CudaBuffer &q, const CudaBuffer &k, const CudaBuffer &v, const CudaBuffer &qn,
-                       const CudaBuffer &kn, const CudaBuffer &inv_freq, const CudaBuffer &kc, const CudaBuffer &vc,
-                       uint32_t heads, uint32_t kvh, uint32_t hd, uint32_t n_rot, uint32_t pos0, uint32_t cap, uint32_t n,
-                       float eps) const {
-        TM_CALL(tm_cuda_qk_prep_chunk, q.raw(), k.raw(), v.raw(), qn.raw(), kn.raw(), inv_freq.raw(), kc.raw(), vc.raw(),
-                heads, kvh, hd, n_rot, pos0, cap, n, eps);
-    }
     void mma_workspace_reserve(size_t bytes) const {
         char e[256] = "";
         cuda_check(tm_cuda_mma_workspace_reserve(ctx_, bytes, e, sizeof e), e);
@@ -450,12 +443,6 @@ public:
                              const CudaBuffer *mirror) const {
         TM_CALL(tm_cuda_argmax_rows_sharded_dev, x.raw(), n_rows, n, index_offset, partial.raw(), pairs.raw(), out.raw(),
                 out_stride, base, pos.raw(), out_cap, mirror ? mirror->raw() : nullptr);
-    }
-
-    void prefetch_l2(std::initializer_list<const CudaBuffer *> bufs) const {
-        std::vector<tm_cuda_buffer *> raw;
-        for (const CudaBuffer *b : bufs) raw.push_back(b->raw());
-        TM_CALL(tm_cuda_prefetch_l2, raw.data(), (uint32_t)raw.size());
     }
 
     // ---- grouping / measurement (crates/tuckcore/src/qwen35_gpu.rs:62-86) ----

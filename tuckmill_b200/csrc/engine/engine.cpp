@@ -957,7 +957,6 @@ struct EngineModel::Impl {
     // Several sequences: positions pos_buf[s], token logs tokens[s * log_stride ..], logits [s][head_rows];
     // one recorded step advances all of them.
     size_t seqs = 1, log_stride = 0;
-    size_t l2_ahead = 0;  // layers whose weights the decode step asks into L2 ahead of use (0: off)
     CudaGraph batch_graph;
     std::vector<size_t> pos_b;  // host copy of every sequence's position
     const CudaBuffer &head_buf() const { return tied ? (sh.world > 1 ? tied_view : embedding.buf) : head_own.buf; }
@@ -1160,19 +1159,11 @@ std::unique_ptr<EngineModel> EngineModel::load_with(std::shared_ptr<CudaContext>
     // model allows it the step becomes one persistent kernel, else a graph of kernels.
     I.persistent = persistent_decode_applies(g, src, opts);
     {
-        // Layers whose weights a side branch asks into L2 ahead of use: off unless TM_ENGINE_L2_AHEAD asks for it.  The
-        // multiplies ask for their own first weights before their inputs are ready, and a second reader beside them
-        // delays them: the 1B-class shape, the last that gained from a layer ahead, 81.4 ms with it for 700 + 64 tokens,
-        // 78.3 without; F16 layers 5-7 us per projection.
-        size_t ahead = 0;
-        if (const char *e = std::getenv("TM_ENGINE_L2_AHEAD")) ahead = (size_t)std::max(0, std::min(8, std::atoi(e)));
         const char *fold = std::getenv("TM_ENGINE_FOLD_NORMS");
         I.ffn_blocks = !(fold && fold[0] == '1') && !opts.exact && !I.persistent && opts.shard_world == 1 && !I.layers.empty();
         for (const Layer &L : I.layers) I.ffn_blocks = I.ffn_blocks && L.ffn_block_applies(g.hidden);
         I.attn_blocks = I.ffn_blocks;
         for (const Layer &L : I.layers) I.attn_blocks = I.attn_blocks && L.attn_block_applies(g.hidden);
-        if (opts.shard_world > 1 || I.persistent || I.ffn_blocks || I.head_type() == 1) ahead = 0;
-        I.l2_ahead = ahead;
         // Folding the output norms into the next projection (Layer::decode_folded) saves two launches per
         // layer and is bit-identical, but measured slower on the Gemma-3-1B shape (1344 against 1299 us per
         // token: every CTA of the wide gate|up projection repeats a second reduction and two more vector
@@ -1180,7 +1171,6 @@ std::unique_ptr<EngineModel> EngineModel::load_with(std::shared_ptr<CudaContext>
         I.fold_norms = fold && fold[0] == '1' && !I.persistent && opts.shard_world == 1 && I.head_type() == 8 &&
                        !I.layers.empty();
         for (const Layer &L : I.layers) I.fold_norms = I.fold_norms && L.norms_fold(g.hidden);
-        if (ahead) c.prefetch_l2({&I.final_norm});  // the context's side stream comes into being outside a group
     }
     if (I.persistent) {
         const DecodeProgramSize ps = decode_program_size(g, capacity);
@@ -1233,15 +1223,6 @@ void EngineModel::encode_decode_step() {
     else
         c.row_indirect_dev(I.embedding.buf, I.embedding.rows, I.embedding.cols, I.tokens, 0, I.pos_buf, 0, 0,
                            g.embedding_scale, I.x);
-    // Where it pays (see load_with), the weights of the layer(s) ahead are asked into L2 on a side
-    // branch of the recorded graph.
-    const size_t ahead = I.l2_ahead;
-    auto prefetch = [&](size_t l) {
-        if (ahead == 0 || l >= I.layers.size()) return;
-        const Layer &P = I.layers[l];
-        c.prefetch_l2({&P.mixer.qkv.buf, &P.mixer.o.buf, &P.ffn.gate_up.buf, &P.ffn.down.buf});
-    };
-    for (size_t l = 0; l < ahead; ++l) prefetch(l);
     if (I.ffn_blocks) {
         SlotResidual R;
         R.cur = &I.x;
@@ -1255,13 +1236,11 @@ void EngineModel::encode_decode_step() {
         R.cur = &I.x;
         R.alt = &I.x2;
         for (size_t l = 0; l < I.layers.size(); ++l) {
-            prefetch(l + ahead);
             I.layers[l].decode_folded(c, R, I.pos_buf, I.status, g.hidden, g.eps, opts_.exact);
         }
         R.project(c, I.head_buf(), I.head_rows, I.head_cols(), I.final_norm, I.logits, g.eps);
     } else {
         for (size_t l = 0; l < I.layers.size(); ++l) {
-            prefetch(l + ahead);
             I.layers[l].decode(c, I.x, I.pos_buf, I.status, g.hidden, g.eps, opts_.exact);
         }
         I.project_head(c, g.eps);
