@@ -102,6 +102,24 @@ def test_a_request_that_ends_on_its_first_token_leaves_the_prompts_state(ctx, ar
     eng.close()
 
 
+@pytest.mark.parametrize("sequences", [1, 2])
+def test_a_request_without_a_first_token_leaves_the_prompts_state(ctx, tmp_path, sequences):
+    path, shape = tmp_path / "nan.gguf", T.TINY_QWEN3
+    _, _, at, size = T.write_gguf(path, shape, seed=3)["output_norm.weight"]
+    with open(path, "r+b") as f:
+        f.seek(at)
+        f.write(np.full(size // 4, np.nan, np.float32).tobytes())
+    prompt = T.token_ids(13, 15, shape.vocab)
+    eng = E.Engine(path, context=16, prefill_batch=16, sequences=sequences)
+    for _ in range(2):
+        with pytest.raises(E.EngineError) as e:
+            eng.generate(prompt, 2) if sequences == 1 else eng.generate_batch([prompt, prompt], 2)
+        assert e.value.code == "INTERNAL"
+        # the one position behind the prompt is still free
+        eng.step(7) if sequences == 1 else eng.step_batch([7, 7])
+    eng.close()
+
+
 def test_ledger_equals_plan_and_info(ctx, artifact):
     path, shape = artifact
     eng = E.Engine(path, context=48)

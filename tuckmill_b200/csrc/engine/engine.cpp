@@ -1621,15 +1621,8 @@ std::vector<std::vector<uint32_t>> EngineModel::generate_batch(const std::vector
         return f;
     };
     std::vector<Flight> inflight;
-    const uint64_t prefilled = ctx_->committed();
-    // The first step needs no token read before it, unless every request may end on its first token: the step would
-    // then move the state past the prompts.
-    if (I.sh.world <= 1 && !may_stop && any_wants()) inflight.push_back(submit());
     for (size_t s = 0; s < R; ++s) {
-        uint32_t tok = 0;
-        const size_t at = s * I.log_stride + I.pos_b[s];
-        if (I.sh.world > 1) tok = prefill_token_of(s);  // a split model's prefill has no mirror
-        else I.tokens_mirror.download_after(at * 4, &tok, 4, prefilled);
+        const uint32_t tok = prefill_token_of(s);
         if (tok == 0xFFFFFFFFu)
             throw TuckmillError(ErrorCode::Internal, "every logit was NaN; refusing to guess a token");
         out[s].push_back(tok);
@@ -1637,7 +1630,8 @@ std::vector<std::vector<uint32_t>> EngineModel::generate_batch(const std::vector
     }
     const uint64_t t_first = now_ns();
     uint64_t t_last = t_first;
-    if (inflight.empty() && any_wants()) inflight.push_back(submit());
+    // (only now: a request that ends on its first token, or throws for it, leaves the state that its prompt made)
+    if (any_wants()) inflight.push_back(submit());
     while (!inflight.empty()) {
         if (any_wants()) inflight.push_back(submit());
         const Flight f = inflight.front();
@@ -1729,18 +1723,14 @@ std::vector<uint32_t> EngineModel::generate(const uint32_t *prompt, size_t n_pro
     reset();
     prefill(prompt, n_prompt, true);
     // Step i+1 is submitted before step i is collected (executor.rs:1080-1087): the device already has token i in its
-    // log.  So is the first one before the prompt's own token is read, unless the request may end on that token: its
-    // position and logits are then the prompt's.
+    // log.  The first one waits for the prompt's own token: a request that ends on it, or throws for it, leaves the
+    // prompt's position and logits.
     std::vector<Ticket> inflight;
     size_t submitted = 0;
     const size_t want = max_new - 1;
     auto can_submit = [&] { return submitted < want && pos_ < capacity_; };
-    const size_t first_slot = pos_;
-    const uint64_t first_dispatch = ctx_->committed();
-    const uint32_t first_split = impl_->sh.world > 1 ? prefill_token() : 0u;  // a split model's prefill has no mirror
     const bool may_stop = !ignore_eos && graph_.has_eos;
-    if (!may_stop && can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
-    uint32_t tok = impl_->sh.world > 1 ? first_split : collect_greedy(Ticket{first_dispatch, first_slot});
+    uint32_t tok = prefill_token();
     const uint64_t t_first = now_ns();
     uint64_t t_last = t_first;
     auto is_stop = [&](uint32_t t) { return t == 0xFFFFFFFFu || (may_stop && t == graph_.eos_token_id); };
@@ -1748,7 +1738,7 @@ std::vector<uint32_t> EngineModel::generate(const uint32_t *prompt, size_t n_pro
     if (tok == 0xFFFFFFFFu)
         throw TuckmillError(ErrorCode::Internal, "every logit was NaN; refusing to guess a token");
     if (!is_stop(tok)) {
-        if (inflight.empty() && can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
+        if (can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
         while (!inflight.empty()) {
             if (can_submit()) { inflight.push_back(submit_greedy()); ++submitted; }
             const Ticket t = inflight.front();
