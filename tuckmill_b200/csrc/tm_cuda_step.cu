@@ -35,8 +35,8 @@
 //     still being read.  Every poll is bounded; when one runs out the CTA raises a
 //     status bit, stops producing and returns, and the others follow.
 //
-// Attention is the latency-optimised decode kernel of tm_cuda_ops.cu (same
-// arithmetic and key split) run by groups of four warps, two (KV head, key
+// Attention computes what the stand-alone decode kernel does (tm_cuda_attn_decode.cu;
+// its own key split, sums in another order), run by groups of four warps, two (KV head, key
 // split) items per CTA at a time; the splits of a KV head are merged by the group
 // that holds the newest key, which polls the other groups' flagged partials.
 #include <cuda.h>
@@ -681,8 +681,8 @@ struct attn_shared {
 };
 
 // One (KV head, 64-key split) item by 128 threads: q/k RMS norm, RoPE, f16 KV store (the split that
-// holds the new position), scores, split softmax, values.  The arithmetic and the merge order are
-// those of attention_decode_fast_kernel (tm_cuda_ops.cu), so both give the same bits; the splits'
+// holds the new position), scores, split softmax, values: the stand-alone decode attention
+// (tm_cuda_attn_decode.cu) but for the order of its sums; the splits'
 // partial results travel as flagged words and the group of the newest split merges them.
 template <int G, int HD>
 __device__ __forceinline__ void attn_item(const step_params &P, const step_op &op, uint32_t oi, uint32_t pos, uint32_t kvh,
