@@ -112,6 +112,12 @@ def test_feed_forward_block(ctx, hidden, width, n_slots, normed, gelu):
     assert rel_err(so.download(0, 8 * hidden * 4, np.float32).reshape(8, hidden).astype(np.float64).sum(axis=0), want) <= 2e-6
 
 
+# the narrowest width that takes eight clusters, the widest that takes six, clusters with one chunk of columns and with two
+@pytest.mark.parametrize("hidden,width,n_slots", [(1024, 4096, 8), (1024, 3136, 2), (1024, 3072, 0), (192, 704, 5)])
+def test_feed_forward_block_by_clusters(ctx, hidden, width, n_slots):
+    test_feed_forward_block(ctx, hidden, width, n_slots, False, False)
+
+
 @pytest.mark.parametrize("hidden,heads,kvh,hd,pos,window", [(1024, 16, 8, 128, 700, 0), (256, 4, 2, 128, 0, 0), (64, 3, 3, 128, 129, 50),
                                                             (128, 4, 1, 256, 1030, 40), (1088, 8, 8, 128, 15, 0)])
 def test_attention_block_equals_the_operators_it_replaces(ctx, oracle, hidden, heads, kvh, hd, pos, window):

@@ -6,6 +6,7 @@
 // value sum never leave its registers, so the tiles need no barrier; the warps' states meet once at the end.  (With
 // the softmax of a tile as a CTA-wide step, three barriers around it were most of the time at short contexts.)
 //
+// (Stand-alone form; the fused block has its projections between the wait and the scores and reads no row before it.)
 // Cached rows are read before the predecessor kernel finishes.  The position read at that moment only says which
 // rows to ask for; it is read again afterwards, and a changed one reloads them.  Row pos - 1 is always read after the
 // wait: the attention call of the previous token may still be storing it.  Calls further back have finished, because
@@ -104,17 +105,49 @@ struct keys {
     }
     __device__ __forceinline__ void load_v(int p, uint32_t j) { vraw[p] = __ldcg((const int4 *)(vp + (size_t)j * HD + vd)); }
 
-    // Before the dependency wait: rows up to hint - 2 of the first tile.
-    __device__ __forceinline__ void early(const __half *k_plane, const __half *v_plane, uint32_t pos_hint, uint32_t window,
-                                          uint32_t C, uint32_t rank) {
-        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    __device__ __forceinline__ void place(const __half *k_plane, const __half *v_plane) {
+        const uint32_t lane = threadIdx.x & 31u, warp = tmdev::warp_index();
         kp = k_plane;
         vp = v_plane;
-        hint = pos_hint;
         kk = warp * 8u + (lane >> 2);
         kq = lane & 3u;
         vr = warp * 8u + lane / TV;
         vd = (lane % TV) * 8u;
+    }
+    // Rows from `from` on: towards L2.
+    __device__ __forceinline__ void prefetch(uint32_t from) const {
+#pragma unroll 1
+        for (uint32_t t = from; t < hi; t += kTile) {
+            const uint32_t j = min(t + threadIdx.x / (kT / kTile), hi - 1u);
+#pragma unroll 1
+            for (uint32_t b = (threadIdx.x & 1u) * 128u; b < HD * 2u; b += 256u)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)((threadIdx.x & 2u ? vp : kp) + (size_t)j * HD) + b));
+        }
+    }
+    // Before the dependency wait, where there is work between it and the scores: all rows towards L2 (no value is read) ...
+    __device__ __forceinline__ void ask(const __half *k_plane, const __half *v_plane, uint32_t pos_hint, uint32_t window,
+                                        uint32_t C, uint32_t rank) {
+        place(k_plane, v_plane);
+        key_range(pos_hint, window, C, rank, lo, hi);
+        prefetch(lo);
+    }
+    // ... and after it the first tile.
+    __device__ __forceinline__ void first_tile(uint32_t pos, uint32_t window, uint32_t C, uint32_t rank) {
+        key_range(pos, window, C, rank, lo, hi);
+        load_tile(lo);
+    }
+    // Rows past the range are read as its last one (whose weight there is 0).
+    __device__ __forceinline__ void load_tile(uint32_t t0) {
+        load_k(min(t0 + kk, hi - 1u));
+#pragma unroll
+        for (int p = 0; p < VP; ++p) load_v(p, min(t0 + vr + p * RV, hi - 1u));
+    }
+
+    // Before the dependency wait: rows up to hint - 2 of the first tile.
+    __device__ __forceinline__ void early(const __half *k_plane, const __half *v_plane, uint32_t pos_hint, uint32_t window,
+                                          uint32_t C, uint32_t rank) {
+        place(k_plane, v_plane);
+        hint = pos_hint;
         key_range(hint, window, C, rank, lo, hi);
 #pragma unroll
         for (int i = 0; i < NL; ++i) kraw[i] = make_int4(0, 0, 0, 0);
@@ -125,13 +158,7 @@ struct keys {
             vraw[p] = make_int4(0, 0, 0, 0);
             if (j < hi && j + 1u < hint) load_v(p, j);
         }
-        // the rows after those: towards L2
-#pragma unroll 1
-        for (uint32_t t = lo + kTile; t < hi; t += kTile) {
-            const uint32_t j = min(t + threadIdx.x / (kT / kTile), hi - 1u);
-            for (uint32_t b = (threadIdx.x & 1u) * 128u; b < HD * 2u; b += 256u)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)((threadIdx.x & 2u ? vp : kp) + (size_t)j * HD) + b));
-        }
+        prefetch(lo + kTile);  // the rows after those
     }
     // After it: the rows of the first tile that were not to be read early.
     __device__ __forceinline__ void late(uint32_t pos, uint32_t window, uint32_t C, uint32_t rank) {
@@ -146,7 +173,7 @@ struct keys {
     }
     // All tiles; s.qs, s.kh and s.vh are set (one barrier ago).  Leaves every warp's (max, sum, output) in s.
     __device__ __forceinline__ void attend(S &s, uint32_t pos, float scale) {
-        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+        const uint32_t lane = threadIdx.x & 31u, warp = tmdev::warp_index();
         float acc[G][8], m[G], l[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -158,8 +185,8 @@ struct keys {
 #pragma unroll 1
         for (uint32_t t0 = lo; t0 + warp * 8u < hi; t0 += kTile) {  // uniform over the warp
             // ---- scores: four lanes per key, interleaved 8-dim pieces ----
-            const uint32_t j = t0 + kk;
-            if (j == pos)
+            const uint32_t j = t0 + kk, last = hi - 1u;
+            if (min(j, last) == pos)
 #pragma unroll
                 for (int i = 0; i < NL; ++i) kraw[i] = *(const int4 *)(s.kh + i * 32 + kq * 8u);
             float p[G];
@@ -185,7 +212,7 @@ struct keys {
                     p[g] = t;
                 }
             }
-            if (t0 + kTile + kk < hi && t0 + kTile + kk != pos) load_k(t0 + kTile + kk);  // the next tile's
+            load_k(min(j + kTile, last));  // the next tile's
             // ---- softmax weights against the warp's running maximum ----
             float al[G];
 #pragma unroll
@@ -213,8 +240,7 @@ struct keys {
             for (int v = 0; v < VP; ++v) {
                 const uint32_t row = lane / TV + v * RV, jv = t0 + vr + v * RV;
                 int4 raw = vraw[v];
-                if (jv == pos) raw = *(const int4 *)(s.vh + vd);
-                if (jv >= hi) raw = make_int4(0, 0, 0, 0);  // weight 0 there; never multiply stale bytes
+                if (min(jv, last) == pos) raw = *(const int4 *)(s.vh + vd);
                 const __half2 *h2 = (const __half2 *)&raw;
                 float f[8];
 #pragma unroll
@@ -229,7 +255,7 @@ struct keys {
 #pragma unroll
                     for (int e = 0; e < 8; ++e) acc[g][e] = fmaf(pj, f[e], acc[g][e]);
                 }
-                if (jv + kTile < hi && jv + kTile != pos) load_v(v, jv + kTile);
+                load_v(v, min(jv + kTile, last));
             }
         }
 #pragma unroll
@@ -256,7 +282,7 @@ struct keys {
     static __device__ __forceinline__ void combine(S &s) {
         constexpr int W = kT / 32;
         static_assert(W == 8, "a warp holds eight warps' states of four heads");
-        if (threadIdx.x < 32u) {
+        if (tmdev::warp_index() == 0u) {
             const uint32_t g = threadIdx.x / W < G ? threadIdx.x / W : 0u, w = threadIdx.x % W;
             const float m = s.m[g][w];
             float M = m;

@@ -38,14 +38,14 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
     __shared__ float recv_ml[kMaxCluster][G][2];  // every CTA's max and sum
     const uint32_t C = cluster_size(), rank = cluster_rank();
     const uint32_t kvh = blockIdx.x / C, seq_i = blockIdx.z, cap = a.cap;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tmdev::warp_index();
     cluster_arrive();  // before any peer's shared memory is written, every CTA must have started
     const float *q = a.q + seq_i * a.sq + (size_t)kvh * G * HD, *k = a.k + seq_i * a.sk + (size_t)kvh * HD;
     const float *v = a.v + seq_i * a.sv + (size_t)kvh * HD;
     __half *kp = a.kc + seq_i * a.scache + (size_t)kvh * cap * HD, *vp = a.vc + seq_i * a.scache + (size_t)kvh * cap * HD;
     const volatile uint32_t *pos_p = a.pos + seq_i;
     keys<G, HD> K;
-    const uint32_t hint = min(*pos_p, cap - 1u);
+    const uint32_t hint = tmdev::uniform(min(*pos_p, cap - 1u));
     K.early(kp, vp, hint, a.window, C, rank);
     rotation<HD> rot;  // as if the position stood already
     rot.set(a.inv_freq, hint);
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
             vx[r] = is_k ? v[lane + 32 * r] : 0.0f;
         }
     }
-    const uint32_t pos = *pos_p;
+    const uint32_t pos = tmdev::uniform(*pos_p);
     if (pos >= cap) {  // uniform over the cluster
         if (tid == 0 && rank == 0) atomicOr(a.status, 1u);
         cluster_wait();

@@ -67,6 +67,12 @@ static __device__ float block_sumsq(const float *x, uint32_t n, float *red /* [k
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 
+// A value that all lanes of the (whole, converged) warp hold, told to the compiler: it then knows that a branch on it
+// keeps the warp together.  Behind a branch that may split the warp, every shuffle is compiled twice, the second time
+// with the code that gathers the lanes first.
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ uint32_t warp_index() { return uniform(threadIdx.x >> 5); }
+
 __device__ __forceinline__ float silu_f(float g) { return g / (1.0f + expf(-g)); }
 __device__ __forceinline__ float gelu_tanh_f(float x) {
     const float inner = 0.7978845608028654f * x * (1.0f + 0.044715f * x * x);
@@ -92,14 +98,16 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1,
 
 // Four consecutive values of a thread as digits (at `dst` of each plane, unless the thread is past the row); eight
 // adjacent lanes own a 32-column block, whose four coefficients 2^(e - 7k) go to `coef`.  Whole warps call it.
-__device__ __forceinline__ void digitise_quad(const float (&v)[4], bool live, signed char *dst, uint32_t plane, float *coef, uint32_t lane) {
+// (`shift` > 0: 2^shift adjacent lanes hold the same four values.)
+__device__ __forceinline__ void digitise_quad(const float (&v)[4], bool live, signed char *dst, uint32_t plane, float *coef, uint32_t lane,
+                                              uint32_t shift = 0) {
     float amax = 0.0f;
 #pragma unroll
     for (int j = 0; j < 4; ++j)  // a non-finite value poisons its block (amax = inf -> NaN coefficient)
         amax = fmaxf(amax, fabsf(v[j]) <= 3.402823466e38f ? fabsf(v[j]) : INFINITY);
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1u << shift));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2u << shift));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4u << shift));
     if (!live) return;
     const bool bad = !(amax <= 3.402823466e38f);
     int e = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 127 - 5;
@@ -123,7 +131,7 @@ __device__ __forceinline__ void digitise_quad(const float (&v)[4], bool live, si
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) *(uint32_t *)(dst + k * plane) = w[k];
-    const uint32_t k = lane & 7u;
+    const uint32_t k = (lane >> shift) & 7u;
     if (k < 4u) {
         const int ex = 127 + e - 7 * (int)k;  // 2^(e - 7k); below the normal range -> 0
         float sc = ex > 0 ? __uint_as_float((uint32_t)ex << 23) : 0.0f;

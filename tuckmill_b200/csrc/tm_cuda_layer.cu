@@ -12,8 +12,15 @@
 //     anyway; one cluster also stores the sum.  A layer's output norm is applied there too;
 //   * weights never wait for activations: every warp copies its own 16-row x 64-column pieces of both projections to
 //     shared memory before the dependency wait; both blocks' CTAs fit on an SM together, so a block's weights arrive
-//     while the block before it computes.  (Only 7 of the 8 GPCs have the 16 SMs of a cluster: a block that fills more
-//     than half an SM's shared memory runs its eighth cluster after the others, 20 us a layer instead of 11.)
+//     while the block before it computes.  Only 7 of the 8 GPCs have the 16 SMs of a cluster, so 14 clusters are in
+//     flight at two CTAs an SM: eight of attention (a KV head each) and six of feed-forward.  With eight of each the last
+//     two of a block started when the block before it had gone, and loaded their weights after that (0.6B shape, 512 +
+//     256 tokens: 138.3 -> 134.7 ms, although a warp multiplies 12 pieces instead of 9).
+//   * the code is short, because every launch runs it once: a chain of two kernels of 66 and 33 KB never finds it in
+//     an SM's 32 KB instruction cache.  Both projections go through the same digit split and products (one loop of two
+//     turns), and branches are on values that the compiler knows to be the same in a warp (tmdev::uniform): behind
+//     others it repeats every shuffle in a form that gathers the lanes first, 200 cycles each instead of 30.  From the
+//     dependency wait on, attention 23.0 -> 17.7 thousand cycles, feed-forward 13.1 -> 10.4 (143.8 -> 138.3 ms).
 // Products are the decode GEMV's (tm_cuda_q8.cu): int8 tensor-core MMAs on activations split into four 7-bit digits,
 // exact sums per 32-column block.  How a row's columns are cut over warps, CTAs and clusters depends on the shape
 // alone, and every sum has a fixed order.
@@ -27,6 +34,7 @@ constexpr int kWarps = kT / 32;
 constexpr uint32_t kSlotBytes = 1024u + 64u;  // 16 rows x 64 quants, 16 rows x 2 scales
 constexpr uint32_t kC = 16;                   // CTAs per cluster
 constexpr uint32_t kSlots = TM_CUDA_DECODE_SLOTS;
+constexpr uint32_t kFfnClusters = 6;          // where a warp can keep its pieces, else kSlots
 constexpr uint32_t kResident = 12;            // most pieces a warp keeps in shared memory
 
 __host__ __device__ inline uint32_t plane_bytes(uint32_t cols) {  // 64 mod 128: the four digit planes hit distinct banks
@@ -49,11 +57,6 @@ struct residual_in {
 
 using tmdev::mma_s8;
 
-// Four consecutive columns of a vector into the digit planes (tmdev::digitise_quad; dead lanes with zeros).
-__device__ __forceinline__ void digitise(const float (&v)[4], uint32_t c, bool live, unsigned char *dig, uint32_t plane) {
-    tmdev::digitise_quad(v, live, (signed char *)dig + c, plane, (float *)(dig + 4u * plane) + (c >> 5) * 4u, threadIdx.x);
-}
-
 // Sum of every thread's value: one barrier (`red` is 8 floats no other sum between two barriers uses).
 __device__ __forceinline__ float cta_sum(float v, float *red) {
 #pragma unroll
@@ -64,13 +67,13 @@ __device__ __forceinline__ float cta_sum(float v, float *red) {
     return ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
 }
 
-// x + [norm](sum of the slots), stored by cluster 0, then normed and split into digits: NB quads of columns per
-// thread.  `red`: 16 floats.
+// v = rmsnorm(x + [norm](sum of the slots)): NB quads of columns per thread, the sum stored by cluster 0.  `red`: 16
+// floats.
 template <int NB>
-__device__ __forceinline__ void stage_residual(const residual_in &r, bool store, uint32_t rank, unsigned char *dig, float *red) {
-    const uint32_t H = r.hidden, quads = H / 4u, plane = plane_bytes(H);
+__device__ __forceinline__ void residual_norm(const residual_in &r, bool store, uint32_t rank, float4 (&v)[NB], float *red) {
+    const uint32_t H = r.hidden, quads = H / 4u;
     const float inv_h = 1.0f / (float)H;
-    float4 v[NB], nw[NB];
+    float4 nw[NB];
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
         const uint32_t q = threadIdx.x + i * kT;
@@ -81,13 +84,12 @@ __device__ __forceinline__ void stage_residual(const residual_in &r, bool store,
         }
     }
     if (r.n_slots) {
-        float4 p[NB], aw[NB];
+        float4 p[NB];
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
             const uint32_t q = threadIdx.x + i * kT;
-            p[i] = aw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (q < quads) {
-                if (r.add_w) aw[i] = __ldg((const float4 *)r.add_w + q);
                 float4 s[kSlots];
 #pragma unroll
                 for (uint32_t k = 0; k < kSlots; ++k)
@@ -108,10 +110,12 @@ __device__ __forceinline__ void stage_residual(const residual_in &r, bool store,
             const float inv = inv_sqrt(fmaf(cta_sum(sq, red + 8), inv_h, r.eps));
 #pragma unroll
             for (int i = 0; i < NB; ++i) {
-                p[i].x = p[i].x * inv * aw[i].x;
-                p[i].y = p[i].y * inv * aw[i].y;
-                p[i].z = p[i].z * inv * aw[i].z;
-                p[i].w = p[i].w * inv * aw[i].w;
+                const uint32_t q = threadIdx.x + i * kT;
+                const float4 aw = q < quads ? __ldg((const float4 *)r.add_w + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                p[i].x = p[i].x * inv * aw.x;
+                p[i].y = p[i].y * inv * aw.y;
+                p[i].z = p[i].z * inv * aw.z;
+                p[i].w = p[i].w * inv * aw.w;
             }
         }
 #pragma unroll
@@ -124,20 +128,18 @@ __device__ __forceinline__ void stage_residual(const residual_in &r, bool store,
     }
     float sq = 0.0f;
 #pragma unroll
-    for (int i = 0; i < NB; ++i) sq = tmdev::sumsq_quad(sq, v[i]);
+    for (int i = 0; i < NB; ++i) {
+        const uint32_t q = threadIdx.x + i * kT;
+        sq = tmdev::sumsq_quad(sq, v[i]);
+        if (store && q < quads && q % kC == rank) ((float4 *)r.x_out)[q] = v[i];
+    }
     const float inv = inv_sqrt(fmaf(cta_sum(sq, red), inv_h, r.eps));
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
-        const uint32_t q = threadIdx.x + i * kT;
-        if ((q & ~31u) < quads) {
-            const float y[4] = {v[i].x * inv * nw[i].x, v[i].y * inv * nw[i].y, v[i].z * inv * nw[i].z, v[i].w * inv * nw[i].w};
-            digitise(y, q * 4u, q < quads, dig, plane);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NB; ++i) {
-        const uint32_t q = threadIdx.x + i * kT;
-        if (store && q < quads && q % kC == rank) ((float4 *)r.x_out)[q] = v[i];
+        v[i].x = v[i].x * inv * nw[i].x;
+        v[i].y = v[i].y * inv * nw[i].y;
+        v[i].z = v[i].z * inv * nw[i].z;
+        v[i].w = v[i].w * inv * nw[i].w;
     }
 }
 
@@ -154,135 +156,117 @@ struct matrix_part {
 // group with one wait.  Every lane copies, and later reads back, its own 16 bytes of rows g and g + 8 of a piece; the 32
 // block scales ride along as 4-byte copies.  Every piece leaves its own partial sum: no bookkeeping between pieces (a
 // commit, a wait and a running sum per piece cost more than 400 cycles each in a chain that multiplies six).
-template <class RowOf1, class RowOf2>
-struct weight_pieces {
-    matrix_part m1, m2;
-    RowOf1 row1;  // (tile, r): the weight row of row r of a tile
-    RowOf2 row2;
-    uint32_t base, slot;             // this warp's slots, the one consumed next
-    const signed char *pa, *pb;      // next piece: this lane's bytes of rows g and g + 8
-    const unsigned short *ps;        // and its scale pair
-    uint32_t left_tile, left, tile;  // pieces left in the tile and in the projection, the tile's number
-    bool second;
-
-    __device__ __forceinline__ uint32_t lane() const { return threadIdx.x & 31u; }
-    __device__ __forceinline__ uint32_t warp() const { return threadIdx.x >> 5; }
-
-    __device__ __forceinline__ void point(const matrix_part &m, size_t ra, size_t rb, uint32_t chunk) {
-        const uint32_t t4 = lane() & 3u, col = (m.chunk0 + chunk) * 64u;
-        pa = m.q + ra * m.cols + col + t4 * 16u;
-        pb = m.q + rb * m.cols + col + t4 * 16u;
-        ps = m.d + ((t4 & 1u) ? rb : ra) * (m.cols / 32u) + col / 32u;
-    }
-    __device__ __forceinline__ void open_tile(uint32_t chunk) {
-        const uint32_t g = lane() >> 2;
-        if (second) point(m2, row2(tile, g), row2(tile, g + 8u), chunk);
-        else point(m1, row1(tile, g), row1(tile, g + 8u), chunk);
-        left_tile = (second ? m2.chunks : m1.chunks) - chunk;
-    }
-    __device__ __forceinline__ void open(bool sec) {
-        second = sec;
-        const uint32_t n = sec ? m2.chunks : m1.chunks;
-        const uint32_t i0 = sec ? m2.first(warp()) : m1.first(warp());
-        left = (sec ? m2.first(warp() + 1u) : m1.first(warp() + 1u)) - i0;
-        tile = i0 / n;
-        if (left) open_tile(i0 - tile * n);
-    }
-    // The next piece, if one is left, into slot `to`.
-    __device__ __forceinline__ void issue(uint32_t to) {
-        if (left) {
-            const uint32_t dst = base + to * kSlotBytes, l = lane(), t4 = l & 3u;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + l * 16u), "l"(pa) : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512u + l * 16u), "l"(pb) : "memory");
+// `row_of(second, tile)` is the weight row of row 0 of a tile, and where row 8 lies from it.
+template <class RowOf>
+__device__ __forceinline__ void load_pieces(const matrix_part &m1, const matrix_part &m2, uint32_t ring, RowOf row_of) {
+    const uint32_t lane = threadIdx.x & 31u, warp = tmdev::warp_index(), g = lane >> 2, t4 = lane & 3u;
+    uint32_t dst = ring + lane * 16u, dst_s = ring + 1024u + (g + 8u * t4) * 4u;
+#pragma unroll 1
+    for (uint32_t sec = 0; sec < 2u; ++sec) {
+        const signed char *q = sec ? m2.q : m1.q;
+        const unsigned short *d = sec ? m2.d : m1.d;
+        const uint32_t cols = sec ? m2.cols : m1.cols, chunk0 = sec ? m2.chunk0 : m1.chunk0, chunks = sec ? m2.chunks : m1.chunks;
+        const uint32_t all = chunks * (sec ? m2.tiles : m1.tiles), end = all * (warp + 1u) / kWarps;
+        uint32_t i = all * warp / kWarps, tile = i / chunks, ch = i - tile * chunks;
+#pragma unroll 1
+        for (; i < end; ++i) {
+            const uint2 row = row_of(sec, tile);
+            const size_t ra = row.x + g, rb = ra + row.y, col = (chunk0 + ch) * 64u;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(q + ra * cols + col + t4 * 16u) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512u), "l"(q + rb * cols + col + t4 * 16u) : "memory");
             if (t4 < 2u)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 1024u + ((l >> 2) + 8u * t4) * 4u), "l"(ps) : "memory");
-            pa += 64;
-            pb += 64;
-            ps += 2;
-            if (--left != 0u && --left_tile == 0u) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst_s), "l"(d + ((t4 ? rb : ra) * cols + col) / 32u) : "memory");
+            dst += kSlotBytes;
+            dst_s += kSlotBytes;
+            if (++ch == chunks) {
+                ch = 0u;
                 ++tile;
-                open_tile(0u);
             }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    static __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-    __device__ __forceinline__ void start(uint32_t ring) {
-        base = ring;
-        slot = 0;
-        open(false);
-#pragma unroll 1
-        while (left) issue(slot++);
-        commit();
-        open(true);
-#pragma unroll 1
-        while (left) issue(slot++);
-        commit();
-        slot = 0;
-    }
-    // One piece: this lane's digits' share of rows g (x) and g + 8 (y).
-    __device__ __forceinline__ float2 piece(uint32_t at, const unsigned char *dig, uint32_t plane, uint32_t ch) const {
-        const uint32_t l = lane(), g = l >> 2, t4 = l & 3u, src = base + at * kSlotBytes, c0 = ch * 64u + t4 * 16u;
-        int4 qa, qb;
-        unsigned short sa, sb;
-        asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(qa.x), "=r"(qa.y), "=r"(qa.z), "=r"(qa.w) : "r"(src + l * 16u));
-        asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(qb.x), "=r"(qb.y), "=r"(qb.z), "=r"(qb.w) : "r"(src + 512u + l * 16u));
-        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sa) : "r"(src + 1024u + g * 4u + (t4 >> 1) * 2u));
-        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(src + 1056u + g * 4u + (t4 >> 1) * 2u));
-        int4 bx = make_int4(0, 0, 0, 0);
-        if ((t4 >> 1) == (g >> 2)) bx = *(const int4 *)(dig + (size_t)(g & 3u) * plane + c0);
-        const float2 cx = *(const float2 *)(dig + 4u * plane + ((size_t)(c0 >> 5) * 4u + 2u * (t4 & 1u)) * 4u);
-        int dd[4] = {0, 0, 0, 0};
-        mma_s8(dd, qa.x, qb.x, qa.y, qb.y, bx.x, bx.y);
-        mma_s8(dd, qa.z, qb.z, qa.w, qb.w, bx.z, bx.w);
-        return make_float2(__half2float(__ushort_as_half(sa)) * fmaf((float)dd[1], cx.y, (float)dd[0] * cx.x),
-                           __half2float(__ushort_as_half(sb)) * fmaf((float)dd[3], cx.y, (float)dd[2] * cx.x));
-    }
-    // This warp's pieces of one projection: piece i leaves its sums in part[i][16 rows].
-    __device__ __forceinline__ void multiply(const matrix_part &m, bool sec, const unsigned char *dig, uint32_t plane, float *part) {
-        const uint32_t l = lane(), g = l >> 2, t4 = l & 3u, i0 = m.first(warp()), end = m.first(warp() + 1u);
-        uint32_t ch = i0 % m.chunks;
-        if (sec) asm volatile("cp.async.wait_group 0;" ::: "memory");
-        else asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncwarp();  // scales were copied by other lanes
-#pragma unroll 1
-        for (uint32_t i = i0; i < end; i += 3u) {
-            float2 v[3];
-#pragma unroll
-            for (uint32_t k = 0; k < 3u; ++k) {
-                v[k] = make_float2(0.0f, 0.0f);
-                if (i + k < end) v[k] = piece(slot + k, dig, plane, ch);
-                ch = ch + 1u == m.chunks ? 0u : ch + 1u;
-            }
-            slot += min(3u, end - i);
-#pragma unroll
-            for (uint32_t k = 0; k < 3u; ++k) {
-                v[k].x += __shfl_xor_sync(0xffffffffu, v[k].x, 1);
-                v[k].y += __shfl_xor_sync(0xffffffffu, v[k].y, 1);
-                v[k].x += __shfl_xor_sync(0xffffffffu, v[k].x, 2);
-                v[k].y += __shfl_xor_sync(0xffffffffu, v[k].y, 2);
-                if (t4 == 0u && i + k < end) {
-                    part[(i + k) * 16u + g] = v[k].x;
-                    part[(i + k) * 16u + g + 8u] = v[k].y;
-                }
-            }
-        }
+}
+
+// One piece (in shared memory at `src`): this lane's digits' share of rows g (x) and g + 8 (y).
+__device__ __forceinline__ float2 piece(uint32_t src, const unsigned char *dig, uint32_t plane, uint32_t ch) {
+    const uint32_t l = threadIdx.x & 31u, g = l >> 2, t4 = l & 3u, c0 = ch * 64u + t4 * 16u;
+    int4 qa, qb;
+    unsigned short sa, sb;
+    asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(qa.x), "=r"(qa.y), "=r"(qa.z), "=r"(qa.w) : "r"(src + l * 16u));
+    asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(qb.x), "=r"(qb.y), "=r"(qb.z), "=r"(qb.w) : "r"(src + 512u + l * 16u));
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sa) : "r"(src + 1024u + g * 4u + (t4 >> 1) * 2u));
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(src + 1056u + g * 4u + (t4 >> 1) * 2u));
+    int4 bx = make_int4(0, 0, 0, 0);
+    if ((t4 >> 1) == (g >> 2)) bx = *(const int4 *)(dig + (size_t)(g & 3u) * plane + c0);
+    const float2 cx = *(const float2 *)(dig + 4u * plane + ((size_t)(c0 >> 5) * 4u + 2u * (t4 & 1u)) * 4u);
+    int dd[4] = {0, 0, 0, 0};
+    mma_s8(dd, qa.x, qb.x, qa.y, qb.y, bx.x, bx.y);
+    mma_s8(dd, qa.z, qb.z, qa.w, qb.w, bx.z, bx.w);
+    return make_float2(__half2float(__ushort_as_half(sa)) * fmaf((float)dd[1], cx.y, (float)dd[0] * cx.x),
+                       __half2float(__ushort_as_half(sb)) * fmaf((float)dd[3], cx.y, (float)dd[2] * cx.x));
+}
+// This warp's items [first, end) of a projection, the first one's chunk, and where its pieces lie.
+struct span {
+    uint32_t first, end, chunk, src;
+    __device__ __forceinline__ span(const matrix_part &m, uint32_t at) {
+        const uint32_t warp = tmdev::warp_index();
+        first = m.first(warp);
+        end = m.first(warp + 1u);
+        chunk = first % m.chunks;
+        src = at;
     }
 };
-
-// Row r of tile t: the sum over the tile's pieces, by one thread (row_sum) or by the 16 lanes of half a warp, which all
-// receive it (half_sum).
-__device__ __forceinline__ float row_sum(const float *part, const matrix_part &m, uint32_t t, uint32_t r) {
-    float v = 0.0f;
-#pragma unroll 4
-    for (uint32_t k = 0; k < m.chunks; ++k) v += part[(t * m.chunks + k) * 16u + r];
-    return v;
-}
-__device__ __forceinline__ float half_sum(const float *part, const matrix_part &m, uint32_t t, uint32_t r) {
-    float v = 0.0f;
-    for (uint32_t k = threadIdx.x & 15u; k < m.chunks; k += 16u) v += part[(t * m.chunks + k) * 16u + r];
+// Item i leaves its sums in part[i][16 rows].
+__device__ __forceinline__ void multiply(const span &w, uint32_t chunks, bool sec, const unsigned char *dig, uint32_t plane, float *part) {
+    const uint32_t l = threadIdx.x & 31u, g = l >> 2, t4 = l & 3u;
+    uint32_t ch = w.chunk, src = w.src;
+    if (sec) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();  // scales were copied by other lanes
+#pragma unroll 1
+    for (uint32_t i = w.first; i < w.end; i += 4u) {
+        float2 v[4];
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+        for (uint32_t k = 0; k < 4u; ++k) {  // (past the end: the last piece again)
+            v[k] = piece(src, dig, plane, ch);
+            if (i + k + 1u < w.end) {
+                src += kSlotBytes;
+                ch = ch + 1u == chunks ? 0u : ch + 1u;
+            }
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k) {
+            v[k].x += __shfl_xor_sync(0xffffffffu, v[k].x, 1);
+            v[k].y += __shfl_xor_sync(0xffffffffu, v[k].y, 1);
+            v[k].x += __shfl_xor_sync(0xffffffffu, v[k].x, 2);
+            v[k].y += __shfl_xor_sync(0xffffffffu, v[k].y, 2);
+            if (t4 == 0u && i + k < w.end) {
+                part[(i + k) * 16u + g] = v[k].x;
+                part[(i + k) * 16u + g + 8u] = v[k].y;
+            }
+        }
+    }
+}
+
+// Row `row` (16 tile + r) of a projection: the sum over its tile's pieces, by four adjacent lanes, which all receive it.
+__device__ __forceinline__ float quad_sum(const float *part, uint32_t chunks, uint32_t row) {
+    const uint32_t sub = threadIdx.x & 3u;
+    const float *p = part + ((row >> 4) * chunks + sub) * 16u + (row & 15u);
+    float v = 0.0f;
+#pragma unroll 2
+    for (uint32_t k = 0; k < chunks; k += 4u)
+        if (k + sub < chunks) v += p[k * 16u];
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+// This CTA's rows of the second projection, into the cluster's slot.
+__device__ __forceinline__ void store_slot(const float *part, const matrix_part &m, float *out) {
+#pragma unroll 1
+    for (uint32_t i0 = tmdev::warp_index() * 8u; i0 < m.tiles * 16u; i0 += kT / 4u) {
+        const uint32_t i = i0 + (threadIdx.x & 31u) / 4u;
+        const float v = quad_sum(part, m.chunks, i);
+        if ((threadIdx.x & 3u) == 0u) out[i] = v;
+    }
 }
 
 // ---------------- feed-forward block ----------------
@@ -291,17 +275,16 @@ struct ffn_args {
     const signed char *gu_q, *dn_q;          // [2 width][hidden], [hidden][width]
     const unsigned short *gu_d, *dn_d;
     float *slots_out;                        // [clusters][hidden]
-    uint32_t width, gelu, tiles1, tiles2, acts;  // most tiles / activations a CTA / cluster has
+    uint32_t width, gelu, clusters, tiles1, tiles2, acts;  // most tiles / activations a CTA / cluster has
 };
 
-// Shared memory: digits of x, digits of the activations, activations, partial sums, ring.
+// Shared memory: digits (of x, then of the activations), activations, partial sums, ring.
 struct ffn_smem {
-    uint32_t dig2, acts, part, red, ring, bytes;
+    uint32_t acts, part, red, ring, bytes;
 };
 __host__ __device__ inline ffn_smem ffn_layout(uint32_t hidden, uint32_t acts, uint32_t tiles1, uint32_t tiles2, uint32_t slots) {
     ffn_smem s;
-    s.dig2 = digit_bytes(hidden);
-    s.acts = s.dig2 + digit_bytes(acts);
+    s.acts = digit_bytes(max_of(hidden, acts));
     s.part = s.acts + acts * 4u;
     s.red = s.part + 64u * max_of(tiles1 * (hidden / 64u), tiles2 * (acts / 64u));
     s.ring = s.red + 64u;
@@ -312,51 +295,64 @@ __host__ __device__ inline ffn_smem ffn_layout(uint32_t hidden, uint32_t acts, u
 template <int NB>
 __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint32_t ring_slots) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t rank = cluster_rank(), cluster = blockIdx.x / kC, n_clusters = gridDim.x / kC;
+    const uint32_t rank = cluster_rank(), cluster = blockIdx.x / kC;
     const uint32_t H = a.in.hidden, F = a.width, chunks = F / 64u;
-    const uint32_t fc0 = chunks * cluster / n_clusters, nfc = chunks * (cluster + 1u) / n_clusters - fc0;  // FFN chunks
+    const uint32_t fc0 = chunks * cluster / a.clusters, nfc = chunks * (cluster + 1u) / a.clusters - fc0;  // FFN chunks
     const uint32_t groups = nfc * 8u;                  // of 8 gate rows and the 8 up rows they gate: one tile
     const uint32_t g0 = groups * rank / kC, n1 = groups * (rank + 1u) / kC - g0;
     const uint32_t row_tiles = H / 16u, t0 = row_tiles * rank / kC, n2 = row_tiles * (rank + 1u) / kC - t0;
     const ffn_smem L = ffn_layout(H, a.acts, a.tiles1, a.tiles2, ring_slots);
-    unsigned char *dig1 = smem, *dig2 = smem + L.dig2;
     float *acts = (float *)(smem + L.acts), *part = (float *)(smem + L.part), *red = (float *)(smem + L.red);
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tmdev::warp_index();
     cluster_arrive();
-    auto row1 = [=](uint32_t tile, uint32_t r) -> size_t {
-        return fc0 * 64u + (g0 + tile) * 8u + (r & 7u) + (r & 8u ? F : 0u);
-    };
-    auto row2 = [=](uint32_t tile, uint32_t r) -> size_t { return (t0 + tile) * 16u + r; };
-    weight_pieces<decltype(row1), decltype(row2)> W = {
-        {a.gu_q, a.gu_d, H, 0u, n1, H / 64u}, {a.dn_q, a.dn_d, F, fc0, n2, nfc}, row1, row2};
-    W.start(smem_addr(smem + L.ring) + warp * ring_slots * kSlotBytes);
+    const matrix_part m1 = {a.gu_q, a.gu_d, H, 0u, n1, H / 64u}, m2 = {a.dn_q, a.dn_d, F, fc0, n2, nfc};
+    const uint32_t ring = smem_addr(smem + L.ring) + warp * ring_slots * kSlotBytes;
+    load_pieces(m1, m2, ring, [=](uint32_t sec, uint32_t tile) {
+        return sec ? make_uint2((t0 + tile) * 16u, 8u) : make_uint2(fc0 * 64u + (g0 + tile) * 8u, F);
+    });
+    const span w1(m1, ring), w2(m2, ring + (w1.end - w1.first) * kSlotBytes);
     tmdev::pdl_trigger();
     tmdev::pdl_wait();
-    stage_residual<NB>(a.in, cluster == 0u, rank, dig1, red);
-    __syncthreads();
-    W.multiply(W.m1, false, dig1, plane_bytes(H), part);
-    __syncthreads();
-    cluster_wait();  // every CTA of the cluster has started
-    // A warp finishes an activation: gate in its lower half, up in its upper; lane c of the lower half sends it to CTA c.
-    for (uint32_t i = warp; i < n1 * 8u; i += kWarps) {
-        const float sum = half_sum(part, W.m1, i >> 3, (i & 7u) + (lane & 16u) / 2u);
-        const float up = __shfl_down_sync(0xffffffffu, sum, 16);
-        const float v = (a.gelu ? tmdev::gelu_tanh_f(sum) : tmdev::silu_f(sum)) * up;
-        if (lane < kC) st_cluster(smem_addr(acts + g0 * 8u + i), lane, v);
+#pragma unroll 1
+    for (uint32_t sec = 0; sec < 2u; ++sec) {
+        const uint32_t quads = sec ? nfc * 16u : H / 4u, plane = plane_bytes(sec ? a.acts : H);
+        float4 v[NB];
+        if (sec == 0u) {
+            residual_norm<NB>(a.in, cluster == 0u, rank, v, red);
+        } else {
+            cluster_wait();  // every CTA of the cluster has started
+            // A warp finishes four activations: the gate rows in its lower half, the up rows in its upper; the four lanes
+            // of an activation send it to four CTAs each.
+#pragma unroll 1
+            for (uint32_t i = warp; i < n1 * 2u; i += kWarps) {
+                const uint32_t act = i * 4u + ((lane >> 2) & 3u);
+                const float sum = quad_sum(part, m1.chunks, (act >> 3) * 16u + (act & 7u) + (lane & 16u) / 2u);
+                const float up = __shfl_down_sync(0xffffffffu, sum, 16);
+                const float z = (a.gelu ? tmdev::gelu_tanh_f(sum) : tmdev::silu_f(sum)) * up;
+                if (lane < 16u)
+#pragma unroll
+                    for (uint32_t k = 0; k < kC / 4u; ++k) st_cluster(smem_addr(acts + g0 * 8u + act), (lane & 3u) * (kC / 4u) + k, z);
+            }
+            cluster_arrive();
+            cluster_wait();
+        }
+#pragma unroll 1
+        for (uint32_t q0 = warp * 32u; q0 < quads; q0 += NB * kT)
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                const uint32_t q = q0 + i * kT + lane;
+                if (q0 + i * kT >= quads) break;
+                if (sec) v[i] = q < quads ? *(const float4 *)(acts + q * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float y[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+                tmdev::digitise_quad(y, q < quads, (signed char *)smem + q * 4u, plane, (float *)(smem + 4u * plane) + (q >> 3) * 4u, lane);
+            }
+        __syncthreads();
+        multiply(sec ? w2 : w1, sec ? m2.chunks : m1.chunks, sec, smem, plane, part);
+        __syncthreads();
     }
-    cluster_arrive();
-    cluster_wait();
-    for (uint32_t q = threadIdx.x; (q & ~31u) < nfc * 16u; q += kT) {
-        const bool live = q < nfc * 16u;
-        const float4 v = live ? *(const float4 *)(acts + q * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float y[4] = {v.x, v.y, v.z, v.w};
-        digitise(y, q * 4u, live, dig2, plane_bytes(a.acts));
-    }
-    __syncthreads();
-    W.multiply(W.m2, true, dig2, plane_bytes(a.acts), part);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n2 * 16u; i += kT)
-        a.slots_out[(size_t)cluster * H + t0 * 16u + i] = row_sum(part, W.m2, i >> 4, i & 15u);
+    store_slot(part, m2, a.slots_out + (size_t)cluster * H + t0 * 16u);
+    for (uint32_t s = cluster + a.clusters; s < kSlots; s += a.clusters)  // slots without a cluster
+        for (uint32_t i = tid; i < n2 * 16u; i += kT) a.slots_out[(size_t)s * H + t0 * 16u + i] = 0.0f;
 }
 
 // ---------------- attention block ----------------
@@ -374,18 +370,16 @@ struct attn_block_args {
 };
 
 struct attn_smem {
-    uint32_t dig2, state, qkv, recv, recv_ml, wgt, part, red, ring, bytes;
+    uint32_t state, qkv, recv, recv_ml, part, red, ring, bytes;
 };
 template <int G, int HD>
 __host__ __device__ inline attn_smem attn_layout(uint32_t hidden, uint32_t tiles1, uint32_t tiles2, uint32_t slots) {
     attn_smem s;
-    s.dig2 = digit_bytes(hidden);
-    s.state = s.dig2 + digit_bytes(G * HD);
+    s.state = digit_bytes(max_of(hidden, G * HD));
     s.qkv = s.state + (uint32_t)((sizeof(shared_state<G, HD>) + 15u) & ~15u);
     s.recv = s.qkv + (G + 2) * HD * 4u;
     s.recv_ml = s.recv + kC * G * HD * 4u;
-    s.wgt = s.recv_ml + kC * G * 2u * 4u;
-    s.part = s.wgt + kC * G * 4u;
+    s.part = s.recv_ml + kC * G * 2u * 4u;
     s.red = s.part + 64u * max_of(tiles1 * (hidden / 64u), tiles2 * (G * HD / 64u));
     s.ring = s.red + 64u;
     s.bytes = s.ring + kWarps * slots * kSlotBytes;
@@ -398,131 +392,160 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
     constexpr int EPL = HD / 32;
     constexpr uint32_t kTiles = (G + 2) * HD / 16u;  // of this KV head's q, k and v rows
     const uint32_t rank = cluster_rank(), kvh = blockIdx.x / kC, H = a.in.hidden, cap = a.cap;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, tid = threadIdx.x;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tmdev::warp_index();
     const uint32_t u0 = kTiles * rank / kC, n1 = kTiles * (rank + 1u) / kC - u0;
     const uint32_t row_tiles = H / 16u, t0 = row_tiles * rank / kC, n2 = row_tiles * (rank + 1u) / kC - t0;
     const attn_smem L = attn_layout<G, HD>(H, a.tiles1, a.tiles2, ring_slots);
-    unsigned char *dig1 = smem, *dig2 = smem + L.dig2;
     shared_state<G, HD> &sh = *(shared_state<G, HD> *)(smem + L.state);
     float *qkv = (float *)(smem + L.qkv), *recv = (float *)(smem + L.recv), *recv_ml = (float *)(smem + L.recv_ml);
-    float *wgt = (float *)(smem + L.wgt), *part = (float *)(smem + L.part), *red = (float *)(smem + L.red);
+    float *part = (float *)(smem + L.part), *red = (float *)(smem + L.red);
     cluster_arrive();
-    // Row r of tile t, counted over this head's q rows, then its k rows, then its v rows.
     const uint32_t kvw = a.kv_heads * HD;
-    auto row1 = [=](uint32_t tile, uint32_t r) -> size_t {
-        const uint32_t i = (u0 + tile) * 16u + r;
-        return i < G * HD         ? kvh * (G * HD) + i
-               : i < (G + 1) * HD ? kvw * G + kvh * HD + (i - G * HD)
-                                  : kvw * (G + 1) + kvh * HD + (i - (G + 1) * HD);
-    };
-    auto row2 = [=](uint32_t tile, uint32_t r) -> size_t { return (t0 + tile) * 16u + r; };
-    weight_pieces<decltype(row1), decltype(row2)> W = {
-        {a.qkv_q, a.qkv_d, H, 0u, n1, H / 64u}, {a.o_q, a.o_d, kvw * G, kvh * (G * HD / 64u), n2, G * HD / 64u}, row1, row2};
-    W.start(smem_addr(smem + L.ring) + warp * ring_slots * kSlotBytes);
+    const matrix_part m1 = {a.qkv_q, a.qkv_d, H, 0u, n1, H / 64u}, m2 = {a.o_q, a.o_d, kvw * G, kvh * (G * HD / 64u), n2, G * HD / 64u};
+    const uint32_t ring = smem_addr(smem + L.ring) + warp * ring_slots * kSlotBytes;
+    // Tiles are counted over this head's q rows, then its k rows, then its v rows.
+    load_pieces(m1, m2, ring, [=](uint32_t sec, uint32_t tile) {
+        const uint32_t i = (u0 + tile) * 16u;
+        return make_uint2(sec             ? (t0 + tile) * 16u
+                          : i < G * HD    ? kvh * (G * HD) + i
+                          : i < (G + 1) * HD ? kvw * G + kvh * HD + (i - G * HD)
+                                          : kvw * (G + 1) + kvh * HD + (i - (G + 1) * HD),
+                          8u);
+    });
+    const span w1(m1, ring), w2(m2, ring + (w1.end - w1.first) * kSlotBytes);
     __half *kp = a.kc + (size_t)kvh * cap * HD, *vp = a.vc + (size_t)kvh * cap * HD;
     const volatile uint32_t *pos_p = a.pos;
     keys<G, HD> K;
-    K.early(kp, vp, min(*pos_p, cap - 1u), a.window, kC, rank);
-    tmdev::pdl_wait();
-    tmdev::pdl_trigger();  // only now: see tm_cuda_attn_core.cuh
-    const uint32_t pos = *pos_p;
-    stage_residual<NB>(a.in, kvh == 0u, rank, dig1, red);
-    if (pos >= cap) {  // uniform over the cluster; the pieces's copies land before the CTA's memory goes away
+    float nw[EPL];  // warp g < G: query head g; warp G: the new key
+    rotation<HD> rot;
+    uint32_t pos = tmdev::uniform(min(*pos_p, cap - 1u));
+    K.ask(kp, vp, pos, a.window, kC, rank);
+#pragma unroll
+    for (int r = 0; r < EPL; ++r) nw[r] = __ldg((warp == G ? a.k_norm : a.q_norm) + lane + 32 * r);
+#pragma unroll 1
+    for (uint32_t hint = pos;;) {  // the angles of the position as it reads before the wait, again where it was another
+        if (warp <= G) rot.set(a.inv_freq, min(pos, cap - 1u));
+        if (hint == ~0u) break;
+        tmdev::pdl_wait();
+        tmdev::pdl_trigger();  // only now: see tm_cuda_attn_core.cuh
+        pos = tmdev::uniform(*pos_p);
+        if (pos == hint) break;
+        hint = ~0u;
+    }
+    if (pos >= cap) {  // uniform over the cluster; the pieces' copies land before the CTA's memory goes away
         if (tid == 0 && rank == 0) atomicOr(a.status, 1u);
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         cluster_wait();
         return;
     }
-    K.late(pos, a.window, kC, rank);
-    float nw[EPL];  // warp g < G: query head g; warp G: the new key
-    rotation<HD> rot;
-    if (warp <= G) {
-        const float *src = warp == G ? a.k_norm : a.q_norm;
+#pragma unroll 1
+    for (uint32_t sec = 0; sec < 2u; ++sec) {
+        const uint32_t quads = (sec ? G * HD : H) / 4u, plane = plane_bytes(sec ? G * HD : H);
+        float4 v[NB];
+        if (sec == 0u) {
+            residual_norm<NB>(a.in, kvh == 0u, rank, v, red);
+            K.first_tile(pos, a.window, kC, rank);
+        } else {
+            cluster_wait();  // every CTA of the cluster has started
+            // Four lanes finish a row and send it to four CTAs each.
+#pragma unroll 1
+            for (uint32_t i0 = warp * 8u; i0 < n1 * 16u; i0 += kT / 4u) {
+                const uint32_t i = i0 + lane / 4u;
+                const float z = quad_sum(part, m1.chunks, i);
 #pragma unroll
-        for (int r = 0; r < EPL; ++r) nw[r] = __ldg(src + lane + 32 * r);
-        rot.set(a.inv_freq, pos);
-    }
-    __syncthreads();
-    W.multiply(W.m1, false, dig1, plane_bytes(H), part);
-    __syncthreads();
-    cluster_wait();  // every CTA of the cluster has started
-    // Half a warp finishes a row; its lane c sends it to CTA c.
-    for (uint32_t i = warp * 2u + (lane >> 4); i < n1 * 16u; i += 2u * kWarps)
-        st_cluster(smem_addr(qkv + u0 * 16u + i), lane & 15u, half_sum(part, W.m1, i >> 4, i & 15u));
-    cluster_arrive();
-    cluster_wait();
-    // ---- every CTA has the head's q, k and v ----
-    if (warp < G || (warp == G && K.lo <= pos && pos < K.hi)) {
-        float x[EPL];
-#pragma unroll
-        for (int r = 0; r < EPL; ++r) x[r] = qkv[warp * HD + lane + 32 * r];
-        norm_rope<HD>(x, nw, rot, a.in.eps);
-#pragma unroll
-        for (int r = 0; r < EPL; ++r) {
-            const uint32_t e = lane + 32 * r;
-            if (warp == G) {
-                const __half hk = __float2half_rn(x[r]), hv = __float2half_rn(qkv[(G + 1) * HD + e]);
-                sh.kh[e] = hk;
-                sh.vh[e] = hv;
-                kp[(size_t)pos * HD + e] = hk;
-                vp[(size_t)pos * HD + e] = hv;
-            } else {
-                sh.qs[warp][e] = x[r];
+                for (uint32_t k = 0; k < kC / 4u; ++k) st_cluster(smem_addr(qkv + u0 * 16u + i), (lane & 3u) * (kC / 4u) + k, z);
             }
-        }
-    }
-    __syncthreads();
-    K.attend(sh, pos, a.scale);
-    __syncthreads();
-    keys<G, HD>::combine(sh);
-    // ---- this CTA's (max, sum, output) to every CTA: each needs all of the head's output for its rows of o ----
-    for (uint32_t i = tid; i < G * HD; i += kT) {
-        const float o = keys<G, HD>::value(sh, i);
-        const uint32_t at = smem_addr(recv + rank * G * HD + i);
+            cluster_arrive();
+            cluster_wait();
+            // ---- every CTA has the head's q, k and v ----
+            if (warp < G || (warp == G && K.lo <= pos && pos < K.hi)) {
+                float x[EPL];
 #pragma unroll
-        for (uint32_t to = 0; to < kC; ++to) st_cluster(at, (to + warp) % kC, o);
-    }
-    for (uint32_t i = tid; i < kC * G * 2u; i += kT) {
-        const uint32_t e = i % (2u * G);
-        st_cluster(smem_addr(recv_ml + rank * 2u * G + e), i / (2u * G), sh.l[e % G][e / G]);
-    }
-    cluster_arrive();
-    cluster_wait();
-    if (warp < G) {  // weight of source CTA `lane` in head `warp`
-        const float m = lane < kC ? recv_ml[lane * 2u * G + warp] : -INFINITY;
-        float M = m;
+                for (int r = 0; r < EPL; ++r) x[r] = qkv[warp * HD + lane + 32 * r];
+                norm_rope<HD>(x, nw, rot, a.in.eps);
 #pragma unroll
-        for (int off = 8; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
-        const float f = lane < kC ? expf(m - M) : 0.0f;  // a CTA without keys: exp(-inf) = 0
-        float l = lane < kC ? f * recv_ml[lane * 2u * G + G + warp] : 0.0f;
-#pragma unroll
-        for (int off = 8; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
-        if (lane < kC) wgt[warp * kC + lane] = f / l;
-    }
-    __syncthreads();
-    for (uint32_t q = tid; (q & ~31u) < G * HD / 4u; q += kT) {
-        const bool live = q < G * HD / 4u;
-        float y[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (live) {
-            const float *wg = wgt + (q * 4u / HD) * kC;
-#pragma unroll
-            for (uint32_t s = 0; s < kC; ++s) {
-                const float4 o = *(const float4 *)(recv + s * G * HD + q * 4u);
-                const float f = wg[s];
-                y[0] = fmaf(f, o.x, y[0]);
-                y[1] = fmaf(f, o.y, y[1]);
-                y[2] = fmaf(f, o.z, y[2]);
-                y[3] = fmaf(f, o.w, y[3]);
+                for (int r = 0; r < EPL; ++r) {
+                    const uint32_t e = lane + 32 * r;
+                    if (warp == G) {
+                        const __half hk = __float2half_rn(x[r]), hv = __float2half_rn(qkv[(G + 1) * HD + e]);
+                        sh.kh[e] = hk;
+                        sh.vh[e] = hv;
+                        kp[(size_t)pos * HD + e] = hk;
+                        vp[(size_t)pos * HD + e] = hv;
+                    } else {
+                        sh.qs[warp][e] = x[r];
+                    }
+                }
             }
+            __syncthreads();
+            K.attend(sh, pos, a.scale);
+            __syncthreads();
+            // ---- this CTA's (max, sum, output) to every CTA: each needs all of the head's output for its rows of o ----
+            keys<G, HD>::combine(sh);
+#pragma unroll 1
+            for (uint32_t i = tid; i < G * HD; i += kT) {
+                const float o = keys<G, HD>::value(sh, i);
+                const uint32_t at = smem_addr(recv + rank * G * HD + i);
+#pragma unroll 4
+                for (uint32_t to = 0; to < kC; ++to) st_cluster(at, (to + warp) % kC, o);
+            }
+#pragma unroll 1
+            for (uint32_t i = tid; i < kC * G * 2u; i += kT) {
+                const uint32_t e = i % (2u * G);
+                st_cluster(smem_addr(recv_ml + rank * 2u * G + e), i / (2u * G), sh.l[e % G][e / G]);
+            }
+            cluster_arrive();
+            cluster_wait();
         }
-        digitise(y, q * 4u, live, dig2, plane_bytes(G * HD));
+        // Four lanes to a quad of the attention's output, each with a quarter of the source CTAs.
+        const uint32_t shift = sec ? 2u : 0u;
+#pragma unroll 1
+        for (uint32_t q0 = (warp * 32u) >> shift; q0 < quads; q0 += NB * (kT >> shift))
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                const uint32_t q = q0 + i * (kT >> shift) + (lane >> shift);
+                if (q0 + i * (kT >> shift) >= quads) break;
+                if (sec) {
+                    const uint32_t head = q * 4u / HD, c0 = (lane & 3u) * (kC / 4u);
+                    float m[kC / 4u], M = -INFINITY, l = 0.0f;
+#pragma unroll
+                    for (uint32_t k = 0; k < kC / 4u; ++k) {
+                        m[k] = recv_ml[(c0 + k) * 2u * G + head];
+                        M = fmaxf(M, m[k]);
+                    }
+                    M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 1));
+                    M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 2));
+                    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (uint32_t k = 0; k < kC / 4u; ++k) {
+                        const float4 o = *(const float4 *)(recv + (c0 + k) * G * HD + q * 4u);
+                        const float f = expf(m[k] - M);  // a CTA without keys: exp(-inf) = 0
+                        l = fmaf(f, recv_ml[(c0 + k) * 2u * G + G + head], l);
+                        v[i].x = fmaf(f, o.x, v[i].x);
+                        v[i].y = fmaf(f, o.y, v[i].y);
+                        v[i].z = fmaf(f, o.z, v[i].z);
+                        v[i].w = fmaf(f, o.w, v[i].w);
+                    }
+#pragma unroll
+                    for (int off = 1; off < 4; off <<= 1) {
+                        l += __shfl_xor_sync(0xffffffffu, l, off);
+                        v[i].x += __shfl_xor_sync(0xffffffffu, v[i].x, off);
+                        v[i].y += __shfl_xor_sync(0xffffffffu, v[i].y, off);
+                        v[i].z += __shfl_xor_sync(0xffffffffu, v[i].z, off);
+                        v[i].w += __shfl_xor_sync(0xffffffffu, v[i].w, off);
+                    }
+                    const float inv = 1.0f / l;
+                    v[i] = make_float4(v[i].x * inv, v[i].y * inv, v[i].z * inv, v[i].w * inv);
+                }
+                const float y[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+                tmdev::digitise_quad(y, q < quads, (signed char *)smem + q * 4u, plane, (float *)(smem + 4u * plane) + (q >> 3) * 4u, lane, shift);
+            }
+        __syncthreads();
+        multiply(sec ? w2 : w1, sec ? m2.chunks : m1.chunks, sec, smem, plane, part);
+        __syncthreads();
     }
-    __syncthreads();
-    W.multiply(W.m2, true, dig2, plane_bytes(G * HD), part);
-    __syncthreads();
-    for (uint32_t i = tid; i < n2 * 16u; i += kT)
-        a.slots_out[(size_t)kvh * H + t0 * 16u + i] = row_sum(part, W.m2, i >> 4, i & 15u);
+    store_slot(part, m2, a.slots_out + (size_t)kvh * H + t0 * 16u);
 }
 
 // ---------------- launches ----------------
@@ -575,7 +598,7 @@ cudaError_t launch_clusters(tm_cuda_ctx *ctx, Kernel kernel, std::atomic<bool> *
 template <int NB>
 cudaError_t launch_ffn(tm_cuda_ctx *ctx, const ffn_args &a, uint32_t slots) {
     static std::atomic<bool> attr_set[64] = {};  // per device; contexts of a process share it
-    return launch_clusters(ctx, ffn_block_kernel<NB>, attr_set, kSlots,
+    return launch_clusters(ctx, ffn_block_kernel<NB>, attr_set, a.clusters,
                            ffn_layout(a.in.hidden, a.acts, a.tiles1, a.tiles2, slots).bytes, a, slots);
 }
 template <int G, int HD, int NB>
@@ -618,18 +641,22 @@ bool attn_shape(uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t hd)
     return hidden >= 64u && hidden % 64u == 0u && hidden <= 2048u && (hd == 128u || hd == 256u) && kv_heads >= 1u &&
            kv_heads <= kSlots && heads == g * kv_heads && (g == 1u || g == 2u || g == 4u) && attn_items(hidden, g, hd) <= kResident;
 }
+uint32_t ffn_items(const ffn_args &a) {
+    return ceil_div(a.tiles1 * (a.in.hidden / 64u), kWarps) + ceil_div(a.tiles2 * (a.acts / 64u), kWarps);
+}
 ffn_args ffn_shape(uint32_t hidden, uint32_t width) {
     ffn_args a = {};
     a.in.hidden = hidden;
     a.width = width;
-    const uint32_t nfc = ceil_div(width / 64u, kSlots);
-    a.acts = nfc * 64u;
-    a.tiles1 = ceil_div(nfc * 8u, kC);
-    a.tiles2 = ceil_div(hidden / 16u, kC);
+    for (uint32_t clusters : {kFfnClusters, kSlots}) {
+        const uint32_t nfc = ceil_div(width / 64u, clusters);
+        a.clusters = clusters;
+        a.acts = nfc * 64u;
+        a.tiles1 = ceil_div(nfc * 8u, kC);
+        a.tiles2 = ceil_div(hidden / 16u, kC);
+        if (ffn_items(a) <= kResident) break;
+    }
     return a;
-}
-uint32_t ffn_items(const ffn_args &a) {
-    return ceil_div(a.tiles1 * (a.in.hidden / 64u), kWarps) + ceil_div(a.tiles2 * (a.acts / 64u), kWarps);
 }
 bool ffn_shape_ok(uint32_t hidden, uint32_t width) {
     return hidden >= 64u && hidden % 64u == 0u && hidden <= 2048u && width % 64u == 0u && width / 64u >= kSlots &&
