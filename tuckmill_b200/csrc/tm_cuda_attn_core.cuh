@@ -300,6 +300,25 @@ struct keys {
         }
         __syncthreads();
     }
+    // After the same barrier: dims d .. d + 3 of head g (not yet divided by the sum) by one thread, with the CTA's maximum
+    // and sum.  For a thread that finishes one quad: every factor once, and no barrier.
+    static __device__ __forceinline__ float2 combined(const S &s, uint32_t g, uint32_t d, float4 &o) {
+        float m[kT / 32], M = -INFINITY, L = 0.0f;
+        o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < kT / 32; ++w) M = fmaxf(M, m[w] = s.m[g][w]);
+#pragma unroll
+        for (int w = 0; w < kT / 32; ++w) {
+            const float f = M == -INFINITY ? 0.0f : expf(m[w] - M);
+            const float4 v = *(const float4 *)&s.opart[w][g][d];
+            L = fmaf(f, s.l[g][w], L);
+            o.x = fmaf(f, v.x, o.x);
+            o.y = fmaf(f, v.y, o.y);
+            o.z = fmaf(f, v.z, o.z);
+            o.w = fmaf(f, v.w, o.w);
+        }
+        return make_float2(M, L);
+    }
     // After combine: value i (head i / HD, dim i % HD), not yet divided by the sum.
     static __device__ __forceinline__ float value(const S &s, uint32_t i) {
         const uint32_t g = i / HD, d = i % HD;

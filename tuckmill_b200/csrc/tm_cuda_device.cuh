@@ -172,4 +172,40 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {
     return v;
 }
 
+
+// ---- values sent to a peer's shared memory that arrive at a barrier of the peer's, counted in bytes ----
+// A cluster barrier takes a release of everything a CTA has stored and the last CTA's arrival; a CTA that waits for the
+// bytes it needs goes on as soon as they are there.
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t bytes) {  // one use: `bytes` will arrive
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ void send(uint32_t addr, uint32_t bar, uint32_t rank, float v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(map_rank(addr, rank)), "f"(v),
+                 "r"(map_rank(bar, rank)) : "memory");
+}
+__device__ __forceinline__ void send(uint32_t addr, uint32_t bar, uint32_t rank, float2 v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(map_rank(addr, rank)),
+                 "f"(v.x), "f"(v.y), "r"(map_rank(bar, rank)) : "memory");
+}
+__device__ __forceinline__ void send(uint32_t addr, uint32_t bar, uint32_t rank, float4 v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(map_rank(addr, rank)),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(map_rank(bar, rank)) : "memory");
+}
+// Waits for a barrier's one use, at most some tenths of a second; a wait that runs out sets `flag` and returns.
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t *flag) {
+    uint32_t done = 0;
+#pragma unroll 1
+    for (uint32_t i = 0; i < (1u << 20) && !done; ++i)
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.b32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done) : "r"(bar) : "memory");
+    if (!done) *(volatile uint32_t *)flag = 1u;
+}
+
 }  // namespace tmdev

@@ -97,8 +97,8 @@ struct tm_cuda_ctx {
     // Scratch owned by the context for the tensor-core GEMM (f16 copy of X).
     unsigned char *mma_scratch = nullptr;
     size_t mma_scratch_bytes = 0;
-    // Set by a tensor-core GEMM whose bounded wait ran out: host memory the device can write, so that the
-    // host looks at it without a copy.
+    // Set by a kernel whose bounded wait for a pipeline stage (tensor-core GEMM) or for a peer CTA's values (decode
+    // layer blocks) ran out: host memory the device can write, so that the host looks at it without a copy.
     volatile uint32_t *mma_abort = nullptr;
     int mma_last_bn = 0;                 // token sub-tile width of the last tensor-core GEMM launch
     int mma_last_sets = 0;               // its sets of converter warps
@@ -210,6 +210,16 @@ int tm_op_end(tm_cuda_ctx *ctx, uint64_t kernels, char *err, size_t err_cap);
                            cudaGetErrorString(le_));                                \
         return tm_op_end(ctx, (kernels), err, err_cap);                             \
     } while (0)
+
+inline cudaError_t tm_ensure_abort_flag(tm_cuda_ctx *ctx) {
+    if (ctx->mma_abort) return cudaSuccess;
+    void *f = nullptr;
+    const cudaError_t e = cudaHostAlloc(&f, 4, cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    ctx->mma_abort = (volatile uint32_t *)f;
+    *ctx->mma_abort = 0u;
+    return e;
+}
 
 inline size_t tm_round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 inline size_t tm_q8_qplane_bytes(uint32_t rows, uint32_t cols) {

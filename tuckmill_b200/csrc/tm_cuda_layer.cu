@@ -51,6 +51,7 @@ struct residual_in {
     const float *add_w;   // RMS norm weight of their sum (a layer's output norm), or null
     const float *norm_w;  // the block's own input norm
     float *x_out;         // the updated stream
+    uint32_t *late;       // set when an exchange inside a cluster did not arrive
     uint32_t n_slots, hidden;
     float eps;
 };
@@ -280,14 +281,15 @@ struct ffn_args {
 
 // Shared memory: digits (of x, then of the activations), activations, partial sums, ring.
 struct ffn_smem {
-    uint32_t acts, part, red, ring, bytes;
+    uint32_t acts, part, red, bar, ring, bytes;
 };
 __host__ __device__ inline ffn_smem ffn_layout(uint32_t hidden, uint32_t acts, uint32_t tiles1, uint32_t tiles2, uint32_t slots) {
     ffn_smem s;
     s.acts = digit_bytes(max_of(hidden, acts));
     s.part = s.acts + acts * 4u;
     s.red = s.part + 64u * max_of(tiles1 * (hidden / 64u), tiles2 * (acts / 64u));
-    s.ring = s.red + 64u;
+    s.bar = s.red + 64u;
+    s.ring = s.bar + 16u;
     s.bytes = s.ring + kWarps * slots * kSlotBytes;
     return s;
 }
@@ -304,6 +306,8 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
     const ffn_smem L = ffn_layout(H, a.acts, a.tiles1, a.tiles2, ring_slots);
     float *acts = (float *)(smem + L.acts), *part = (float *)(smem + L.part), *red = (float *)(smem + L.red);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tmdev::warp_index();
+    const uint32_t bar = smem_addr(smem + L.bar);
+    if (tid == 0) tmdev::mbar_init(bar, nfc * 256u);  // all activations of the cluster
     cluster_arrive();
     const matrix_part m1 = {a.gu_q, a.gu_d, H, 0u, n1, H / 64u}, m2 = {a.dn_q, a.dn_d, F, fc0, n2, nfc};
     const uint32_t ring = smem_addr(smem + L.ring) + warp * ring_slots * kSlotBytes;
@@ -331,10 +335,9 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
                 const float z = (a.gelu ? tmdev::gelu_tanh_f(sum) : tmdev::silu_f(sum)) * up;
                 if (lane < 16u)
 #pragma unroll
-                    for (uint32_t k = 0; k < kC / 4u; ++k) st_cluster(smem_addr(acts + g0 * 8u + act), (lane & 3u) * (kC / 4u) + k, z);
+                    for (uint32_t k = 0; k < kC / 4u; ++k) tmdev::send(smem_addr(acts + g0 * 8u + act), bar, (lane & 3u) * (kC / 4u) + k, z);
             }
-            cluster_arrive();
-            cluster_wait();
+            tmdev::mbar_wait(bar, a.in.late);
         }
 #pragma unroll 1
         for (uint32_t q0 = warp * 32u; q0 < quads; q0 += NB * kT)
@@ -370,7 +373,7 @@ struct attn_block_args {
 };
 
 struct attn_smem {
-    uint32_t state, qkv, recv, recv_ml, part, red, ring, bytes;
+    uint32_t state, qkv, recv, recv_ml, part, red, bar, ring, bytes;
 };
 template <int G, int HD>
 __host__ __device__ inline attn_smem attn_layout(uint32_t hidden, uint32_t tiles1, uint32_t tiles2, uint32_t slots) {
@@ -381,7 +384,8 @@ __host__ __device__ inline attn_smem attn_layout(uint32_t hidden, uint32_t tiles
     s.recv_ml = s.recv + kC * G * HD * 4u;
     s.part = s.recv_ml + kC * G * 2u * 4u;
     s.red = s.part + 64u * max_of(tiles1 * (hidden / 64u), tiles2 * (G * HD / 64u));
-    s.ring = s.red + 64u;
+    s.bar = s.red + 64u;
+    s.ring = s.bar + 16u;
     s.bytes = s.ring + kWarps * slots * kSlotBytes;
     return s;
 }
@@ -399,6 +403,11 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
     shared_state<G, HD> &sh = *(shared_state<G, HD> *)(smem + L.state);
     float *qkv = (float *)(smem + L.qkv), *recv = (float *)(smem + L.recv), *recv_ml = (float *)(smem + L.recv_ml);
     float *part = (float *)(smem + L.part), *red = (float *)(smem + L.red);
+    const uint32_t bar = smem_addr(smem + L.bar);
+    if (tid == 0) {
+        tmdev::mbar_init(bar, (G + 2) * HD * 4u);               // this head's q, k and v
+        tmdev::mbar_init(bar + 8u, kC * (G * HD + 2 * G) * 4u);  // every CTA's (max, sum, output)
+    }
     cluster_arrive();
     const uint32_t kvw = a.kv_heads * HD;
     const matrix_part m1 = {a.qkv_q, a.qkv_d, H, 0u, n1, H / 64u}, m2 = {a.o_q, a.o_d, kvw * G, kvh * (G * HD / 64u), n2, G * HD / 64u};
@@ -454,10 +463,9 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                 const uint32_t i = i0 + lane / 4u;
                 const float z = quad_sum(part, m1.chunks, i);
 #pragma unroll
-                for (uint32_t k = 0; k < kC / 4u; ++k) st_cluster(smem_addr(qkv + u0 * 16u + i), (lane & 3u) * (kC / 4u) + k, z);
+                for (uint32_t k = 0; k < kC / 4u; ++k) tmdev::send(smem_addr(qkv + u0 * 16u + i), bar, (lane & 3u) * (kC / 4u) + k, z);
             }
-            cluster_arrive();
-            cluster_wait();
+            tmdev::mbar_wait(bar, a.in.late);
             // ---- every CTA has the head's q, k and v ----
             if (warp < G || (warp == G && K.lo <= pos && pos < K.hi)) {
                 float x[EPL];
@@ -482,21 +490,18 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
             K.attend(sh, pos, a.scale);
             __syncthreads();
             // ---- this CTA's (max, sum, output) to every CTA: each needs all of the head's output for its rows of o ----
-            keys<G, HD>::combine(sh);
+            {
+                constexpr uint32_t kQuads = G * HD / 4, kDest = kC * kQuads / kT;  // a thread's quad goes to kDest CTAs
+                const uint32_t quad = tid % kQuads, to = tid / kQuads * kDest, head = quad * 4u / HD;
+                float4 o;
+                const float2 ml = keys<G, HD>::combined(sh, head, quad * 4u % HD, o);
 #pragma unroll 1
-            for (uint32_t i = tid; i < G * HD; i += kT) {
-                const float o = keys<G, HD>::value(sh, i);
-                const uint32_t at = smem_addr(recv + rank * G * HD + i);
-#pragma unroll 4
-                for (uint32_t to = 0; to < kC; ++to) st_cluster(at, (to + warp) % kC, o);
+                for (uint32_t k = 0; k < kDest; ++k) {
+                    tmdev::send(smem_addr(recv + (rank * kQuads + quad) * 4u), bar + 8u, to + k, o);
+                    if (quad % (HD / 4u) == 0u) tmdev::send(smem_addr(recv_ml + (rank * G + head) * 2u), bar + 8u, to + k, ml);
+                }
             }
-#pragma unroll 1
-            for (uint32_t i = tid; i < kC * G * 2u; i += kT) {
-                const uint32_t e = i % (2u * G);
-                st_cluster(smem_addr(recv_ml + rank * 2u * G + e), i / (2u * G), sh.l[e % G][e / G]);
-            }
-            cluster_arrive();
-            cluster_wait();
+            tmdev::mbar_wait(bar + 8u, a.in.late);
         }
         // Four lanes to a quad of the attention's output, each with a quarter of the source CTAs.
         const uint32_t shift = sec ? 2u : 0u;
@@ -511,7 +516,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                     float m[kC / 4u], M = -INFINITY, l = 0.0f;
 #pragma unroll
                     for (uint32_t k = 0; k < kC / 4u; ++k) {
-                        m[k] = recv_ml[(c0 + k) * 2u * G + head];
+                        m[k] = recv_ml[((c0 + k) * G + head) * 2u];
                         M = fmaxf(M, m[k]);
                     }
                     M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 1));
@@ -521,7 +526,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                     for (uint32_t k = 0; k < kC / 4u; ++k) {
                         const float4 o = *(const float4 *)(recv + (c0 + k) * G * HD + q * 4u);
                         const float f = expf(m[k] - M);  // a CTA without keys: exp(-inf) = 0
-                        l = fmaf(f, recv_ml[(c0 + k) * 2u * G + G + head], l);
+                        l = fmaf(f, recv_ml[((c0 + k) * G + head) * 2u + 1u], l);
                         v[i].x = fmaf(f, o.x, v[i].x);
                         v[i].y = fmaf(f, o.y, v[i].y);
                         v[i].z = fmaf(f, o.z, v[i].z);
@@ -689,6 +694,8 @@ int check_residual(tm_cuda_ctx *ctx, residual_in &r, tm_cuda_buffer *x, tm_cuda_
                                o.name, i.name);
     if (((size_t)x->dev | (size_t)x_out->dev | (size_t)norm_w->dev | (n_slots ? (size_t)slots->dev : 0) | (add_w ? (size_t)add_w->dev : 0)) & 15u)
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "residual operands are not 16-byte aligned");
+    TM_CUDA_TRY(tm_ensure_abort_flag(ctx));
+    r.late = (uint32_t *)ctx->mma_abort;
     r.x = (const float *)x->dev;
     r.slots = n_slots ? (const float *)slots->dev : nullptr;
     r.add_w = n_slots && add_w ? (const float *)add_w->dev : nullptr;

@@ -819,14 +819,9 @@ int tm_cuda_mma_workspace_reserve(tm_cuda_ctx *ctx, size_t bytes, char *err, siz
         ctx->mma_scratch_bytes = 0;
     }
     void *p = nullptr;
-    if (!ctx->mma_abort) {
-        void *f = nullptr;
-        if (cudaHostAlloc(&f, 4, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-            cudaGetLastError();
-            return tm_fail(err, err_cap, TM_CUDA_ERR_ALLOC, "allocating the GEMM's status word failed");
-        }
-        ctx->mma_abort = (volatile uint32_t *)f;
-        *ctx->mma_abort = 0u;
+    if (tm_ensure_abort_flag(ctx) != cudaSuccess) {
+        cudaGetLastError();
+        return tm_fail(err, err_cap, TM_CUDA_ERR_ALLOC, "allocating the GEMM's status word failed");
     }
     const size_t total = tm_round_up(bytes, 256);
     if (cudaMalloc(&p, total) != cudaSuccess) {
