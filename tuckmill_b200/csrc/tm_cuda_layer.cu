@@ -68,42 +68,47 @@ __device__ __forceinline__ float cta_sum(float v, float *red) {
     return ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
 }
 
-// v = rmsnorm(x + [norm](sum of the slots)): NB quads of columns per thread, the sum stored by cluster 0.  `red`: 16
-// floats.
+// The weights of the input norm, asked for before the dependency wait.  (What is left of the residual, 3 thousand cycles,
+// is 128 CTAs that ask for the same 36 KB.)
 template <int NB>
-__device__ __forceinline__ void residual_norm(const residual_in &r, bool store, uint32_t rank, float4 (&v)[NB], float *red) {
-    const uint32_t H = r.hidden, quads = H / 4u;
-    const float inv_h = 1.0f / (float)H;
-    float4 nw[NB];
+__device__ __forceinline__ void norm_weights(const residual_in &r, float4 (&nw)[NB]) {
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
         const uint32_t q = threadIdx.x + i * kT;
-        v[i] = nw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (q < quads) {
-            v[i] = __ldcg((const float4 *)r.x + q);
-            nw[i] = __ldg((const float4 *)r.norm_w + q);
+        nw[i] = q < r.hidden / 4u ? __ldg((const float4 *)r.norm_w + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+// v = rmsnorm(x + [norm](sum of the slots)): NB quads of columns per thread, the sum stored by cluster 0.  `red`: 16
+// floats.  `meanwhile` runs while the loads are on their way.
+template <int NB, class F>
+__device__ __forceinline__ void residual_norm(const residual_in &r, bool store, uint32_t rank, const float4 (&nw)[NB], float4 (&v)[NB],
+                                              float *red, F meanwhile) {
+    const uint32_t H = r.hidden, quads = H / 4u;
+    const float inv_h = 1.0f / (float)H;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const uint32_t q = threadIdx.x + i * kT;
+        v[i] = q < quads ? __ldcg((const float4 *)r.x + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float4 p[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const uint32_t q = threadIdx.x + i * kT;
+        float4 s[kSlots];
+#pragma unroll
+        for (uint32_t k = 0; k < kSlots; ++k)
+            s[k] = q < quads && k < r.n_slots ? __ldcg((const float4 *)(r.slots + (size_t)k * H) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i == 0) meanwhile();
+        p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (uint32_t k = 0; k < kSlots; ++k) {
+            p[i].x += s[k].x;
+            p[i].y += s[k].y;
+            p[i].z += s[k].z;
+            p[i].w += s[k].w;
         }
     }
     if (r.n_slots) {
-        float4 p[NB];
-#pragma unroll
-        for (int i = 0; i < NB; ++i) {
-            const uint32_t q = threadIdx.x + i * kT;
-            p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (q < quads) {
-                float4 s[kSlots];
-#pragma unroll
-                for (uint32_t k = 0; k < kSlots; ++k)
-                    s[k] = k < r.n_slots ? __ldcg((const float4 *)(r.slots + (size_t)k * H) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (uint32_t k = 0; k < kSlots; ++k) {
-                    p[i].x += s[k].x;
-                    p[i].y += s[k].y;
-                    p[i].z += s[k].z;
-                    p[i].w += s[k].w;
-                }
-            }
-        }
         if (r.add_w) {
             float sq = 0.0f;
 #pragma unroll
@@ -314,6 +319,8 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
     load_pieces(m1, m2, ring, [=](uint32_t sec, uint32_t tile) {
         return sec ? make_uint2((t0 + tile) * 16u, 8u) : make_uint2(fc0 * 64u + (g0 + tile) * 8u, F);
     });
+    float4 nw[NB];
+    norm_weights<NB>(a.in, nw);
     const span w1(m1, ring), w2(m2, ring + (w1.end - w1.first) * kSlotBytes);
     tmdev::pdl_trigger();
     tmdev::pdl_wait();
@@ -322,7 +329,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
         const uint32_t quads = sec ? nfc * 16u : H / 4u, plane = plane_bytes(sec ? a.acts : H);
         float4 v[NB];
         if (sec == 0u) {
-            residual_norm<NB>(a.in, cluster == 0u, rank, v, red);
+            residual_norm<NB>(a.in, cluster == 0u, rank, nw, v, red, [] {});
         } else {
             cluster_wait();  // every CTA of the cluster has started
             // A warp finishes four activations: the gate rows in its lower half, the up rows in its upper; the four lanes
@@ -421,16 +428,18 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                                           : kvw * (G + 1) + kvh * HD + (i - (G + 1) * HD),
                           8u);
     });
+    float4 nw[NB];
+    norm_weights<NB>(a.in, nw);
     const span w1(m1, ring), w2(m2, ring + (w1.end - w1.first) * kSlotBytes);
     __half *kp = a.kc + (size_t)kvh * cap * HD, *vp = a.vc + (size_t)kvh * cap * HD;
     const volatile uint32_t *pos_p = a.pos;
     keys<G, HD> K;
-    float nw[EPL];  // warp g < G: query head g; warp G: the new key
+    float hw[EPL];  // warp g < G: query head g; warp G: the new key
     rotation<HD> rot;
     uint32_t pos = tmdev::uniform(min(*pos_p, cap - 1u));
     K.ask(kp, vp, pos, a.window, kC, rank);
 #pragma unroll
-    for (int r = 0; r < EPL; ++r) nw[r] = __ldg((warp == G ? a.k_norm : a.q_norm) + lane + 32 * r);
+    for (int r = 0; r < EPL; ++r) hw[r] = __ldg((warp == G ? a.k_norm : a.q_norm) + lane + 32 * r);
 #pragma unroll 1
     for (uint32_t hint = pos;;) {  // the angles of the position as it reads before the wait, again where it was another
         if (warp <= G) rot.set(a.inv_freq, min(pos, cap - 1u));
@@ -453,8 +462,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
         const uint32_t quads = (sec ? G * HD : H) / 4u, plane = plane_bytes(sec ? G * HD : H);
         float4 v[NB];
         if (sec == 0u) {
-            residual_norm<NB>(a.in, kvh == 0u, rank, v, red);
-            K.first_tile(pos, a.window, kC, rank);
+            residual_norm<NB>(a.in, kvh == 0u, rank, nw, v, red, [&] { K.first_tile(pos, a.window, kC, rank); });
         } else {
             cluster_wait();  // every CTA of the cluster has started
             // Four lanes finish a row and send it to four CTAs each.
@@ -471,7 +479,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                 float x[EPL];
 #pragma unroll
                 for (int r = 0; r < EPL; ++r) x[r] = qkv[warp * HD + lane + 32 * r];
-                norm_rope<HD>(x, nw, rot, a.in.eps);
+                norm_rope<HD>(x, hw, rot, a.in.eps);
 #pragma unroll
                 for (int r = 0; r < EPL; ++r) {
                     const uint32_t e = lane + 32 * r;
