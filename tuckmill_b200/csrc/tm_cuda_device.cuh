@@ -7,6 +7,12 @@ namespace tmdev {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 
+// A value that all lanes of the (whole, converged) warp hold, told to the compiler: it then knows that a branch on it
+// keeps the warp together.  Behind a branch that may split the warp, every shuffle is compiled twice, the second time
+// with the code that gathers the lanes first.
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ uint32_t warp_index() { return uniform(threadIdx.x >> 5); }
+
 // Canonical sum of squares of a vector, shared by every kernel that computes an
 // RMS norm so all of them produce the same bits:
 //   * elements are taken in quads; quad Q belongs to thread Q % 256, which adds
@@ -54,7 +60,11 @@ static __device__ float block_sumsq(const float *x, uint32_t n, float *red /* [k
     const bool vec = quads_vectorizable(x, n);
     const uint32_t quads = (n + 3u) / 4u;
     float s = 0.0f;
-    for (uint32_t q = threadIdx.x; q < quads; q += kThreads) s = sumsq_quad(s, load_quad(x, n, q, vec));
+#pragma unroll 2
+    for (uint32_t q0 = warp_index() * 32u; q0 < quads; q0 += kThreads) {
+        const uint32_t q = q0 + (threadIdx.x & 31u);
+        if (q < quads) s = sumsq_quad(s, load_quad(x, n, q, vec));
+    }
     return block_reduce_sumsq(s, red);
 }
 
@@ -66,12 +76,6 @@ static __device__ float block_sumsq(const float *x, uint32_t n, float *red /* [k
 // says which (TM_CHECK_AHEAD in tm_cuda_internal.cuh).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
-
-// A value that all lanes of the (whole, converged) warp hold, told to the compiler: it then knows that a branch on it
-// keeps the warp together.  Behind a branch that may split the warp, every shuffle is compiled twice, the second time
-// with the code that gathers the lanes first.
-__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
-__device__ __forceinline__ uint32_t warp_index() { return uniform(threadIdx.x >> 5); }
 
 __device__ __forceinline__ float silu_f(float g) { return g / (1.0f + expf(-g)); }
 __device__ __forceinline__ float gelu_tanh_f(float x) {

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kThreads) f16_gemv_kernel(const f16_args args)
     __shared__ float red[kWarps];
     constexpr int U = M == 1 ? (R == 1 ? 4 : 2) : 1;  // 256-column trips requested together
     const uint32_t cols = a.cols, rows = a.rows, octets = (cols + 7u) / 8u;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31, warp = tmdev::warp_index();
     const bool vec = (cols & 7u) == 0u && (((size_t)a.w) & 15u) == 0u;
     auto load = [&](uint32_t row, uint32_t o) -> int4 {
         if (o >= octets || row >= rows) return make_int4(0, 0, 0, 0);

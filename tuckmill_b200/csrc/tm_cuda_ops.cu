@@ -169,7 +169,7 @@ __device__ void argmax_block(float &v, uint32_t &i, float *tv, uint32_t *ti) {
         const uint32_t oi = __shfl_down_sync(0xffffffffu, i, o);
         if (better(ov, oi, v, i)) { v = ov; i = oi; }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = (int)tmdev::warp_index();
     if (lane == 0) { tv[warp] = v; ti[warp] = i; }
     __syncthreads();
     if (warp == 0) {
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) attention_decode_kernel(
     __shared__ __align__(16) float ks[32 * DPL];  // (one block holds the new position)
     __shared__ __align__(16) __half kh[32 * DPL];
     __shared__ __align__(16) __half vh[32 * DPL];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = (int)tmdev::warp_index();
     float *qs = qs_all[warp];
     const uint32_t head = blockIdx.x, blk = blockIdx.y * kDecodeWarps + warp, group = heads / kv_heads, kvh = head / group;
     const uint32_t nblk = (cap + kAttnBlock - 1) / kAttnBlock;

@@ -53,6 +53,35 @@ struct gemv_args {
     float *x_out = nullptr;
 };
 
+// The first n of a thread's quads (n is the same in a warp), after the elementwise prologue, to put(i, values): ONE copy
+// of the prologue and of what put does (the quads move down a register), because these kernels run their code once a
+// launch.  Four copies of three prologues and of the digit split were most of q8_gemv_kernel's 61 KB, twice an SM's
+// instruction cache.
+template <int B, class Put>
+__device__ __forceinline__ void finish_quads(float4 (&vs)[B], float4 (&ps)[B], int n, int prologue, float inv_rms, Put put) {
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+        float v[4] = {vs[0].x, vs[0].y, vs[0].z, vs[0].w};
+        const float pw[4] = {ps[0].x, ps[0].y, ps[0].z, ps[0].w};
+#pragma unroll
+        for (int k = 0; k + 1 < B; ++k) {
+            vs[k] = vs[k + 1];
+            ps[k] = ps[k + 1];
+        }
+        if (prologue == TM_CUDA_PRO_RMSNORM) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = v[j] * inv_rms * pw[j];
+        } else if (prologue == TM_CUDA_PRO_SILU_MUL) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = silu_f(v[j]) * pw[j];
+        } else if (prologue == TM_CUDA_PRO_GELU_MUL) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = gelu_tanh_f(v[j]) * pw[j];
+        }
+        put(i, v);
+    }
+}
+
 // Bytes of shared memory one token's staged activations take.
 __host__ __device__ inline size_t token_smem(uint32_t cols, uint32_t plane) {
     return 4u * (size_t)plane + (size_t)(cols / 32u) * 16u;
@@ -90,7 +119,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
     __shared__ float partial[kWarps][M][16];
     const uint32_t cols = a.cols, rows = a.rows, nb = cols / 32u, plane = a.plane;
     const size_t tok = token_smem(cols, plane);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = (int)tmdev::warp_index();
     const int g = lane >> 2, t4 = lane & 3;
 
     // Paired split (ks = 32): split v takes the chunk pairs v, v + 32, ...; a warp has the four splits 8 s + warp.
@@ -189,7 +218,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if constexpr (kAsync) {
-#pragma unroll
+#pragma unroll 1
         for (int i = 0; i < H; ++i) async_issue((uint32_t)i);
     } else {
         load_half(half0{});
@@ -293,23 +322,13 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
                 for (int i = 0; i < kBatch; ++i) sq = tmdev::sumsq_quad(sq, vs[i]);
                 inv_rms = 1.0f / sqrtf(tmdev::block_reduce_sumsq(sq, red) / (float)cols + a.eps);
             }
-#pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
+            // Whole warps have a quad or not: 32 lanes x 4 columns = 128 columns, and cols is a multiple of 32, so a
+            // partially filled warp keeps its out-of-range lanes (zeros) in the shuffles of the digit split.
+            const int left = (int)(cols - cb) - warp * 128, live = (left + kThreads * 4 - 1) / (kThreads * 4);
+            finish_quads(vs, ps, live < kBatch ? live : kBatch, a.prologue, inv_rms, [&](int i, const float (&v)[4]) {
                 const uint32_t c = cb + (i * kThreads + threadIdx.x) * 4u;
-                // Whole warps leave together: 32 lanes x 4 columns = 128 columns, and
-                // cols is a multiple of 32, so a partially filled warp keeps its
-                // out-of-range lanes (zeros) in the shuffles below.
-                if (cb + (i * kThreads + (threadIdx.x & ~31u)) * 4u >= cols) break;
-                float v[4] = {vs[i].x, vs[i].y, vs[i].z, vs[i].w};
-                const float pw[4] = {ps[i].x, ps[i].y, ps[i].z, ps[i].w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (a.prologue == TM_CUDA_PRO_RMSNORM) v[j] = v[j] * inv_rms * pw[j];
-                    else if (a.prologue == TM_CUDA_PRO_SILU_MUL) v[j] = silu_f(v[j]) * pw[j];
-                    else if (a.prologue == TM_CUDA_PRO_GELU_MUL) v[j] = gelu_tanh_f(v[j]) * pw[j];
-                }
                 digitise_quad(v, c < cols, dig + c, plane, coef + (c >> 5) * 4u, lane);
-            }
+            });
         }
     }
     __syncthreads();
@@ -476,6 +495,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemv_kernel(const gemv_args args)
                 }
             }
             __syncthreads();
+#pragma unroll 1
             for (uint32_t i = threadIdx.x; i < tiles_per_cta * M * 16u; i += kThreads) {
                 const uint32_t r16 = i & 15u, m = (i >> 4) % M, tl = i / (16u * M);
                 const uint32_t row = (base + tl) * 16u + r16;
@@ -519,7 +539,7 @@ __global__ void __launch_bounds__(kClusterThreads, 2) q8_gemv_cluster_kernel(con
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float red[kWarps];
     const uint32_t cols = a.cols, rows = a.rows, nb = cols / 32u, plane = a.plane;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, t4 = lane & 3u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tmdev::warp_index(), g = lane >> 2, t4 = lane & 3u;
     const uint32_t rank = blockIdx.x & (kClusterCtas - 1u), cluster = blockIdx.x / kClusterCtas;
     const uint32_t clusters = gridDim.x / kClusterCtas, n_tiles = (rows + 15u) / 16u, n_chunks = cols / kChunkCols;
     const uint32_t v = kClusterWarps * rank + warp;
@@ -555,7 +575,7 @@ __global__ void __launch_bounds__(kClusterThreads, 2) q8_gemv_cluster_kernel(con
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-#pragma unroll
+#pragma unroll 1
     for (uint32_t i = 0; i < kRing; ++i) issue(i);
     tmdev::pdl_trigger();
     tmdev::pdl_wait();
@@ -565,8 +585,12 @@ __global__ void __launch_bounds__(kClusterThreads, 2) q8_gemv_cluster_kernel(con
     if (a.prologue == TM_CUDA_PRO_RMSNORM) {  // the sum of squares of the 256-thread kernels
         const bool vec = tmdev::quads_vectorizable(a.x, cols);
         float ss = 0.0f;
-        if (tid < (uint32_t)kThreads)
-            for (uint32_t q = tid; q < cols / 4u; q += kThreads) ss = tmdev::sumsq_quad(ss, tmdev::load_quad(a.x, cols, q, vec));
+        if (warp < (uint32_t)kWarps)
+#pragma unroll 4
+            for (uint32_t q0 = warp * 32u; q0 < cols / 4u; q0 += kThreads) {
+                const uint32_t q = q0 + lane;
+                if (q < cols / 4u) ss = tmdev::sumsq_quad(ss, tmdev::load_quad(a.x, cols, q, vec));
+            }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         if (lane == 0u && warp < (uint32_t)kWarps) red[warp] = ss;
@@ -579,30 +603,31 @@ __global__ void __launch_bounds__(kClusterThreads, 2) q8_gemv_cluster_kernel(con
     const bool vec_ok = (((size_t)a.x | (size_t)a.pro) & 15u) == 0;
     const bool has_pro = a.prologue != TM_CUDA_PRO_NONE;
     const uint32_t segs = (cols + 4095u) / 4096u;
-#pragma unroll 4
-    for (uint32_t q = 0; q < segs; ++q) {
-        const uint32_t c = (kPairSplit * q + v) * 128u + lane * 4u, lc = q * 2048u + tid * 4u;
-        if (c - lane * 4u >= cols) break;  // (whole pairs of warps: cols may end with half a pair, whose lanes stay as zeros)
-        float x[4] = {0.f, 0.f, 0.f, 0.f}, pw[4] = {1.f, 1.f, 1.f, 1.f};
-        if (c < cols) {
-            if (vec_ok) {
-                *(float4 *)x = *(const float4 *)(a.x + c);
-                if (has_pro) *(float4 *)pw = *(const float4 *)(a.pro + c);
-            } else {
+    constexpr int kBatch = 4;
+#pragma unroll 1
+    for (uint32_t q0 = 0; q0 < segs; q0 += kBatch) {
+        float4 vs[kBatch], ps[kBatch];
+        int live = 0;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    x[j] = a.x[c + j];
-                    if (has_pro) pw[j] = a.pro[c + j];
+        for (uint32_t i = 0; i < kBatch; ++i) {
+            const uint32_t c = (kPairSplit * (q0 + i) + v) * 128u + lane * 4u;
+            vs[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            ps[i] = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (c - lane * 4u < cols) live = (int)i + 1;  // (cols may end with half a warp, whose lanes stay as zeros)
+            if (c < cols) {
+                if (vec_ok) {
+                    vs[i] = *(const float4 *)(a.x + c);
+                    if (has_pro) ps[i] = *(const float4 *)(a.pro + c);
+                } else {
+                    vs[i] = make_float4(a.x[c], a.x[c + 1], a.x[c + 2], a.x[c + 3]);
+                    if (has_pro) ps[i] = make_float4(a.pro[c], a.pro[c + 1], a.pro[c + 2], a.pro[c + 3]);
                 }
             }
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (a.prologue == TM_CUDA_PRO_RMSNORM) x[j] = x[j] * inv_rms * pw[j];
-            else if (a.prologue == TM_CUDA_PRO_SILU_MUL) x[j] = silu_f(x[j]) * pw[j];
-            else if (a.prologue == TM_CUDA_PRO_GELU_MUL) x[j] = gelu_tanh_f(x[j]) * pw[j];
-        }
-        digitise_quad(x, true, dig + lc, plane, coef + (lc >> 5) * 4u, lane);
+        finish_quads(vs, ps, live, a.prologue, inv_rms, [&](int i, const float (&x)[4]) {
+            const uint32_t lc = (q0 + i) * 2048u + tid * 4u;
+            digitise_quad(x, true, dig + lc, plane, coef + (lc >> 5) * 4u, lane);
+        });
     }
     __syncthreads();
 

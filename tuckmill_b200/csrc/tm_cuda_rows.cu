@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kThreads) q8_gemm_rows_kernel(const rows_args 
     constexpr uint32_t kTok = NT * 8;
     const uint32_t P = cluster_size(), rank = P > 1 ? cluster_rank() : 0u;
     const uint32_t n_clusters = gridDim.x / P, cluster = blockIdx.x / P;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const uint32_t warp = tmdev::warp_index(), lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     const uint32_t n_chunks = a.cols / 64u, nb = a.cols / 32u;
     const uint32_t c0 = n_chunks * rank / P, c1 = n_chunks * (rank + 1) / P;
     const uint32_t kc_max = (n_chunks + P - 1) / P;
