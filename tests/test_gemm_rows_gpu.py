@@ -66,3 +66,23 @@ def test_gemm_rows_parts_and_limits(ctx):
     for rows_of, batch in (([48, 48, 64], 3), ([64, 32, 64], 33)):
         with pytest.raises(cuda.CudaError):
             ctx.q8_0_gemm_rows(w, xb, 160, 128, batch, ys, rows_of)
+
+
+# X read where it lies: units of one part and of several, warps without a chunk, more units than find a place at once, the
+# staged form (8 tokens by many units); binary16 rows that lie on a 16-byte boundary only take half-width loads
+@pytest.mark.parametrize("rows,cols,batch", [(64, 64, 1), (1024, 3072, 32), (1056, 6912, 7), (4096, 4096, 24), (9504, 576, 31),
+                                             (9504, 64, 8), (9504, 5120, 8), (9504, 5120, 9)])
+def test_gemm_rows_x_at_either_alignment(ctx, rows, cols, batch):
+    raw = T.q8_0_matrix(14, rows + cols, rows, cols)
+    X = T.activations(14, 5, batch * cols).reshape(batch, cols).astype(np.float16)
+    w, yb = ctx.q8_0_matrix(raw, rows, cols), ctx.buffer(batch * rows * 4)
+    flat = ctx.buffer(batch * cols * 2 + 32)
+    got = []
+    for off in (0, 16):
+        x = flat.view(off, batch * cols * 2)
+        x.upload(0, X)
+        yb.zero()
+        ctx.q8_0_gemm_rows(w, x, rows, cols, batch, [yb], [rows], cuda.PRO_F16)
+        got.append(yb.download(0, batch * rows * 4, np.float32).reshape(batch, rows))
+    assert rel_err(got[0], f16_profile_reference(raw, X)) <= 2e-5
+    np.testing.assert_array_equal(got[0], got[1])

@@ -11,10 +11,19 @@
 // issue slots the weight stream leaves, so mma.sync suffices; from 33 rows on the tcgen05 kernel serves.
 //
 // Split.  A unit is 32 weight rows (two 16-row tiles, so that one read of the token fragments feeds two tiles).
-// A cluster of P CTAs owns a unit, each CTA a P-th of K, each of its 8 warps every 8th 64-column chunk of that;
-// the CTA's share of X (f16) stays in shared memory for all units it serves.  Sums meet in a fixed order: the
-// 8 warps through shared memory, the P CTAs through distributed shared memory -- no workspace, no counters.
-// P is the smallest cost of rounds x chunks a warp streams (see plan_rows).
+// A cluster of P CTAs serves a unit, each CTA a P-th of K, each of its 8 warps every 8th 64-column chunk of that.
+// Sums meet in a fixed order: the 8 warps through shared memory, the P CTAs through distributed shared memory -- no
+// workspace, no counters.  P is the part count of least cost (see plan_rows).
+//
+// X.  A unit's columns of X are read by one warp each, so nothing is gained by keeping them in shared memory for one
+// unit: a lane loads the 32 bytes of its 16 columns of a token straight into the B operand, while the weights that the
+// warp asked for before the dependency wait are on their way.  That takes the round trip through shared memory and its
+// barrier out of a chain that is all latency, and 40 KB of shared memory in place of 100-220 let two CTAs share an SM,
+// so the next launch's weights are in flight while this one ends.  32 tokens by 6144 x 1024 6.9 -> 4.9 us, 1024 x 3072
+// 5.7 -> 4.6, 4096 x 4096 13.2 -> 9.8, 1152 x 6912 15.6 -> 7.0; 19 tokens by 4096 x 1024 5.6 -> 4.0.
+// Only 8 tokens by a matrix of many units keep X staged, in CTAs that stay (STAGED): 12288 x 4096 15.4 us against 17.4,
+// 24576 x 4096 27.7 / 29.7, 151936 x 4096 128 / 143.  (At 16 tokens 18.5 / 19.1, 33.8 / 33.9, 152 / 163: two tiles of
+// tokens are not worth a second form, and from 24 tokens on it is the slower one, 26 / 20.)
 #include "tm_cuda_internal.cuh"
 #include "tm_cuda_device.cuh"
 
@@ -34,6 +43,7 @@ struct rows_args {
     uint32_t part_end[3];  // exclusive row bound of each (multiples of 32 but the last)
     __half *act;           // gated forms: act(gate) * up, [batch][rows / 2]
     uint32_t rows, cols, batch, units, accumulate, mode, ring;
+    uint32_t x32;          // X is 32-byte aligned: one load takes a lane's 16 columns
 };
 
 using tmdev::cluster_rank;
@@ -53,8 +63,13 @@ __device__ __forceinline__ void dequant4(uint32_t w, __half2 d2, uint32_t &lo, u
     hi = *(const uint32_t *)&b;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(kThreads) q8_gemm_rows_kernel(const rows_args a) {
+// Shared memory of a CTA that stages no activations: its ring, then its sums.
+__host__ __device__ constexpr uint32_t ring_or_sums(uint32_t tok, uint32_t ring) {
+    return kWarps * (ring * kSlot > tok * kRowPad * 4u ? ring * kSlot : tok * kRowPad * 4u);
+}
+
+template <int NT, bool STAGED>
+__global__ void __launch_bounds__(kThreads, STAGED ? 1 : 2) q8_gemm_rows_kernel(const rows_args a) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr uint32_t kTok = NT * 8;
     const uint32_t P = cluster_size(), rank = P > 1 ? cluster_rank() : 0u;
@@ -65,9 +80,11 @@ __global__ void __launch_bounds__(kThreads) q8_gemm_rows_kernel(const rows_args 
     const uint32_t kc_max = (n_chunks + P - 1) / P;
     const uint32_t xstride = kc_max * 128u + 16u;  // 16 mod 128: the 16-byte reads of 8 lanes hit distinct banks
     unsigned char *xs = smem;
-    float *red = (float *)(smem + kTok * xstride);      // [warp][token][kRowPad]
-    float *part = red + kWarps * kTok * kRowPad;        // [2][token][32]
-    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(part + (P > 1 ? 2 * kTok * 32 : 0)) + warp * a.ring * kSlot;
+    // [warp][token][kRowPad]; not STAGED, a CTA has one unit and the sums take the ring's place once it has been read
+    float *red = (float *)(smem + (STAGED ? kTok * xstride : 0u));
+    float *part = STAGED ? red + kWarps * kTok * kRowPad : (float *)(smem + ring_or_sums(kTok, a.ring));  // [2][token][32]
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(STAGED ? (unsigned char *)(part + (P > 1 ? 2 * kTok * 32 : 0)) : smem) +
+                          warp * a.ring * kSlot;
     const uint32_t half_rows = a.rows / 2u;
 
     // Row r (0..31) of a unit: consecutive rows, or 16 gate rows and the 16 up rows they gate.
@@ -100,7 +117,28 @@ __global__ void __launch_bounds__(kThreads) q8_gemm_rows_kernel(const rows_args 
 
     tmdev::pdl_trigger();
     tmdev::pdl_wait();
-    {   // this CTA's columns of X; rows past the batch are zero
+    uint32_t xb[STAGED ? 1 : NT][8];  // this lane's 16 columns of the chunk at hand, of token 8 n + g
+    auto load_x = [&](int n, uint32_t c) {
+        uint32_t(&v)[8] = xb[STAGED ? 0 : n];
+        const uint32_t tok = (uint32_t)n * 8u + g;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = 0u;
+        if (c >= c1 || tok >= a.batch) return;
+        const __half *p = a.x + (size_t)tok * a.cols + c * 64u + t4 * 16u;
+        if (a.x32) {
+            asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                         : "l"(p)
+                         : "memory");
+        } else {
+            const uint4 lo = __ldcg((const uint4 *)p), hi = __ldcg((const uint4 *)p + 1);
+            v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
+        }
+    };
+    if (!STAGED) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n) load_x(n, c0 + warp);
+    } else {  // this CTA's columns of X; rows past the batch are zero
         const uint32_t q16 = (c1 - c0) * 8u, total = kTok * q16;  // 16-byte pieces
         constexpr uint32_t kBatch = 8;
         for (uint32_t b = threadIdx.x; b < total; b += kThreads * kBatch) {
@@ -117,8 +155,8 @@ __global__ void __launch_bounds__(kThreads) q8_gemm_rows_kernel(const rows_args 
                 if (at < total) *(int4 *)(xs + t * xstride + c * 16u) = v[i];
             }
         }
+        __syncthreads();
     }
-    __syncthreads();
 
     uint32_t slot = 0, it = 0;
     for (uint32_t unit = cluster; unit < a.units; unit += n_clusters, ++it) {
@@ -163,16 +201,23 @@ __global__ void __launch_bounds__(kThreads) q8_gemm_rows_kernel(const rows_args 
                     }
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
-                    const uint4 b = *(const uint4 *)(xp + n * 8u * xstride + h * 16u);
+                    const uint32_t(&v)[8] = xb[STAGED ? 0 : n];
+                    const uint4 b = STAGED ? *(const uint4 *)(xp + n * 8u * xstride + h * 16u)
+                                           : make_uint4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
 #pragma unroll
                     for (int m = 0; m < 2; ++m) {
                         mma_f16(acc[m][n], af[0][m][0], af[0][m][1], af[0][m][2], af[0][m][3], b.x, b.y);
                         mma_f16(acc[m][n], af[1][m][0], af[1][m][1], af[1][m][2], af[1][m][3], b.z, b.w);
                     }
+                    if (!STAGED && h == 1) load_x(n, c + kWarps);
                 }
             }
         }
         // ---- the 8 warps' sums, then the CTAs' ----
+        if (!STAGED) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+        }
 #pragma unroll
         for (int m = 0; m < 2; ++m)
 #pragma unroll
@@ -234,38 +279,60 @@ __global__ void __launch_bounds__(kThreads) q8_gemm_rows_kernel(const rows_args 
     if (P > 1) cluster_sync();  // nobody leaves while its sums are being read
 }
 
-size_t rows_smem(uint32_t cols, uint32_t nt, uint32_t p, uint32_t ring) {
+size_t rows_smem(uint32_t cols, uint32_t nt, uint32_t p, uint32_t ring, bool staged) {
     const uint32_t tok = nt * 8u, kc = (cols / 64u + p - 1u) / p;
+    if (!staged) return ring_or_sums(tok, ring) + (p > 1 ? 2u * tok * 32u * 4u : 0u);
     return (size_t)tok * (kc * 128u + 16u) + (size_t)kWarps * tok * kRowPad * 4u + (p > 1 ? 2u * tok * 32u * 4u : 0u) +
            (size_t)kWarps * ring * kSlot;
 }
 
 struct rows_plan {
     uint32_t p = 0, ring = 0;
+    bool staged = false;
 };
 
-// K parts and ring depth.  A CTA's time in cycles, fitted to measurements at 8 and 32 tokens (151936 x 1024:
-// 2.7k and 4.6k cycles per unit of two chunks a warp): its rounds of units, each the chunks one warp streams plus
-// the ordered sum, and once its share of X.  P is the part count with the least of that whose share of X leaves
-// room for a ring; the ring is as deep as a warp's stream is long, at most 6.
+// K parts.  Not staged: a CTA's time in hundredths of a microsecond, fitted to measurements at 8, 19 and 32 tokens and
+// P = 1..8: per chunk of a warp 0.35 us of latency and, times the CTAs that share an SM, 0.35 + 0.1 per 8 tokens for the
+// weights, the products and X from L2; 0.5 us for the CTAs' sums.  The parts of a unit have to be resident together, and
+// clusters of three and more find a place each only well below two CTAs an SM (1152 x 6912 by 32 tokens: 6 parts, 216
+// CTAs, 6.7 us; 8 parts, 288 CTAs, 10.4), so P stops there; units alone may take turns.  The ring is as deep as a warp's
+// stream is long, at most 6.
+// Staged: a CTA's time in cycles, its rounds of units, each the chunks one warp streams plus the ordered sum, and once
+// its share of X; P is the part count with the least of that whose share of X leaves room for a ring.
 rows_plan plan_rows(const tm_cuda_ctx *ctx, uint32_t units, uint32_t cols, uint32_t nt) {
     const uint32_t chunks = cols / 64u, sms = (uint32_t)ctx->sm_count;
     rows_plan best;
     uint32_t cost = 0;
+    // Staged: units for several rounds of every SM and a stream that is longer than X is wide (13824 x 1152, 432 units of
+    // 18 chunks: 7.3 us staged, 7.2 not; 12288 x 4096, 384 of 64: 15.4, 17.4; 4096 x 12288, 128 of 192: 17.5, 15.3).
+    if (nt == 1u && units > 2u * sms && units * chunks >= 24000u) {
+        best.staged = true;
+        for (uint32_t p = 1; p <= 8u && p <= chunks; ++p) {
+            const uint32_t kc = (chunks + p - 1u) / p, rounds = (units * p + sms - 1u) / sms;
+            const uint32_t per_warp = (kc + kWarps - 1u) / kWarps;
+            const uint32_t c = rounds * (per_warp * 700u + 1100u + (p > 1u ? 300u : 0u)) + kc * 20u;
+            if (best.p && c >= cost) continue;
+            uint32_t ring = 0;
+            for (uint32_t r : {6u, 4u, 3u, 2u})
+                if ((r <= rounds * per_warp || r == 2u) && rows_smem(cols, nt, p, r, true) <= ctx->smem_optin) {
+                    ring = r;
+                    break;
+                }
+            if (!ring) continue;
+            best.p = p;
+            best.ring = ring;
+            cost = c;
+        }
+        if (best.p) return best;
+        best = rows_plan();
+    }
     for (uint32_t p = 1; p <= 8u && p <= chunks; ++p) {
-        const uint32_t kc = (chunks + p - 1u) / p, rounds = (units * p + sms - 1u) / sms;
-        const uint32_t per_warp = (kc + kWarps - 1u) / kWarps;
-        const uint32_t c = rounds * (per_warp * (500u + 200u * nt) + 900u + 200u * nt + (p > 1u ? 300u : 0u)) + kc * 20u * nt;
+        const uint32_t ctas = units * p, per_warp = ((chunks + p - 1u) / p + kWarps - 1u) / kWarps;
+        if (p > 1u && ctas > (p == 2u ? 2u * sms : sms + sms / 2u)) break;
+        const uint32_t c = (uint32_t)((uint64_t)per_warp * (35ull * sms + (35ull + 10ull * nt) * ctas) / sms) + (p > 1u ? 50u : 0u);
         if (best.p && c >= cost) continue;
-        uint32_t ring = 0;
-        for (uint32_t r : {6u, 4u, 3u, 2u})
-            if ((r <= rounds * per_warp || r == 2u) && rows_smem(cols, nt, p, r) <= ctx->smem_optin) {
-                ring = r;
-                break;
-            }
-        if (!ring) continue;
         best.p = p;
-        best.ring = ring;
+        best.ring = per_warp >= 6u ? 6u : per_warp >= 4u ? 4u : per_warp == 3u ? 3u : 2u;
         cost = c;
     }
     return best;
@@ -276,15 +343,15 @@ bool rows_ok(uint32_t rows, uint32_t cols, uint32_t batch, bool gated) {
            cols <= 16384u && (!gated || rows % 32u == 0u);
 }
 
-template <int NT>
-cudaError_t launch_rows(tm_cuda_ctx *ctx, const rows_args &args, const rows_plan &pl) {
+template <int NT, bool STAGED>
+cudaError_t launch_rows_as(tm_cuda_ctx *ctx, const rows_args &args, const rows_plan &pl) {
     rows_args a = args;
     a.ring = pl.ring;
-    const size_t smem = rows_smem(a.cols, NT, pl.p, pl.ring);
+    const size_t smem = rows_smem(a.cols, NT, pl.p, pl.ring, STAGED);
     static std::atomic<bool> attr_set[64] = {};  // per device; contexts of a process share it
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(q8_gemm_rows_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const cudaError_t e = cudaFuncSetAttribute(q8_gemm_rows_kernel<NT, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)ctx->smem_optin);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
@@ -292,8 +359,15 @@ cudaError_t launch_rows(tm_cuda_ctx *ctx, const rows_args &args, const rows_plan
     // Resident clusters: by shared memory (1 KB per CTA is the system's) and registers at most two CTAs per SM.
     const uint32_t per_sm = 2u * (smem + 1024u) <= 228u * 1024u ? 2u : 1u;
     uint32_t clusters = (uint32_t)ctx->sm_count * per_sm / pl.p;
-    if (clusters > a.units) clusters = a.units;
-    return tm_launch_cluster_pdl(ctx, pl.p, q8_gemm_rows_kernel<NT>, dim3(clusters * pl.p), dim3(kThreads), smem, a);
+    if (!STAGED || clusters > a.units) clusters = a.units;
+    return tm_launch_cluster_pdl(ctx, pl.p, q8_gemm_rows_kernel<NT, STAGED>, dim3(clusters * pl.p), dim3(kThreads), smem, a);
+}
+
+template <int NT>
+cudaError_t launch_rows(tm_cuda_ctx *ctx, const rows_args &a, const rows_plan &pl) {
+    if constexpr (NT == 1)
+        if (pl.staged) return launch_rows_as<NT, true>(ctx, a, pl);
+    return launch_rows_as<NT, false>(ctx, a, pl);
 }
 
 }  // namespace
@@ -302,13 +376,15 @@ extern "C" {
 
 // Where the multiply for a few rows beats the tcgen05 GEMM: the more tokens, the sooner its MMAs and token fragments cost
 // more than the other kernel's hand-overs.  Measured, us against us, both with the f16 copy of X, at either side of the
-// lines: 8 tokens 24576 x 4096 30.6 / 33.9, 151936 x 1024 48.4 / 45.8; 16 tokens 6144 x 4096 15.9 / 16.1, 12288 x 4096
-// 21.6 / 21.6, 4096 x 12288 33.5 / 21.5; 24 tokens 4096 x 4096 13.5 / 14.0, 6144 x 4096 17.1 / 16.3; 32 tokens 6144 x 1024
-// 8.5 / 9.9, 13824 x 1152 13.6 / 11.6.  (On the wrong side of them: 151936 x 4096 at 8 tokens, 140 / 152; 13824 x 1152 and
-// 1152 x 6912 at 24, 11.8 / 11.6 and 15.1 / 13.8.)
+// lines: 8 tokens 24576 x 4096 27.7 / 32.3, 151936 x 4096 128 / 150, 262144 x 1152 86 / 79; 16 tokens 12288 x 4096 19.1 /
+// 19.6, 4096 x 12288 17.6 / 19.4, 24576 x 4096 33.9 / 32.2; 24 tokens 6144 x 4096 12.3 / 13.6, 12288 x 4096 20.3 / 19.9; 32
+// tokens 4096 x 4096 9.8 / 10.6, 1152 x 6912 7.0 / 10.1, 6144 x 4096 14.0 / 13.5, 13824 x 1152 10.3 / 8.6 (its units are more
+// than find a place at once).  (On the wrong side of them: 13824 x 1152 at 24, 9.0 / 8.6.)
 int tm_cuda_q8_0_gemm_rows_pays(uint32_t rows, uint32_t cols, uint32_t batch, int gated) {
     if (!rows_ok(rows, cols, batch, gated != 0)) return 0;
-    const uint64_t weights = (uint64_t)rows * cols, limit[4] = {128u << 20, 32u << 20, 17u << 20, 7u << 20};
+    const uint64_t weights = (uint64_t)rows * cols, limit[4] = {128u << 20, 64u << 20, 32u << 20, 17u << 20};
+    if (batch <= 8u && cols >= 4096u) return 1;
+    if (batch > 24u && rows > 8192u) return 0;
     return weights <= limit[(batch - 1u) / 8u];
 }
 
@@ -373,6 +449,7 @@ int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *
         else if (prologue != TM_CUDA_PRO_NONE) TM_CHECK_BUF(pro, (size_t)batch * cols * 4, "gate operand");
         a.x = (const __half *)ctx->mma_scratch;
     }
+    a.x32 = ((size_t)a.x & 31u) == 0;
     TM_OP_BEGIN("q8_0_gemm_rows");
     if (prologue != TM_CUDA_PRO_F16)
         TM_CUDA_TRY(tm_x_prep_launch(ctx, prologue, (const float *)x->dev, pro ? (const float *)pro->dev : nullptr, cols,
