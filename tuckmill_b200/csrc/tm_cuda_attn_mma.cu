@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
     constexpr int DV = C::kDV, SP = C::kSP, BQ = C::kBQ, KR = C::kRound;
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *sQ = smem, *sKV = smem + C::kQBytes;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = (int)tmdev::warp_index(), lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const int rw = warp % RW, sp = warp / RW;
     // Tiles of queries from the last one down (the last of a chunk sees the most keys), heads next to one another.
@@ -187,19 +187,27 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
     // Q: f32 -> f16 into the swizzled tile (rows past the run are zero).
     if (a.q_norm) {
         constexpr int R = HD / 32;
-#pragma unroll 2
+        const uint32_t rows = min((uint32_t)BQ, n - q0);
+        float nx[R];  // the next row, on its way
+        auto fetch = [&](uint32_t r) {
+            const float *src = a.q + ((size_t)(row0 + q0 + min(r, rows - 1u)) * a.heads + head) * HD;
+#pragma unroll
+            for (int i = 0; i < R; ++i) nx[i] = src[lane + 32 * i];
+        };
+        fetch(warp);
+#pragma unroll 1
         for (uint32_t r = warp; r < BQ; r += 8) {
             float x[R];
-            const bool in = q0 + r < n;
-            const float *src = a.q + ((size_t)(row0 + (in ? q0 + r : q0)) * a.heads + head) * HD;
-            const float sign = in ? a.q_sign : 0.0f;
 #pragma unroll
-            for (int i = 0; i < R; ++i) x[i] = src[lane + 32 * i];
-            norm_rope_row<R>(x, a.q_norm, a.inv_freq, a.n_rot, pos0 + q0 + r, a.eps, lane);
+            for (int i = 0; i < R; ++i) x[i] = nx[i];
+            if (r < rows) {
+                fetch(r + 8u);
+                norm_rope_row<R>(x, a.q_norm, a.inv_freq, a.n_rot, pos0 + q0 + r, a.eps, lane);
+            }
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 const uint32_t e = lane + 32u * i;
-                *(__half *)(sQ + sw<C::kQPitch>(r, e >> 3) + (e & 7u) * 2u) = __float2half_rn(x[i] * sign);
+                *(__half *)(sQ + sw<C::kQPitch>(r, e >> 3) + (e & 7u) * 2u) = r < rows ? __float2half_rn(x[i] * a.q_sign) : __half(0);
             }
         }
     } else {
@@ -295,7 +303,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
                 const float m_new = fmaxf(m_run[mt][h], mx * a.scale_log2e);
                 const float m_use = m_new == -INFINITY ? 0.0f : m_new;  // nothing visible yet: every weight is 0
                 alpha[mt][h] = exp2f(m_run[mt][h] - m_use);             // m_run = -inf gives 0
-                moved = moved || m_new != m_run[mt][h];
+                moved = moved || (m_new != m_run[mt][h] && m_run[mt][h] != -INFINITY);  // (nothing to rescale before the first keys)
                 m_run[mt][h] = m_new;
                 float rs = 0.0f;
 #pragma unroll
@@ -365,6 +373,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
             for (int p = 0; p < SP; ++p) l += sL[p * BQ + row] * exp2f(sM[p * BQ + row] - mx);
             inv[mt][h] = exp2f(m_run[mt][h] - mx) / l;
         }
+#pragma unroll 1
     for (int p = 0; p < SP; ++p) {
         if (sp == p) {
 #pragma unroll
