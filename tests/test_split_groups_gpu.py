@@ -30,3 +30,27 @@ def test_groups_of_a_split_sum(ctx, oracle, rows, cols, batch):
     acc = ctx.floats(base)
     ctx.q8_0_gemm_mma_fused(w, xb, rows, cols, batch, [acc], [rows], cuda.PRO_NONE, None, 0.0, cuda.EPI_ADD)
     np.testing.assert_array_equal(acc.download(0, batch * rows * 4, np.float32).reshape(batch, rows), base + runs[0])
+
+
+# Parts that meet in a cluster: 2, 3, 4, 6 and 8 of them, shares of the tokens that are uneven or empty, a last four of
+# tokens that is not whole, rows that end inside a tile, more clusters than have a place (through the workspace)
+@pytest.mark.parametrize("rows,cols,batch", [(6144, 1024, 61), (1500, 2304, 3), (1536, 1152, 130), (4000, 1024, 29),
+                                             (1152, 6912, 35), (1024, 3072, 9), (1024, 2048, 33), (1024, 3072, 200),
+                                             (3000, 4096, 128), (1024, 2048, 512)])
+def test_parts_that_meet_in_a_cluster(ctx, rows, cols, batch):
+    raw = T.q8_0_matrix(6, rows + cols, rows, cols)
+    x = T.activations(6, 2, batch * cols).reshape(batch, cols)
+    w, xb = ctx.q8_0_matrix(raw, rows, cols), ctx.floats(x)
+    base = T.activations(6, 4, batch * rows).reshape(batch, rows)
+    got = []
+    for _ in range(2):
+        y = ctx.floats(np.full((batch, rows), np.nan, np.float32))
+        ctx.q8_0_gemm_mma(w, xb, y, rows, cols, batch)
+        got.append(y.download(0, batch * rows * 4, np.float32).reshape(batch, rows))
+    assert ctx.mma_last_split() > 1 and not ctx.mma_aborted()
+    ref = x.astype(np.float16).astype(np.float64) @ T.q8_0_dequant(raw).astype(np.float16).astype(np.float64).T
+    assert rel_err(got[0], ref) <= 2e-5
+    np.testing.assert_array_equal(got[0], got[1])
+    acc = ctx.floats(base)
+    ctx.q8_0_gemm_mma_fused(w, xb, rows, cols, batch, [acc], [rows], cuda.PRO_NONE, None, 0.0, cuda.EPI_ADD)
+    np.testing.assert_array_equal(acc.download(0, batch * rows * 4, np.float32).reshape(batch, rows), base + got[0])

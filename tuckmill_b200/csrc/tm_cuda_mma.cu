@@ -43,12 +43,14 @@ namespace {
 constexpr int kBM = 128;        // weight rows per tile (UMMA M)
 constexpr int kBK = 64;         // K per stage: 64 f16 = one 128-byte swizzle row
 constexpr int kEpiWarps = 4;
+constexpr uint32_t kQuadBytes = kBM * 16;  // four tokens of a tile's rows, f32
 constexpr uint32_t kSpinLimit = 1u << 20;  // a healthy wait is microseconds; this is ~seconds
 // Split-K: when it shortens the longest CTA's run (few output tiles on many SMs: a decode batch, a narrow
 // projection, a last round that leaves most SMs idle) the K range of every tile is cut into `ksplit`
 // equal parts, each its own tile of the persistent grid;
-// the parts' accumulators meet in a workspace slot per (tile, part) and the warp that arrives last for a
-// (tile, row quarter) adds them IN PART ORDER and runs the epilogue -- no waiting, and a sum that does not
+// the parts' accumulators meet in the shared memory of a cluster, where one holds all parts of a tile and every CTA
+// has one; otherwise in a workspace slot per (tile, part), where the warp that arrives last for a
+// (tile, row quarter) adds them IN PART ORDER and runs the epilogue -- no waiting.  Either way a sum does not
 // depend on which part finished last.
 // The workspace holds 148 slots of the widest split tile (128 rows x 256 tokens); narrower tiles pack
 // more (output tile, part) slots into the same bytes.  Arrival counters: 4 row quarters per output tile.
@@ -78,6 +80,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
             : "r"(addr), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((spin & 1023u) == 1023u && *abort_flag) return false;
+    }
+    *abort_flag = 1u;
+    return false;
+}
+
+// The same for a barrier that other CTAs of the cluster arrive at (its first phase).
+__device__ __forceinline__ bool cluster_bar_wait(uint32_t addr, volatile uint32_t *abort_flag) {
+#pragma unroll 1
+    for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+        uint32_t done;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.b32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(addr)
             : "memory");
         if (done) return true;
         if ((spin & 1023u) == 1023u && *abort_flag) return false;
@@ -267,14 +286,15 @@ struct mma_smem {
     static constexpr uint32_t kRawOff = kBOff + kStages * kBBytes;
     static constexpr uint32_t kBarOff = kRawOff + kRawStages * kRawBytes;
     static constexpr uint32_t kBars = 2 * kRawStages + 2 * kStages + kAccs * (kIssuers + 1);
-    static constexpr uint32_t kBytes = 1024 + kBarOff + kBars * 8 + 16;
+    static constexpr uint32_t kBytes = 1024 + kBarOff + kBars * 8 + 32;
     static constexpr uint32_t kACol0 = kAccs * kIssuers * BN;  // tensor-memory column of A stage 0, after the accumulators
     static constexpr uint32_t kTmemCols = 512;
     static_assert(kStages % SETS == 0 && kStages <= kATmemStages, "each converter set needs its own A stages");
     static_assert(kBytes <= 232448, "shared memory per CTA");
 };
 
-template <int BN, int ISS, int SETS, bool WIDE>
+// CLUSTER: split K with the parts of an output tile in one cluster, one tile a CTA (see the epilogue).
+template <int BN, int ISS, int SETS, bool WIDE, bool CLUSTER>
 __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
     q8_gemm_mma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
                        const mma_args a) {
@@ -286,6 +306,7 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
     constexpr bool kTurns = L::kTurns;
     constexpr uint32_t kAccs = L::kAccs;
     constexpr uint32_t kTB = L::kSubs * BN;  // tokens per tile
+    static_assert(!CLUSTER || (kTB / 4u + 7u) * kQuadBytes <= L::kRawOff, "the sums of a split tile take the token stages' place");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte aligned stage buffers (swizzle atoms), then the barriers.
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -295,6 +316,8 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
     uint64_t *acc_full = empty + kStages, *acc_empty = acc_full + kAccs * kIssuers;
     uint32_t *tmem_slot = (uint32_t *)(acc_empty + kAccs);
     volatile uint32_t *abort_s = tmem_slot + 1;
+    // CLUSTER: every part has multiplied; this CTA's share of every part has arrived
+    const uint32_t bar_ready = smem_u32(tmem_slot + 2), bar_sums = bar_ready + 8u;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // A tile of the grid is (output tile, K part): tile / ksplit and tile % ksplit; nkb K steps each.
@@ -303,6 +326,10 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
     const uint32_t row_tiles = (a.rows + kBM - 1) / kBM, tok_tiles = (a.batch + kTB - 1) / kTB;
     const uint32_t n_tiles = row_tiles * tok_tiles * ksplit;
     // Consecutive tiles share a token tile, so CTAs running side by side read the same X.
+    // CLUSTER: the tile's tokens in fours, and those this part adds up and stores.
+    const uint32_t quads = CLUSTER ? (min(kTB, a.batch - blockIdx.x / ksplit / row_tiles * kTB) + 3u) / 4u : 0u;
+    const uint32_t share = CLUSTER ? (quads + ksplit - 1u) / ksplit : 0u;
+    const uint32_t quad0 = CLUSTER ? min(blockIdx.x % ksplit * share, quads) : 0u, quad1 = min(quad0 + share, quads);
 
     if (tid == 0) {
         for (int s = 0; s < kRawStages; ++s) {
@@ -316,6 +343,10 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
         for (uint32_t s = 0; s < kAccs * kIssuers; ++s) mbar_init(&acc_full[s], 1);  // tcgen05.commit after a tile's last MMA
         for (uint32_t s = 0; s < kAccs; ++s) mbar_init(&acc_empty[s], kEpiWarps);                                    // one arrival per epilogue warp
         *abort_s = 0u;
+        if (CLUSTER) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_ready), "r"(ksplit) : "memory");
+            tmdev::mbar_init(bar_sums, ksplit * (quad1 - quad0) * kQuadBytes);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kWarpMma) {
@@ -328,6 +359,7 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    if (CLUSTER) tmdev::cluster_arrive();  // (waited for before the first word to another CTA, or at the end)
 
     // Programmatic dependent launch: the weight pipeline (TMA of the raw tiles, converters) reads
     // nothing a predecessor writes and starts at once, overlapping the predecessor's tail -- the f16
@@ -445,6 +477,94 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full[sa]);
+            }
+        }
+    } else if (CLUSTER && warp < kWarpRaw) {
+        // ---------------- epilogue of a split tile whose parts are a cluster ----------------
+        // Every part sends its accumulators to the CTAs that add them, each an equal share of the tokens, where they
+        // arrive at a counted barrier in the token stages' place; then the share is added in part order and stored.
+        // Through the workspace (below) a part waits for its stores to be visible, counts itself in at every 32 tokens
+        // and the last one reads everything back: 512 tokens by 1024 x 3072 in four parts spent 6.9 us after the last
+        // MMA on that, 32 tokens by 4096 x 1024 5.7 us of 7.9.
+        const uint32_t quarter = (uint32_t)warp & 3u, part = blockIdx.x % ksplit, ot = blockIdx.x / ksplit;
+        const uint32_t tile_row0 = (ot % row_tiles) * kBM, tile_tok0 = (ot / row_tiles) * kTB;
+        const uint32_t row = quarter * 32u + (uint32_t)lane, rr = tile_row0 + row;
+        const bool p0 = tile_row0 < a.part_end[0], p1 = tile_row0 < a.part_end[1];
+        const uint32_t part_row0 = p0 ? 0u : p1 ? a.part_end[0] : a.part_end[1];
+        const size_t stride = (p0 ? a.part_end[0] : p1 ? a.part_end[1] : a.part_end[2]) - part_row0;
+        float *ybase = (p0 ? a.y[0] : p1 ? a.y[1] : a.y[2]) + (rr - part_row0) + (size_t)tile_tok0 * stride;
+        bool ok = true;
+        tmdev::pdl_wait();
+        tmdev::pdl_trigger();
+        tmdev::cluster_wait();
+#pragma unroll 1
+        for (uint32_t i = 0; i < (uint32_t)kIssuers; ++i)
+            if (ok) ok = mbar_wait(&acc_full[i], 0u, abort_s);
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (quarter == 0u && (uint32_t)lane < ksplit)
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tmdev::map_rank(bar_ready, (uint32_t)lane)) : "memory");
+            ok = cluster_bar_wait(bar_ready, abort_s);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            const uint32_t sums = smem_u32(sB) + part * share * kQuadBytes + row * 16u;
+            uint32_t owner = 0, left = share, at = 0;  // of the next four tokens: their CTA, what is left of its share, the place in it
+#pragma unroll 1
+            for (uint32_t t = 0; t < quads * 4u; t += 16u) {
+                uint32_t u[16];
+                float v[16];
+                const uint32_t acc = tmem_base + ((quarter * 32u) << 16) + t;  // (sub-tiles lie one after the other)
+                tmem_ld(acc, u);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(u[j]);
+                if (kTurns)  // the other issuers' accumulators, in order: each has a K step in every part (see the launcher)
+#pragma unroll 1
+                    for (uint32_t i = 1; i < (uint32_t)kIssuers; ++i) {
+                        tmem_ld(acc + i * BN, u);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(u[j]);
+                    }
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    if (t + (uint32_t)j >= quads * 4u) break;
+                    tmdev::send(sums + at, bar_sums, owner, make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+                    at += kQuadBytes;
+                    if (--left == 0u) {
+                        ++owner;
+                        left = share;
+                        at = 0;
+                    }
+                }
+            }
+        }
+#pragma unroll 1
+        for (uint32_t q = quad0; q < quad1 && ok; q += 4u) {
+            const float4 *src = (const float4 *)(sB + (size_t)(q - quad0) * kQuadBytes) + row;
+            float *p = ybase + (size_t)q * 4u * stride;
+            const uint32_t n = rr < a.rows ? min(min(quad1 - q, 4u) * 4u, a.batch - tile_tok0 - q * 4u) : 0u;  // tokens
+            float old[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) old[j] = a.accumulate && (uint32_t)j < n ? __ldcg(p + (size_t)j * stride) : 0.0f;
+            if (q == quad0) ok = cluster_bar_wait(bar_sums, abort_s);
+            if (!ok) break;
+            float4 v[4];  // (past the share: what lies there, not stored)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = src[j * kBM];
+#pragma unroll 1
+            for (uint32_t pp = 1; pp < ksplit; ++pp) {
+                src += share * kBM;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 f = src[j * kBM];
+                    v[j].x += f.x, v[j].y += f.y, v[j].z += f.z, v[j].w += f.w;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const float o = j % 4 == 0 ? v[j / 4].x : j % 4 == 1 ? v[j / 4].y : j % 4 == 2 ? v[j / 4].z : v[j / 4].w;
+                if ((uint32_t)j < n) p[(size_t)j * stride] = a.accumulate ? old[j] + o : o;
             }
         }
     } else if (warp < kWarpRaw) {
@@ -579,7 +699,7 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
           }
             if (!ok) break;
         }
-        if (a.push_world) __threadfence_system();  // this thread's peer stores, before the CTA counts itself in
+        if (!CLUSTER && a.push_world) __threadfence_system();  // this thread's peer stores, before the CTA counts itself in
     } else if (warp == kWarpRaw) {
         // ---------------- TMA producer of the raw weight tile ----------------
         if (lane == 0) {
@@ -670,10 +790,15 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
         }
     }
     // ---------------- teardown: everyone meets, tensor memory goes back ----------------
+    __syncwarp();
+    if (CLUSTER) {  // nobody leaves while another CTA may still send to it
+        if (warp < kConvWarps || warp >= kWarpRaw) tmdev::cluster_wait();
+        tmdev::cluster_sync();
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (tid == 0 && *abort_s) *(volatile uint32_t *)a.abort_flag = 1u;
-    if (a.push_world) {
+    if (!CLUSTER && a.push_world) {
         __shared__ uint32_t s_flag[2];
         tm_symm_finish(a.peer, a.push_tail, a.push_world, a.push_rank, s_flag);
     }
@@ -787,17 +912,33 @@ encode_tiled_fn get_encode_tiled() {
     return fn;
 }
 
-template <int BN, int ISS, int SETS, bool WIDE>
-cudaError_t launch_mma(tm_cuda_ctx *ctx, const CUtensorMap &wmap, const CUtensorMap &xmap, const mma_args &a, int grid) {
+// CTAs of a launch whose split tiles meet in clusters of `parts`: as many as find a place at once, also while the launch
+// before is on its way out.  us through the workspace and in clusters: two parts 6144 x 1024 at 128 tokens (96 CTAs) 12.8 /
+// 11.0, 4096 x 12288 at 200 (128) 47.7 / 45.5; four 4096 x 4096 at 128 (128) 18.7 / 13.8, 1024 x 3072 at 512 (128) 14.4 /
+// 13.9; six 1152 x 6912 at 64 (54) 11.6 / 8.4, at 200 (108) 16.2 / 14.9; eight 1024 x 3072 at 128 (64) 12.3 / 9.7, but at
+// 200 (128) 12.6 / 16.2: not all clusters of eight that the SMs add up to have a place.
+uint32_t cluster_ctas(uint32_t sms, uint32_t parts) { return parts == 2u ? sms - 4u : parts <= 4u ? sms - sms / 8u : sms - sms / 4u; }
+
+template <int BN, int ISS, int SETS, bool WIDE, bool CLUSTER>
+cudaError_t launch_mma_as(tm_cuda_ctx *ctx, const CUtensorMap &wmap, const CUtensorMap &xmap, const mma_args &a, int grid) {
+    using L = mma_smem<BN, ISS, SETS, WIDE>;
     const int device = ctx->device;
     static std::atomic<bool> attr_done[64] = {};  // per device; contexts of a process share it
     if (device < 0 || device >= 64 || !attr_done[device].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(q8_gemm_mma_kernel<BN, ISS, SETS, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)mma_smem<BN, ISS, SETS, WIDE>::kBytes);
+        const cudaError_t e = cudaFuncSetAttribute(q8_gemm_mma_kernel<BN, ISS, SETS, WIDE, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)L::kBytes);
         if (e != cudaSuccess) return e;
         if (device >= 0 && device < 64) attr_done[device].store(true, std::memory_order_release);
     }
-    return tm_launch_pdl(ctx, q8_gemm_mma_kernel<BN, ISS, SETS, WIDE>, dim3(grid), dim3(mma_smem<BN, ISS, SETS, WIDE>::kThreads), mma_smem<BN, ISS, SETS, WIDE>::kBytes, wmap, xmap, a);
+    return tm_launch_cluster_pdl(ctx, CLUSTER ? a.ksplit : 0u, q8_gemm_mma_kernel<BN, ISS, SETS, WIDE, CLUSTER>, dim3(grid),
+                                 dim3(L::kThreads), (size_t)L::kBytes, wmap, xmap, a);
+}
+
+template <int BN, int ISS, int SETS, bool WIDE>
+cudaError_t launch_mma(tm_cuda_ctx *ctx, const CUtensorMap &wmap, const CUtensorMap &xmap, const mma_args &a, int grid, bool cluster) {
+    if constexpr (WIDE)
+        if (cluster) return launch_mma_as<BN, ISS, SETS, WIDE, true>(ctx, wmap, xmap, a, grid);
+    return launch_mma_as<BN, ISS, SETS, WIDE, false>(ctx, wmap, xmap, a, grid);
 }
 
 }  // namespace
@@ -928,9 +1069,11 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     a.accumulate = accumulate ? 1u : 0u;
     // Split K: the K range of every output tile is cut into `ksplit` equal parts when that shortens the
     // longest CTA's run -- rounds of the persistent grid x (K steps of a part + the fixed cost of a tile,
-    // about 4 steps, + 2 for the ordered reduction) -- and the parts' accumulators fit the workspace
-    // (never for the pushing form).
+    // about 4 steps, + 2 for the ordered reduction through the workspace) -- and the parts' accumulators fit the
+    // workspace (never for the pushing form).  Where all parts find a place at once and a cluster holds a tile's, they
+    // meet there instead.
     a.ksplit = 1;
+    bool cluster = false;
     const uint32_t tile_tokens = batch < 2u * (uint32_t)bn ? (batch + 31u) / 32u * 32u : 2u * (uint32_t)bn;
     a.kslot = 128u * tile_tokens;
     {
@@ -943,10 +1086,12 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
             for (uint32_t cand : {2u, 3u, 4u, 6u, 8u}) {
                 if (nkb % cand != 0 || nkb / cand < 4) continue;
                 if ((uint64_t)out_tiles * cand * a.kslot > (uint64_t)kSplitSlots * kSplitSlotFloats) continue;
-                const uint64_t cost = (uint64_t)((out_tiles * cand + sms - 1) / sms) * (nkb / cand + 6);
+                const bool cl = (few || bn == 64) && out_tiles * cand <= cluster_ctas(sms, cand);
+                const uint64_t cost = (uint64_t)((out_tiles * cand + sms - 1) / sms) * (nkb / cand + (cl ? 4 : 6));
                 if (cost < best && cost * 10 < whole * 9) {  // a split has to pay for its reduction
                     best = cost;
                     a.ksplit = cand;
+                    cluster = cl;
                 }
             }
         }
@@ -968,12 +1113,12 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     ctx->mma_last_ksplit = (int)a.ksplit;
     const uint32_t n_tiles = row_tiles * ((batch + 2 * bn - 1) / (2 * bn)) * a.ksplit;
     const int grid = (int)(n_tiles < (uint32_t)ctx->sm_count ? n_tiles : (uint32_t)ctx->sm_count);
-    TM_CUDA_TRY(few == 32   ? (launch_mma<32, 4, 4, true>(ctx, wmap, xmap, a, grid))
-                : few == 64 ? (launch_mma<64, 2, 4, true>(ctx, wmap, xmap, a, grid))
-                : few == 128 ? (launch_mma<128, 2, 4, true>(ctx, wmap, xmap, a, grid))
-                : bn == 192 ? (launch_mma<192, 2, 2, false>(ctx, wmap, xmap, a, grid))
-                : bn == 128 ? (launch_mma<128, 2, 2, false>(ctx, wmap, xmap, a, grid))
-                            : (launch_mma<64, 2, 2, true>(ctx, wmap, xmap, a, grid)));
+    TM_CUDA_TRY(few == 32   ? (launch_mma<32, 4, 4, true>(ctx, wmap, xmap, a, grid, cluster))
+                : few == 64 ? (launch_mma<64, 2, 4, true>(ctx, wmap, xmap, a, grid, cluster))
+                : few == 128 ? (launch_mma<128, 2, 4, true>(ctx, wmap, xmap, a, grid, cluster))
+                : bn == 192 ? (launch_mma<192, 2, 2, false>(ctx, wmap, xmap, a, grid, cluster))
+                : bn == 128 ? (launch_mma<128, 2, 2, false>(ctx, wmap, xmap, a, grid, cluster))
+                            : (launch_mma<64, 2, 2, true>(ctx, wmap, xmap, a, grid, cluster)));
     return TM_CUDA_OK;
 }
 
