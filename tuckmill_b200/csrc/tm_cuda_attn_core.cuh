@@ -81,8 +81,7 @@ struct shared_state {
     __align__(16) float qs[G][HD];
     __align__(16) __half kh[HD];   // this step's own key and value
     __align__(16) __half vh[HD];
-    // Every warp's maximum and sum; after combine the factors that bring the warps to one maximum, and in l[g][0..1]
-    // the CTA's maximum and sum.
+    // Every warp's maximum, sum and output.
     float m[G][kT / 32], l[G][kT / 32];
     __align__(16) float opart[kT / 32][G][HD];
 };
@@ -276,32 +275,8 @@ struct keys {
             }
         }
     }
-    // After a barrier: the CTA's maximum and sum of every head, and the factors of its warps' values.  A CTA without
-    // keys has maximum -inf, sum 0 and values 0.  (Once per CTA: as a part of value() every thread took eight
-    // exponentials for each of its values: 2.2 us of a call with four heads of 256 dims, now 0.6.)
-    static __device__ __forceinline__ void combine(S &s) {
-        constexpr int W = kT / 32;
-        static_assert(W == 8, "a warp holds eight warps' states of four heads");
-        if (tmdev::warp_index() == 0u) {
-            const uint32_t g = threadIdx.x / W < G ? threadIdx.x / W : 0u, w = threadIdx.x % W;
-            const float m = s.m[g][w];
-            float M = m;
-#pragma unroll
-            for (int off = 1; off < W; off <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
-            const float f = M == -INFINITY ? 0.0f : expf(m - M);
-            float L = f * s.l[g][w];
-#pragma unroll
-            for (int off = 1; off < W; off <<= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
-            __syncwarp();
-            if (threadIdx.x < G * W) {
-                s.m[g][w] = f;
-                if (w < 2u) s.l[g][w] = w == 0u ? M : L;
-            }
-        }
-        __syncthreads();
-    }
-    // After the same barrier: dims d .. d + 3 of head g (not yet divided by the sum) by one thread, with the CTA's maximum
-    // and sum.  For a thread that finishes one quad: every factor once, and no barrier.
+    // After a barrier: dims d .. d + 3 of head g (not yet divided by the sum) by one thread, with the CTA's maximum and sum:
+    // every factor once, and no barrier.  A CTA without keys has maximum -inf, sum 0 and values 0.
     static __device__ __forceinline__ float2 combined(const S &s, uint32_t g, uint32_t d, float4 &o) {
         float m[kT / 32], M = -INFINITY, L = 0.0f;
         o = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -318,14 +293,6 @@ struct keys {
             o.w = fmaf(f, v.w, o.w);
         }
         return make_float2(M, L);
-    }
-    // After combine: value i (head i / HD, dim i % HD), not yet divided by the sum.
-    static __device__ __forceinline__ float value(const S &s, uint32_t i) {
-        const uint32_t g = i / HD, d = i % HD;
-        float o = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kT / 32; ++w) o = fmaf(s.m[g][w], s.opart[w][g][d], o);
-        return o;
     }
 };
 

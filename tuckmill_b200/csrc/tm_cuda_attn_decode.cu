@@ -5,7 +5,7 @@
 // What bounds it: a step's chain, not its bytes (a 0.6B decoder at position 700 reads 2.9 MB per layer).  A cluster
 // of up to 16 CTAs serves the G query heads of one KV head; each CTA takes a contiguous run of the visible keys, 64
 // at a time, and the CTAs' (max, sum, output) meet in distributed shared memory: every CTA pushes each peer the
-// slice of value dims that peer finishes, so one cluster barrier separates partial and final results.  The form this
+// slice of value dims that peer finishes, and goes on when its own slice has arrived at a counted barrier.  The form this
 // replaces met through a scratch buffer in HBM (store, fence, atomic, reload: three dependent memory trips) and
 // launched a CTA per 64 positions of CAPACITY, each reading its rows before it knew whether they exist: 16.8 MB a
 // layer at capacity 4096 and 8.9 us of the step at position 700, against 6.
@@ -32,13 +32,19 @@ struct attn_args {
 template <int G, int HD>
 __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster_kernel(const attn_args a) {
     constexpr int EPL = HD / 32;  // elements of a head vector per lane (strided by 32)
-    constexpr int PER = G * HD / kT > 0 ? G * HD / kT : 1;
+    constexpr uint32_t kQuads = G * HD / 4;
+    static_assert(kQuads <= (uint32_t)kT, "a thread finishes one quad");
     __shared__ __align__(16) shared_state<G, HD> sh;
-    __shared__ float recv[G * HD];                // [source CTA][this CTA's slice]
-    __shared__ float recv_ml[kMaxCluster][G][2];  // every CTA's max and sum
+    __shared__ __align__(16) float recv[G * HD];                // [source CTA][this CTA's slice]
+    __shared__ __align__(16) float recv_ml[kMaxCluster][G][2];  // every CTA's max and sum of the heads in the slice
+    __shared__ __align__(8) uint64_t arrived;
     const uint32_t C = cluster_size(), rank = cluster_rank();
     const uint32_t kvh = blockIdx.x / C, seq_i = blockIdx.z, cap = a.cap;
     const int tid = threadIdx.x, lane = tid & 31, warp = tmdev::warp_index();
+    // Quad i of the G HD values is finished by CTA i / E; C and E are powers of two.
+    const uint32_t logc = 31u - (uint32_t)__clz((int)C), E = (uint32_t)(G * HD) >> logc;
+    const uint32_t slice_heads = E > HD ? E / HD : 1u, bar = smem_addr(&arrived);
+    if (tid == 0) tmdev::mbar_init(bar, C * (E * 4u + slice_heads * 8u));
     cluster_arrive();  // before any peer's shared memory is written, every CTA must have started
     const float *q = a.q + seq_i * a.sq + (size_t)kvh * G * HD, *k = a.k + seq_i * a.sk + (size_t)kvh * HD;
     const float *v = a.v + seq_i * a.sv + (size_t)kvh * HD;
@@ -89,56 +95,42 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
     }
     __syncthreads();
     K.attend(sh, pos, a.scale);
-    __syncthreads();
     cluster_wait();  // every CTA of the cluster has started
-    // ---- value i (head i / HD, dim i % HD) is finished by CTA i / E: push it there, and everyone the max and sum ----
-    const uint32_t logc = 31u - (uint32_t)__clz((int)C), E = (uint32_t)(G * HD) >> logc;  // C, E: powers of two
-    keys<G, HD>::combine(sh);
-#pragma unroll
-    for (int r = 0; r < PER; ++r) {
-        const uint32_t i = tid + r * kT;
-        if (i < G * HD) st_cluster(smem_addr(&recv[rank * E + (i & (E - 1u))]), (i << logc) / (G * HD), keys<G, HD>::value(sh, i));
+    __syncthreads();
+    // ---- a quad of this CTA's values to the CTA that finishes it, the maximum and sum once a slice and head ----
+    if ((uint32_t)warp * 32u < kQuads) {
+        const uint32_t i = (uint32_t)tid * 4u, in = i & (E - 1u), to = i / E;
+        float4 o;
+        const float2 ml = keys<G, HD>::combined(sh, i / HD, i % HD, o);
+        tmdev::send(smem_addr(&recv[rank * E + in]), bar, to, o);
+        if ((in & (HD - 1u)) == 0u) tmdev::send(smem_addr(&recv_ml[rank][in / HD][0]), bar, to, ml);
     }
-    for (uint32_t i = tid; i < C * G * 2u; i += kT) {
-        const uint32_t g = (i >> 1) % G;
-        st_cluster(smem_addr(&recv_ml[rank][g][i & 1u]), i / (2u * G), sh.l[g][i & 1u]);
+    tmdev::mbar_wait(bar, a.status);
+    // ---- C lanes per quad: source s's share, added over the lanes ----
+    if ((uint32_t)warp * 32u >= kQuads) return;
+    const uint32_t src = tid & (C - 1u), in = ((uint32_t)tid >> logc) * 4u;
+    const float M = recv_ml[src][in / HD][0];
+    float L = recv_ml[src][in / HD][1];
+    float4 O = *(const float4 *)&recv[src * E + in];
+    float top = M;
+#pragma unroll 1
+    for (uint32_t off = C >> 1; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+    const float f = expf(M - top);  // a CTA without keys: exp(-inf) = 0
+    L *= f, O.x *= f, O.y *= f, O.z *= f, O.w *= f;
+#pragma unroll 1
+    for (uint32_t off = C >> 1; off > 0; off >>= 1) {
+        L += __shfl_xor_sync(0xffffffffu, L, off);
+        O.x += __shfl_xor_sync(0xffffffffu, O.x, off);
+        O.y += __shfl_xor_sync(0xffffffffu, O.y, off);
+        O.z += __shfl_xor_sync(0xffffffffu, O.z, off);
+        O.w += __shfl_xor_sync(0xffffffffu, O.w, off);
     }
-    cluster_arrive();
-    cluster_wait();
-    // ---- C lanes per value: source s's share, added over the lanes ----
-    const uint32_t src = tid & (C - 1u);
-    float O[PER], L[PER], M[PER];
+    if (src == 0) {
+        float *out = a.out + seq_i * a.so + (size_t)kvh * G * HD + rank * E + in;
+        const float d[4] = {O.x / L, O.y / L, O.z / L, O.w / L};
 #pragma unroll
-    for (int r = 0; r < PER; ++r) {
-        const uint32_t e = (tid + r * kT) >> logc, g = min(rank * E + e, G * HD - 1u) / HD;
-        M[r] = recv_ml[src][g][0];
-        L[r] = recv_ml[src][g][1];
-        O[r] = e < E ? recv[src * E + e] : 0.0f;
+        for (int r = 0; r < 4; ++r) out[r] = d[r];
     }
-    float top[PER];
-#pragma unroll
-    for (int r = 0; r < PER; ++r) top[r] = M[r];
-    for (uint32_t off = C >> 1; off > 0; off >>= 1)
-#pragma unroll
-        for (int r = 0; r < PER; ++r) top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], off));
-#pragma unroll
-    for (int r = 0; r < PER; ++r) {
-        const float f = expf(M[r] - top[r]);  // a CTA without keys: exp(-inf) = 0
-        L[r] *= f;
-        O[r] *= f;
-    }
-    for (uint32_t off = C >> 1; off > 0; off >>= 1)
-#pragma unroll
-        for (int r = 0; r < PER; ++r) {
-            L[r] += __shfl_xor_sync(0xffffffffu, L[r], off);
-            O[r] += __shfl_xor_sync(0xffffffffu, O[r], off);
-        }
-    if (src == 0)
-#pragma unroll
-        for (int r = 0; r < PER; ++r) {
-            const uint32_t e = (tid + r * kT) >> logc;
-            if (e < E) a.out[seq_i * a.so + (size_t)kvh * G * HD + rank * E + e] = O[r] / L[r];
-        }
 }
 
 // The widest cluster this device can hold of the kernel (16 needs the non-portable size).
