@@ -47,3 +47,13 @@ def test_burst_counts_as_one_dispatch(ctx):
     ctx._call("end_burst")
     assert ctx.committed_dispatches() == before + 1 and ctx.kernel_launches() == launches + 2
     np.testing.assert_array_equal(y.download(0, 1200, np.float32), x.download(0, 1200, np.float32) * 4)
+
+
+@pytest.mark.parametrize("n", [65532, 65536, 607744, 1048576, 1048580])  # either side of what passes through pinned memory
+def test_downloads_of_any_length(ctx, n):
+    a = np.random.default_rng(n).integers(0, 256, n + 64, dtype=np.uint8)
+    buf = ctx.from_array(a)
+    np.testing.assert_array_equal(buf.download(64, n, np.uint8), a[64:])
+    b = a[::-1].copy()
+    buf.upload(0, b)
+    np.testing.assert_array_equal(buf.download(0, n, np.uint8), b[:n])

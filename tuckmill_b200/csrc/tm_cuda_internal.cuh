@@ -99,6 +99,7 @@ struct tm_cuda_ctx {
     size_t mma_scratch_bytes = 0;
     // Set by a kernel whose bounded wait for a pipeline stage (tensor-core GEMM) or for a peer CTA's values (decode
     // layer blocks) ran out: host memory the device can write, so that the host looks at it without a copy.
+    unsigned char *stage = nullptr;  // pinned memory that downloads of kStageMin to kStageBytes pass through
     volatile uint32_t *mma_abort = nullptr;
     int mma_last_bn = 0;                 // token sub-tile width of the last tensor-core GEMM launch
     int mma_last_sets = 0;               // its sets of converter warps
