@@ -790,8 +790,8 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
         }
     }
     // ---------------- teardown: everyone meets, tensor memory goes back ----------------
-    __syncwarp();
     if (CLUSTER) {  // nobody leaves while another CTA may still send to it
+        __syncwarp();
         if (warp < kConvWarps || warp >= kWarpRaw) tmdev::cluster_wait();
         tmdev::cluster_sync();
     }
