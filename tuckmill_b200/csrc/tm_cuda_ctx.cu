@@ -399,8 +399,12 @@ int tm_cuda_download(tm_cuda_ctx *ctx, tm_cuda_buffer *src, size_t off, void *ds
     // A row of logits into pageable memory: through pinned memory of the context's, 26 us and 12 for the host's own copy
     // against the driver's 64 (151936 floats behind nothing), with the copy in stream order behind the step.
     cudaPointerAttributes at;
-    const bool staged = ctx->stage && len >= kStageMin && len <= kStageBytes &&
-                        cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+    bool staged = ctx->stage && len >= kStageMin && len <= kStageBytes;
+    if (staged && cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+        cudaGetLastError();
+        staged = false;
+    }
+    staged = staged && at.type == cudaMemoryTypeUnregistered;
     TM_CUDA_TRY(cudaMemcpyAsync(staged ? ctx->stage : dst, src->dev + off, len, cudaMemcpyDefault, ctx->stream));
     TM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     if (staged) memcpy(dst, ctx->stage, len);

@@ -377,8 +377,8 @@ extern "C" {
 // Where the multiply for a few rows beats the tcgen05 GEMM: the more tokens, the sooner its MMAs and token fragments cost
 // more than the other kernel's hand-overs.  Measured, us against us, both with the f16 copy of X, at either side of the
 // lines: 8 tokens 24576 x 4096 27.7 / 32.3, 151936 x 4096 128 / 150, 262144 x 1152 86 / 79; 16 tokens 12288 x 4096 19.1 /
-// 19.6, 4096 x 12288 17.6 / 19.4, 24576 x 4096 33.9 / 32.2; 24 tokens 6144 x 4096 12.3 / 13.6, 12288 x 4096 20.3 / 19.9; 32
-// tokens 4096 x 4096 9.8 / 10.6, 1152 x 6912 7.0 / 10.1, 6144 x 4096 14.0 / 13.5, 13824 x 1152 10.3 / 8.6 (its units are more
+// 19.6, 4096 x 12288 17.6 / 18.8, 24576 x 4096 33.9 / 32.2; 24 tokens 6144 x 4096 12.3 / 12.7, 12288 x 4096 20.3 / 19.9; 32
+// tokens 4096 x 4096 9.9 / 10.2, 1152 x 6912 7.0 / 7.9, 6144 x 4096 14.0 / 12.7, 13824 x 1152 10.3 / 8.6 (its units are more
 // than find a place at once).  (On the wrong side of them: 13824 x 1152 at 24, 9.0 / 8.6.)
 int tm_cuda_q8_0_gemm_rows_pays(uint32_t rows, uint32_t cols, uint32_t batch, int gated) {
     if (!rows_ok(rows, cols, batch, gated != 0)) return 0;
