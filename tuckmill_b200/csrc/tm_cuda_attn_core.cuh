@@ -239,7 +239,8 @@ struct keys {
             for (int v = 0; v < VP; ++v) {
                 const uint32_t row = lane / TV + v * RV, jv = t0 + vr + v * RV;
                 int4 raw = vraw[v];
-                if (min(jv, last) == pos) raw = *(const int4 *)(s.vh + vd);
+                if (jv == pos) raw = *(const int4 *)(s.vh + vd);
+                if (jv > last) raw = make_int4(0, 0, 0, 0);  // weight 0 there, and 0 times an infinity is NaN
                 const __half2 *h2 = (const __half2 *)&raw;
                 float f[8];
 #pragma unroll
