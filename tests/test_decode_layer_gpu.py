@@ -39,9 +39,9 @@ def test_cluster_attention_equals_the_exact_form(ctx, oracle, heads, kvh, hd, wi
     assert int(status.download(0, 4, np.uint32)[0]) == 0
 
 
-# A value that binary16 holds as an infinity stays one: rows past a CTA's run, whose weight is 0, add no NaN.
+# A value that binary16 holds as an infinity stays one: rows past a CTA's run or before the window, whose weight is 0, add no NaN.
 @pytest.mark.parametrize("pos", [0, 7, 8, 63, 100, 1099])
-@pytest.mark.parametrize("heads,kvh,hd,window", [(16, 8, 128, 0), (4, 1, 256, 40)])
+@pytest.mark.parametrize("heads,kvh,hd,window", [(16, 8, 128, 0), (4, 1, 256, 40), (4, 2, 128, 40)])
 def test_attention_of_infinite_values(ctx, oracle, heads, kvh, hd, window, pos):
     cap, eps, scale = 1200, 1e-6, 1.0 / np.sqrt(np.float32(hd))
     one, inv, pb = ctx.floats(np.ones(hd)), ctx.floats(oracle.rope_inv_freq(hd, 1e6)), ctx.from_array(np.array([pos], np.uint32))
@@ -49,6 +49,7 @@ def test_attention_of_infinite_values(ctx, oracle, heads, kvh, hd, window, pos):
     q, k, v = (T.activations(7, t, n * hd).reshape(n, hd) for t, n in ((30, heads), (31, kvh), (32, kvh)))
     fill[1][:, :, 3], v[:, 3] = np.inf, 1e6  # every row
     v[:, 5] = -1e6                           # this step's
+    fill[1][:, :max(0, pos + 1 - window) if window else 0, 7] = np.inf  # not seen
     status = ctx.buffer(4, shared=True)
     status.zero()
     scratch = ctx.buffer(cuda.decode_attention_scratch_bytes(heads, kvh, hd, cap))
@@ -59,10 +60,19 @@ def test_attention_of_infinite_values(ctx, oracle, heads, kvh, hd, window, pos):
         ctx.attention_decode_dev(ctx.floats(q), ctx.floats(k), ctx.floats(v), one, one, inv, kc, vc, out, scratch, pb, 0, status,
                                  heads, kvh, hd, hd, cap, window, eps, scale, exact)
         outs.append(out.download(0, heads * hd * 4, np.float32).reshape(heads, hd))
+    # a batch of two such sequences, on the tensor cores for head size 128
+    kc, vc, out = ctx.from_array(np.stack([fill[0]] * 2)), ctx.from_array(np.stack([fill[1]] * 2)), ctx.buffer(2 * heads * hd * 4)
+    sb = ctx.buffer(2 * cuda.decode_attention_scratch_bytes(heads, kvh, hd, cap))
+    sb.zero()
+    ctx.attention_decode_batch(*(ctx.floats(np.stack([r] * 2)) for r in (q, k, v)), one, one, inv, kc, vc, out, sb,
+                               ctx.from_array(np.array([pos] * 2, np.uint32)), status, 2, heads, kvh, hd, hd, cap, window, eps, scale, False)
+    batch = out.download(0, 2 * heads * hd * 4, np.float32).reshape(2, heads, hd)
     finite = np.delete(np.arange(hd), [3, 5])
-    for o in outs:
+    for o in (*outs, *batch):
         assert np.all(o[:, 3] == np.inf) and np.all(o[:, 5] == -np.inf)
     assert rel_err(outs[1][:, finite], outs[0][:, finite]) <= 2e-5  # (as for finite rows, above)
+    for b in batch:
+        assert rel_err(b[:, finite], outs[0][:, finite]) <= 2e-3  # binary16 queries and weights
 
 
 # A row whose sum of squares overflows is normed with 1 / infinity: zeros, in every form.

@@ -44,6 +44,9 @@ using tmdev::mma_f16;
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void *src, bool read) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(read ? 16u : 0u) : "memory");
+}
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *(const uint32_t *)&h;
@@ -624,9 +627,10 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
         constexpr int CH = HD / 8;  // 16-byte chunks per row
         for (int i = tid; i < kBKV * CH; i += kThreads) {
             const uint32_t r = i / CH, c = i % CH;
-            const uint32_t j = min(j0 + r, pos);  // rows past the position repeat its row (masked below)
+            // Keys past the position repeat its row (masked below); values that weigh 0 are zeros: 0 times an infinity is NaN.
+            const uint32_t j = min(j0 + r, pos);
             cp_async16(smem_u32(sK) + sw<PITCH>(r, c), kc + (size_t)j * HD + c * 8);
-            cp_async16(smem_u32(sV) + sw<PITCH>(r, c), vc + (size_t)j * HD + c * 8);
+            cp_async16_or_zero(smem_u32(sV) + sw<PITCH>(r, c), vc + (size_t)j * HD + c * 8, j0 + r - start <= pos - start);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
