@@ -146,6 +146,7 @@ mod ffi {
         pub fn tm_cuda_program_status(ctx: *mut TmCudaCtx, program: *mut TmCudaGraph, status: *mut u32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_program_trace(ctx: *mut TmCudaCtx, program: *mut TmCudaGraph, out: *mut u64, max_ops: u32, kinds: *mut u32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_program_debug(ctx: *mut TmCudaCtx, program: *mut TmCudaGraph, sequence_skew: u32, spin_limit: u32, err: *mut c_char, err_cap: usize) -> c_int;
+        pub fn tm_cuda_wait_debug(ctx: *mut TmCudaCtx, starve: u32, limit: u32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_fence(ctx: *mut TmCudaCtx, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_committed_dispatches(ctx: *const TmCudaCtx) -> u64;
         pub fn tm_cuda_completed_dispatches(ctx: *const TmCudaCtx) -> u64;

@@ -359,6 +359,12 @@ int tm_cuda_program_trace(tm_cuda_ctx *ctx, tm_cuda_graph *program, uint64_t *ou
 int tm_cuda_program_debug(tm_cuda_ctx *ctx, tm_cuda_graph *program, uint32_t sequence_skew, uint32_t spin_limit,
                           char *err, size_t err_cap);
 
+/* No counterpart, for tests of the waits between the CTAs of a cluster (decode attention, decode layer blocks, split
+ * tiles of the tensor-core GEMM): in kernels launched or recorded from now on a CTA polls at most `limit` times for its
+ * peers' values (0 = normal, about a second), and barrier number `starve` of the kernel, counted from 1 in the order of its
+ * waits (at most 3), expects more than is sent (0 = none): the wait runs out, the kernel says so in its status word and returns. */
+int tm_cuda_wait_debug(tm_cuda_ctx *ctx, uint32_t starve, uint32_t limit, char *err, size_t err_cap);
+
 /* tm_metal.h:291 tm_metal_fence. */
 int tm_cuda_fence(tm_cuda_ctx *ctx, char *err, size_t err_cap);
 /* tm_metal.h:294,301 committed / completed dispatch counters. */
@@ -501,7 +507,9 @@ int tm_cuda_attention_prefill(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffe
  * tm_cuda_qwen35_attention_f16_chunk(n = 1): bit for bit with `exact` = 1;
  * with `exact` = 0 a latency-optimised kernel with the same mathematics and a
  * different summation order (tolerance-qualified) runs where it applies.  A
- * position >= cap writes nothing and sets bit 0 of status[0] (u32, shared).
+ * position >= cap writes nothing and sets bit 0 of status[0] (u32, shared); bit 1 is
+ * set where CTAs that share a KV head did not deliver their parts within a bounded wait
+ * (the call's output is then undefined).
  * `scratch` holds the per-key-block partial results and arrival counters
  * (tm_cuda_attention_decode_scratch_bytes, zero-filled once by the caller;
  * the kernel leaves the counters at zero).  Calls sharing one scratch buffer
@@ -515,6 +523,8 @@ int tm_cuda_attention_prefill(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffe
  * group included).  Rows that something OTHER than this operator wrote (a
  * prefill chunk, a host upload) must be complete when the call is made, which
  * every earlier dispatch group, graph launch or upload is. */
+#define TM_CUDA_STATUS_PAST_CAPACITY 1u
+#define TM_CUDA_STATUS_LATE 2u
 size_t tm_cuda_attention_decode_scratch_bytes(uint32_t heads, uint32_t kv_heads, uint32_t head_dim,
                                               uint32_t cap);
 int tm_cuda_attention_decode_dev(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffer *k,
@@ -594,7 +604,7 @@ int tm_cuda_decode_ffn_block(tm_cuda_ctx *ctx, tm_cuda_buffer *x, tm_cuda_buffer
  * [n_seq][heads * head_dim], scratch n_seq regions of
  * tm_cuda_attention_decode_scratch_bytes (zero-filled once).  Results per sequence are those of the
  * single call, bit for bit (same kernels, one more grid dimension); a sequence whose position is
- * >= cap writes nothing and sets bit 0 of status[0]. */
+ * >= cap writes nothing and sets bit 0 of status[0] (bit 1 as in the single call). */
 int tm_cuda_attention_decode_batch_dev(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_cuda_buffer *k, tm_cuda_buffer *v,
                                        tm_cuda_buffer *q_norm, tm_cuda_buffer *k_norm, tm_cuda_buffer *inv_freq,
                                        tm_cuda_buffer *k_cache, tm_cuda_buffer *v_cache, tm_cuda_buffer *out,

@@ -27,6 +27,7 @@ struct attn_args {
     uint32_t cap, window;
     float eps, scale;
     size_t sq, sk, sv, so, scache;  // elements between consecutive sequences
+    tm_peer_waits waits;
 };
 
 template <int G, int HD>
@@ -44,7 +45,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
     // Quad i of the G HD values is finished by CTA i / E; C and E are powers of two.
     const uint32_t logc = 31u - (uint32_t)__clz((int)C), E = (uint32_t)(G * HD) >> logc;
     const uint32_t slice_heads = E > HD ? E / HD : 1u, bar = smem_addr(&arrived);
-    if (tid == 0) tmdev::mbar_init(bar, C * (E * 4u + slice_heads * 8u));
+    if (tid == 0) tmdev::mbar_init(bar, C * (E * 4u + slice_heads * 8u) + a.waits.more(1u));
     cluster_arrive();  // before any peer's shared memory is written, every CTA must have started
     const float *q = a.q + seq_i * a.sq + (size_t)kvh * G * HD, *k = a.k + seq_i * a.sk + (size_t)kvh * HD;
     const float *v = a.v + seq_i * a.sv + (size_t)kvh * HD;
@@ -71,7 +72,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
     }
     const uint32_t pos = tmdev::uniform(*pos_p);
     if (pos >= cap) {  // uniform over the cluster
-        if (tid == 0 && rank == 0) atomicOr(a.status, 1u);
+        if (tid == 0 && rank == 0) atomicOr(a.status, TM_CUDA_STATUS_PAST_CAPACITY);
         cluster_wait();
         return;
     }
@@ -105,7 +106,11 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
         tmdev::send(smem_addr(&recv[rank * E + in]), bar, to, o);
         if ((in & (HD - 1u)) == 0u) tmdev::send(smem_addr(&recv_ml[rank][in / HD][0]), bar, to, ml);
     }
-    tmdev::mbar_wait(bar, a.status);
+    if (!__all_sync(0xffffffffu, tmdev::mbar_wait(bar, a.waits.limit(), a.status, TM_CUDA_STATUS_LATE))) {
+        if (lane == 0) atomicOr(a.status, TM_CUDA_STATUS_LATE);
+        tmdev::linger(bar);
+        return;
+    }
     // ---- C lanes per quad: source s's share, added over the lanes ----
     if ((uint32_t)warp * 32u >= kQuads) return;
     const uint32_t src = tid & (C - 1u), in = ((uint32_t)tid >> logc) * 4u;
@@ -181,7 +186,7 @@ cudaError_t tm_attention_decode_fast_launch(tm_cuda_ctx *ctx, const float *q, co
                                             uint32_t kv_heads, uint32_t hd, uint32_t cap, uint32_t window, float eps,
                                             float scale, uint32_t n_seq, size_t sq, size_t skv, size_t so, size_t scache) {
     attn_args a = {q, k, v, qn, kn, inv_freq, (__half *)kc, (__half *)vc, out, pos, status, cap, window, eps, scale,
-                   sq, skv, skv, so, scache};
+                   sq, skv, skv, so, scache, ctx->waits};
     switch ((heads / kv_heads) * 1000 + hd) {
         case 1128: return launch<1, 128>(ctx, a, kv_heads, n_seq);
         case 2128: return launch<2, 128>(ctx, a, kv_heads, n_seq);

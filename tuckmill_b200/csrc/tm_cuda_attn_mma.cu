@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
     if (warp <= G) fetch(warp);  // (with the position's own trip)
     const uint32_t pos = a.pos[sidx];
     if (pos >= a.cap) {
-        if (tid == 0 && split == 0 && kvh == 0) atomicOr(a.status, 1u);
+        if (tid == 0 && split == 0 && kvh == 0) atomicOr(a.status, TM_CUDA_STATUS_PAST_CAPACITY);
         return;
     }
     if (pos != hint) {

@@ -630,6 +630,15 @@ void tm_cuda_graph_free(tm_cuda_ctx *ctx, tm_cuda_graph *graph) {
     delete graph;
 }
 
+int tm_cuda_wait_debug(tm_cuda_ctx *ctx, uint32_t starve, uint32_t limit, char *err, size_t err_cap) {
+    TM_ENTER();
+    if (starve > 3u || limit >> 30) return tm_fail(err, err_cap, TM_CUDA_ERR_BOUNDS, "barrier %u, %u polls", starve, limit);
+    ctx->waits = tm_peer_waits();
+    if (limit) ctx->waits.word = limit;
+    ctx->waits.word |= starve << 30;
+    return TM_CUDA_OK;
+}
+
 int tm_cuda_fence(tm_cuda_ctx *ctx, char *err, size_t err_cap) {
     TM_ENTER();
     if (ctx->group_open || ctx->burst_open)

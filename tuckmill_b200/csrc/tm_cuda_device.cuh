@@ -202,14 +202,34 @@ __device__ __forceinline__ void send(uint32_t addr, uint32_t bar, uint32_t rank,
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(map_rank(addr, rank)),
                  "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(map_rank(bar, rank)) : "memory");
 }
-// Waits for a barrier's one use, at most some tenths of a second; a wait that runs out sets `flag` and returns.
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t *flag) {
-    uint32_t done = 0;
+__device__ __forceinline__ bool arrived(uint32_t bar) {
+    uint32_t done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.b32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(bar) : "memory");
+    return done != 0u;
+}
+// Waits for a barrier's one use, at most `limit` polls (of 4.4 us each while nothing arrives); false when they run out, or
+// after 256 where `flag` has a bit of `mask`: a wait has failed already, and nothing that depends on it is worth the full time.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t limit, const volatile uint32_t *flag, uint32_t mask) {
 #pragma unroll 1
-    for (uint32_t i = 0; i < (1u << 20) && !done; ++i)
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.b32 %0, 1, 0, p;\n}\n"
-                     : "=r"(done) : "r"(bar) : "memory");
-    if (!done) *(volatile uint32_t *)flag = 1u;
+    for (uint32_t i = 0; i < limit; ++i) {
+        if (arrived(bar)) return true;
+        if ((i & 255u) == 255u && (*flag & mask) != 0u) return false;
+    }
+    return false;
+}
+// After the peers have sent all they will: what is on its way lands (as far as a millisecond shows; what was never sent does not).
+__device__ __forceinline__ void landed(uint32_t bar) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < 256u && !arrived(bar); ++i) {
+    }
+}
+// The end of a warp that has not received everything: its CTA's shared memory stays until the other warps of the cluster have met it here
+// or have ended (a cluster barrier counts the threads that have not), and until what they had sent has landed.
+__device__ __forceinline__ void linger(uint32_t bar) {
+    __syncwarp();
+    cluster_sync();
+    landed(bar);
 }
 
 }  // namespace tmdev

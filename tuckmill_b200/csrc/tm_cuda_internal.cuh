@@ -61,6 +61,14 @@ struct tm_profile_row {
     uint64_t nanos = 0, count = 0;
 };
 
+// How many times a CTA polls for its peers' values (30 bits).  The upper two bits are for tests: the kernel's barrier of that
+// number (from 1) expects more than is sent, so that the wait for it runs out.
+struct tm_peer_waits {
+    uint32_t word = 1u << 18;  // a second (a healthy wait is microseconds)
+    __device__ __forceinline__ uint32_t limit() const { return word & 0x3fffffffu; }
+    __device__ __forceinline__ uint32_t more(uint32_t bar) const { return word >> 30 == bar ? 4u : 0u; }
+};
+
 struct tm_cuda_ctx {
     int device = 0;
     int sm_count = 0;
@@ -97,10 +105,11 @@ struct tm_cuda_ctx {
     // Scratch owned by the context for the tensor-core GEMM (f16 copy of X).
     unsigned char *mma_scratch = nullptr;
     size_t mma_scratch_bytes = 0;
-    // Set by a kernel whose bounded wait for a pipeline stage (tensor-core GEMM) or for a peer CTA's values (decode
-    // layer blocks) ran out: host memory the device can write, so that the host looks at it without a copy.
     unsigned char *stage = nullptr;  // pinned memory that downloads of kStageMin to kStageBytes pass through
+    // Set by a kernel whose bounded wait for a pipeline stage (tensor-core GEMM) or for a peer CTA's values (its split
+    // tiles, decode layer blocks) ran out: host memory the device can write, so that the host looks at it without a copy.
     volatile uint32_t *mma_abort = nullptr;
+    tm_peer_waits waits;  // (tm_cuda_wait_debug)
     int mma_last_bn = 0;                 // token sub-tile width of the last tensor-core GEMM launch
     int mma_last_sets = 0;               // its sets of converter warps
     int mma_last_ksplit = 0;             // K parts per output tile of that launch

@@ -54,6 +54,7 @@ struct residual_in {
     uint32_t *late;       // set when an exchange inside a cluster did not arrive
     uint32_t n_slots, hidden;
     float eps;
+    tm_peer_waits waits;
 };
 
 using tmdev::mma_s8;
@@ -147,6 +148,20 @@ __device__ __forceinline__ void residual_norm(const residual_in &r, bool store, 
         v[i].z = v[i].z * inv * nw[i].z;
         v[i].w = v[i].w * inv * nw[i].w;
     }
+}
+
+// Waits for an exchange; false (and the word set) when it did not arrive.  The next barrier tells the whole CTA, which then
+// leaves by give_up().
+__device__ __forceinline__ bool await(const residual_in &r, uint32_t bar) {
+    const bool ok = tmdev::mbar_wait(bar, r.waits.limit(), r.late, ~0u);
+    if (!ok) *(volatile uint32_t *)r.late = 1u;
+    return ok;
+}
+// Leaves once no peer writes to this CTA any more (`bars` counted barriers from `bar` on) and its own copies have landed.
+__device__ __forceinline__ void give_up(uint32_t bar, uint32_t bars) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    tmdev::linger(bar);
+    if (bars > 1u) tmdev::landed(bar + 8u);
 }
 
 // One projection of a block as this CTA sees it: `tiles` 16-row tiles of `chunks` 64-column chunks, item i = tile
@@ -312,7 +327,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
     float *acts = (float *)(smem + L.acts), *part = (float *)(smem + L.part), *red = (float *)(smem + L.red);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tmdev::warp_index();
     const uint32_t bar = smem_addr(smem + L.bar);
-    if (tid == 0) tmdev::mbar_init(bar, nfc * 256u);  // all activations of the cluster
+    if (tid == 0) tmdev::mbar_init(bar, nfc * 256u + a.in.waits.more(1u));  // all activations of the cluster
     cluster_arrive();
     const matrix_part m1 = {a.gu_q, a.gu_d, H, 0u, n1, H / 64u}, m2 = {a.dn_q, a.dn_d, F, fc0, n2, nfc};
     const uint32_t ring = smem_addr(smem + L.ring) + warp * ring_slots * kSlotBytes;
@@ -328,6 +343,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
     for (uint32_t sec = 0; sec < 2u; ++sec) {
         const uint32_t quads = sec ? nfc * 16u : H / 4u, plane = plane_bytes(sec ? a.acts : H);
         float4 v[NB];
+        bool ok = true;
         if (sec == 0u) {
             residual_norm<NB>(a.in, cluster == 0u, rank, nw, v, red, [] {});
         } else {
@@ -344,7 +360,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
 #pragma unroll
                     for (uint32_t k = 0; k < kC / 4u; ++k) tmdev::send(smem_addr(acts + g0 * 8u + act), bar, (lane & 3u) * (kC / 4u) + k, z);
             }
-            tmdev::mbar_wait(bar, a.in.late);
+            ok = await(a.in, bar);
         }
 #pragma unroll 1
         for (uint32_t q0 = warp * 32u; q0 < quads; q0 += NB * kT)
@@ -356,7 +372,7 @@ __global__ void __launch_bounds__(kT, 2) ffn_block_kernel(const ffn_args a, uint
                 const float y[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
                 tmdev::digitise_quad(y, q < quads, (signed char *)smem + q * 4u, plane, (float *)(smem + 4u * plane) + (q >> 3) * 4u, lane);
             }
-        __syncthreads();
+        if (__syncthreads_or(!ok)) return give_up(bar, 1u);
         multiply(sec ? w2 : w1, sec ? m2.chunks : m1.chunks, sec, smem, plane, part);
         __syncthreads();
     }
@@ -412,8 +428,8 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
     float *part = (float *)(smem + L.part), *red = (float *)(smem + L.red);
     const uint32_t bar = smem_addr(smem + L.bar);
     if (tid == 0) {
-        tmdev::mbar_init(bar, (G + 2) * HD * 4u);               // this head's q, k and v
-        tmdev::mbar_init(bar + 8u, kC * (G * HD + 2 * G) * 4u);  // every CTA's (max, sum, output)
+        tmdev::mbar_init(bar, (G + 2) * HD * 4u + a.in.waits.more(1u));               // this head's q, k and v
+        tmdev::mbar_init(bar + 8u, kC * (G * HD + 2 * G) * 4u + a.in.waits.more(2u));  // every CTA's (max, sum, output)
     }
     cluster_arrive();
     const uint32_t kvw = a.kv_heads * HD;
@@ -451,7 +467,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
         hint = ~0u;
     }
     if (pos >= cap) {  // uniform over the cluster; the pieces' copies land before the CTA's memory goes away
-        if (tid == 0 && rank == 0) atomicOr(a.status, 1u);
+        if (tid == 0 && rank == 0) atomicOr(a.status, TM_CUDA_STATUS_PAST_CAPACITY);
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         cluster_wait();
@@ -461,6 +477,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
     for (uint32_t sec = 0; sec < 2u; ++sec) {
         const uint32_t quads = (sec ? G * HD : H) / 4u, plane = plane_bytes(sec ? G * HD : H);
         float4 v[NB];
+        bool ok = true;
         if (sec == 0u) {
             residual_norm<NB>(a.in, kvh == 0u, rank, nw, v, red, [&] { K.first_tile(pos, a.window, kC, rank); });
         } else {
@@ -473,7 +490,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
 #pragma unroll
                 for (uint32_t k = 0; k < kC / 4u; ++k) tmdev::send(smem_addr(qkv + u0 * 16u + i), bar, (lane & 3u) * (kC / 4u) + k, z);
             }
-            tmdev::mbar_wait(bar, a.in.late);
+            ok = await(a.in, bar);
             // ---- every CTA has the head's q, k and v ----
             if (warp < G || (warp == G && K.lo <= pos && pos < K.hi)) {
                 float x[EPL];
@@ -494,7 +511,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                     }
                 }
             }
-            __syncthreads();
+            if (__syncthreads_or(!ok)) return give_up(bar, 2u);
             K.attend(sh, pos, a.scale);
             __syncthreads();
             // ---- this CTA's (max, sum, output) to every CTA: each needs all of the head's output for its rows of o ----
@@ -509,7 +526,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                     if (quad % (HD / 4u) == 0u) tmdev::send(smem_addr(recv_ml + (rank * G + head) * 2u), bar + 8u, to + k, ml);
                 }
             }
-            tmdev::mbar_wait(bar + 8u, a.in.late);
+            ok = await(a.in, bar + 8u);
         }
         // Four lanes to a quad of the attention's output, each with a quarter of the source CTAs.
         const uint32_t shift = sec ? 2u : 0u;
@@ -554,7 +571,7 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
                 const float y[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
                 tmdev::digitise_quad(y, q < quads, (signed char *)smem + q * 4u, plane, (float *)(smem + 4u * plane) + (q >> 3) * 4u, lane, shift);
             }
-        __syncthreads();
+        if (__syncthreads_or(!ok)) return give_up(bar, 2u);
         multiply(sec ? w2 : w1, sec ? m2.chunks : m1.chunks, sec, smem, plane, part);
         __syncthreads();
     }
@@ -704,6 +721,7 @@ int check_residual(tm_cuda_ctx *ctx, residual_in &r, tm_cuda_buffer *x, tm_cuda_
         return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "residual operands are not 16-byte aligned");
     TM_CUDA_TRY(tm_ensure_abort_flag(ctx));
     r.late = (uint32_t *)ctx->mma_abort;
+    r.waits = ctx->waits;
     r.x = (const float *)x->dev;
     r.slots = n_slots ? (const float *)slots->dev : nullptr;
     r.add_w = n_slots && add_w ? (const float *)add_w->dev : nullptr;

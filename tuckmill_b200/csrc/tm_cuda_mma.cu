@@ -88,23 +88,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     return false;
 }
 
-// The same for a barrier that other CTAs of the cluster arrive at (its first phase).
-__device__ __forceinline__ bool cluster_bar_wait(uint32_t addr, volatile uint32_t *abort_flag) {
-#pragma unroll 1
-    for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.b32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(addr)
-            : "memory");
-        if (done) return true;
-        if ((spin & 1023u) == 1023u && *abort_flag) return false;
-    }
-    *abort_flag = 1u;
-    return false;
-}
-
 // Shared-memory matrix descriptor, K-major operand in the 128-byte swizzle:
 // rows are 128 bytes apart, groups of 8 rows 1024 bytes apart (SBO), 16-byte
 // chunk c of row r sits at chunk position c ^ (r & 7).
@@ -235,6 +218,7 @@ struct mma_args {
     float *const *peer;
     uint32_t push_world, push_rank, push_off, push_tail;
     uint32_t rows, cols, batch;
+    tm_peer_waits waits;   // 1: every part has multiplied; 2: this CTA's share of the sums
     uint32_t *abort_flag;  // host memory, set when a bounded wait gave up
 };
 
@@ -344,8 +328,8 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
         for (uint32_t s = 0; s < kAccs; ++s) mbar_init(&acc_empty[s], kEpiWarps);                                    // one arrival per epilogue warp
         *abort_s = 0u;
         if (CLUSTER) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_ready), "r"(ksplit) : "memory");
-            tmdev::mbar_init(bar_sums, ksplit * (quad1 - quad0) * kQuadBytes);
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_ready), "r"(ksplit + a.waits.more(1u)) : "memory");
+            tmdev::mbar_init(bar_sums, ksplit * (quad1 - quad0) * kQuadBytes + a.waits.more(2u));
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -505,7 +489,8 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (quarter == 0u && (uint32_t)lane < ksplit)
                 asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tmdev::map_rank(bar_ready, (uint32_t)lane)) : "memory");
-            ok = cluster_bar_wait(bar_ready, abort_s);
+            ok = tmdev::mbar_wait(bar_ready, a.waits.limit(), abort_s, ~0u);
+            if (!ok) *abort_s = 1u;
         }
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
@@ -547,8 +532,11 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
             float old[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) old[j] = a.accumulate && (uint32_t)j < n ? __ldcg(p + (size_t)j * stride) : 0.0f;
-            if (q == quad0) ok = cluster_bar_wait(bar_sums, abort_s);
-            if (!ok) break;
+            if (q == quad0) ok = tmdev::mbar_wait(bar_sums, a.waits.limit(), abort_s, ~0u);
+            if (!ok) {
+                *abort_s = 1u;
+                break;
+            }
             float4 v[4];  // (past the share: what lies there, not stored)
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[j] = src[j * kBM];
@@ -794,6 +782,7 @@ __global__ void __launch_bounds__((mma_smem<BN, ISS, SETS, WIDE>::kThreads), 1)
         __syncwarp();
         if (warp < kConvWarps || warp >= kWarpRaw) tmdev::cluster_wait();
         tmdev::cluster_sync();
+        if (tid == 0 && *abort_s) tmdev::landed(bar_sums);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -1108,6 +1097,7 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     a.cols = cols;
     a.batch = batch;
     a.abort_flag = abort_flag;
+    a.waits = ctx->waits;
     ctx->mma_last_bn = few ? few : bn;
     ctx->mma_last_sets = few ? 4 : 2;
     ctx->mma_last_ksplit = (int)a.ksplit;
@@ -1256,7 +1246,7 @@ int tm_cuda_mma_last_split(tm_cuda_ctx *ctx) {
     return ctx->mma_last_ksplit;
 }
 
-// 1 when a tensor-core GEMM on this context ever gave up a bounded wait.
+// 1 when a tensor-core GEMM or a decode layer block on this context ever gave up a bounded wait.
 int tm_cuda_mma_aborted(tm_cuda_ctx *ctx) {
     if (!ctx) return 0;
     std::lock_guard<std::mutex> lock(ctx->mu);

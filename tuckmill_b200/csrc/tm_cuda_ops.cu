@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) attention_decode_kernel(
     for (int r = 0; r < RP; ++r) fr[r] = lane + 32 * r < half_rot ? inv_freq[lane + 32 * r] : 0.0f;
     const uint32_t pos = *pos_p;
     if (pos >= cap) {
-        if (lane == 0 && blk == 0 && head == 0) atomicOr(status, 1u);
+        if (lane == 0 && blk == 0 && head == 0) atomicOr(status, TM_CUDA_STATUS_PAST_CAPACITY);
         return;
     }
     const uint32_t seq = pos + 1u, start = attn_start(seq, window);

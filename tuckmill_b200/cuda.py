@@ -23,6 +23,7 @@ GEMM_MAX_BATCH = 32
 GEMM_MMA_MAX_BATCH = 8192
 PRO_NONE, PRO_RMSNORM, PRO_SILU_MUL, PRO_GELU_MUL, PRO_F16 = 0, 1, 2, 3, 4
 EPI_STORE, EPI_ADD, EPI_SILU_MUL_F16, EPI_GELU_MUL_F16 = 0, 1, 2, 3
+STATUS_PAST_CAPACITY, STATUS_LATE = 1, 2
 
 
 class CudaError(RuntimeError):
@@ -92,6 +93,7 @@ _OPS = {
     "abort_program": [_P],
     "program_status": [_P, _P, C.POINTER(C.c_uint32)],
     "program_debug": [_P, _P, _U32, _U32],
+    "wait_debug": [_P, _U32, _U32],
     "fence": [_P],
     "u32_add": [_P, _P, _U32, _U32],
     "qwen35_rope_partial": [_P, _P, _P, _P, _U32, _U32, _U32, _U32, _U32],
@@ -416,6 +418,7 @@ class CudaContext:
         self._call("q8_0_gemm_mma", w.handle, x.handle, y.handle, rows, cols, batch, x_off, y_off)
 
     def mma_workspace_reserve(self, nbytes: int): self._call("mma_workspace_reserve", nbytes)
+    def wait_debug(self, starve: int = 0, limit: int = 0): self._call("wait_debug", starve, limit)
     def mma_aborted(self) -> bool: return bool(self._l.tm_cuda_mma_aborted(self.handle))
     def mma_last_tile(self) -> int: return int(self._l.tm_cuda_mma_last_tile(self.handle))
     def mma_last_sets(self) -> int: return int(self._l.tm_cuda_mma_last_sets(self.handle))
