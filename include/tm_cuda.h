@@ -193,8 +193,9 @@ int tm_cuda_q8_0_gemm_mma(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x
  * beforehand with the size tm_cuda_mma_workspace_bytes gives. */
 size_t tm_cuda_mma_workspace_bytes(uint32_t cols, uint32_t batch);
 int tm_cuda_mma_workspace_reserve(tm_cuda_ctx *ctx, size_t bytes, char *err, size_t err_cap);
-/* No counterpart: 1 when a tensor-core GEMM of this context gave up one of its
- * bounded pipeline waits (its output is then undefined); waits for the stream. */
+/* No counterpart: 1 when a kernel of this context gave up a bounded wait, a tensor-core GEMM (for a pipeline stage or the
+ * other parts of a split tile) or a decode layer block (for a CTA of its cluster): the output is then undefined.  The word
+ * stays set.  Waits for the stream. */
 int tm_cuda_mma_aborted(tm_cuda_ctx *ctx);
 /* No counterpart: which instantiation of the tensor-core kernel the context's last GEMM
  * launch used, as its token sub-tile width (32, 64, 128 or 192) and its sets of converter

@@ -1,12 +1,14 @@
 """Waits of a cluster's CTAs for one another's values: every one is bounded, says so in its own status word when it runs
 out, and leaves the context usable.  A barrier that expects more than is sent makes it run out."""
 import contextlib
+import ctypes as C
+import dataclasses
 import time
 
 import numpy as np
 import pytest
 
-from tuckmill_b200 import cuda, testing as T
+from tuckmill_b200 import cuda, engine as E, testing as T
 
 pytestmark = pytest.mark.gpu
 
@@ -116,3 +118,29 @@ def test_a_wait_that_runs_out_says_so_and_ends(ctx, oracle, op, starve):
         c.wait_debug()
         o.run(c)
         np.testing.assert_array_equal(o.result(), want)
+
+
+def starved_engine_message(path, prompt, **kw):
+    """What an engine says after a step whose waits ran out."""
+    eng = E.Engine(path, context=128, **kw)
+    eng.prefill(prompt, want_token=True)
+    err = C.create_string_buffer(256)
+    assert cuda.load_library().tm_cuda_wait_debug(C.c_void_p(eng.cuda_ctx()), 1, LIMIT, err, 256) == 0
+    eng.decode_ungrouped(1)
+    with pytest.raises(E.EngineError) as e:
+        eng.logits()
+    eng.close()
+    assert e.value.code == "INTERNAL"
+    return e.value.message
+
+
+def test_the_engine_names_the_wait(ctx, tmp_path):
+    prompt = T.token_ids(3, 9, 512)
+    # no layer has the blocks' shape: decode attention by itself
+    wide = dataclasses.replace(T.SMALL_QWEN3, hidden=2304)
+    assert not cuda.load_library().tm_cuda_decode_attn_block_supported(2304, wide.heads, wide.kv_heads, wide.head_dim, wide.head_dim)
+    T.write_gguf(tmp_path / "wide.gguf", wide)
+    message = starved_engine_message(tmp_path / "wide.gguf", prompt)
+    assert "decode attention" in message and "capacity" not in message
+    T.write_gguf(tmp_path / "small.gguf", T.SMALL_QWEN3)
+    assert "decode layer" in starved_engine_message(tmp_path / "small.gguf", prompt)

@@ -1313,11 +1313,14 @@ void EngineModel::step_ungrouped() {
 void EngineModel::check_device_status() {
     Impl &I = *impl_;
     ctx_->fence();
-    if (*(const volatile uint32_t *)I.status.contents() != 0)
+    const uint32_t status = *(const volatile uint32_t *)I.status.contents();
+    if (status & TM_CUDA_STATUS_PAST_CAPACITY)
         throw TuckmillError(ErrorCode::Internal, "a decode step ran past the KV capacity on the device");
+    if (status != 0)
+        throw TuckmillError(ErrorCode::Internal, "a bounded wait of decode attention ran out; the step's results are undefined");
     if (!opts_.exact && ctx_->mma_aborted())
         throw TuckmillError(ErrorCode::Internal,
-                            "a pipeline wait of the tensor-core GEMM ran out; the prefill results are undefined");
+                            "a bounded wait of the tensor-core GEMM or of a decode layer block ran out; the results are undefined");
     if (I.sh.world > 1 && ctx_->symm_status(I.arena.buf) != 0)
         throw TuckmillError(ErrorCode::Internal,
                             "a peer-memory exchange wait ran out; gathered activations of a step are stale");
