@@ -574,8 +574,10 @@ int tm_cuda_attention_decode_dev_static(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_
  *   attention block:    slots_out[h] = the columns of KV head h's query heads of  o * attention(rmsnorm(x_out) * norm_w),
  *                       with q / k norm, RoPE, the f16 KV store and attention at pos_buf[pos_index] folded in
  *                       (tm_cuda_attention_decode_dev); kv_heads slots;
- *   feed-forward block: slots_out[c] = the c-th eighth of  down * (act(gate x') * up x'), x' = rmsnorm(x_out) * norm_w;
- *                       gate_up holds width gate rows above width up rows; TM_CUDA_DECODE_SLOTS slots.
+ *   feed-forward block: the sum of the TM_CUDA_DECODE_SLOTS slots_out = down * (act(gate x') * up x'), x' = rmsnorm(x_out) *
+ *                       norm_w; gate_up holds width gate rows above width up rows.  The k = width / 64 chunks of columns are
+ *                       cut into n shares: slot c < n holds the product of chunks [c k / n, (c + 1) k / n), the slots from n on
+ *                       are zeros.  n is 6 where a warp of 6 x 16 CTAs can keep its weights in shared memory, else 8.
  * The slots are for the next block's slots_in (or tm_cuda_reduce_ranks_add_f32).  x_out and slots_out share no storage
  * with x, slots_in or the norm weights: such a call is refused.  `supported`: whether the shape has these forms and the
  * current device can hold their clusters. */

@@ -130,7 +130,7 @@ def f64_layer(x, slots, add_w, norm_w, eps):
 @pytest.mark.parametrize("hidden,width,n_slots,normed", [(1024, 3072, 8, False), (64, 512, 0, False), (320, 576, 1, True),
                                                          (1088, 1024, 3, True), (1024, 2112, 8, True)])
 @pytest.mark.parametrize("gelu", [False, True])
-def test_feed_forward_block(ctx, hidden, width, n_slots, normed, gelu):
+def test_feed_forward_block(ctx, hidden, width, n_slots, normed, gelu, clusters=0):
     eps = 1e-6
     raw_gu, raw_dn = T.q8_0_matrix(3, 1, 2 * width, hidden), T.q8_0_matrix(3, 2, hidden, width)
     x, nw = T.activations(3, 3, hidden), (1 + 0.1 * T.activations(3, 4, hidden)).astype(np.float32)
@@ -145,13 +145,19 @@ def test_feed_forward_block(ctx, hidden, width, n_slots, normed, gelu):
                          ctx.floats(nw), xo, ctx.q8_0_matrix(raw_gu, 2 * width, hidden), ctx.q8_0_matrix(raw_dn, hidden, width),
                          so, hidden, width, gelu, eps)
     assert rel_err(xo.download(0, hidden * 4, np.float32), want_x) <= 2e-6
-    assert rel_err(so.download(0, 8 * hidden * 4, np.float32).reshape(8, hidden).astype(np.float64).sum(axis=0), want) <= 2e-6
+    out = so.download(0, 8 * hidden * 4, np.float32).reshape(8, hidden).astype(np.float64)
+    assert rel_err(out.sum(axis=0), want) <= 2e-6
+    if clusters:  # every slot is its share of the width, the rest are zeros
+        cut = [64 * (width // 64 * c // clusters) for c in range(clusters + 1)]
+        shares = [T.q8_0_dequant(raw_dn).astype(np.float64)[:, a:b] @ act[a:b] for a, b in zip(cut, cut[1:])]
+        assert rel_err(out[:clusters], np.array(shares)) <= 2e-6
+        assert np.all(out[clusters:] == 0)
 
 
 # the narrowest width that takes eight clusters, the widest that takes six, clusters with one chunk of columns and with two
-@pytest.mark.parametrize("hidden,width,n_slots", [(1024, 4096, 8), (1024, 3136, 2), (1024, 3072, 0), (192, 704, 5)])
-def test_feed_forward_block_by_clusters(ctx, hidden, width, n_slots):
-    test_feed_forward_block(ctx, hidden, width, n_slots, False, False)
+@pytest.mark.parametrize("hidden,width,n_slots,clusters", [(1024, 4096, 8, 8), (1024, 3136, 2, 8), (1024, 3072, 0, 6), (192, 704, 5, 6)])
+def test_feed_forward_block_by_clusters(ctx, hidden, width, n_slots, clusters):
+    test_feed_forward_block(ctx, hidden, width, n_slots, False, False, clusters)
 
 
 @pytest.mark.parametrize("hidden,heads,kvh,hd,pos,window", [(1024, 16, 8, 128, 700, 0), (256, 4, 2, 128, 0, 0), (64, 3, 3, 128, 129, 50),

@@ -6,8 +6,8 @@
 // load, norm + digit split, products, cross-warp sum and completion.  Here the operators that only exchange a few
 // hundred values meet inside a cluster of 16 CTAs through distributed shared memory:
 //   * cluster h of the attention block owns KV head h: its q, k and v rows, its keys, and the columns of o that its
-//     heads feed; cluster c of the feed-forward block owns an eighth of the FFN width: its gate and up rows and its
-//     columns of down.  Both end in one full-width partial product per cluster, a "slot";
+//     heads feed; cluster c of the feed-forward block owns a sixth (or an eighth, see ffn_shape) of the FFN width: its gate
+//     and up rows and its columns of down.  Both end in one full-width partial product per cluster, a "slot";
 //   * the slots are added (in order) to the residual stream by whoever reads it next, as the first thing its CTAs do
 //     anyway; one cluster also stores the sum.  A layer's output norm is applied there too;
 //   * weights never wait for activations: every warp copies its own 16-row x 64-column pieces of both projections to
@@ -674,6 +674,7 @@ bool attn_shape(uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t hd)
 uint32_t ffn_items(const ffn_args &a) {
     return ceil_div(a.tiles1 * (a.in.hidden / 64u), kWarps) + ceil_div(a.tiles2 * (a.acts / 64u), kWarps);
 }
+// Six clusters find a place beside attention's eight (above); eight where a sixth's pieces do not stay in shared memory.
 ffn_args ffn_shape(uint32_t hidden, uint32_t width) {
     ffn_args a = {};
     a.in.hidden = hidden;
