@@ -573,7 +573,8 @@ int tm_cuda_attention_decode_dev_static(tm_cuda_ctx *ctx, tm_cuda_buffer *q, tm_
  * add_w, + rmsnorm(that sum) * add_w (a layer's output norm); x_out is a buffer other than x.  Then
  *   attention block:    slots_out[h] = the columns of KV head h's query heads of  o * attention(rmsnorm(x_out) * norm_w),
  *                       with q / k norm, RoPE, the f16 KV store and attention at pos_buf[pos_index] folded in
- *                       (tm_cuda_attention_decode_dev); kv_heads slots;
+ *                       (tm_cuda_attention_decode_dev); kv_heads slots.  At a position >= cap x_out is stored, nothing else,
+ *                       and bit 0 of status[0] set;
  *   feed-forward block: the sum of the TM_CUDA_DECODE_SLOTS slots_out = down * (act(gate x') * up x'), x' = rmsnorm(x_out) *
  *                       norm_w; gate_up holds width gate rows above width up rows.  The k = width / 64 chunks of columns are
  *                       cut into n shares: slot c < n holds the product of chunks [c k / n, (c + 1) k / n), the slots from n on

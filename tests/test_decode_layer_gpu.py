@@ -202,6 +202,32 @@ def test_attention_block_equals_the_operators_it_replaces(ctx, oracle, hidden, h
     assert int(status.download(0, 4, np.uint32)[0]) == 1
 
 
+# x_out does not hang on the position: it is stored where the rest of the block is not
+@pytest.mark.parametrize("hidden,heads,kvh,hd,n_slots,normed", [(256, 4, 2, 128, 2, True), (128, 4, 1, 256, 0, False),
+                                                                 (1088, 8, 8, 128, 8, False)])
+@pytest.mark.parametrize("past", [0, 1, 2**32 - 65])
+def test_attention_block_past_the_capacity_stores_the_sum_alone(ctx, oracle, hidden, heads, kvh, hd, n_slots, normed, past):
+    cap, rows, eps = 64, (heads + 2 * kvh) * hd, 1e-6
+    qkv = ctx.q8_0_matrix(T.q8_0_matrix(4, 1, rows, hidden), rows, hidden)
+    o = ctx.q8_0_matrix(T.q8_0_matrix(4, 2, hidden, heads * hd), hidden, heads * hd)
+    x, nw = T.activations(4, 3, hidden), (1 + 0.1 * T.activations(4, 4, hidden)).astype(np.float32)
+    aw = (1 + 0.1 * T.activations(4, 6, hidden)).astype(np.float32) if normed else None
+    slots = T.activations(4, 5, n_slots * hidden).reshape(n_slots, hidden)
+    fill, so_fill = T.activations(4, 30, kvh * cap * hd).astype(np.float16), T.activations(4, 7, 8 * hidden)
+    kc, vc, xo = ctx.from_array(fill), ctx.from_array(fill), ctx.buffer(hidden * 4)
+    so, status = ctx.floats(so_fill), ctx.buffer(4, shared=True)
+    xo.zero(), status.zero()
+    one, inv = ctx.floats(np.ones(hd)), ctx.floats(oracle.rope_inv_freq(hd, 1e6))
+    ctx.decode_attn_block(ctx.floats(x), ctx.floats(slots) if n_slots else None, n_slots, ctx.floats(aw) if normed else None,
+                          ctx.floats(nw), xo, qkv, o, one, one, inv, kc, vc,
+                          ctx.from_array(np.array([cap + past], np.uint32)), 0, status, so, hidden, heads, kvh, hd, cap, 0, eps, hd ** -0.5)
+    assert int(status.download(0, 4, np.uint32)[0]) == cuda.STATUS_PAST_CAPACITY
+    assert rel_err(xo.download(0, hidden * 4, np.float32), f64_layer(x, slots, aw, nw, eps)[0]) <= 2e-6
+    for c in (kc, vc):
+        np.testing.assert_array_equal(c.download(0, fill.nbytes, np.float16), fill)
+    np.testing.assert_array_equal(so.download(0, so_fill.nbytes, np.float32), so_fill)
+
+
 @pytest.mark.parametrize("block", ["attention", "feed-forward"])
 def test_blocks_refuse_outputs_in_what_other_clusters_read(ctx, oracle, block):
     hidden, width, heads, kvh, hd, cap = 256, 1024, 4, 2, 128, 64

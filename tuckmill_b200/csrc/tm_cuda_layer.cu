@@ -466,20 +466,22 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attn_block_kernel(const 
         if (pos == hint) break;
         hint = ~0u;
     }
-    if (pos >= cap) {  // uniform over the cluster; the pieces' copies land before the CTA's memory goes away
-        if (tid == 0 && rank == 0) atomicOr(a.status, TM_CUDA_STATUS_PAST_CAPACITY);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-        cluster_wait();
-        return;
-    }
 #pragma unroll 1
     for (uint32_t sec = 0; sec < 2u; ++sec) {
         const uint32_t quads = (sec ? G * HD : H) / 4u, plane = plane_bytes(sec ? G * HD : H);
         float4 v[NB];
         bool ok = true;
         if (sec == 0u) {
-            residual_norm<NB>(a.in, kvh == 0u, rank, nw, v, red, [&] { K.first_tile(pos, a.window, kC, rank); });
+            residual_norm<NB>(a.in, kvh == 0u, rank, nw, v, red, [&] { K.first_tile(min(pos, cap - 1u), a.window, kC, rank); });
+            // The sum is stored whatever the position is; past the capacity nothing else.  Uniform over the cluster; the
+            // pieces' copies land before the CTA's memory goes away.
+            if (pos >= cap) {
+                if (tid == 0 && rank == 0) atomicOr(a.status, TM_CUDA_STATUS_PAST_CAPACITY);
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncthreads();
+                cluster_wait();
+                return;
+            }
         } else {
             cluster_wait();  // every CTA of the cluster has started
             // Four lanes finish a row and send it to four CTAs each.
