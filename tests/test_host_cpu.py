@@ -139,3 +139,15 @@ def test_product_never_touches_the_oracle():
         if p.suffix in (".py", ".cu", ".cuh", ".cpp", ".hpp", ".h") and "build" not in p.parts:
             text = p.read_text()
             assert "liboracle" not in text and "import oracle" not in text and "tm_oracle" not in text, p
+
+
+# either side of where the two multiplies of up to 32 tokens cross, at shapes where the times differ by 8 % or more, and
+# shapes that the few-row one refuses
+@pytest.mark.parametrize("rows,cols,batch,pays", [(4096, 1024, 19, 1), (20480, 2048, 16, 1), (16384, 4096, 16, 0), (131072, 512, 16, 0),
+                                                  (8192, 3072, 24, 1), (16384, 2048, 24, 0), (250803, 128, 23, 0), (8704, 2048, 32, 1),
+                                                  (12288, 2048, 32, 0), (1152, 6912, 32, 1), (24576, 4096, 32, 0), (98304, 3072, 8, 1),
+                                                  (262144, 1152, 8, 0), (151936, 4096, 1, 1), (1, 64, 1, 1), (1, 16384, 32, 1),
+                                                  (0, 64, 1, 0), (64, 0, 1, 0), (64, 96, 1, 0), (64, 16448, 9, 0), (64, 64, 0, 0),
+                                                  (64, 64, 33, 0), (2**32 - 1, 16384, 9, 0)])
+def test_where_the_few_row_multiply_is_taken(rows, cols, batch, pays):
+    assert cuda.load_library().tm_cuda_q8_0_gemm_rows_pays(*(ctypes.c_uint32(v) for v in (rows, cols, batch)), 0) == pays

@@ -301,6 +301,7 @@ cudaError_t tm_attention_decode_fast_launch(tm_cuda_ctx *ctx, const float *q, co
 extern "C" int tm_mma_ensure_workspace(tm_cuda_ctx *ctx, uint32_t cols, uint32_t batch, char *err, size_t err_cap);
 cudaError_t tm_x_prep_launch(tm_cuda_ctx *ctx, int prologue, const float *x, const float *pro, uint32_t cols, uint32_t batch,
                              float eps);
+uint32_t tm_mma_few_tokens_cost(uint32_t sms, uint32_t rows, uint32_t cols);
 
 cudaError_t tm_argmax_partial_launch(tm_cuda_ctx *ctx, const float *x, uint32_t n, float *pv, uint32_t *pi);
 cudaError_t tm_argmax_rows_partial_launch(tm_cuda_ctx *ctx, const float *x, uint32_t n_rows, uint32_t n, float *pv,

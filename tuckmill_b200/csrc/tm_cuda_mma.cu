@@ -908,6 +908,33 @@ encode_tiled_fn get_encode_tiled() {
 // 200 (128) 12.6 / 16.2: not all clusters of eight that the SMs add up to have a place.
 uint32_t cluster_ctas(uint32_t sms, uint32_t parts) { return parts == 2u ? sms - 4u : parts <= 4u ? sms - sms / 8u : sms - sms / 4u; }
 
+// Split K: the K range of every output tile is cut into `parts` equal parts when that shortens the longest CTA's run --
+// rounds of the persistent grid x (K steps of a part + the fixed cost of a tile, about 4 steps, + 2 for the ordered
+// reduction through the workspace) -- and the parts' accumulators (`kslot` floats each) fit the workspace.  Where all
+// parts find a place at once and a cluster holds a tile's, they meet there instead.
+struct split_plan {
+    uint32_t parts = 1;
+    bool cluster = false;
+};
+split_plan plan_split(uint32_t sms, uint32_t out_tiles, uint32_t nkb, uint32_t kslot, bool wide) {
+    split_plan plan;
+    if (out_tiles > kSplitTiles) return plan;
+    const uint64_t whole = (uint64_t)((out_tiles + sms - 1) / sms) * (nkb + 4);
+    uint64_t best = whole;
+    for (uint32_t cand : {2u, 3u, 4u, 6u, 8u}) {
+        if (nkb % cand != 0 || nkb / cand < 4) continue;
+        if ((uint64_t)out_tiles * cand * kslot > (uint64_t)kSplitSlots * kSplitSlotFloats) continue;
+        const bool cl = wide && out_tiles * cand <= cluster_ctas(sms, cand);
+        const uint64_t cost = (uint64_t)((out_tiles * cand + sms - 1) / sms) * (nkb / cand + (cl ? 4 : 6));
+        if (cost < best && cost * 10 < whole * 9) {  // a split has to pay for its reduction
+            best = cost;
+            plan.parts = cand;
+            plan.cluster = cl;
+        }
+    }
+    return plan;
+}
+
 template <int BN, int ISS, int SETS, bool WIDE, bool CLUSTER>
 cudaError_t launch_mma_as(tm_cuda_ctx *ctx, const CUtensorMap &wmap, const CUtensorMap &xmap, const mma_args &a, int grid) {
     using L = mma_smem<BN, ISS, SETS, WIDE>;
@@ -931,6 +958,15 @@ cudaError_t launch_mma(tm_cuda_ctx *ctx, const CUtensorMap &wmap, const CUtensor
 }
 
 }  // namespace
+
+// Time of a multiply of up to 32 tokens in hundredths of a microsecond, its f16 copy of X included, fitted to measurements
+// at 9 to 32 tokens (see tm_cuda_q8_0_gemm_rows_pays): rounds of the grid, their K steps, and the workspace's reduction.
+uint32_t tm_mma_few_tokens_cost(uint32_t sms, uint32_t rows, uint32_t cols) {
+    const uint32_t out_tiles = rows / kBM + (rows % kBM != 0u), nkb = (cols + kBK - 1) / kBK;
+    const split_plan p = plan_split(sms, out_tiles, nkb, 128u * 32u, true);
+    const uint64_t rounds = ((uint64_t)out_tiles * p.parts + sms - 1) / sms;
+    return (uint32_t)(712u + rounds * (nkb / p.parts * 25u + 83u + (p.parts > 1u && !p.cluster ? 253u : 0u)));
+}
 
 extern "C" {
 
@@ -1056,35 +1092,15 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
         a.part_end[p] = part_end[p];
     }
     a.accumulate = accumulate ? 1u : 0u;
-    // Split K: the K range of every output tile is cut into `ksplit` equal parts when that shortens the
-    // longest CTA's run -- rounds of the persistent grid x (K steps of a part + the fixed cost of a tile,
-    // about 4 steps, + 2 for the ordered reduction through the workspace) -- and the parts' accumulators fit the
-    // workspace (never for the pushing form).  Where all parts find a place at once and a cluster holds a tile's, they
-    // meet there instead.
-    a.ksplit = 1;
-    bool cluster = false;
     const uint32_t tile_tokens = batch < 2u * (uint32_t)bn ? (batch + 31u) / 32u * 32u : 2u * (uint32_t)bn;
     a.kslot = 128u * tile_tokens;
-    {
-        const uint32_t out_tiles = row_tiles * ((batch + 2 * bn - 1) / (2 * bn)), nkb = (cols + kBK - 1) / kBK;
-        static const bool off = [] { const char *e = getenv("TM_CUDA_MMA_SPLITK"); return e && e[0] == '0'; }();
-        if (!off && push.world == 0 && bn <= 128 && cols % kBK == 0 && out_tiles <= kSplitTiles &&
-            ctx->mma_scratch_bytes >= kSplitBytes) {
-            const uint64_t whole = (uint64_t)((out_tiles + sms - 1) / sms) * (nkb + 4);
-            uint64_t best = whole;
-            for (uint32_t cand : {2u, 3u, 4u, 6u, 8u}) {
-                if (nkb % cand != 0 || nkb / cand < 4) continue;
-                if ((uint64_t)out_tiles * cand * a.kslot > (uint64_t)kSplitSlots * kSplitSlotFloats) continue;
-                const bool cl = (few || bn == 64) && out_tiles * cand <= cluster_ctas(sms, cand);
-                const uint64_t cost = (uint64_t)((out_tiles * cand + sms - 1) / sms) * (nkb / cand + (cl ? 4 : 6));
-                if (cost < best && cost * 10 < whole * 9) {  // a split has to pay for its reduction
-                    best = cost;
-                    a.ksplit = cand;
-                    cluster = cl;
-                }
-            }
-        }
-    }
+    const uint32_t out_tiles = row_tiles * ((batch + 2 * bn - 1) / (2 * bn));
+    static const bool off = [] { const char *e = getenv("TM_CUDA_MMA_SPLITK"); return e && e[0] == '0'; }();
+    // (never for the pushing form)
+    const bool may_split = !off && push.world == 0 && bn <= 128 && cols % kBK == 0 && ctx->mma_scratch_bytes >= kSplitBytes;
+    const split_plan split = may_split ? plan_split(sms, out_tiles, nk, a.kslot, few || bn == 64) : split_plan();
+    a.ksplit = split.parts;
+    const bool cluster = split.cluster;
     unsigned char *split_base = ctx->mma_scratch + ((ctx->mma_scratch_bytes >= kSplitBytes ? ctx->mma_scratch_bytes - kSplitBytes : 0) & ~(size_t)255);
     a.kpart = (float *)split_base;
     a.kcount = (uint32_t *)(split_base + (size_t)kSplitSlots * kSplitSlotFloats * 4);
@@ -1101,7 +1117,7 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     ctx->mma_last_bn = few ? few : bn;
     ctx->mma_last_sets = few ? 4 : 2;
     ctx->mma_last_ksplit = (int)a.ksplit;
-    const uint32_t n_tiles = row_tiles * ((batch + 2 * bn - 1) / (2 * bn)) * a.ksplit;
+    const uint32_t n_tiles = out_tiles * a.ksplit;
     const int grid = (int)(n_tiles < (uint32_t)ctx->sm_count ? n_tiles : (uint32_t)ctx->sm_count);
     TM_CUDA_TRY(few == 32   ? (launch_mma<32, 4, 4, true>(ctx, wmap, xmap, a, grid, cluster))
                 : few == 64 ? (launch_mma<64, 2, 4, true>(ctx, wmap, xmap, a, grid, cluster))

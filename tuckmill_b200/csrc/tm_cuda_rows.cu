@@ -299,13 +299,16 @@ struct rows_plan {
 // stream is long, at most 6.
 // Staged: a CTA's time in cycles, its rounds of units, each the chunks one warp streams plus the ordered sum, and once
 // its share of X; P is the part count with the least of that whose share of X leaves room for a ring.
-rows_plan plan_rows(const tm_cuda_ctx *ctx, uint32_t units, uint32_t cols, uint32_t nt) {
-    const uint32_t chunks = cols / 64u, sms = (uint32_t)ctx->sm_count;
+rows_plan plan_rows(uint32_t sms, size_t smem_optin, uint32_t units, uint32_t cols, uint32_t nt) {
+    const uint32_t chunks = cols / 64u;
     rows_plan best;
     uint32_t cost = 0;
-    // Staged: units for several rounds of every SM and a stream that is longer than X is wide (13824 x 1152, 432 units of
-    // 18 chunks: 7.3 us staged, 7.2 not; 12288 x 4096, 384 of 64: 15.4, 17.4; 4096 x 12288, 128 of 192: 17.5, 15.3).
-    if (nt == 1u && units > 2u * sms && units * chunks >= 24000u) {
+    // Staged: units for more than two rounds of every SM, and a stream that is longer than X is wide or (8 chunks, one a
+    // warp) so short that the CTAs that come and go cost more than it.  us staged / not, at 8 tokens: 512 columns 12288
+    // rows 5.4 / 5.9, 24576 9.0 / 8.4, 65536 16.2 / 17.7; 1024 24576 12.3 / 11.8, 32768 14.0 / 14.7; 1536 16384 11.7 / 11.2,
+    // 24576 15.1 / 15.4; 2048 16384 14.4 / 14.1, 20480 16.7 / 17.2; 4096 9504 (297 units) 17.7 / 17.3, 12288 18.5 / 18.9;
+    // 5120 9504 21.7 / 20.4, 12288 21.3 / 22.0; 3072 98304 70 / 85.
+    if (nt == 1u && 2u * units > 5u * sms && (units * chunks >= 16000u || chunks <= 8u)) {
         best.staged = true;
         for (uint32_t p = 1; p <= 8u && p <= chunks; ++p) {
             const uint32_t kc = (chunks + p - 1u) / p, rounds = (units * p + sms - 1u) / sms;
@@ -314,7 +317,7 @@ rows_plan plan_rows(const tm_cuda_ctx *ctx, uint32_t units, uint32_t cols, uint3
             if (best.p && c >= cost) continue;
             uint32_t ring = 0;
             for (uint32_t r : {6u, 4u, 3u, 2u})
-                if ((r <= rounds * per_warp || r == 2u) && rows_smem(cols, nt, p, r, true) <= ctx->smem_optin) {
+                if ((r <= rounds * per_warp || r == 2u) && rows_smem(cols, nt, p, r, true) <= smem_optin) {
                     ring = r;
                     break;
                 }
@@ -374,18 +377,26 @@ cudaError_t launch_rows(tm_cuda_ctx *ctx, const rows_args &a, const rows_plan &p
 
 extern "C" {
 
-// Where the multiply for a few rows beats the tcgen05 GEMM: the more tokens, the sooner its MMAs and token fragments cost
-// more than the other kernel's hand-overs.  Measured, us against us, both with the f16 copy of X, at either side of the
-// lines: 8 tokens 24576 x 4096 27.7 / 32.3, 151936 x 4096 128 / 150, 262144 x 1152 86 / 79; 16 tokens 12288 x 4096 19.1 /
-// 19.6, 4096 x 12288 17.6 / 18.8, 24576 x 4096 33.9 / 32.2; 24 tokens 6144 x 4096 12.3 / 12.7, 12288 x 4096 20.3 / 19.9; 32
-// tokens 4096 x 4096 9.9 / 10.2, 1152 x 6912 7.0 / 7.9, 6144 x 4096 14.0 / 12.7, 13824 x 1152 10.3 / 8.6 (its units are more
-// than find a place at once).  (On the wrong side of them: 13824 x 1152 at 24, 9.0 / 8.6.)
+// Where the multiply for a few rows beats the tcgen05 GEMM, both with the f16 copy of X.  Up to 8 tokens: everywhere but in
+// narrow matrices of many bytes (us, this form / tcgen05: 65536 x 1536 30 / 34, 98304 x 3072 70 / 87, 98304 x 4096 96 / 118,
+// but 262144 x 1152 86 / 79).  From 9 tokens on the two cross wherever the one's units or the other's 128-row tiles have
+// just begun another round of the SMs, so both times are estimated, in hundredths of a microsecond, fitted to 279 shapes of
+// 64 to 16384 columns and 3 to 130 M weights at 9 to 32 tokens: one of nine takes the slower form, by 4 % (11 at most).
+// At 16 tokens 20480 x 2048 19.4 / 23.7, 16384 x 4096 26.7 / 24.2, 131072 x 512 38 / 26; at 24 8192 x 3072 13.4 / 15.0,
+// 6144 x 4096 15.5 / 16.4, 16384 x 2048 17.7 / 15.9; at 32 8704 x 2048 11.5 / 13.2, 4096 x 4096 12.5 / 13.3, 12288 x 2048
+// 16.1 / 14.9.  (Lines at a number of weights, 64, 32 and 17 M, cost 5, 5 and 2 % in the mean and up to 97.)
+static bool rows_are_faster(uint32_t rows, uint32_t cols, uint32_t batch) {
+    constexpr uint32_t kSms = 148;  // of the part that the times were taken on
+    if (batch <= 8u) return cols >= 1536u || (uint64_t)rows * cols <= 128u << 20;
+    const uint32_t nt = (batch + 7u) / 8u, units = rows / 32u + (rows % 32u != 0u);
+    const rows_plan pl = plan_rows(kSms, 0, units, cols, nt);
+    // Rounds of two CTAs an SM, and the chunks that the warps of the fullest SM stream (some of it behind the launch).
+    const int64_t ctas = (int64_t)units * pl.p, turns = (ctas + 2 * kSms - 1) / (2 * kSms), per_sm = (ctas + kSms - 1) / kSms;
+    const int64_t cost = 191 + turns * 227 + per_sm * ((int64_t)cols * (35 + 14 * nt) / (512 * pl.p) - 36) + (pl.p > 1u ? 109 : 0);
+    return cost < (int64_t)tm_mma_few_tokens_cost(kSms, rows, cols);
+}
 int tm_cuda_q8_0_gemm_rows_pays(uint32_t rows, uint32_t cols, uint32_t batch, int gated) {
-    if (!rows_ok(rows, cols, batch, gated != 0)) return 0;
-    const uint64_t weights = (uint64_t)rows * cols, limit[4] = {128u << 20, 64u << 20, 32u << 20, 17u << 20};
-    if (batch <= 8u && cols >= 4096u) return 1;
-    if (batch > 24u && rows > 8192u) return 0;
-    return weights <= limit[(batch - 1u) / 8u];
+    return rows_ok(rows, cols, batch, gated != 0) && rows_are_faster(rows, cols, batch);
 }
 
 int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, uint32_t rows, uint32_t cols,
@@ -437,7 +448,7 @@ int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *
     a.batch = batch;
     a.accumulate = epilogue == TM_CUDA_EPI_ADD;
     const uint32_t nt = (batch + 7u) / 8u;
-    const rows_plan pl = plan_rows(ctx, a.units, cols, nt);
+    const rows_plan pl = plan_rows((uint32_t)ctx->sm_count, ctx->smem_optin, a.units, cols, nt);
     if (!pl.p) return tm_fail(err, err_cap, TM_CUDA_ERR_UNSUPPORTED, "cols %u exceeds the activation stage of a cluster", cols);
     if (prologue == TM_CUDA_PRO_F16) {
         TM_CHECK_BUF(x, (size_t)batch * cols * 2, "activation");
