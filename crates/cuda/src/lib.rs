@@ -115,6 +115,7 @@ mod ffi {
         pub fn tm_cuda_mma_last_tile(ctx: *mut TmCudaCtx) -> c_int;
         pub fn tm_cuda_mma_last_sets(ctx: *mut TmCudaCtx) -> c_int;
         pub fn tm_cuda_mma_last_split(ctx: *mut TmCudaCtx) -> c_int;
+        pub fn tm_cuda_mma_last_cluster(ctx: *mut TmCudaCtx) -> c_int;
         pub fn tm_cuda_q8_0_row_f32(ctx: *mut TmCudaCtx, w: *mut TmCudaBuffer, out: *mut TmCudaBuffer, row: u32, cols: u32, out_off: u32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_f16_gemv(ctx: *mut TmCudaCtx, w: *mut TmCudaBuffer, x: *mut TmCudaBuffer, y: *mut TmCudaBuffer, rows: u32, cols: u32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_f16_gemm(ctx: *mut TmCudaCtx, w: *mut TmCudaBuffer, x: *mut TmCudaBuffer, y: *mut TmCudaBuffer, rows: u32, cols: u32, batch: u32, x_off: u32, y_off: u32, err: *mut c_char, err_cap: usize) -> c_int;
@@ -169,6 +170,7 @@ mod ffi {
         pub fn tm_cuda_qwen35_attention_f16_chunk(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, out: *mut TmCudaBuffer, scratch: *mut TmCudaBuffer, heads: u32, pos0: u32, cap: u32, head_dim: u32, group: u32, scale: f32, n: u32, window: u32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_q8_0_gemm_mma_fused(ctx: *mut TmCudaCtx, w: *mut TmCudaBuffer, x: *mut TmCudaBuffer, rows: u32, cols: u32, batch: u32, n_parts: u32, y_parts: *const *mut TmCudaBuffer, part_rows: *const u32, prologue: c_int, pro: *mut TmCudaBuffer, eps: f32, epilogue: c_int, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_q8_0_gemm_rows_pays(rows: u32, cols: u32, batch: u32, gated: c_int) -> c_int;
+        pub fn tm_cuda_gemm_rows_last_form(ctx: *mut TmCudaCtx) -> c_int;
         pub fn tm_cuda_q8_0_gemm_rows(ctx: *mut TmCudaCtx, w: *mut TmCudaBuffer, x: *mut TmCudaBuffer, rows: u32, cols: u32, batch: u32, n_parts: u32, y_parts: *const *mut TmCudaBuffer, part_rows: *const u32, prologue: c_int, pro: *mut TmCudaBuffer, eps: f32, epilogue: c_int, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_qk_prep_chunk(ctx: *mut TmCudaCtx, q: *mut TmCudaBuffer, k: *mut TmCudaBuffer, v: *mut TmCudaBuffer, q_norm: *mut TmCudaBuffer, k_norm: *mut TmCudaBuffer, inv_freq: *mut TmCudaBuffer, k_cache: *mut TmCudaBuffer, v_cache: *mut TmCudaBuffer, heads: u32, kv_heads: u32, head_dim: u32, n_rot: u32, pos0: u32, cap: u32, n: u32, eps: f32, err: *mut c_char, err_cap: usize) -> c_int;
         pub fn tm_cuda_attention_chunk_mma_supported(head_dim: u32) -> c_int;

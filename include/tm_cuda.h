@@ -206,9 +206,10 @@ int tm_cuda_mma_last_sets(tm_cuda_ctx *ctx);
 /* No counterpart: how many parts the last GEMM launch cut the K range of every output tile into
  * (1: none; 0 before the first launch).  A call with fewer output tiles than half the SMs (a batch of
  * decode rows, a narrow projection) is split so that the whole machine streams its weights; the
- * parts' sums are added in part order by whichever part finishes last, so the result does not depend
- * on timing. */
+ * parts' sums are added in part order, by the CTAs of a cluster that holds a tile's parts (_last_cluster: 1) or,
+ * through the workspace, by whichever part finishes last (0), so the result does not depend on timing. */
 int tm_cuda_mma_last_split(tm_cuda_ctx *ctx);
+int tm_cuda_mma_last_cluster(tm_cuda_ctx *ctx);
 /* tm_metal.h:138 tm_metal_q8_0_row_f32: dequantise one row to out[out_off..]. */
 int tm_cuda_q8_0_row_f32(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *out, uint32_t row,
                          uint32_t cols, uint32_t out_off, char *err, size_t err_cap);
@@ -461,6 +462,9 @@ int tm_cuda_q8_0_gemm_mma_fused(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buf
  * the two kernels for this size. */
 #define TM_CUDA_GEMM_ROWS_MAX_BATCH 32
 int tm_cuda_q8_0_gemm_rows_pays(uint32_t rows, uint32_t cols, uint32_t batch, int gated);
+/* No counterpart: K parts of the context's last such multiply (0 before the first), negative for the form that keeps its
+ * activations in shared memory. */
+int tm_cuda_gemm_rows_last_form(tm_cuda_ctx *ctx);
 int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, uint32_t rows, uint32_t cols,
                            uint32_t batch, uint32_t n_parts, tm_cuda_buffer *const *y_parts, const uint32_t *part_rows,
                            int prologue, tm_cuda_buffer *pro, float eps, int epilogue, char *err, size_t err_cap);

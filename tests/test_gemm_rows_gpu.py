@@ -68,11 +68,11 @@ def test_gemm_rows_parts_and_limits(ctx):
             ctx.q8_0_gemm_rows(w, xb, 160, 128, batch, ys, rows_of)
 
 
-# X read where it lies: units of one part and of several, warps without a chunk, more units than find a place at once, the
-# staged form (8 tokens by many units); binary16 rows that lie on a 16-byte boundary only take half-width loads
+# X read where it lies: units of one part and of several, warps without a chunk, more units than find a place at once;
+# binary16 rows that lie on a 16-byte boundary only take half-width loads
 @pytest.mark.parametrize("rows,cols,batch", [(64, 64, 1), (1024, 3072, 32), (1056, 6912, 7), (4096, 4096, 24), (9504, 576, 31),
                                              (9504, 64, 8), (9504, 5120, 8), (9504, 5120, 9)])
-def test_gemm_rows_x_at_either_alignment(ctx, rows, cols, batch):
+def test_gemm_rows_x_at_either_alignment(ctx, rows, cols, batch, staged=False):
     raw = T.q8_0_matrix(14, rows + cols, rows, cols)
     X = T.activations(14, 5, batch * cols).reshape(batch, cols).astype(np.float16)
     w, yb = ctx.q8_0_matrix(raw, rows, cols), ctx.buffer(batch * rows * 4)
@@ -84,5 +84,36 @@ def test_gemm_rows_x_at_either_alignment(ctx, rows, cols, batch):
         yb.zero()
         ctx.q8_0_gemm_rows(w, x, rows, cols, batch, [yb], [rows], cuda.PRO_F16)
         got.append(yb.download(0, batch * rows * 4, np.float32).reshape(batch, rows))
+    assert (ctx.gemm_rows_last_form() < 0) == staged
     assert rel_err(got[0], f16_profile_reference(raw, X)) <= 2e-5
     np.testing.assert_array_equal(got[0], got[1])
+    base = T.activations(14, 9, batch * rows).reshape(batch, rows)
+    yb.upload(0, base)
+    ctx.q8_0_gemm_rows(w, x, rows, cols, batch, [yb], [rows], cuda.PRO_F16, epilogue=cuda.EPI_ADD)
+    np.testing.assert_array_equal(yb.download(0, batch * rows * 4, np.float32).reshape(batch, rows), base + got[0])
+
+
+# X staged for CTAs that serve several units (up to 8 tokens): either side of both lines, fewer chunks than warps, one
+# round of units and many, a last unit that is not whole
+@pytest.mark.parametrize("rows,cols,batch,staged", [(11840, 512, 8, False), (11841, 512, 8, True), (11841, 576, 8, False),
+                                                    (13632, 2368, 8, False), (13632, 2432, 8, True), (12007, 64, 3, True),
+                                                    (50001, 704, 5, True), (11872, 8192, 1, True), (13632, 2432, 9, False)])
+def test_gemm_rows_with_x_staged(ctx, rows, cols, batch, staged):
+    test_gemm_rows_x_at_either_alignment(ctx, rows, cols, batch, staged)
+
+
+def test_gemm_rows_staged_in_parts_and_gated(ctx):
+    rows, cols, batch = 32768, 1088, 6
+    raw = T.q8_0_matrix(15, 1, rows, cols)
+    X = T.activations(15, 5, batch * cols).reshape(batch, cols)
+    w, xb, part_rows = ctx.q8_0_matrix(raw, rows, cols), ctx.floats(X), [32, 16384, 16352]
+    ys = [ctx.buffer(batch * n * 4) for n in part_rows]
+    want = f16_profile_reference(raw, X)
+    ctx.q8_0_gemm_rows(w, xb, rows, cols, batch, ys, part_rows)
+    assert ctx.gemm_rows_last_form() < 0
+    got = np.concatenate([y.download(0, batch * n * 4, np.float32).reshape(batch, n) for y, n in zip(ys, part_rows)], axis=1)
+    assert rel_err(got, want) <= 2e-5
+    h, (g, u) = ctx.buffer(batch * rows), np.split(want, 2, axis=1)
+    ctx.q8_0_gemm_rows(w, xb, rows, cols, batch, [h], [rows // 2], epilogue=cuda.EPI_SILU_MUL_F16)
+    assert ctx.gemm_rows_last_form() < 0
+    assert rel_err(h.download(0, batch * rows, np.float16).reshape(batch, rows // 2).astype(np.float64), g / (1 + np.exp(-g)) * u) <= 2e-3

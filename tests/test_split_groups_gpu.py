@@ -33,11 +33,11 @@ def test_groups_of_a_split_sum(ctx, oracle, rows, cols, batch):
 
 
 # Parts that meet in a cluster: 2, 3, 4, 6 and 8 of them, shares of the tokens that are uneven or empty, a last four of
-# tokens that is not whole, rows that end inside a tile, more clusters than have a place (through the workspace)
+# tokens that is not whole, rows that end inside a tile
 @pytest.mark.parametrize("rows,cols,batch", [(6144, 1024, 61), (1500, 2304, 3), (1536, 1152, 130), (4000, 1024, 29),
                                              (1152, 6912, 35), (1024, 3072, 9), (1024, 2048, 33), (1024, 3072, 200),
                                              (3000, 4096, 128), (1024, 2048, 512)])
-def test_parts_that_meet_in_a_cluster(ctx, rows, cols, batch):
+def test_parts_that_meet_in_a_cluster(ctx, rows, cols, batch, parts=None):
     raw = T.q8_0_matrix(6, rows + cols, rows, cols)
     x = T.activations(6, 2, batch * cols).reshape(batch, cols)
     w, xb = ctx.q8_0_matrix(raw, rows, cols), ctx.floats(x)
@@ -48,9 +48,19 @@ def test_parts_that_meet_in_a_cluster(ctx, rows, cols, batch):
         ctx.q8_0_gemm_mma(w, xb, y, rows, cols, batch)
         got.append(y.download(0, batch * rows * 4, np.float32).reshape(batch, rows))
     assert ctx.mma_last_split() > 1 and not ctx.mma_aborted()
+    assert ctx.mma_last_cluster() == (parts is None) and parts in (None, ctx.mma_last_split())
     ref = x.astype(np.float16).astype(np.float64) @ T.q8_0_dequant(raw).astype(np.float16).astype(np.float64).T
     assert rel_err(got[0], ref) <= 2e-5
     np.testing.assert_array_equal(got[0], got[1])
     acc = ctx.floats(base)
     ctx.q8_0_gemm_mma_fused(w, xb, rows, cols, batch, [acc], [rows], cuda.PRO_NONE, None, 0.0, cuda.EPI_ADD)
     np.testing.assert_array_equal(acc.download(0, batch * rows * 4, np.float32).reshape(batch, rows), base + got[0])
+
+
+# Parts that meet in the workspace, because not all clusters have a place: 2, 3, 6 and 8 of them, in the forms with four
+# converter sets and with two, fewer groups of 32 tokens than parts and more, a last group of one token; 128-token sub-tiles
+# (which have no cluster form)
+@pytest.mark.parametrize("rows,cols,batch,parts", [(9344, 2048, 33, 2), (6144, 1152, 29, 3), (6100, 1152, 33, 3), (6144, 1152, 97, 3),
+                                                   (2432, 2304, 64, 6), (2432, 2304, 32, 6), (1024, 2048, 161, 8), (1000, 2048, 200, 8)])
+def test_parts_that_meet_in_the_workspace(ctx, rows, cols, batch, parts):
+    test_parts_that_meet_in_a_cluster(ctx, rows, cols, batch, parts)

@@ -28,7 +28,6 @@ using tmdev::cluster_rank;
 using tmdev::cluster_size;
 using tmdev::cluster_wait;
 using tmdev::smem_addr;
-using tmdev::st_cluster;
 
 // CTA `rank` of C owns keys [lo, hi) of a step at position p: equal contiguous runs of whole eights.
 __device__ __forceinline__ void key_range(uint32_t p, uint32_t window, uint32_t C, uint32_t rank, uint32_t &lo, uint32_t &hi) {

@@ -113,6 +113,8 @@ struct tm_cuda_ctx {
     int mma_last_bn = 0;                 // token sub-tile width of the last tensor-core GEMM launch
     int mma_last_sets = 0;               // its sets of converter warps
     int mma_last_ksplit = 0;             // K parts per output tile of that launch
+    int mma_last_cluster = 0;            // whether they were a cluster
+    int rows_last_form = 0;              // K parts of the last multiply for a few rows, negative if it staged X
     void *comm = nullptr;  // multi-GPU communicator state (tm_cuda_comm.cu)
     void *program = nullptr;  // the persistent program being recorded (tm_step_program), if any
 };

@@ -44,7 +44,7 @@ constexpr int kBM = 128;        // weight rows per tile (UMMA M)
 constexpr int kBK = 64;         // K per stage: 64 f16 = one 128-byte swizzle row
 constexpr int kEpiWarps = 4;
 constexpr uint32_t kQuadBytes = kBM * 16;  // four tokens of a tile's rows, f32
-constexpr uint32_t kSpinLimit = 1u << 20;  // a healthy wait is microseconds; this is ~seconds
+constexpr uint32_t kSpinLimit = 1u << 20;  // polls of 4.4 us each while nothing arrives: 4.6 s (a healthy wait is microseconds)
 // Split-K: when it shortens the longest CTA's run (few output tiles on many SMs: a decode batch, a narrow
 // projection, a last round that leaves most SMs idle) the K range of every tile is cut into `ksplit`
 // equal parts, each its own tile of the persistent grid;
@@ -1117,6 +1117,7 @@ static int mma_launch(tm_cuda_ctx *ctx, const tm_cuda_buffer *w, uint32_t rows, 
     ctx->mma_last_bn = few ? few : bn;
     ctx->mma_last_sets = few ? 4 : 2;
     ctx->mma_last_ksplit = (int)a.ksplit;
+    ctx->mma_last_cluster = cluster;
     const uint32_t n_tiles = out_tiles * a.ksplit;
     const int grid = (int)(n_tiles < (uint32_t)ctx->sm_count ? n_tiles : (uint32_t)ctx->sm_count);
     TM_CUDA_TRY(few == 32   ? (launch_mma<32, 4, 4, true>(ctx, wmap, xmap, a, grid, cluster))
@@ -1260,6 +1261,11 @@ int tm_cuda_mma_last_split(tm_cuda_ctx *ctx) {
     if (!ctx) return 0;
     std::lock_guard<std::mutex> lock(ctx->mu);
     return ctx->mma_last_ksplit;
+}
+int tm_cuda_mma_last_cluster(tm_cuda_ctx *ctx) {
+    if (!ctx) return 0;
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return ctx->mma_last_cluster;
 }
 
 // 1 when a tensor-core GEMM or a decode layer block on this context ever gave up a bounded wait.

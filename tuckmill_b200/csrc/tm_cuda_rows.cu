@@ -399,6 +399,12 @@ int tm_cuda_q8_0_gemm_rows_pays(uint32_t rows, uint32_t cols, uint32_t batch, in
     return rows_ok(rows, cols, batch, gated != 0) && rows_are_faster(rows, cols, batch);
 }
 
+int tm_cuda_gemm_rows_last_form(tm_cuda_ctx *ctx) {
+    if (!ctx) return 0;
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return ctx->rows_last_form;
+}
+
 int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *x, uint32_t rows, uint32_t cols,
                            uint32_t batch, uint32_t n_parts, tm_cuda_buffer *const *y_parts, const uint32_t *part_rows,
                            int prologue, tm_cuda_buffer *pro, float eps, int epilogue, char *err, size_t err_cap) {
@@ -461,6 +467,7 @@ int tm_cuda_q8_0_gemm_rows(tm_cuda_ctx *ctx, tm_cuda_buffer *w, tm_cuda_buffer *
         a.x = (const __half *)ctx->mma_scratch;
     }
     a.x32 = ((size_t)a.x & 31u) == 0;
+    ctx->rows_last_form = pl.staged ? -(int)pl.p : (int)pl.p;
     TM_OP_BEGIN("q8_0_gemm_rows");
     if (prologue != TM_CUDA_PRO_F16)
         TM_CUDA_TRY(tm_x_prep_launch(ctx, prologue, (const float *)x->dev, pro ? (const float *)pro->dev : nullptr, cols,
