@@ -71,7 +71,7 @@ def test_gemm_rows_parts_and_limits(ctx):
 # X read where it lies: units of one part and of several, warps without a chunk, more units than find a place at once;
 # binary16 rows that lie on a 16-byte boundary only take half-width loads
 @pytest.mark.parametrize("rows,cols,batch", [(64, 64, 1), (1024, 3072, 32), (1056, 6912, 7), (4096, 4096, 24), (9504, 576, 31),
-                                             (9504, 64, 8), (9504, 5120, 8), (9504, 5120, 9)])
+                                             (9472, 64, 8), (9504, 5120, 8), (9504, 5120, 9)])
 def test_gemm_rows_x_at_either_alignment(ctx, rows, cols, batch, staged=False):
     raw = T.q8_0_matrix(14, rows + cols, rows, cols)
     X = T.activations(14, 5, batch * cols).reshape(batch, cols).astype(np.float16)
@@ -93,11 +93,14 @@ def test_gemm_rows_x_at_either_alignment(ctx, rows, cols, batch, staged=False):
     np.testing.assert_array_equal(yb.download(0, batch * rows * 4, np.float32).reshape(batch, rows), base + got[0])
 
 
-# X staged for CTAs that serve several units (up to 8 tokens): either side of both lines, fewer chunks than warps, one
-# round of units and many, a last unit that is not whole
-@pytest.mark.parametrize("rows,cols,batch,staged", [(11840, 512, 8, False), (11841, 512, 8, True), (11841, 576, 8, False),
-                                                    (13632, 2368, 8, False), (13632, 2432, 8, True), (12007, 64, 3, True),
-                                                    (50001, 704, 5, True), (11872, 8192, 1, True), (13632, 2432, 9, False)])
+# X staged for CTAs that serve several units (up to 8 tokens, up to 16 in a narrow matrix): either side of every line, fewer
+# chunks than warps, one round of units and many, a last unit that is not whole
+@pytest.mark.parametrize("rows,cols,batch,staged", [(9472, 512, 8, False), (9473, 512, 8, True), (9473, 576, 8, False),
+                                                    (13632, 1920, 8, False), (13632, 1984, 8, True), (11840, 5952, 8, False),
+                                                    (11840, 6080, 8, True), (9504, 64, 8, True), (12007, 64, 3, True), (50001, 704, 5, True),
+                                                    (11872, 8192, 1, True), (13632, 1984, 9, False), (9472, 512, 9, False),
+                                                    (9473, 512, 9, True), (20481, 192, 16, True), (9473, 576, 16, False),
+                                                    (9473, 512, 17, False)])
 def test_gemm_rows_with_x_staged(ctx, rows, cols, batch, staged):
     test_gemm_rows_x_at_either_alignment(ctx, rows, cols, batch, staged)
 

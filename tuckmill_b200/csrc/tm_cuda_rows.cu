@@ -21,9 +21,9 @@
 // barrier out of a chain that is all latency, and 40 KB of shared memory in place of 100-220 let two CTAs share an SM,
 // so the next launch's weights are in flight while this one ends.  32 tokens by 6144 x 1024 6.9 -> 4.9 us, 1024 x 3072
 // 5.7 -> 4.6, 4096 x 4096 13.2 -> 9.8, 1152 x 6912 15.6 -> 7.0; 19 tokens by 4096 x 1024 5.6 -> 4.0.
-// Only 8 tokens by a matrix of many units keep X staged, in CTAs that stay (STAGED): 12288 x 4096 15.4 us against 17.4,
-// 24576 x 4096 27.7 / 29.7, 151936 x 4096 128 / 143.  (At 16 tokens 18.5 / 19.1, 33.8 / 33.9, 152 / 163: two tiles of
-// tokens are not worth a second form, and from 24 tokens on it is the slower one, 26 / 20.)
+// Only up to 8 tokens, or 16 in a narrow matrix, by many units keep X staged, in CTAs that stay (STAGED): at 8 tokens 12288 x
+// 4096 15.4 us against 17.4, 24576 x 4096 27.7 / 29.7, 151936 x 4096 128 / 143.  (At 16 tokens 18.5 / 19.1, 33.8 / 33.9, 152 /
+// 163: two tiles of tokens are not worth it there, and from 24 tokens on it is the slower one, 26 / 20.)
 #include "tm_cuda_internal.cuh"
 #include "tm_cuda_device.cuh"
 
@@ -286,6 +286,10 @@ size_t rows_smem(uint32_t cols, uint32_t nt, uint32_t p, uint32_t ring, bool sta
            (size_t)kWarps * ring * kSlot;
 }
 
+// Clusters of p CTAs, one CTA to an SM, that find a place at once.  (Where more were launched than that, 12288 x 12288 at 8
+// tokens took 75 us in three parts; 47 without staging.)
+uint32_t cluster_places(uint32_t sms, uint32_t p) { return (p <= 2u ? sms : p <= 4u ? sms - sms / 8u : sms - sms / 4u) / p; }
+
 struct rows_plan {
     uint32_t p = 0, ring = 0;
     bool staged = false;
@@ -303,17 +307,20 @@ rows_plan plan_rows(uint32_t sms, size_t smem_optin, uint32_t units, uint32_t co
     const uint32_t chunks = cols / 64u;
     rows_plan best;
     uint32_t cost = 0;
-    // Staged: units for more than two rounds of every SM, and a stream that is longer than X is wide or (8 chunks, one a
-    // warp) so short that the CTAs that come and go cost more than it.  us staged / not, at 8 tokens: 512 columns 12288
-    // rows 5.4 / 5.9, 24576 9.0 / 8.4, 65536 16.2 / 17.7; 1024 24576 12.3 / 11.8, 32768 14.0 / 14.7; 1536 16384 11.7 / 11.2,
-    // 24576 15.1 / 15.4; 2048 16384 14.4 / 14.1, 20480 16.7 / 17.2; 4096 9504 (297 units) 17.7 / 17.3, 12288 18.5 / 18.9;
-    // 5120 9504 21.7 / 20.4, 12288 21.3 / 22.0; 3072 98304 70 / 85.
-    if (nt == 1u && 2u * units > 5u * sms && (units * chunks >= 16000u || chunks <= 8u)) {
+    // Staged: units for more than two rounds of every SM, and either at most 8 chunks, one a warp, so that the CTAs that come
+    // and go cost more than they stream, or (up to 8 tokens) a stream that is longer than X is wide; where the third round
+    // is hardly begun, a still longer one.  us staged / not: 8 tokens by 10464 x 320 4.7 / 5.3, 12288 x 512 5.4 / 5.9, 24576 x
+    // 512 9.0 / 8.4, 24576 x 1024 12.3 / 11.8, 32768 x 1024 14.0 / 14.7, 16384 x 1536 11.7 / 11.2, 24576 x 1536 15.1 / 15.4,
+    // 12288 x 2048 12.0 / 11.8, 20480 x 2048 16.7 / 17.2, 12288 x 4096 18.5 / 18.9, 98304 x 3072 70 / 85, and with 297 to 364
+    // units 9504 x 6144 24.3 / 23.8, 9504 x 8192 29.2 / 30.1, 10240 x 11264 37 / 45; 16 tokens by 20480 x 128 6.0 / 7.1, 20480 x
+    // 512 8.1 / 8.9, 16384 x 640 9.4 / 8.2.  (24 tokens by 16384 x 128 5.9 / 6.4, x 512 9.3 / 7.8: no third form for that.)
+    const bool long_stream = units * chunks >= (2u * units > 5u * sms ? 13000u : 35000u);
+    if (nt <= 2u && units > 2u * sms && (chunks <= 8u || (nt == 1u && long_stream))) {
         best.staged = true;
         for (uint32_t p = 1; p <= 8u && p <= chunks; ++p) {
-            const uint32_t kc = (chunks + p - 1u) / p, rounds = (units * p + sms - 1u) / sms;
+            const uint32_t kc = (chunks + p - 1u) / p, at_once = cluster_places(sms, p), rounds = (units + at_once - 1u) / at_once;
             const uint32_t per_warp = (kc + kWarps - 1u) / kWarps;
-            const uint32_t c = rounds * (per_warp * 700u + 1100u + (p > 1u ? 300u : 0u)) + kc * 20u;
+            const uint32_t c = rounds * (per_warp * (500u + 200u * nt) + 900u + 200u * nt + (p > 1u ? 300u : 0u)) + kc * 20u * nt;
             if (best.p && c >= cost) continue;
             uint32_t ring = 0;
             for (uint32_t r : {6u, 4u, 3u, 2u})
@@ -361,14 +368,14 @@ cudaError_t launch_rows_as(tm_cuda_ctx *ctx, const rows_args &args, const rows_p
     }
     // Resident clusters: by shared memory (1 KB per CTA is the system's) and registers at most two CTAs per SM.
     const uint32_t per_sm = 2u * (smem + 1024u) <= 228u * 1024u ? 2u : 1u;
-    uint32_t clusters = (uint32_t)ctx->sm_count * per_sm / pl.p;
+    uint32_t clusters = cluster_places((uint32_t)ctx->sm_count, pl.p) * per_sm;
     if (!STAGED || clusters > a.units) clusters = a.units;
     return tm_launch_cluster_pdl(ctx, pl.p, q8_gemm_rows_kernel<NT, STAGED>, dim3(clusters * pl.p), dim3(kThreads), smem, a);
 }
 
 template <int NT>
 cudaError_t launch_rows(tm_cuda_ctx *ctx, const rows_args &a, const rows_plan &pl) {
-    if constexpr (NT == 1)
+    if constexpr (NT <= 2)
         if (pl.staged) return launch_rows_as<NT, true>(ctx, a, pl);
     return launch_rows_as<NT, false>(ctx, a, pl);
 }
@@ -389,7 +396,7 @@ static bool rows_are_faster(uint32_t rows, uint32_t cols, uint32_t batch) {
     constexpr uint32_t kSms = 148;  // of the part that the times were taken on
     if (batch <= 8u) return cols >= 1536u || (uint64_t)rows * cols <= 128u << 20;
     const uint32_t nt = (batch + 7u) / 8u, units = rows / 32u + (rows % 32u != 0u);
-    const rows_plan pl = plan_rows(kSms, 0, units, cols, nt);
+    const rows_plan pl = plan_rows(kSms, 0, units, cols, nt);  // (no shared memory: X not staged)
     // Rounds of two CTAs an SM, and the chunks that the warps of the fullest SM stream (some of it behind the launch).
     const int64_t ctas = (int64_t)units * pl.p, turns = (ctas + 2 * kSms - 1) / (2 * kSms), per_sm = (ctas + kSms - 1) / kSms;
     const int64_t cost = 191 + turns * 227 + per_sm * ((int64_t)cols * (35 + 14 * nt) / (512 * pl.p) - 36) + (pl.p > 1u ? 109 : 0);
