@@ -560,8 +560,10 @@ struct decode_seq_strides {
 // warp a CTA (2048 of them at 4096 positions of a 0.6B decoder, each fetching all small inputs before it looked at the
 // position, and the key loads only after the norm) a layer's call took 15.8 us at 150 positions, now 10.4.
 constexpr int kDecodeWarps = 4;
+// (Three CTAs an SM: at head size 128 the compiler takes two registers more than let the third one in, and 32 heads at
+// position 1500 take 31 us in place of 26.)
 template <int DPL>
-__global__ void __launch_bounds__(32 * kDecodeWarps) attention_decode_kernel(
+__global__ void __launch_bounds__(32 * kDecodeWarps, 3) attention_decode_kernel(
     const float *q, const float *k, const float *v, const float *q_norm, const float *k_norm,
     const float *inv_freq, __half *kc, __half *vc, float *out, float *scratch, const uint32_t *pos_p,
     uint32_t *status, uint32_t heads, uint32_t kv_heads, uint32_t hd, uint32_t n_rot, uint32_t cap,
