@@ -44,9 +44,6 @@ using tmdev::mma_f16;
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void *src, bool read) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(read ? 16u : 0u) : "memory");
-}
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *(const uint32_t *)&h;
@@ -627,10 +624,9 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
         constexpr int CH = HD / 8;  // 16-byte chunks per row
         for (int i = tid; i < kBKV * CH; i += kThreads) {
             const uint32_t r = i / CH, c = i % CH;
-            // Keys past the position repeat its row (masked below); values that weigh 0 are zeros: 0 times an infinity is NaN.
-            const uint32_t j = min(j0 + r, pos);
+            const uint32_t j = min(j0 + r, pos);  // rows past the position repeat its row (masked below)
             cp_async16(smem_u32(sK) + sw<PITCH>(r, c), kc + (size_t)j * HD + c * 8);
-            cp_async16_or_zero(smem_u32(sV) + sw<PITCH>(r, c), vc + (size_t)j * HD + c * 8, j0 + r - start <= pos - start);
+            cp_async16(smem_u32(sV) + sw<PITCH>(r, c), vc + (size_t)j * HD + c * 8);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -742,12 +738,14 @@ __global__ void __launch_bounds__(kThreads) attention_decode_mma_kernel(const de
             o[i][0] *= alpha;
             o[i][1] *= alpha;
         }
-        // ---- O += P V over this warp's 16 keys ----
+        // ---- O += P V over this warp's 16 keys.  A row that weighs 0 is read as zeros (from Q's last row), because 0 times an
+        // infinity is NaN; zero-filled copies of such rows took 3 to 8 % longer with one head a KV head. ----
+        const uint32_t vm = lane >> 3, vr = warp * 16 + (vm & 1u) * 8 + (lane & 7), zeros = smem_u32(sQ) + sw<PITCH>(15u, 0u);
+        const bool seen = j0 + vr - start <= pos - start;
 #pragma unroll
         for (int dp = 0; dp < HD / 16; ++dp) {
             uint32_t b0, b1, b2, b3;
-            const uint32_t m = lane >> 3;
-            ldsm_x4_t(sV + sw<PITCH>(warp * 16 + (m & 1u) * 8 + (lane & 7), dp * 2 + (m >> 1)), b0, b1, b2, b3);
+            ldsm_x4_t(seen ? sV + sw<PITCH>(vr, dp * 2 + (vm >> 1)) : zeros, b0, b1, b2, b3);
             mma_f16(o[2 * dp], pa0, 0u, pa2, 0u, b0, b1);
             mma_f16(o[2 * dp + 1], pa0, 0u, pa2, 0u, b2, b3);
         }
