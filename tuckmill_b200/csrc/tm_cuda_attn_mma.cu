@@ -141,7 +141,9 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
     constexpr int DV = C::kDV, SP = C::kSP, BQ = C::kBQ, KR = C::kRound;
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *sQ = smem, *sKV = smem + C::kQBytes;
-    const int tid = threadIdx.x, warp = (int)tmdev::warp_index(), lane = tid & 31;
+    // (With a warp index that the compiler knows to be uniform the rounds of keys take 3 % longer; nor does it pay to leave out
+    // the rescale of an empty sum: both together 512 rows at position 1000 32.8 -> 34.9 us.)
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const int rw = warp % RW, sp = warp / RW;
     // Tiles of queries from the last one down (the last of a chunk sees the most keys), heads next to one another.
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
             for (int i = 0; i < R; ++i) nx[i] = src[lane + 32 * i];
         };
         fetch(warp);
-#pragma unroll 1
+#pragma unroll 2
         for (uint32_t r = warp; r < BQ; r += 8) {
             float x[R];
 #pragma unroll
@@ -303,7 +305,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) attention_chunk_mma_kernel(c
                 const float m_new = fmaxf(m_run[mt][h], mx * a.scale_log2e);
                 const float m_use = m_new == -INFINITY ? 0.0f : m_new;  // nothing visible yet: every weight is 0
                 alpha[mt][h] = exp2f(m_run[mt][h] - m_use);             // m_run = -inf gives 0
-                moved = moved || (m_new != m_run[mt][h] && m_run[mt][h] != -INFINITY);  // (nothing to rescale before the first keys)
+                moved = moved || m_new != m_run[mt][h];
                 m_run[mt][h] = m_new;
                 float rs = 0.0f;
 #pragma unroll
