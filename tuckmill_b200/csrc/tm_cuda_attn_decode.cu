@@ -106,36 +106,36 @@ __global__ void __launch_bounds__(kT, HD > 128 ? 1 : 2) attention_decode_cluster
         tmdev::send(smem_addr(&recv[rank * E + in]), bar, to, o);
         if ((in & (HD - 1u)) == 0u) tmdev::send(smem_addr(&recv_ml[rank][in / HD][0]), bar, to, ml);
     }
-    if (!__all_sync(0xffffffffu, tmdev::mbar_wait(bar, a.waits.limit(), a.status, TM_CUDA_STATUS_LATE))) {
-        if (lane == 0) atomicOr(a.status, TM_CUDA_STATUS_LATE);
-        tmdev::linger(bar);
+    if (__all_sync(0xffffffffu, tmdev::mbar_wait(bar, a.waits.limit(), a.status, TM_CUDA_STATUS_LATE))) {
+        // ---- C lanes per quad: source s's share, added over the lanes ----
+        if ((uint32_t)warp * 32u >= kQuads) return;
+        const uint32_t src = tid & (C - 1u), in = ((uint32_t)tid >> logc) * 4u;
+        const float M = recv_ml[src][in / HD][0];
+        float L = recv_ml[src][in / HD][1];
+        float4 O = *(const float4 *)&recv[src * E + in];
+        float top = M;
+#pragma unroll 1
+        for (uint32_t off = C >> 1; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+        const float f = expf(M - top);  // a CTA without keys: exp(-inf) = 0
+        L *= f, O.x *= f, O.y *= f, O.z *= f, O.w *= f;
+#pragma unroll 1
+        for (uint32_t off = C >> 1; off > 0; off >>= 1) {
+            L += __shfl_xor_sync(0xffffffffu, L, off);
+            O.x += __shfl_xor_sync(0xffffffffu, O.x, off);
+            O.y += __shfl_xor_sync(0xffffffffu, O.y, off);
+            O.z += __shfl_xor_sync(0xffffffffu, O.z, off);
+            O.w += __shfl_xor_sync(0xffffffffu, O.w, off);
+        }
+        if (src == 0) {
+            float *out = a.out + seq_i * a.so + (size_t)kvh * G * HD + rank * E + in;
+            const float d[4] = {O.x / L, O.y / L, O.z / L, O.w / L};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) out[r] = d[r];
+        }
         return;
     }
-    // ---- C lanes per quad: source s's share, added over the lanes ----
-    if ((uint32_t)warp * 32u >= kQuads) return;
-    const uint32_t src = tid & (C - 1u), in = ((uint32_t)tid >> logc) * 4u;
-    const float M = recv_ml[src][in / HD][0];
-    float L = recv_ml[src][in / HD][1];
-    float4 O = *(const float4 *)&recv[src * E + in];
-    float top = M;
-#pragma unroll 1
-    for (uint32_t off = C >> 1; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-    const float f = expf(M - top);  // a CTA without keys: exp(-inf) = 0
-    L *= f, O.x *= f, O.y *= f, O.z *= f, O.w *= f;
-#pragma unroll 1
-    for (uint32_t off = C >> 1; off > 0; off >>= 1) {
-        L += __shfl_xor_sync(0xffffffffu, L, off);
-        O.x += __shfl_xor_sync(0xffffffffu, O.x, off);
-        O.y += __shfl_xor_sync(0xffffffffu, O.y, off);
-        O.z += __shfl_xor_sync(0xffffffffu, O.z, off);
-        O.w += __shfl_xor_sync(0xffffffffu, O.w, off);
-    }
-    if (src == 0) {
-        float *out = a.out + seq_i * a.so + (size_t)kvh * G * HD + rank * E + in;
-        const float d[4] = {O.x / L, O.y / L, O.z / L, O.w / L};
-#pragma unroll
-        for (int r = 0; r < 4; ++r) out[r] = d[r];
-    }
+    if (lane == 0) atomicOr(a.status, TM_CUDA_STATUS_LATE);  // (behind the code of every call)
+    tmdev::linger(bar);
 }
 
 // The widest cluster this device can hold of the kernel (16 needs the non-portable size).
